@@ -319,8 +319,9 @@ extern "C" int vec_create(const vec_params *p, vec_ctx **out)
         }
         aky2[E.ny / 2] = -(double)(E.ny / 2) * (double)(E.ny / 2) * cy * cy;
     }
-    if ((st = line_tables_make<double>(E.nx, akx1.data(), akx2.data(), E.k.icutoffx, &E.tx64)) ||
-        (st = line_tables_make<double>(E.ny, aky1.data(), aky2.data(), E.k.icutoffy, &E.ty64)) ||
+    if ((st = fx_plan_make(E.nx, &E.fpx)) || (st = fx_plan_make(E.ny, &E.fpy)) ||
+        (st = fx_tables_make(E.nx, E.fpx, akx1.data(), akx2.data(), E.k.icutoffx, &E.fxx)) ||
+        (st = fx_tables_make(E.ny, E.fpy, aky1.data(), aky2.data(), E.k.icutoffy, &E.fxy)) ||
         (st = line_tables_make<float>(E.nx, akx1.data(), akx2.data(), E.k.icutoffx, &E.tx32)) ||
         (st = line_tables_make<float>(E.ny, aky1.data(), aky2.data(), E.k.icutoffy, &E.ty32))) {
         vec_destroy(c);
@@ -442,8 +443,8 @@ extern "C" int vec_destroy(vec_ctx *c)
     if (E.ht) cudaFree(E.ht);
     if (E.wblock) cudaFree(E.wblock);
     for (int i = 0; i < 6; i++) if (E.s64[i]) cudaFree(E.s64[i]);
-    if (E.tx64.tw) line_tables_free(&E.tx64);
-    if (E.ty64.tw) line_tables_free(&E.ty64);
+    fx_tables_free(&E.fxx);
+    fx_tables_free(&E.fxy);
     if (E.tx32.tw) line_tables_free(&E.tx32);
     if (E.ty32.tw) line_tables_free(&E.ty32);
     if (E.hs) cudaFreeHost(E.hs);

@@ -60,6 +60,31 @@ struct LineTables {
     R *mda;                 // dealias mask (1/n or 0)
 };
 
+// the FP64 line kernel's passes for a length n (lines_fx.cu): radix, block and
+// stride of each, ceil(2^31 / stride), and where its twiddles start
+struct FxPlan {
+    int n, nb;              // length; elements of a buffer (n rounded up to 8)
+    int np;                 // passes
+    int R[6], L[6], M[6], tw[6];
+    unsigned mg[6];
+    int ntw;                // twiddles in all
+    int halvings;           // of one transform
+    int gb;                 // its values stay below 2^gb times the norm
+    int Q;                  // sequences per warp
+    int pow2;
+    float rn;               // 1 / n
+};
+// its tables: twiddles by pass; position of wavenumber k in the spectrum and
+// back; per operator (and 1 / n) the multipliers by position, scaled by 2^-p to
+// at most one
+struct TwX;
+struct FxTables {
+    TwX *tw;
+    unsigned short *pos, *kof;
+    int2 *m1, *m2, *mda, *minv;
+    int p1, p2, pda, pinv;
+};
+
 // horizontal wavenumber tables in one precision: akx1, aky1 and the
 // plane table akx2[i] + aky2[j] (summed in FP64, then rounded once)
 template <typename R>

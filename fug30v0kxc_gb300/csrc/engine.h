@@ -51,7 +51,8 @@ struct Engine {
 
     LinePlan plx, ply;          // precision of the bulk path
     LinePlan plx64, ply64;      // FP64 plans (per-operator entry points)
-    LineTables<double> tx64, ty64;
+    FxPlan fpx = {}, fpy = {};  // FP64 line passes and tables
+    FxTables fxx = {}, fxy = {};
     LineTables<float> tx32, ty32;
 
     // FP64 state (src/arrays.f90)
@@ -108,7 +109,7 @@ struct Engine {
     // tunables (the ensemble autotuner sets them per grid)
     int kc_pass2 = 16;          // planes per z chunk of hydro pass 2 (z-pencil or z-marching kernel)
     int ct_s = 0;               // sequences per line tile (0: default for the size)
-    bool ct_warp = true;        // x-line tiles synchronised per warp (VEC_CT_WARP=0: per CTA)
+    bool ct_warp = true;        // x-line tiles synchronised per warp (FP32; VEC_CT_WARP=0: per CTA)
     bool prof_kinds = false;    // VEC_PROF_KINDS=1: line launches profiled per job kind
     bool pdl = true;            // programmatic dependent launches (VEC_PDL=0: ordinary launches)
     bool vec4 = true;           // four-point (16-byte) forms of the split pointwise kernels (VEC_VEC4=0: one point)
@@ -140,7 +141,6 @@ struct Engine {
     int prof_flush();
 };
 
-template <> inline const LineTables<double> &Engine::tables<double>(int dir) const { return dir == 0 ? tx64 : ty64; }
 // A kernel launch on the engine's stream.  With E.pdl (the default) it is a
 // programmatic dependent launch: the launch of the next kernel overlaps the
 // end of this one, which hides most of the gap between the step's kernels;
@@ -208,11 +208,16 @@ int line_plan_make(int n, int lines, int elem_bytes, LinePlan *pl, int force_p =
 template <typename R> int line_tables_make(int n, const double *k1, const double *k2, int icut, LineTables<R> *tb);
 template <typename R> void line_tables_free(LineTables<R> *tb);
 template <typename R> int launch_lines(Engine *E, int dir, const LineJob<R> *jobs, int njobs);
+template <> int launch_lines<double>(Engine *E, int dir, const LineJob<double> *jobs, int njobs);   // lines_fx.cu
 int line_kernels_configure();
 // physics.cu: calcdt scratch (floats per context, initialisation of its keys)
 int cdt_chunks(size_t n);
 int cdt_init(float *cdt);
 int line_ct_configure();
+int line_fx_configure();
+int fx_plan_make(int n, FxPlan *pl);
+int fx_tables_make(int n, const FxPlan &pl, const double *k1, const double *k2, int icut, FxTables *tb);
+void fx_tables_free(FxTables *tb);
 template <typename R> int launch_lines_ct(Engine *E, int dir, const LineJob<R> *jobs, int njobs);
 
 template <typename R>

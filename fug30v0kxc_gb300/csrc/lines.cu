@@ -1,5 +1,5 @@
 // lines.cu -- horizontal spectral operators of src/fft.F90 as batched
-// shared-memory FFT kernels for sm_103a.
+// shared-memory FFT kernels for sm_103a, in FP32 (FP64: lines_fx.cu).
 //
 // One CTA takes 2P real lines of one z-plane (rows of nx values for the x
 // direction, columns of ny values at stride nx for the y direction), packs
@@ -445,8 +445,7 @@ int launch_lines(Engine *E, int dir, const LineJob<R> *jobs, int njobs)
         for (int j = 0; j < nj; j++) pk.j[j] = jobs[j0 + j];
         dim3 grid((unsigned)(pl.tiles * E->nz), (unsigned)nj);
         size_t smem = (size_t)(2 * pl.P * (pl.n + 1) + pl.n) * sizeof(typename CT<R>::T);
-        const char *name = dir == 0 ? (sizeof(R) == 8 ? "line_x_f64" : "line_x_f32")
-                                    : (sizeof(R) == 8 ? "line_y_f64" : "line_y_f32");
+        const char *name = dir == 0 ? "line_x_f32" : "line_y_f32";
         double fields = 0.0;
         for (int j = 0; j < nj; j++) {
             const LineJob<R> &q = pk.j[j];
@@ -467,17 +466,12 @@ int launch_lines(Engine *E, int dir, const LineJob<R> *jobs, int njobs)
 int line_kernels_configure()
 {
     int st = line_ct_configure();
-    if (st) return st;
-    CUDA_TRY(cudaFuncSetAttribute(line_kernel<double, 0>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
-    CUDA_TRY(cudaFuncSetAttribute(line_kernel<double, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
+    if (st || (st = line_fx_configure())) return st;
     CUDA_TRY(cudaFuncSetAttribute(line_kernel<float, 0>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
     CUDA_TRY(cudaFuncSetAttribute(line_kernel<float, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
     return VEC_OK;
 }
 
-template int line_tables_make<double>(int, const double *, const double *, int, LineTables<double> *);
 template int line_tables_make<float>(int, const double *, const double *, int, LineTables<float> *);
-template void line_tables_free<double>(LineTables<double> *);
 template void line_tables_free<float>(LineTables<float> *);
-template int launch_lines<double>(Engine *, int, const LineJob<double> *, int);
 template int launch_lines<float>(Engine *, int, const LineJob<float> *, int);

@@ -1,5 +1,5 @@
-// lines_ct.cu -- horizontal spectral operators (src/fft.F90) for line
-// lengths n = N1*N2 = 2^a or 3*2^a (64..1024), the hot path of the time step.
+// lines_ct.cu -- horizontal spectral operators (src/fft.F90) in FP32 for line
+// lengths n = N1*N2 = 2^a or 3*2^a (64..1024), the hot path of the split step.
 //
 // Per tile a CTA owns 2S real lines of one z-plane (S complex sequences
 // z = a + ib).  The tile is brought into shared memory by TMA bulk copies
@@ -35,16 +35,12 @@ struct TmapPack { CUtensorMap m[MAX_JOBS]; };
 // W_32^q = exp(-2 pi i q/32), q = 0..31, and W_96^q (the in-register radix
 // kernels; radix-3 factors take their twiddles from the second table)
 __constant__ float2 c_tw32f[32];
-__constant__ double2 c_tw32d[32];
 __constant__ float2 c_tw96f[96];
-__constant__ double2 c_tw96d[96];
 
 template <typename C> __device__ __forceinline__ C tw32(int q);
 template <> __device__ __forceinline__ float2 tw32<float2>(int q) { return c_tw32f[q]; }
-template <> __device__ __forceinline__ double2 tw32<double2>(int q) { return c_tw32d[q]; }
 template <typename C> __device__ __forceinline__ C tw96(int q);
 template <> __device__ __forceinline__ float2 tw96<float2>(int q) { return c_tw96f[q]; }
-template <> __device__ __forceinline__ double2 tw96<double2>(int q) { return c_tw96d[q]; }
 
 // x mod N for x >= 0 (N a compile-time constant)
 template <int N> __device__ __forceinline__ int modn(int x) { return (N & (N - 1)) == 0 ? (x & (N - 1)) : x % N; }
@@ -168,7 +164,7 @@ __host__ __device__ constexpr int ybox_rows(int n) { return n <= 256 ? n : (n % 
 // N1 + 1, the spectra's separation N + N/32 padded elements: the stride
 // covers the largest.  A shared-memory wavefront serves U = 128 /
 // sizeof(complex) consecutive elements.  x lines: the threads of a
-// half-warp (quarter-warp in FP64) belong to one or two sequences, and a
+// half-warp belong to one or two sequences, and a
 // stride of 1 mod 16 keeps them on distinct banks.  y lines: thread tid is
 // lane tid / S of sequence tid % S, so a wavefront's threads are G = U / S
 // lanes of U / G sequences; a stride of G mod U puts them on distinct banks
@@ -190,7 +186,7 @@ __host__ __device__ constexpr size_t ct_smem_bytes()
 {
     constexpr int N = N1 * N2;
     constexpr int LDS = ct_lds<R, DIR, N1, N2, S>();
-    return 2 * (size_t)(2 * S * N) * sizeof(R) + ((size_t)S * LDS + (sizeof(R) == 4 ? 2 : 1) * (size_t)N) * 2 * sizeof(R)
+    return 2 * (size_t)(2 * S * N) * sizeof(R) + ((size_t)S * LDS + 2 * (size_t)N) * 2 * sizeof(R)
            + 3 * (size_t)N * sizeof(R);
 }
 // two CTAs per SM where their shared memory fits (227 KB per SM), else one
@@ -221,16 +217,14 @@ line_ct(JobPackCT<R> jobs, const __grid_constant__ TmapPack tmaps, LineTables<R>
     R *tile0 = reinterpret_cast<R *>(smem);
     R *tile1 = tile0 + TILE;
     C *ex = reinterpret_cast<C *>(tile1 + TILE);
-    // FP32: twiddles W_N^(m2 k1) as two N1 x N2 tables, one row per value of
+    // twiddles W_N^(m2 k1) as two N1 x N2 tables, one row per value of
     // the loop index, so that the 16 threads of a sequence read consecutive
     // entries (indexed by (m2 k1) mod N, a thread stride of k1 made up to
-    // eight-way bank conflicts).  FP64: one table of N (the second would
-    // cost the second CTA per SM).
-    constexpr bool TW2 = sizeof(R) == 4;
-    static_assert(!TW2 || (N1 % 4 == 0 && N2 % 4 == 0), "FP32 twiddles factor the index as 4 a + b");
-    C *twf = ex + (size_t)S * LDS;                    // twf[k1 N2 + m2] (FP64: tw[e])
+    // eight-way bank conflicts)
+    static_assert(N1 % 4 == 0 && N2 % 4 == 0, "twiddles factor the index as 4 a + b");
+    C *twf = ex + (size_t)S * LDS;                    // twf[k1 N2 + m2]
     C *twi = twf + N;                                 // twi[m2 N1 + k1]
-    R *sm1 = reinterpret_cast<R *>(twi + (TW2 ? N : 0));   // spectral multipliers
+    R *sm1 = reinterpret_cast<R *>(twi + N);   // spectral multipliers
     R *sm2 = sm1 + N;
     R *smda = sm2 + N;
     __shared__ __align__(8) uint64_t bar[4];          // full[2], empty[2]
@@ -245,14 +239,10 @@ line_ct(JobPackCT<R> jobs, const __grid_constant__ TmapPack tmaps, LineTables<R>
     };
 
     for (int e = tid; e < N; e += NT) {
-        if constexpr (TW2) {
-            const int k1 = e / N2, m2 = e - k1 * N2;
-            twf[e] = tb.tw[modn<N>(m2 * k1)];
-            const int m2i = e / N1, k1i = e - m2i * N1;
-            twi[e] = tb.tw[modn<N>(m2i * k1i)];
-        } else {
-            twf[e] = tb.tw[e];
-        }
+        const int k1 = e / N2, m2 = e - k1 * N2;
+        twf[e] = tb.tw[modn<N>(m2 * k1)];
+        const int m2i = e / N1, k1i = e - m2i * N1;
+        twi[e] = tb.tw[modn<N>(m2i * k1i)];
         sm1[e] = tb.m1[e];
         sm2[e] = tb.m2[e];
         smda[e] = tb.mda[e];
@@ -340,7 +330,7 @@ line_ct(JobPackCT<R> jobs, const __grid_constant__ TmapPack tmaps, LineTables<R>
         // that start on the same bank; the odd one reads its columns in pairs
         // swapped (index ^ 1), so that the two half-warps hit different banks,
         // and swaps the registers back.  The values are the same.
-        constexpr bool XSW = WS && DIR == 0 && NP == 16 && sizeof(R) == 4 && N1 % 2 == 0 && N2 % 2 == 0;
+        constexpr bool XSW = WS && DIR == 0 && NP == 16 && N1 % 2 == 0 && N2 % 2 == 0;
         const int sw = XSW ? (sidx & 1) : 0;
         auto unswap = [&](C *v, int n) {
             if constexpr (XSW) {
@@ -362,24 +352,17 @@ line_ct(JobPackCT<R> jobs, const __grid_constant__ TmapPack tmaps, LineTables<R>
                 for (int m1 = 0; m1 < N1; m1++) a[m1] = tile_z(N2 * (m1 ^ sw) + lane);
                 unswap(a, N1);
                 RDft<N1, false>::run(a);
-                // FP32: W^(lane k1) = W^(lane 4 (k1 / 4)) W^(lane (k1 % 4)): 3 + N1/4 - 1
+                // W^(lane k1) = W^(lane 4 (k1 / 4)) W^(lane (k1 % 4)): 3 + N1/4 - 1
                 // table reads instead of N1 - 1, one product more per twiddle
                 C lo[4], hi[N1 / 4];
-                if constexpr (TW2) {
 #pragma unroll
-                    for (int j = 1; j < 4; j++) lo[j] = twf[j * N2 + lane];
+                for (int j = 1; j < 4; j++) lo[j] = twf[j * N2 + lane];
 #pragma unroll
-                    for (int j = 1; j < N1 / 4; j++) hi[j] = twf[4 * j * N2 + lane];
-                }
+                for (int j = 1; j < N1 / 4; j++) hi[j] = twf[4 * j * N2 + lane];
 #pragma unroll
                 for (int k1 = 0; k1 < N1; k1++) {
-                    C w;
-                    if constexpr (TW2) {
-                        const int ja = k1 >> 2, jb = k1 & 3;
-                        w = ja == 0 ? lo[jb] : (jb == 0 ? hi[ja] : cmul_(hi[ja], lo[jb]));
-                    } else {
-                        w = twf[modn<N>(lane * k1)];
-                    }
+                    const int ja = k1 >> 2, jb = k1 & 3;
+                    const C w = ja == 0 ? lo[jb] : (jb == 0 ? hi[ja] : cmul_(hi[ja], lo[jb]));
                     ex_s[k1 * LXF + lane] = k1 == 0 ? a[k1] : cmul_(a[k1], w);
                 }
             }
@@ -465,23 +448,16 @@ line_ct(JobPackCT<R> jobs, const __grid_constant__ TmapPack tmaps, LineTables<R>
                 }
                 // inverse, first level: thread k1 = lane, N2-point DFT over k2
                 RDft<N2, true>::run(Y);
-                // (FP32: the same factorisation of W^(m2 lane), m2 = 4 (m2 / 4) + m2 % 4)
+                // (the same factorisation of W^(m2 lane), m2 = 4 (m2 / 4) + m2 % 4)
                 C lo[4], hi[N2 / 4];
-                if constexpr (TW2) {
 #pragma unroll
-                    for (int j = 1; j < 4; j++) lo[j] = twi[j * N1 + lane];
+                for (int j = 1; j < 4; j++) lo[j] = twi[j * N1 + lane];
 #pragma unroll
-                    for (int j = 1; j < N2 / 4; j++) hi[j] = twi[4 * j * N1 + lane];
-                }
+                for (int j = 1; j < N2 / 4; j++) hi[j] = twi[4 * j * N1 + lane];
 #pragma unroll
                 for (int m2 = 0; m2 < N2; m2++) {
-                    C w;
-                    if constexpr (TW2) {
-                        const int ja = m2 >> 2, jb = m2 & 3;
-                        w = ja == 0 ? lo[jb] : (jb == 0 ? hi[ja] : cmul_(hi[ja], lo[jb]));
-                    } else {
-                        w = twf[modn<N>(m2 * lane)];
-                    }
+                    const int ja = m2 >> 2, jb = m2 & 3;
+                    C w = ja == 0 ? lo[jb] : (jb == 0 ? hi[ja] : cmul_(hi[ja], lo[jb]));
                     w.y = -w.y;
                     ex_s[m2 * LXI + lane] = m2 == 0 ? Y[m2] : cmul_(Y[m2], w);
                 }
@@ -546,31 +522,17 @@ extern "C" int vec_selftest_wait(vec_ctx *c, long long polls)
 // ---- host side ------------------------------------------------------------------------
 int line_ct_configure()
 {
-    float2 tf[32];
-    double2 td[32];
-    for (int q = 0; q < 32; q++) {
-        // exp(-2 pi i q/32) with exact quadrant values
-        double a = 2.0 * M_PI * (double)q / 32.0;
-        double c = cos(a), s = sin(a);
-        if (q % 8 == 0) {
-            c = (q == 0) ? 1.0 : (q == 16 ? -1.0 : 0.0);
-            s = (q == 8) ? 1.0 : (q == 24 ? -1.0 : 0.0);
-        }
-        td[q].x = c; td[q].y = -s;
-        tf[q].x = (float)c; tf[q].y = (float)(-s);
+    float2 tf[32], uf[96];
+    for (int q = 0; q < 96; q++) {
+        double c, v;
+        sincos2pi_host(q, 96, &c, &v);
+        uf[q].x = (float)c; uf[q].y = (float)(-v);
+        if (q >= 32) continue;
+        sincos2pi_host(q, 32, &c, &v);
+        tf[q].x = (float)c; tf[q].y = (float)(-v);
     }
     CUDA_TRY(cudaMemcpyToSymbol(c_tw32f, tf, sizeof(tf)));
-    CUDA_TRY(cudaMemcpyToSymbol(c_tw32d, td, sizeof(td)));
-    float2 uf[96];
-    double2 ud[96];
-    for (int q = 0; q < 96; q++) {
-        double c, s;
-        sincos2pi_host(q, 96, &c, &s);
-        ud[q].x = c; ud[q].y = -s;
-        uf[q].x = (float)c; uf[q].y = (float)(-s);
-    }
     CUDA_TRY(cudaMemcpyToSymbol(c_tw96f, uf, sizeof(uf)));
-    CUDA_TRY(cudaMemcpyToSymbol(c_tw96d, ud, sizeof(ud)));
     return VEC_OK;
 }
 
@@ -603,7 +565,7 @@ static int encode_ymap(CUtensorMap *m, const R *base, int nx, int ny, int nz, in
     cuuint64_t strides[2] = { (cuuint64_t)nx * sizeof(R), (cuuint64_t)nx * ny * sizeof(R) };
     cuuint32_t box[3] = { (cuuint32_t)(2 * S), (cuuint32_t)BR, 1 };
     cuuint32_t es[3] = { 1, 1, 1 };
-    CUresult r = g_encode(m, sizeof(R) == 4 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT32 : CU_TENSOR_MAP_DATA_TYPE_FLOAT64, 3,
+    CUresult r = g_encode(m, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 3,
                           (void *)base, dims, strides, box, es, CU_TENSOR_MAP_INTERLEAVE_NONE,
                           CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
                           CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
@@ -624,7 +586,7 @@ static int run_ct(Engine *E, const LineJob<R> *jobs, int nj, const char *name)
     constexpr int LDS = ct_lds<R, DIR, N1, N2, S>();
     static bool attr_set = false;
     const size_t smem = ct_smem_bytes<R, DIR, N1, N2, S>();
-    static_assert(ct_smem_bytes<R, DIR, N1, N2, S>() == 2 * TILE * sizeof(R) + ((size_t)S * LDS + (sizeof(R) == 4 ? 2 : 1) * N) * sizeof(C) + 3 * (size_t)N * sizeof(R),
+    static_assert(ct_smem_bytes<R, DIR, N1, N2, S>() == 2 * TILE * sizeof(R) + ((size_t)S * LDS + 2 * N) * sizeof(C) + 3 * (size_t)N * sizeof(R),
                   "shared memory layout");
     static_assert(ct_smem_bytes<R, DIR, N1, N2, S>() + 128 <= 232448, "tile does not fit one SM's shared memory");
     static_assert(LDS >= N1 * (N2 + 1) && LDS >= N2 * (N1 + 1) && LDS >= N + N / 32 + 1, "exchange rows");
@@ -675,20 +637,19 @@ int launch_lines_ct(Engine *E, int dir, const LineJob<R> *jobs, int njobs)
 {
     const int n = dir == 0 ? E->nx : E->ny;
     const int L = dir == 0 ? E->ny : E->nx;
-    constexpr bool F = sizeof(R) == 4;
     // sequences per tile
     int S = 0;
     switch (n) {
-    case 64: case 96: case 128: case 192: case 256: S = F ? 16 : 8; break;
-    case 384: case 512: S = F ? 8 : 4; break;
-    // (n >= 768, FP32: 8 sequences make the y tiles' rows 64 bytes wide and
+    case 64: case 96: case 128: case 192: case 256: S = 16; break;
+    case 384: case 512: S = 8; break;
+    // (n >= 768: 8 sequences make the y tiles' rows 64 bytes wide and
     // give 8 warps per SM; with 4 the 1024-point passes ran at 1.7-1.8 TB/s,
     // with 8 at 3.2-3.4 TB/s, measured at 1024^2 x 17)
-    case 768: case 1024: S = F ? 8 : 2; break;
+    case 768: case 1024: S = 8; break;
     default: return 0;
     }
-    if (F && n <= 256 && E->ct_s == 8) S = 8;    // autotuned alternatives
-    if (F && n >= 768 && E->ct_s == 4) S = 4;
+    if (n <= 256 && E->ct_s == 8) S = 8;    // autotuned alternatives
+    if (n >= 768 && E->ct_s == 4) S = 4;
     if (L % (2 * S) != 0) return 0;
     if ((E->nx * (int)sizeof(R)) % 16 != 0) return 0;
     for (int j = 0; j < njobs; j++) {
@@ -699,16 +660,14 @@ int launch_lines_ct(Engine *E, int dir, const LineJob<R> *jobs, int njobs)
     for (int j0 = 0; j0 < njobs; j0 += MAX_JOBS) {
         const int nj = njobs - j0 < MAX_JOBS ? njobs - j0 : MAX_JOBS;
         const LineJob<R> *jb = jobs + j0;
-        const char *name = dir == 0 ? (F ? "line_x_f32" : "line_x_f64") : (F ? "line_y_f32" : "line_y_f64");
+        const char *name = dir == 0 ? "line_x_f32" : "line_y_f32";
         if (E->prof_kinds) {
             // per job kind (profiling aid): forward, inverse, accumulate, derivative pair, other
-            static const char *kinds[2][2][5] = {
-                { { "line_x_f64_fwd", "line_x_f64_inv", "line_x_f64_acc", "line_x_f64_d12", "line_x_f64_op" },
-                  { "line_x_f32_fwd", "line_x_f32_inv", "line_x_f32_acc", "line_x_f32_d12", "line_x_f32_op" } },
-                { { "line_y_f64_fwd", "line_y_f64_inv", "line_y_f64_acc", "line_y_f64_d12", "line_y_f64_op" },
-                  { "line_y_f32_fwd", "line_y_f32_inv", "line_y_f32_acc", "line_y_f32_d12", "line_y_f32_op" } } };
+            static const char *kinds[2][5] = {
+                { "line_x_f32_fwd", "line_x_f32_inv", "line_x_f32_acc", "line_x_f32_d12", "line_x_f32_op" },
+                { "line_y_f32_fwd", "line_y_f32_inv", "line_y_f32_acc", "line_y_f32_d12", "line_y_f32_op" } };
             const int kd = jb[0].op1 == OP_FWD ? 0 : jb[0].op1 == OP_INV ? 1 : jb[0].acc1 ? 2 : jb[0].op2 != OP_NONE ? 3 : 4;
-            name = kinds[dir][F ? 1 : 0][kd];
+            name = kinds[dir][kd];
         }
         int st = -1;
 #define CT_CASE(NN, A, B, SS)                                                                       \
@@ -716,17 +675,11 @@ int launch_lines_ct(Engine *E, int dir, const LineJob<R> *jobs, int njobs)
         st = dir == 1 ? run_ct<R, 1, A, B, SS, false>(E, jb, nj, name)                            \
                       : (ws ? run_ct<R, 0, A, B, SS, true>(E, jb, nj, name)                       \
                             : run_ct<R, 0, A, B, SS, false>(E, jb, nj, name));
-        if constexpr (F) {
-            CT_CASE(64, 8, 8, 16) CT_CASE(128, 16, 8, 16) CT_CASE(256, 16, 16, 16)
-            CT_CASE(64, 8, 8, 8) CT_CASE(128, 16, 8, 8) CT_CASE(256, 16, 16, 8)
-            CT_CASE(512, 32, 16, 8) CT_CASE(1024, 32, 32, 4) CT_CASE(1024, 32, 32, 8)
-            CT_CASE(96, 8, 12, 16) CT_CASE(192, 16, 12, 16) CT_CASE(96, 8, 12, 8) CT_CASE(192, 16, 12, 8)
-            CT_CASE(384, 16, 24, 8) CT_CASE(768, 32, 24, 4) CT_CASE(768, 32, 24, 8)
-        } else {
-            CT_CASE(64, 8, 8, 8) CT_CASE(128, 16, 8, 8) CT_CASE(256, 16, 16, 8)
-            CT_CASE(512, 32, 16, 4) CT_CASE(1024, 32, 32, 2)
-            CT_CASE(96, 8, 12, 8) CT_CASE(192, 16, 12, 8) CT_CASE(384, 16, 24, 4) CT_CASE(768, 32, 24, 2)
-        }
+        CT_CASE(64, 8, 8, 16) CT_CASE(128, 16, 8, 16) CT_CASE(256, 16, 16, 16)
+        CT_CASE(64, 8, 8, 8) CT_CASE(128, 16, 8, 8) CT_CASE(256, 16, 16, 8)
+        CT_CASE(512, 32, 16, 8) CT_CASE(1024, 32, 32, 4) CT_CASE(1024, 32, 32, 8)
+        CT_CASE(96, 8, 12, 16) CT_CASE(192, 16, 12, 16) CT_CASE(96, 8, 12, 8) CT_CASE(192, 16, 12, 8)
+        CT_CASE(384, 16, 24, 8) CT_CASE(768, 32, 24, 4) CT_CASE(768, 32, 24, 8)
 #undef CT_CASE
         if (st < 0) return 0;
         if (st) return st;
@@ -735,4 +688,3 @@ int launch_lines_ct(Engine *E, int dir, const LineJob<R> *jobs, int njobs)
 }
 
 template int launch_lines_ct<float>(Engine *, int, const LineJob<float> *, int);
-template int launch_lines_ct<double>(Engine *, int, const LineJob<double> *, int);
