@@ -257,6 +257,7 @@ extern "C" int vec_create(const vec_params *p, vec_ctx **out)
     E.np = (size_t)E.nx * E.ny;
     E.n = E.np * E.nz;
     E.split = p->precision == VEC_PREC_SPLIT;
+    E.dev = dev;
     cudaDeviceGetAttribute(&E.num_sms, cudaDevAttrMultiProcessorCount, dev);
     {
         const char *g = getenv("VEC_GENERIC_LINES");
@@ -411,7 +412,12 @@ extern "C" int vec_create(const vec_params *p, vec_ctx **out)
     ALLOC(E.ds, sizeof(DevScalars));
     ALLOC(E.cdt, sizeof(float) * (4 + 3 * (size_t)cdt_chunks(E.n)));
     if ((st = cdt_init(E.cdt))) { vec_destroy(c); return st; }
-    ALLOC(E.dev_err, sizeof(int) * 4);
+    if (cudaHostAlloc((void **)&E.dev_err, sizeof(int) * 4, cudaHostAllocMapped | cudaHostAllocPortable) != cudaSuccess) {
+        cudaGetLastError();
+        vec_destroy(c);
+        return VEC_ERR_ALLOC;
+    }
+    memset(E.dev_err, 0, sizeof(int) * 4);
     if (cudaMallocHost(&E.hs, sizeof(DevScalars)) != cudaSuccess) { vec_destroy(c); return VEC_ERR_ALLOC; }
     memset(E.hs, 0, sizeof(DevScalars));
     E.hs->first = 1;
@@ -432,7 +438,7 @@ extern "C" int vec_destroy(vec_ctx *c)
     if (E.stream) cudaStreamSynchronize(E.stream);
     E.drop_graphs();
     void *ptrs[] = { E.r, E.t, E.u, E.v, E.w, E.bx, E.by, E.bz, E.jsq, E.pol, E.tor, E.bxbar, E.bybar,
-                     E.kappa, E.dkappa, E.eta, E.deta, E.akx1, E.akx2, E.aky1, E.aky2, E.w1d, E.red, E.ds, E.dev_err, E.cdt,
+                     E.kappa, E.dkappa, E.eta, E.deta, E.akx1, E.akx2, E.aky1, E.aky2, E.w1d, E.red, E.ds, E.cdt,
                      E.r32, E.t32, E.u32, E.v32, E.w32, E.bx32, E.by32, E.bz32, E.jsq32, E.pol32, E.tor32,
                      E.rho0, E.t0, E.hres, E.corr, E.corr_bx };
     for (void *q : ptrs) if (q) cudaFree(q);
@@ -448,6 +454,7 @@ extern "C" int vec_destroy(vec_ctx *c)
     if (E.tx32.tw) line_tables_free(&E.tx32);
     if (E.ty32.tw) line_tables_free(&E.ty32);
     if (E.hs) cudaFreeHost(E.hs);
+    if (E.dev_err) cudaFreeHost(E.dev_err);
     for (auto &pd : E.pending) { cudaEventDestroy(pd.a); cudaEventDestroy(pd.b); }
     for (auto ev : E.ev_pool) cudaEventDestroy(ev);
     if (E.stream2) { cudaStreamSynchronize(E.stream2); cudaStreamDestroy(E.stream2); }
@@ -464,11 +471,11 @@ extern "C" int vec_sync(vec_ctx *c)
 {
     if (!c) return VEC_ERR_ARG;
     CUDA_TRY(cudaStreamSynchronize(c->E.stream));
-    int err = 0;
-    CUDA_TRY(cudaMemcpy(&err, c->E.dev_err, sizeof(int), cudaMemcpyDeviceToHost));
+    volatile int *flag = c->E.dev_err;
+    const int err = *flag;
     if (err) {
         // reported once: the flag is cleared, the context stays usable
-        CUDA_TRY(cudaMemset(c->E.dev_err, 0, sizeof(int)));
+        *flag = 0;
         vec_set_error(err == 2 ? "a bounded device wait ran out (wait self-test)"
                                : "a bounded device wait ran out (TMA tile load did not complete)");
         return VEC_ERR_CUDA;
@@ -485,6 +492,33 @@ static bool is_device_ptr(const void *p)
         return false;
     }
     return a.type == cudaMemoryTypeDevice || a.type == cudaMemoryTypeManaged;
+}
+
+// Whether an operator may work on the caller's array itself: memory of the
+// context's device, aligned for the kernels' 16-byte accesses.  Anything else
+// (host, managed, another device's, an odd address) goes through the context's
+// scratch.
+static bool in_place(const Engine &E, const void *p)
+{
+    if ((uintptr_t)p & 15) return false;
+    cudaPointerAttributes a;
+    if (cudaPointerGetAttributes(&a, p) != cudaSuccess) {
+        cudaGetLastError();
+        return false;
+    }
+    return a.type == cudaMemoryTypeDevice && a.device == E.dev;
+}
+static bool overlap(const void *a, const void *b, size_t bytes)
+{
+    const uintptr_t x = (uintptr_t)a, y = (uintptr_t)b;
+    return x < y + bytes && y < x + bytes;
+}
+// The line kernels read a line before they write it, so an output may be the
+// input itself; arrays that overlap in another way go through the scratch.
+static bool lines_in_place(const Engine &E, const void *in, const void *f1, const void *f2, size_t bytes)
+{
+    return in_place(E, in) && in_place(E, f1) && (!f2 || in_place(E, f2)) && (f1 == in || !overlap(in, f1, bytes)) &&
+           (!f2 || ((f2 == in || !overlap(in, f2, bytes)) && !overlap(f1, f2, bytes)));
 }
 
 // copy count doubles from src (host or device) into device dst
@@ -522,15 +556,17 @@ static double *state_ptr(Engine &E, int field)
     return nullptr;
 }
 
-__global__ void k_f2d(const float *a, double *b, size_t n)
+// the logical history slot s of field f, as doubles (the kernel reads the slot
+// table: no copy of it to the host)
+template <typename R> __global__ void k_hist_get(const HistTable *ht, int f, int s, double *b, size_t n)
 {
     size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < n) b[i] = (double)a[i];
+    if (i < n) b[i] = (double)((const R *)ht->p[f][s])[i];
 }
-__global__ void k_d2f(const double *a, float *b, size_t n)
+template <typename R> __global__ void k_hist_set(const HistTable *ht, int f, int s, const double *b, size_t n)
 {
     size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < n) b[i] = (float)a[i];
+    if (i < n) ((R *)ht->p[f][s])[i] = (R)b[i];
 }
 
 extern "C" int vec_set_field(vec_ctx *c, int field, const double *src)
@@ -548,12 +584,16 @@ extern "C" int vec_set_field(vec_ctx *c, int field, const double *src)
     }
     int f, s;
     if (hist_index(field, &f, &s)) return VEC_ERR_ARG;
-    HistTable h;
-    int st = hist_table_host(&E, &h);
-    if (st) return st;
-    if (!E.split) return stage_in(E, (double *)h.p[f][s], src, E.n) ? VEC_ERR_CUDA : vec_sync(c);
-    if ((st = stage_in(E, E.s64[0], src, E.n))) return st;
-    k_d2f<<<(unsigned)((E.n + 255) / 256), 256, 0, E.stream>>>(E.s64[0], (float *)h.p[f][s], E.n);
+    int st;
+    const double *a = src;
+    if (!in_place(E, src)) {
+        if ((st = stage_in(E, E.s64[0], src, E.n))) return st;
+        a = E.s64[0];
+    }
+    const unsigned nb = (unsigned)((E.n + 255) / 256);
+    if (E.split) k_hist_set<float><<<nb, 256, 0, E.stream>>>(E.ht, f, s, a, E.n);
+    else k_hist_set<double><<<nb, 256, 0, E.stream>>>(E.ht, f, s, a, E.n);
+    CUDA_TRY(cudaGetLastError());
     return vec_sync(c);
 }
 
@@ -569,12 +609,15 @@ extern "C" int vec_get_field(vec_ctx *c, int field, double *dst)
     }
     int f, s;
     if (hist_index(field, &f, &s)) return VEC_ERR_ARG;
-    HistTable h;
-    int st = hist_table_host(&E, &h);
-    if (st) return st;
-    if (!E.split) return stage_out(E, dst, (const double *)h.p[f][s], E.n);
-    k_f2d<<<(unsigned)((E.n + 255) / 256), 256, 0, E.stream>>>((const float *)h.p[f][s], E.s64[0], E.n);
-    return stage_out(E, dst, E.s64[0], E.n);
+    const bool direct = in_place(E, dst);
+    double *b = direct ? dst : E.s64[0];
+    const unsigned nb = (unsigned)((E.n + 255) / 256);
+    if (E.split) k_hist_get<float><<<nb, 256, 0, E.stream>>>(E.ht, f, s, b, E.n);
+    else k_hist_get<double><<<nb, 256, 0, E.stream>>>(E.ht, f, s, b, E.n);
+    CUDA_TRY(cudaGetLastError());
+    if (!direct) return stage_out(E, dst, b, E.n);
+    CUDA_TRY(cudaStreamSynchronize(E.stream));
+    return VEC_OK;
 }
 
 static double *mean_ptr(Engine &E, int m)
@@ -694,6 +737,12 @@ static int line_op(vec_ctx *c, int dir, const double *fin, double *f1, int op1, 
     if (!c || !fin || !f1 || (op2 != OP_NONE && !f2)) return VEC_ERR_ARG;
     Engine &E = c->E;
     int st;
+    if (lines_in_place(E, fin, f1, op2 != OP_NONE ? f2 : nullptr, sizeof(double) * E.n)) {
+        LineJob<double> j = ljob<double>(fin, f1, op1, op2 != OP_NONE ? f2 : nullptr, op2);
+        if ((st = launch_lines<double>(&E, dir, &j, 1))) return st;
+        CUDA_TRY(cudaStreamSynchronize(E.stream));
+        return VEC_OK;
+    }
     if ((st = stage_in(E, E.s64[0], fin, E.n))) return st;
     LineJob<double> j = ljob<double>(E.s64[0], E.s64[1], op1, op2 != OP_NONE ? E.s64[2] : nullptr, op2);
     if ((st = launch_lines<double>(&E, dir, &j, 1))) return st;
@@ -712,6 +761,11 @@ extern "C" int vec_line_f32(vec_ctx *c, int dir, int op1, int op2, const float *
                                                            (op1 == OP_INV && op2 != OP_D1) || !f2)))
         return VEC_ERR_ARG;
     Engine &E = c->E;
+    if (lines_in_place(E, fin, f1, op2 != OP_NONE ? f2 : nullptr, sizeof(float) * E.n)) {
+        LineJob<float> j = ljob<float>(fin, f1, op1, op2 != OP_NONE ? f2 : nullptr, op2);
+        const int st = launch_lines<float>(&E, dir, &j, 1);
+        return st ? st : vec_sync(c);
+    }
     // each FP64 scratch field holds 2n floats
     float *in = reinterpret_cast<float *>(E.s64[0]), *o1 = reinterpret_cast<float *>(E.s64[1]);
     float *o2 = reinterpret_cast<float *>(E.s64[2]);
@@ -742,35 +796,34 @@ extern "C" int vec_dealias(vec_ctx *c, double *z)
     if (!c || !z) return VEC_ERR_ARG;
     Engine &E = c->E;
     int st;
-    if ((st = stage_in(E, E.s64[0], z, E.n))) return st;
-    LineJob<double> j = ljob<double>(E.s64[0], E.s64[0], OP_DEALIAS);
+    const bool direct = in_place(E, z);
+    double *a = direct ? z : E.s64[0];
+    if (!direct && (st = stage_in(E, a, z, E.n))) return st;
+    LineJob<double> j = ljob<double>(a, a, OP_DEALIAS);
     if ((st = launch_lines<double>(&E, 0, &j, 1)) || (st = launch_lines<double>(&E, 1, &j, 1))) return st;
-    return stage_out(E, z, E.s64[0], E.n);
+    if (!direct) return stage_out(E, z, a, E.n);
+    CUDA_TRY(cudaStreamSynchronize(E.stream));
+    return VEC_OK;
 }
 
-extern "C" int vec_forwardfft(vec_ctx *c, const double *fin, double *fout)
+// x pass into the output, y pass in place there
+static int fft2(vec_ctx *c, const double *fin, double *fout, int op)
 {
     if (!c || !fin || !fout) return VEC_ERR_ARG;
     Engine &E = c->E;
     int st;
-    if ((st = stage_in(E, E.s64[0], fin, E.n))) return st;
-    LineJob<double> jx = ljob<double>(E.s64[0], E.s64[1], OP_FWD);
-    LineJob<double> jy = ljob<double>(E.s64[1], E.s64[1], OP_FWD);
+    const bool direct = lines_in_place(E, fin, fout, nullptr, sizeof(double) * E.n);
+    const double *in = direct ? fin : E.s64[0];
+    double *out = direct ? fout : E.s64[1];
+    if (!direct && (st = stage_in(E, E.s64[0], fin, E.n))) return st;
+    LineJob<double> jx = ljob<double>(in, out, op), jy = ljob<double>(out, out, op);
     if ((st = launch_lines<double>(&E, 0, &jx, 1)) || (st = launch_lines<double>(&E, 1, &jy, 1))) return st;
-    return stage_out(E, fout, E.s64[1], E.n);
+    if (!direct) return stage_out(E, fout, out, E.n);
+    CUDA_TRY(cudaStreamSynchronize(E.stream));
+    return VEC_OK;
 }
-
-extern "C" int vec_inversefft(vec_ctx *c, const double *fin, double *fout)
-{
-    if (!c || !fin || !fout) return VEC_ERR_ARG;
-    Engine &E = c->E;
-    int st;
-    if ((st = stage_in(E, E.s64[0], fin, E.n))) return st;
-    LineJob<double> jx = ljob<double>(E.s64[0], E.s64[1], OP_INV);
-    LineJob<double> jy = ljob<double>(E.s64[1], E.s64[1], OP_INV);
-    if ((st = launch_lines<double>(&E, 0, &jx, 1)) || (st = launch_lines<double>(&E, 1, &jy, 1))) return st;
-    return stage_out(E, fout, E.s64[1], E.n);
-}
+extern "C" int vec_forwardfft(vec_ctx *c, const double *fin, double *fout) { return fft2(c, fin, fout, OP_FWD); }
+extern "C" int vec_inversefft(vec_ctx *c, const double *fin, double *fout) { return fft2(c, fin, fout, OP_INV); }
 
 static int zop(vec_ctx *c, const double *fin, double *fout, int flag, int kind, int oned)
 {
@@ -779,12 +832,19 @@ static int zop(vec_ctx *c, const double *fin, double *fout, int flag, int kind, 
     const size_t cnt = oned ? (size_t)E.nz : E.n;
     int np = oned ? 1 : (int)E.np;
     int st;
-    if ((st = stage_in(E, E.s64[0], fin, cnt))) return st;
-    if (kind == 0) st = op_d1z(&E, E.s64[0], E.s64[1], flag, np, E.nz);
-    else if (kind == 1) st = op_d1upz(&E, E.s64[0], E.s64[1], flag);
-    else st = op_d2z(&E, E.s64[0], E.s64[1], flag, np, E.nz);
+    // (a stencil reads other planes than it writes)
+    const bool direct = in_place(E, fin) && in_place(E, fout) && !overlap(fin, fout, sizeof(double) * cnt) &&
+                        !(kind == 1 && overlap(E.w, fout, sizeof(double) * cnt));
+    const double *in = direct ? fin : E.s64[0];
+    double *out = direct ? fout : E.s64[1];
+    if (!direct && (st = stage_in(E, E.s64[0], fin, cnt))) return st;
+    if (kind == 0) st = op_d1z(&E, in, out, flag, np, E.nz);
+    else if (kind == 1) st = op_d1upz(&E, in, out, flag);
+    else st = op_d2z(&E, in, out, flag, np, E.nz);
     if (st) return st;
-    return stage_out(E, fout, E.s64[1], cnt);
+    if (!direct) return stage_out(E, fout, out, cnt);
+    CUDA_TRY(cudaStreamSynchronize(E.stream));
+    return VEC_OK;
 }
 
 extern "C" int vec_d1bydz(vec_ctx *c, const double *fin, double *fout, int dflag) { return zop(c, fin, fout, dflag, 0, 0); }

@@ -46,7 +46,9 @@ struct Engine {
     int par_mag = 1;            // mag_deriv on stream2 (FP64 form; VEC_SERIAL_MAG=0/1 forces it)
     long long launches = 0;
     int num_sms = 152;
-    int *dev_err = nullptr;     // set by kernels whose bounded waits ran out
+    int *dev_err = nullptr;     // set by kernels whose bounded waits ran out (mapped host
+                                // memory: read after a stream synchronisation, without a copy)
+    int dev = 0;                // the context's device
     int generic_lines = 0;      // force the generic line kernel (VEC_GENERIC_LINES=1)
 
     LinePlan plx, ply;          // precision of the bulk path
