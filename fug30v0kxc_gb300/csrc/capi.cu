@@ -321,8 +321,8 @@ extern "C" int vec_create(const vec_params *p, vec_ctx **out)
         aky2[E.ny / 2] = -(double)(E.ny / 2) * (double)(E.ny / 2) * cy * cy;
     }
     if ((st = fx_plan_make(E.nx, &E.fpx)) || (st = fx_plan_make(E.ny, &E.fpy)) ||
-        (st = fx_tables_make(E.nx, E.fpx, akx1.data(), akx2.data(), E.k.icutoffx, &E.fxx)) ||
-        (st = fx_tables_make(E.ny, E.fpy, aky1.data(), aky2.data(), E.k.icutoffy, &E.fxy)) ||
+        (st = fx_tables_make(E.nx, &E.fpx, akx1.data(), akx2.data(), E.k.icutoffx, &E.fxx)) ||
+        (st = fx_tables_make(E.ny, &E.fpy, aky1.data(), aky2.data(), E.k.icutoffy, &E.fxy)) ||
         (st = line_tables_make<float>(E.nx, akx1.data(), akx2.data(), E.k.icutoffx, &E.tx32)) ||
         (st = line_tables_make<float>(E.ny, aky1.data(), aky2.data(), E.k.icutoffy, &E.ty32))) {
         vec_destroy(c);

@@ -65,24 +65,23 @@ struct LineTables {
 struct FxPlan {
     int n, nb;              // length; elements of a buffer (n rounded up to 8)
     int np;                 // passes
-    int R[6], L[6], M[6], tw[6];
+    int R[6], L[6], M[6], tw[6], kind[6];
     unsigned mg[6];
     int ntw;                // twiddles in all
     int halvings;           // of one transform
     int gb;                 // its values stay below 2^gb times the norm
     int Q;                  // sequences per warp
-    int pow2;
+    int cut;                // wavenumbers below it survive the dealiasing
     float rn;               // 1 / n
+    float floor1, floor2;   // least sums of squares of a first, second derivative's spectrum
 };
 // its tables: twiddles by pass; position of wavenumber k in the spectrum and
-// back; per operator (and 1 / n) the multipliers by position, scaled by 2^-p to
-// at most one
+// back; the constants of dealias and inverse, d1 and d2
 struct TwX;
 struct FxTables {
-    TwX *tw;
+    TwX *tw;                // (one allocation with pos and kof)
     unsigned short *pos, *kof;
-    int2 *m1, *m2, *mda, *minv;
-    int p1, p2, pda, pinv;
+    double c0, c1, c2;
 };
 
 // horizontal wavenumber tables in one precision: akx1, aky1 and the

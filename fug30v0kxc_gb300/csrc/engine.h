@@ -218,7 +218,7 @@ int cdt_init(float *cdt);
 int line_ct_configure();
 int line_fx_configure();
 int fx_plan_make(int n, FxPlan *pl);
-int fx_tables_make(int n, const FxPlan &pl, const double *k1, const double *k2, int icut, FxTables *tb);
+int fx_tables_make(int n, FxPlan *pl, const double *k1, const double *k2, int icut, FxTables *tb);
 void fx_tables_free(FxTables *tb);
 template <typename R> int launch_lines_ct(Engine *E, int dir, const LineJob<R> *jobs, int njobs);
 

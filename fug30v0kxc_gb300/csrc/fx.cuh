@@ -61,14 +61,20 @@ __device__ __forceinline__ X2 fx_mulc(X2 a, TwX w) { return fx_mulw<false>(a, w)
 __device__ __forceinline__ X2 fx_mulcj(X2 a, TwX w) { return fx_mulw<true>(a, w); }
 __device__ __forceinline__ X2 fx_half(X2 a) { X2 r; r.x = a.x >> 1; r.y = a.y >> 1; return r; }
 
-// a m 2^(d - 1) for -1 <= d <= 30 where the result is below 2^62 (a itself
-// times 2^d need not be)
-__device__ __forceinline__ long long fx_muls(long long a, int mh, int ml, int d)
+// a k 2^-t for -20 <= t <= 31 where the result is below 2^62, |k| < 2^21
+__device__ __forceinline__ long long fx_mulk(long long a, int k, int t)
 {
-    const int h = fx_h(a), l = (int)a;
-    const long long mid = fx_wide(h, ml) + fx_wide(l, mh) + (fx_wide(l, ml) >> 32) + (1LL << (30 - d));
-    return (fx_wide(h, mh) << (1 + d)) + (mid >> (31 - d));
+    if (t <= 0) {
+        a <<= -t;
+        const long long p = fx_wide((int)a, k);
+        return (long long)(((unsigned long long)(unsigned)(fx_hi(p) + fx_h(a) * k) << 32) | (unsigned)p);
+    }
+    const long long p = fx_wide((int)a, k) + (1LL << (t - 1));
+    const long long q = fx_wide(fx_h(a), k) + (p >> 32);
+    return (q << (32 - t)) + (long long)((unsigned)p >> t);
 }
+// a signed 23-bit integer as a float, without the conversion unit
+__device__ __forceinline__ float fx_float(int v) { return __int_as_float(0x4b400000 + v) - 12582912.0f; }
 
 // ---- double <-> fixed ---------------------------------------------------------
 // The FP64 pipe converts 1.9 values per clock and SM, beside the integer pipe.

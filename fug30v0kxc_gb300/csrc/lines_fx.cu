@@ -6,7 +6,7 @@
 // forward transform is a chain of radix-8/6/5/4/3/2 passes by decimation in
 // frequency, in place, which leaves the spectrum in digit-reversed order; the
 // Hermitian multipliers of the operators (+ik, -k^2, 2/3 truncation) are
-// stored in that order, and the inverse runs the same passes backwards, so
+// applied in that order, and the inverse runs the same passes backwards, so
 // that nothing is reordered (only the halfcomplex transforms read or write
 // through the permutation).  Passes are synchronised per warp.  x lines:
 // warps are independent.  y lines: a CTA's sequences are adjacent columns,
@@ -19,12 +19,17 @@
 // in 57 % (three CTAs per SM at 80 registers).
 //
 // Measured at 256^2 x 129, mean of d2bydx and d1bydx: 618 us in FP64 (the FP64
-// pipe 83 % busy) -> 168 us, y the same; the 12 passes of an FP64 time step:
-// 14.6 -> 7.3 ms; error against long double 2 to 3 times smaller for white
-// noise, 10^3 times for a constant plus little.
+// pipe 83 % busy) -> 150 us, y the same.  (168 us with every element's place
+// computed, a table of multipliers, and x results stored by a loop of their
+// own.)  It issues in 45 % of the cycles, the rest being instruction fetches and
+// the latency of shared memory and conversions; synchronising the passes of a
+// CTA's warps, so that they fetch the same code, changed nothing.  Error against
+// long double: 2 to 3 times smaller than in FP64 for white noise, 10^4 times for
+// a constant plus little.
 #include <math.h>
 #include <string.h>
 
+#include <type_traits>
 #include <vector>
 
 #include "common.cuh"
@@ -41,74 +46,201 @@ struct FxPack { LineJob<double> j[MAX_JOBS]; };
 // different banks
 __device__ __forceinline__ int fx_at(int i, int s7) { return i ^ ((i >> 3) & 7) ^ s7; }
 
+// One pass of a sequence: radix R over the elements j + m M of every block of
+// L = R M.  KIND: how the elements' places in the buffer follow from the first's
+// (the permutation of fx_at costs three instructions per element in general):
+// K64: M a multiple of 64, K8: R = M = 8, K1: R = 8, M = 1.
+enum { KG, K64, K8, K1 };
 struct FxPassArgs { int n, L, M, G, l, s7; unsigned mg; const TwX *tw; };
 
-// one decimation-in-frequency pass: DFT_R over the elements j + m M of every
-// block of L, then W_L^(j r) / 2.  FIRST: the elements are (a - mean) 2^sh.
-template <int R, bool FIRST>
-__device__ __forceinline__ void fx_fwd(X2 *buf, const FxPassArgs &a, long long mx, long long my, int sh)
+template <int R, int KIND>
+__device__ __forceinline__ void fx_places(const FxPassArgs &a, int b, int &j, int *at)
 {
+    if (KIND == K1) {
+        j = 0;
+        const int base = 8 * b + ((b & 7) ^ a.s7);
+#pragma unroll
+        for (int m = 0; m < R; m++) at[m] = base ^ m;
+    } else if (KIND == K8) {
+        j = b & 7;
+        const int base = 8 * (b - j) + (j ^ a.s7);
+#pragma unroll
+        for (int m = 0; m < R; m++) at[m] = (base ^ m) + 8 * m;
+    } else {
+        const int q = (int)(((unsigned long long)(unsigned)b * a.mg) >> 31);
+        j = b - q * a.M;
+        const int i = q * a.L + j;
+        at[0] = fx_at(i, a.s7);
+#pragma unroll
+        for (int m = 1; m < R; m++) at[m] = KIND == K64 ? at[0] + m * a.M : fx_at(i + m * a.M, a.s7);
+    }
+}
+template <int KIND> __device__ __forceinline__ int fx_stride(const FxPassArgs &a) { return KIND == K8 ? 8 : a.M; }
+
+// decimation in frequency: DFT_R, then W_L^(j r) / 2
+template <int R, int KIND>
+__device__ __forceinline__ void fx_fwd(X2 *buf, const FxPassArgs &a)
+{
+    const int M = fx_stride<KIND>(a);
     for (int b = a.l; b < a.n / R; b += a.G) {
-        const int q = (int)(((unsigned long long)(unsigned)b * a.mg) >> 31), j = b - q * a.M;
-        int at[R];
+        int j, at[R];
         X2 v[R];
+        fx_places<R, KIND>(a, b, j, at);
 #pragma unroll
-        for (int m = 0; m < R; m++) {
-            at[m] = fx_at(q * a.L + j + m * a.M, a.s7);
-            v[m] = buf[at[m]];
-            if (FIRST) { v[m].x = fx_shift(v[m].x - mx, sh); v[m].y = fx_shift(v[m].y - my, sh); }
-        }
+        for (int m = 0; m < R; m++) v[m] = buf[at[m]];
         XDft<R, false>::run(v);
-        buf[at[0]] = a.M > 1 ? fx_half(v[0]) : v[0];
+        buf[at[0]] = fx_half(v[0]);
+        const TwX *w = a.tw + j;
 #pragma unroll
-        for (int r = 1; r < R; r++) buf[at[r]] = a.M > 1 ? fx_mulc(v[r], a.tw[(r - 1) * a.M + j]) : v[r];
+        for (int r = 1; r < R; r++) buf[at[r]] = fx_mulc(v[r], w[(r - 1) * M]);
     }
     __syncwarp();
 }
-// the reverse: conj(W_L^(j r)) / 2, then the inverse DFT_R.  MUL: the elements
-// are those of src times 2^(d - 1) and the multiplier (i times it for D1).
-template <int R, bool MUL>
-__device__ __forceinline__ void fx_inv(X2 *buf, const X2 *src, const FxPassArgs &a, const int2 *mul, bool d1, int d)
+// The last pass (M = 1) has no twiddles.  Its results are the spectrum: with
+// key, the sums of |k X|^2 (s1) and |k^2 X|^2 (s2) over it, in units of 2^39
+// for X.  (Its element m of butterfly b is wavenumber kof[b R] + m n / R.)
+template <int R, int KIND>
+__device__ __forceinline__ void fx_last(X2 *buf, const FxPassArgs &a, const unsigned short *kof, bool key, float &s1, float &s2)
 {
     for (int b = a.l; b < a.n / R; b += a.G) {
-        const int q = (int)(((unsigned long long)(unsigned)b * a.mg) >> 31), j = b - q * a.M;
-        int at[R];
+        int j, at[R];
         X2 v[R];
+        fx_places<R, KIND>(a, b, j, at);
 #pragma unroll
-        for (int r = 0; r < R; r++) {
-            const int i = q * a.L + j + r * a.M;
-            at[r] = fx_at(i, a.s7);
-            if (MUL) {
-                const X2 z = src[at[r]];
-                const int2 m = __ldg(mul + i);
-                const long long p = fx_muls(z.x, m.x, m.y, d), w = fx_muls(z.y, m.x, m.y, d);
-                v[r].x = d1 ? -w : p;
-                v[r].y = d1 ? p : w;
-            } else {
-                v[r] = buf[at[r]];
-                if (r == 0) v[r] = a.M > 1 ? fx_half(v[r]) : v[r];
-                else if (a.M > 1) v[r] = fx_mulcj(v[r], a.tw[(r - 1) * a.M + j]);
+        for (int m = 0; m < R; m++) v[m] = buf[at[m]];
+        XDft<R, false>::run(v);
+#pragma unroll
+        for (int m = 0; m < R; m++) buf[at[m]] = v[m];
+        if (key) {
+            const int k0 = __ldg(kof + b * R), dk = a.n / R;
+#pragma unroll
+            for (int m = 0; m < R; m++) {
+                const int k = k0 + m * dk;
+                const float kf = (float)min(k, a.n - k), x = fx_float((fx_hi(v[m].x) + 64) >> 7), y = fx_float((fx_hi(v[m].y) + 64) >> 7);
+                const float p = x * x + y * y, k2 = kf * kf;
+                s1 = fmaf(p, k2, s1);
+                s2 = fmaf(p * k2, k2, s2);
             }
         }
+    }
+    __syncwarp();
+}
+// what the first inverse pass does to the spectrum: the operators' multipliers
+// are i k, -k^2 and a mask, up to the constant in the results' scale
+__device__ __forceinline__ X2 fx_op(X2 z, int op, int k, int n, int t, int cut)
+{
+    if (op == OP_INV) return z;
+    const int kk = min(k, n - k);
+    X2 y;
+    if (op == OP_DEALIAS) {
+        y.x = kk < cut ? z.x >> t : 0;
+        y.y = kk < cut ? z.y >> t : 0;
+        return y;
+    }
+    const bool d1 = op == OP_D1;
+    const int m = !d1 ? kk * kk : 2 * k < n ? k : 2 * k == n ? 0 : k - n;
+    y.x = fx_mulk(d1 ? z.y : z.x, d1 ? -m : m, t);
+    y.y = fx_mulk(d1 ? z.x : z.y, m, t);
+    return y;
+}
+// the reverse of fx_last, from src into buf
+template <int R, int KIND>
+__device__ __forceinline__ void fx_inv_first(X2 *buf, const X2 *src, const FxPassArgs &a, const unsigned short *kof, int op, int t,
+                                             int cut)
+{
+    for (int b = a.l; b < a.n / R; b += a.G) {
+        int j, at[R];
+        X2 v[R];
+        fx_places<R, KIND>(a, b, j, at);
+        const int k0 = op == OP_INV ? 0 : (int)__ldg(kof + b * R), dk = a.n / R;
+#pragma unroll
+        for (int m = 0; m < R; m++) v[m] = fx_op(src[at[m]], op, k0 + m * dk, a.n, t, cut);
         XDft<R, true>::run(v);
 #pragma unroll
-        for (int r = 0; r < R; r++) buf[at[r]] = v[r];
+        for (int m = 0; m < R; m++) buf[at[m]] = v[m];
+    }
+    __syncwarp();
+}
+// conj(W_L^(j r)) / 2, then the inverse DFT_R.  With oa (the last pass of an x
+// line): the results times sc, plus c, to the two rows.
+template <int R, int KIND, bool OUT>
+__device__ __forceinline__ void fx_inv(X2 *buf, const FxPassArgs &a, double *oa, double *ob, double sc, double ca, double cb, bool con)
+{
+    const int M = fx_stride<KIND>(a);
+    for (int b = a.l; b < a.n / R; b += a.G) {
+        int j, at[R];
+        X2 v[R];
+        fx_places<R, KIND>(a, b, j, at);
+        const TwX *w = a.tw + j;
+        v[0] = fx_half(buf[at[0]]);
+#pragma unroll
+        for (int r = 1; r < R; r++) v[r] = fx_mulcj(buf[at[r]], w[(r - 1) * M]);
+        XDft<R, true>::run(v);
+        if (OUT) {
+            // (one block: elements j + r M)
+            if (con) {
+#pragma unroll
+                for (int r = 0; r < R; r++) {
+                    oa[j + r * M] = fma(__ll2double_rn(v[r].x), sc, ca);
+                    ob[j + r * M] = fma(__ll2double_rn(v[r].y), sc, cb);
+                }
+            } else {
+#pragma unroll
+                for (int r = 0; r < R; r++) {
+                    oa[j + r * M] = __ll2double_rn(v[r].x) * sc;
+                    ob[j + r * M] = __ll2double_rn(v[r].y) * sc;
+                }
+            }
+        } else {
+#pragma unroll
+            for (int r = 0; r < R; r++) buf[at[r]] = v[r];
+        }
     }
     __syncwarp();
 }
 
-#define FX_RADIX(R, CALL)                                                                  \
-    switch (R) {                                                                           \
-    case 8: { constexpr int RR = 8; CALL; break; }                                         \
-    case 6: { constexpr int RR = 6; CALL; break; }                                         \
-    case 5: { constexpr int RR = 5; CALL; break; }                                         \
-    case 4: { constexpr int RR = 4; CALL; break; }                                         \
-    case 3: { constexpr int RR = 3; CALL; break; }                                         \
-    default: { constexpr int RR = 2; CALL; break; }                                        \
+// a pass's template by its radix and kind
+#define FX_SWITCH(pl, p, CALL)                                                             \
+    if (pl.kind[p] == K64) {                                                               \
+        switch (pl.R[p]) {                                                                 \
+        case 8: CALL(8, K64); break;                                                       \
+        case 6: CALL(6, K64); break;                                                       \
+        case 5: CALL(5, K64); break;                                                       \
+        case 4: CALL(4, K64); break;                                                       \
+        case 3: CALL(3, K64); break;                                                       \
+        default: CALL(2, K64); break;                                                      \
+        }                                                                                  \
+    } else if (pl.kind[p] == K8) {                                                         \
+        CALL(8, K8);                                                                       \
+    } else {                                                                               \
+        switch (pl.R[p]) {                                                                 \
+        case 8: CALL(8, KG); break;                                                        \
+        case 6: CALL(6, KG); break;                                                        \
+        case 5: CALL(5, KG); break;                                                        \
+        case 4: CALL(4, KG); break;                                                        \
+        case 3: CALL(3, KG); break;                                                        \
+        default: CALL(2, KG); break;                                                       \
+        }                                                                                  \
+    }
+// the last pass: K1 or general
+#define FX_SWITCH_LAST(pl, CALL)                                                           \
+    if (pl.kind[pl.np - 1] == K1) {                                                        \
+        CALL(8, K1);                                                                       \
+    } else {                                                                               \
+        switch (pl.R[pl.np - 1]) {                                                         \
+        case 8: CALL(8, KG); break;                                                        \
+        case 6: CALL(6, KG); break;                                                        \
+        case 5: CALL(5, KG); break;                                                        \
+        case 4: CALL(4, KG); break;                                                        \
+        case 3: CALL(3, KG); break;                                                        \
+        default: CALL(2, KG); break;                                                       \
+        }                                                                                  \
     }
 
-// what the store of a sequence needs (y lines: through shared memory)
-struct FxOut { double cx, cy; int xe, nonfin; };
+// what the store of a sequence needs (y lines: through shared memory): results
+// are integers times sc, plus c; or, where sc would leave the normal range or
+// the line is not finite, times con 2^xe
+struct FxOut { double cx, cy, sc; int xe, bad; };
 
 // DIR 0: x lines (sequence = two rows), DIR 1: y lines (two columns).  tpp
 // tiles per plane: of Q sequences (one warp's, x) or S = warps Q (a CTA's, y).
@@ -120,10 +252,10 @@ line_fx(const __grid_constant__ FxPack jobs, const __grid_constant__ FxPlan pl, 
     PDL_WAIT();
     extern __shared__ __align__(128) unsigned char smem[];
     const int n = pl.n, Q = pl.Q, G = 32 / Q, W = (int)blockDim.x / 32, S = W * Q;
-    TwX *tw = reinterpret_cast<TwX *>(smem);
-    X2 *bufA = reinterpret_cast<X2 *>(tw + pl.ntw);
+    X2 *bufA = reinterpret_cast<X2 *>(smem);
     X2 *bufB = bufA + (size_t)S * pl.nb;               // (two)
-    FxOut *so = reinterpret_cast<FxOut *>(bufB + (two ? (size_t)S * pl.nb : 0));
+    TwX *tw = reinterpret_cast<TwX *>(bufB + (two ? (size_t)S * pl.nb : 0));
+    FxOut *so = reinterpret_cast<FxOut *>(tw + pl.ntw);
     const int tid = threadIdx.x, wid = tid >> 5, g = (tid & 31) / G, l = (tid & 31) % G;
     const int s = wid * Q + g;
     const int s7 = DIR == 1 ? s & 7 : 0;
@@ -144,91 +276,79 @@ line_fx(const __grid_constant__ FxPack jobs, const __grid_constant__ FxPlan pl, 
         const int plane = rem / tpp, tile = rem - plane * tpp;
         const LineJob<double> &jb = jobs.j[job];
         const int op1 = jb.op1, op2 = jb.op2;
+        const bool inv = op1 == OP_INV;
         const size_t pb = (size_t)plane * np;
         const int pair = tile * (DIR == 0 ? Q : S) + (DIR == 0 ? g : s);     // this group's lines 2 pair, 2 pair + 1
         const bool valid = pair < pairs;
 
-        // ---- load the bits
-        unsigned mxh = 0u;
-        if (DIR == 0) {
-            const double *r0 = jb.in + pb + (size_t)(valid ? 2 * pair : 0) * nx, *r1 = r0 + nx;
-            for (int e0 = l; e0 < n; e0 += 8 * G) {
-                X2 v[8];
-#pragma unroll
-                for (int c = 0; c < 8; c++) {
-                    const int e = e0 + c * G;
-                    const bool in = valid && e < n;
-                    v[c].x = in ? __double_as_longlong(r0[e]) : 0;
-                    v[c].y = in ? __double_as_longlong(r1[e]) : 0;
-                }
-#pragma unroll
-                for (int c = 0; c < 8; c++) {
-                    const int e = e0 + c * G;
-                    if (e >= n) break;
-                    mxh = max(mxh, (unsigned)fx_hi(v[c].x) & 0x7fffffffu);
-                    mxh = max(mxh, (unsigned)fx_hi(v[c].y) & 0x7fffffffu);
-                    A[fx_at(e, s7)] = v[c];
-                }
-            }
-        } else {
-            const int ls = 31 - __clz(S);
-            const double *in = jb.in + pb + 2 * (size_t)tile * S;
-            for (int i0 = tid; i0 < n * S; i0 += 8 * (int)blockDim.x) {
+        // ---- y lines: the bits into shared memory, row by row
+        const double *r0 = jb.in + pb + (size_t)(valid ? 2 * pair : 0) * nx;
+        if (DIR == 1) {
+            const int ls = 31 - __clz(S), q = tid & (S - 1), de = (int)blockDim.x >> ls;     // (S divides the CTA)
+            const double *in = jb.in + pb + 2 * ((size_t)tile * S + q);
+            const bool have = tile * S + q < pairs;
+            double2 *to = reinterpret_cast<double2 *>(bufA + (size_t)q * pl.nb);
+            for (int e0 = tid >> ls; e0 < n; e0 += 8 * de) {
                 double2 v[8];
 #pragma unroll
                 for (int c = 0; c < 8; c++) {
-                    const int i = i0 + c * (int)blockDim.x, e = i >> ls, q = i & (S - 1);
-                    v[c] = i < n * S && tile * S + q < pairs ? *reinterpret_cast<const double2 *>(in + (size_t)e * nx + 2 * q)
-                                                             : make_double2(0.0, 0.0);
+                    const int e = e0 + c * de;
+                    v[c] = have && e < n ? *reinterpret_cast<const double2 *>(in + (size_t)e * nx) : make_double2(0.0, 0.0);
                 }
 #pragma unroll
-                for (int c = 0; c < 8; c++) {
-                    const int i = i0 + c * (int)blockDim.x, e = i >> ls, q = i & (S - 1);
-                    if (i < n * S) *reinterpret_cast<double2 *>(bufA + (size_t)q * pl.nb + fx_at(e, q & 7)) = v[c];
-                }
+                for (int c = 0; c < 8; c++)
+                    if (e0 + c * de < n) to[fx_at(e0 + c * de, q & 7)] = v[c];
             }
             __syncthreads();
-            for (int e = l; e < n; e += G) {
-                const X2 v = A[fx_at(e, s7)];
-                mxh = max(mxh, (unsigned)fx_hi(v.x) & 0x7fffffffu);
-                mxh = max(mxh, (unsigned)fx_hi(v.y) & 0x7fffffffu);
-            }
         }
-        for (int o = G >> 1; o > 0; o >>= 1) mxh = max(mxh, __shfl_xor_sync(0xffffffffu, mxh, o));
-        const int E = (int)max(mxh >> 20, 1u);
-        FxOut out;
-        out.nonfin = E == 0x7ff;
-        out.cx = out.cy = 0.0;
+        auto raw = [&](int e) -> X2 {
+            X2 v;
+            if (DIR == 0) {
+                v.x = valid ? __double_as_longlong(r0[e]) : 0;
+                v.y = valid ? __double_as_longlong(r0[e + nx]) : 0;
+            } else {
+                v = A[fx_at(e, s7)];
+            }
+            return v;
+        };
+        auto top = [](unsigned m, const X2 &v) {
+            return max(max(m, (unsigned)fx_hi(v.x) & 0x7fffffffu), (unsigned)fx_hi(v.y) & 0x7fffffffu);
+        };
+        auto group_max = [&](unsigned m) {
+            for (int o = G >> 1; o > 0; o >>= 1) m = max(m, __shfl_xor_sync(0xffffffffu, m, o));
+            return (int)max(m >> 20, 1u);
+        };
+        auto group_sum = [&](float f) {
+            for (int o = G >> 1; o > 0; o >>= 1) f += __shfl_xor_sync(0xffffffffu, f, o);
+            return f;
+        };
 
-        // ---- to integers; the mean of a real line, or a spectrum's constant, off
-        int sx = 0, sy = 0;
-        const bool low = E < 64;
-        const bool inv = op1 == OP_INV;
+        // ---- to integers; the mean of a real line, or a spectrum's constant, off;
+        // then the norm and with it the exponent F
+        FxOut out;
+        out.cx = out.cy = 0.0;
+        int E = 1, F = 0, sx = 0, sy = 0;
+        long long mx = 0, my = 0;
         double dcx = 0.0, dcy = 0.0;
-        for (int e = l; e < n; e += G) {
-            X2 v = A[fx_at(e, s7)];
+        auto conv = [&](int e, X2 v) {
             if (inv && e == 0) {
                 dcx = __longlong_as_double(v.x);
                 dcy = __longlong_as_double(v.y);
                 v.x = v.y = 0;
             }
-            if (low) {
-                v.x = fx_from_low((unsigned)fx_hi(v.x), (unsigned)v.x, E);
-                v.y = fx_from_low((unsigned)fx_hi(v.y), (unsigned)v.y, E);
-            } else {
-                v.x = fx_from((unsigned)fx_hi(v.x), (unsigned)v.x, E);
-                v.y = fx_from((unsigned)fx_hi(v.y), (unsigned)v.y, E);
-            }
+            v.x = fx_from((unsigned)fx_hi(v.x), (unsigned)v.x, E);
+            v.y = fx_from((unsigned)fx_hi(v.y), (unsigned)v.y, E);
             sx += fx_hi(v.x) >> 9;
             sy += fx_hi(v.y) >> 9;
-            A[fx_at(e, s7)] = v;
-        }
-        long long mx = 0, my = 0;
-        if (inv) {
-            const int src = (tid & 31) - l;
-            out.cx = __shfl_sync(0xffffffffu, dcx, src) / (double)n;
-            out.cy = __shfl_sync(0xffffffffu, dcy, src) / (double)n;
-        } else {
+            return v;
+        };
+        auto means = [&]() {
+            if (inv) {
+                const int src = (tid & 31) - l;
+                out.cx = __shfl_sync(0xffffffffu, dcx, src) / (double)n;
+                out.cy = __shfl_sync(0xffffffffu, dcy, src) / (double)n;
+                return;
+            }
             for (int o = G >> 1; o > 0; o >>= 1) {
                 sx += __shfl_xor_sync(0xffffffffu, sx, o);
                 sy += __shfl_xor_sync(0xffffffffu, sy, o);
@@ -236,53 +356,167 @@ line_fx(const __grid_constant__ FxPack jobs, const __grid_constant__ FxPlan pl, 
             // (to 21 bits, a multiple of 2^41 units)
             mx = (long long)(int)((float)sx * pl.rn) << 41;
             my = (long long)(int)((float)sy * pl.rn) << 41;
+        };
+        auto square = [&](const X2 &v) {     // in units of 2^41
+            const float x = fx_float(fx_hi(v.x) >> 9), y = fx_float(fx_hi(v.y) >> 9);
+            return x * x + y * y;
+        };
+        auto shift = [&](float sq) {
+            // (the squares are of truncated values: 8 n for what they leave out; a
+            // halfcomplex element stands for two of the spectrum)
+            const int K = fx_log2((sq + 8.0f * (float)n) * (inv ? 2.0f : 1.0f));
+            const int sh = 20 - pl.gb - ((K + 1) >> 1);
+            F = E - 1084 - sh;
+            return sh;
+        };
+        // (rare: near the bottom of the exponent range, where subnormals count,
+        // the elements become integers one by one, in shared memory)
+        auto conv_low = [&](int e) {
+            X2 v = A[fx_at(e, s7)];
+            if (inv && e == 0) {
+                dcx = __longlong_as_double(v.x);
+                dcy = __longlong_as_double(v.y);
+                v.x = v.y = 0;
+            }
+            v.x = fx_from_low((unsigned)fx_hi(v.x), (unsigned)v.x, E);
+            v.y = fx_from_low((unsigned)fx_hi(v.y), (unsigned)v.y, E);
+            sx += fx_hi(v.x) >> 9;
+            sy += fx_hi(v.y) >> 9;
+            A[fx_at(e, s7)] = v;
+        };
+        // CH elements per lane in registers
+        auto in_registers = [&](auto chunk) {
+            constexpr int CH = decltype(chunk)::value;
+            X2 v[CH];
+            unsigned m = 0u;
+#pragma unroll
+            for (int c = 0; c < CH; c++) {
+                const int e = l + c * G;
+                if (e < n) v[c] = raw(e);
+                else v[c].x = v[c].y = 0;
+            }
+#pragma unroll
+            for (int c = 0; c < CH; c++) m = top(m, v[c]);
+            E = group_max(m);
+            if (E >= 64) {
+#pragma unroll
+                for (int c = 0; c < CH; c++) v[c] = conv(l + c * G, v[c]);
+            } else {
+#pragma unroll
+                for (int c = 0; c < CH; c++)
+                    if (l + c * G < n) A[fx_at(l + c * G, s7)] = v[c];
+                for (int e = l; e < n; e += G) conv_low(e);
+#pragma unroll
+                for (int c = 0; c < CH; c++)
+                    if (l + c * G < n) v[c] = A[fx_at(l + c * G, s7)];
+            }
+            means();
+            float sq = 0.0f;
+#pragma unroll
+            for (int c = 0; c < CH; c++) {
+                if (l + c * G < n) {
+                    v[c].x -= mx;
+                    v[c].y -= my;
+                }
+                sq += square(v[c]);
+            }
+            const int sh = shift(group_sum(sq));
+#pragma unroll
+            for (int c = 0; c < CH; c++) {
+                const int e = l + c * G;
+                v[c].x = fx_shift(v[c].x, sh);
+                v[c].y = fx_shift(v[c].y, sh);
+                if (e < n) A[fx_at(e, s7)] = v[c];
+            }
+        };
+        if (n <= 2 * G) {
+            in_registers(std::integral_constant<int, 2>());
+        } else if (n <= 8 * G) {
+            in_registers(std::integral_constant<int, 8>());
+        } else {
+            unsigned m = 0u;
+            for (int e0 = l; e0 < n; e0 += 8 * G) {
+                X2 v[8];
+#pragma unroll
+                for (int c = 0; c < 8; c++) {
+                    const int e = e0 + c * G;
+                    if (e < n) v[c] = raw(e);
+                    else v[c].x = v[c].y = 0;
+                }
+#pragma unroll
+                for (int c = 0; c < 8; c++) {
+                    m = top(m, v[c]);
+                    if (DIR == 0 && e0 + c * G < n) A[fx_at(e0 + c * G, s7)] = v[c];
+                }
+            }
+            E = group_max(m);
+            if (E >= 64)
+                for (int e = l; e < n; e += G) A[fx_at(e, s7)] = conv(e, A[fx_at(e, s7)]);
+            else
+                for (int e = l; e < n; e += G) conv_low(e);
+            means();
+            float sq = 0.0f;
+            for (int e = l; e < n; e += G) {
+                X2 v = A[fx_at(e, s7)];
+                v.x -= mx;
+                v.y -= my;
+                sq += square(v);
+            }
+            const int sh = shift(group_sum(sq));
+            for (int e = l; e < n; e += G) {
+                X2 v = A[fx_at(e, s7)];
+                v.x = fx_shift(v.x - mx, sh);
+                v.y = fx_shift(v.y - my, sh);
+                A[fx_at(e, s7)] = v;
+            }
+        }
+        out.bad = E == 0x7ff;
+        if (op1 == OP_FWD || op1 == OP_DEALIAS || op2 == OP_DEALIAS) {
             const int ex = E - 1084;
             out.cx = fx_to(mx, ex, fx_safe(ex));
             out.cy = fx_to(my, ex, fx_safe(ex));
         }
-        // ---- the norm and with it the exponent
-        long long ss = 0;
-        for (int e = l; e < n; e += G) {
-            const X2 v = A[fx_at(e, s7)];
-            const int qx = fx_hi(v.x - mx) >> 4, qy = fx_hi(v.y - my) >> 4;
-            ss += fx_wide(qx, qx) + fx_wide(qy, qy);
-        }
-        auto log2sum = [&](long long v) {
-            float f = (float)v;
-            for (int o = G >> 1; o > 0; o >>= 1) f += __shfl_xor_sync(0xffffffffu, f, o);
-            return fx_log2(f);
-        };
-        // (a halfcomplex element stands for two of the spectrum)
-        const int K = log2sum(ss) + (inv ? 1 : 0);
-        const int sh = min(25 - pl.gb - ((K + 1) >> 1), 15);
-        const int F = E - 1084 - sh;
         __syncwarp();
 
+        // ---- forward
+        float s1 = 0.0f, s2 = 0.0f;
         if (!inv) {
-            { const FxPassArgs a = args(0); FX_RADIX(pl.R[0], (fx_fwd<RR, true>(A, a, mx, my, sh))) }
-            for (int p = 1; p < pl.np; p++) { const FxPassArgs a = args(p); FX_RADIX(pl.R[p], (fx_fwd<RR, false>(A, a, 0, 0, 0))) }
+            for (int p = 0; p < pl.np - 1; p++) {
+                const FxPassArgs a = args(p);
+#define CALL(R, K) fx_fwd<R, K>(A, a)
+                FX_SWITCH(pl, p, CALL)
+#undef CALL
+            }
+            const bool key = op1 == OP_D1 || op1 == OP_D2 || op2 == OP_D1 || op2 == OP_D2;
+            const FxPassArgs a = args(pl.np - 1);
+#define CALL(R, K) fx_last<R, K>(A, a, tb.kof, key, s1, s2)
+            FX_SWITCH_LAST(pl, CALL)
+#undef CALL
+            if (key) {
+                s1 = group_sum(s1);
+                s2 = group_sum(s2);
+            }
         }
 
         if (op1 == OP_FWD) {
             // separate Z into the halfcomplex spectra of the two real lines
             out.xe = F + pl.halvings - 1;
             const bool scale = jb.alpha1 != 1.0;
-            auto sep = [&](const X2 *Z, int z7, int p, const FxOut &o, bool safe, double *va, double *vb) {
+            auto sep = [&](const X2 *Z, int z7, int p, const FxOut &o, double *va, double *vb) {
                 const X2 zp = Z[fx_at(__ldg(tb.pos + p), z7)], zq = Z[fx_at(__ldg(tb.pos + (p == 0 ? 0 : n - p)), z7)];
-                const bool re = 2 * p <= n;
+                const bool re = 2 * p <= n, safe = fx_safe(o.xe);
                 *va = fx_to(re ? zp.x + zq.x : zq.y - zp.y, o.xe, safe);
                 *vb = fx_to(re ? zp.y + zq.y : zp.x - zq.x, o.xe, safe);
                 if (p == 0) { *va += (double)n * o.cx; *vb += (double)n * o.cy; }
-                if (o.nonfin) *va = *vb = FX_NAN;
+                if (o.bad) *va = *vb = FX_NAN;
                 if (scale) { *va *= jb.alpha1; *vb *= jb.alpha1; }
             };
             if (DIR == 0) {
                 if (valid) {
                     double *oa = jb.out1 + pb + 2 * (size_t)pair * nx, *ob = oa + nx;
-                    const bool safe = fx_safe(out.xe);
                     for (int p = l; p < n; p += G) {
                         double va, vb;
-                        sep(A, s7, p, out, safe, &va, &vb);
+                        sep(A, s7, p, out, &va, &vb);
                         oa[p] = jb.acc1 ? oa[p] + va : va;
                         ob[p] = jb.acc1 ? ob[p] + vb : vb;
                     }
@@ -291,147 +525,148 @@ line_fx(const __grid_constant__ FxPack jobs, const __grid_constant__ FxPlan pl, 
             } else {
                 if (l == 0) so[s] = out;
                 __syncthreads();
-                const int ls = 31 - __clz(S);
-                double *op = jb.out1 + pb + 2 * (size_t)tile * S;
-                for (int i = tid; i < n * S; i += (int)blockDim.x) {
-                    const int p = i >> ls, q = i & (S - 1);
-                    if (tile * S + q >= pairs) continue;
+                const int ls = 31 - __clz(S), q = tid & (S - 1);
+                if (tile * S + q < pairs) {
                     const FxOut o = so[q];
-                    double2 v;
-                    sep(bufA + (size_t)q * pl.nb, q & 7, p, o, fx_safe(o.xe), &v.x, &v.y);
-                    double2 *d = reinterpret_cast<double2 *>(op + (size_t)p * nx + 2 * q);
-                    if (jb.acc1) { const double2 w = *d; v.x = w.x + v.x; v.y = w.y + v.y; }
-                    *d = v;
+                    double *op = jb.out1 + pb + 2 * ((size_t)tile * S + q);
+                    for (int p = tid >> ls; p < n; p += (int)blockDim.x >> ls) {
+                        double2 v;
+                        sep(bufA + (size_t)q * pl.nb, q & 7, p, o, &v.x, &v.y);
+                        double2 *d = reinterpret_cast<double2 *>(op + (size_t)p * nx);
+                        if (jb.acc1) { const double2 w = *d; v.x = w.x + v.x; v.y = w.y + v.y; }
+                        *d = v;
+                    }
                 }
                 __syncthreads();
             }
             continue;
         }
 
+        // ---- one or two inverse transforms
         const int nout = op2 != OP_NONE && (!inv || op2 == OP_D1) ? 2 : 1;
         for (int o = 0; o < nout; o++) {
             const int op = o == 0 ? op1 : op2;
             const X2 *src = A;
             X2 *dst = o + 1 < nout ? B : A;
-            int sh1 = 0;               // exponent of the multiplier step
             if (inv) {
                 // Z_k = A_k + i B_k from the halfcomplex lines a (re), b (im),
                 // into the digit-reversed order of the passes
+                float q1 = 0.0f;
                 for (int i = l; i < n; i += G) {
-                    const int k = __ldg(tb.kof + i), kk = 2 * k <= n ? k : n - k;
+                    const int k = __ldg(tb.kof + i), kk = min(k, n - k);
                     const bool edge = kk == 0 || 2 * kk == n;
-                    X2 pa = A[fx_at(kk, s7)], pbb = A[fx_at(edge ? 0 : n - kk, s7)];
-                    if (edge) pbb.x = pbb.y = 0;
-                    pa.x = fx_shift(pa.x, sh); pa.y = fx_shift(pa.y, sh);
-                    pbb.x = fx_shift(pbb.x, sh); pbb.y = fx_shift(pbb.y, sh);
-                    if (2 * k > n) { pbb.x = -pbb.x; pbb.y = -pbb.y; }
+                    const X2 pa = A[fx_at(kk, s7)];
+                    X2 pc = A[fx_at(edge ? 0 : n - kk, s7)];
+                    if (edge) pc.x = pc.y = 0;
+                    if (2 * k > n) { pc.x = -pc.x; pc.y = -pc.y; }
                     X2 z;
-                    z.x = pa.x - pbb.y;
-                    z.y = pbb.x + pa.y;
+                    z.x = pa.x - pc.y;
+                    z.y = pc.x + pa.y;
                     B[fx_at(i, s7)] = z;
+                    const float x = fx_float((fx_hi(z.x) + 64) >> 7), y = fx_float((fx_hi(z.y) + 64) >> 7), kf = (float)kk;
+                    q1 = fmaf((x * x + y * y) * kf, kf, q1);
                 }
+                if (op == OP_D1) s1 = group_sum(q1);
                 __syncwarp();
                 src = dst = B;
             }
-            const int2 *mul = op == OP_D1 ? tb.m1 : op == OP_D2 ? tb.m2 : tb.mda;
-            int d = 1 - pl.gb;
-            if (op == OP_D1 || op == OP_D2) {
-                // the spectrum's norm from a quarter of the products to 27 bits
-                long long sy2 = 0;
-                for (int i = l; i < n; i += G) {
-                    const X2 z = src[fx_at(i, s7)];
-                    const int m = __ldg(&mul[i].x);
-                    const int qx = fx_hi(fx_wide(fx_hi(z.x), m)), qy = fx_hi(fx_wide(fx_hi(z.y), m));
-                    sy2 += fx_wide(qx, qx) + fx_wide(qy, qy);
+            // the multiplier's shift: a derivative's from its norm (what the
+            // squares cannot resolve counted in), a mask's for the growth
+            int sh = 0;
+            if (op == OP_D1) sh = max(((fx_log2(s1 + pl.floor1) + 1) >> 1) + pl.gb - 22, -20);
+            else if (op == OP_D2) sh = max(((fx_log2(s2 + pl.floor2) + 1) >> 1) + pl.gb - 22, -20);
+            else if (op == OP_DEALIAS) sh = pl.gb;
+            {
+                const FxPassArgs a = args(pl.np - 1);
+                if (op == OP_INV && pl.kind[pl.np - 1] == K1) {
+                    fx_inv_first<8, K1>(dst, src, a, tb.kof, OP_INV, 0, 0);
+                } else {
+#define CALL(R, K) fx_inv_first<R, K>(dst, src, a, tb.kof, op, sh, pl.cut)
+                    FX_SWITCH_LAST(pl, CALL)
+#undef CALL
                 }
-                d = min(max(28 - pl.gb - ((log2sum(sy2) + 1) >> 1), -1), 20);
-                __syncwarp();
             }
-            int p = pl.np - 1;
-            if (op != OP_INV || !pl.pow2) {
-                sh1 = 1 - d + (op == OP_D1 ? tb.p1 : op == OP_D2 ? tb.p2 : op == OP_INV ? tb.pinv : tb.pda);
-                const int2 *mm = op == OP_INV ? tb.minv : mul;
-                const FxPassArgs a = args(p);
-                FX_RADIX(pl.R[p], (fx_inv<RR, true>(dst, src, a, mm, op == OP_D1, d)))
-                p--;
-            } else {
-                sh1 = tb.pinv;
-            }
-            for (; p >= 0; p--) { const FxPassArgs a = args(p); FX_RADIX(pl.R[p], (fx_inv<RR, false>(dst, dst, a, nullptr, false, 0))) }
-
-            out.xe = F + sh1 + (inv ? 1 : 2) * pl.halvings;
+            out.xe = F + sh + (inv ? 1 : 2) * pl.halvings;
+            const double con = op == OP_D1 ? tb.c1 : op == OP_D2 ? tb.c2 : tb.c0;
+            // (con 2^xe, and with it every result, in the normal range)
+            const bool safe = out.xe >= -700 && out.xe <= 700;
+            out.sc = safe ? con * __hiloint2double((1023 + out.xe) << 20, 0) : 0.0;
             const double alpha = o == 0 ? jb.alpha1 : jb.alpha2;
             const int acc = o == 0 ? jb.acc1 : jb.acc2;
             double *ot = o == 0 ? jb.out1 : jb.out2;
             // what is added back: the mean of a dealiased line, the constant of an
-            // inverse and its addk, addc
-            const bool con = op == OP_DEALIAS || op == OP_INV;
+            // inverse, and its addk, addc.  (What is only stored takes paths of its
+            // own: FP64 operations, predicated off or not, would keep the FP64 pipe
+            // busier than the conversions do.)
+            const bool add = op == OP_DEALIAS || op == OP_INV;
             double addv = 0.0;
             if (op == OP_INV) addv = (jb.addk ? jb.addk[plane] : 0.0) + jb.addc;
-            // (what is only stored takes loops of its own: FP64 operations,
-            // predicated off or not, would keep the FP64 pipe busier than the
-            // conversions do)
             const bool store = !acc && alpha == 1.0;
-            if (store && op == OP_INV) { out.cx += addv; out.cy += addv; }
-            auto fin = [&](const X2 v, const FxOut &q, const double *old, double *va, double *vb, size_t step) {
-                const bool safe = fx_safe(q.xe);
-                *va = fx_to(v.x, q.xe, safe);
-                *vb = fx_to(v.y, q.xe, safe);
-                if (con) { *va += q.cx; *vb += q.cy; }
-                if (q.nonfin) *va = *vb = FX_NAN;
+            double ca = out.cx, cb = out.cy;
+            if (store && op == OP_INV) { ca += addv; cb += addv; }
+            double *oa = ot + pb + 2 * (size_t)pair * nx, *ob = oa + nx;
+            const bool plain = store && safe && !out.bad;
+            // x lines: the last pass stores its results
+            const bool fused = DIR == 0 && pl.np > 1 && __all_sync(0xffffffffu, plain && valid);
+            for (int p = pl.np - 2; p >= (fused ? 1 : 0); p--) {
+                const FxPassArgs a = args(p);
+#define CALL(R, K) fx_inv<R, K, false>(dst, a, nullptr, nullptr, 0.0, 0.0, 0.0, false)
+                FX_SWITCH(pl, p, CALL)
+#undef CALL
+            }
+            if (fused) {
+                const FxPassArgs a = args(0);
+#define CALL(R, K) fx_inv<R, K, true>(dst, a, oa, ob, out.sc, ca, cb, add)
+                FX_SWITCH(pl, 0, CALL)
+#undef CALL
+                continue;
+            }
+            auto fin = [&](const X2 v, const FxOut &q, double *va, double *vb, const double *old, size_t step) {
+                const bool ok = q.xe >= -700 && q.xe <= 700;
+                *va = ok ? __ll2double_rn(v.x) * q.sc : fx_to_slow(v.x, q.xe) * con;
+                *vb = ok ? __ll2double_rn(v.y) * q.sc : fx_to_slow(v.y, q.xe) * con;
+                if (add) { *va += q.cx; *vb += q.cy; }
+                if (q.bad) *va = *vb = FX_NAN;
                 *va *= alpha;
                 *vb *= alpha;
                 if (acc) { *va = old[0] + *va; *vb = old[step] + *vb; }
                 if (op == OP_INV && !store) { *va += addv; *vb += addv; }
             };
+            const FxOut mine = { ca, cb, out.sc, out.xe, out.bad };
             if (DIR == 0) {
-                double *oa = ot + pb + 2 * (size_t)pair * nx, *ob = oa + nx;
-                if (valid && store && !out.nonfin && fx_safe(out.xe)) {
-                    if (con)
-                        for (int e = l; e < n; e += G) {
-                            const X2 v = dst[fx_at(e, s7)];
-                            oa[e] = fx_to(v.x, out.xe, true) + out.cx;
-                            ob[e] = fx_to(v.y, out.xe, true) + out.cy;
-                        }
-                    else
-                        for (int e = l; e < n; e += G) {
-                            const X2 v = dst[fx_at(e, s7)];
-                            oa[e] = fx_to(v.x, out.xe, true);
-                            ob[e] = fx_to(v.y, out.xe, true);
-                        }
-                } else if (valid) {
+                if (valid)
                     for (int e = l; e < n; e += G) {
                         double va, vb;
-                        fin(dst[fx_at(e, s7)], out, oa + e, &va, &vb, nx);
+                        fin(dst[fx_at(e, s7)], mine, &va, &vb, oa + e, nx);
                         oa[e] = va;
                         ob[e] = vb;
                     }
-                }
                 __syncwarp();
             } else {
-                if (l == 0) so[s] = out;
-                const bool fast = __syncthreads_and(store && !out.nonfin && fx_safe(out.xe));
-                const int ls = 31 - __clz(S), q = tid & (S - 1);     // (S divides the CTA: one sequence per thread)
+                if (l == 0) so[s] = mine;
+                const bool fast = __syncthreads_and(plain);
+                const int ls = 31 - __clz(S), q = tid & (S - 1), de = (int)blockDim.x >> ls;
                 const X2 *bs = (dst == A ? bufA : bufB) + (size_t)q * pl.nb;
                 double *od = ot + pb + 2 * ((size_t)tile * S + q);
                 if (tile * S + q < pairs) {
                     const FxOut f = so[q];
-                    if (fast && con) {
-                        for (int e = tid >> ls; e < n; e += (int)blockDim.x >> ls) {
+                    if (fast && add) {
+                        for (int e = tid >> ls; e < n; e += de) {
                             const X2 v = bs[fx_at(e, q & 7)];
                             *reinterpret_cast<double2 *>(od + (size_t)e * nx) =
-                                make_double2(fx_to(v.x, f.xe, true) + f.cx, fx_to(v.y, f.xe, true) + f.cy);
+                                make_double2(fma(__ll2double_rn(v.x), f.sc, f.cx), fma(__ll2double_rn(v.y), f.sc, f.cy));
                         }
                     } else if (fast) {
-                        for (int e = tid >> ls; e < n; e += (int)blockDim.x >> ls) {
+                        for (int e = tid >> ls; e < n; e += de) {
                             const X2 v = bs[fx_at(e, q & 7)];
-                            *reinterpret_cast<double2 *>(od + (size_t)e * nx) = make_double2(fx_to(v.x, f.xe, true), fx_to(v.y, f.xe, true));
+                            *reinterpret_cast<double2 *>(od + (size_t)e * nx) =
+                                make_double2(__ll2double_rn(v.x) * f.sc, __ll2double_rn(v.y) * f.sc);
                         }
                     } else {
-                        for (int e = tid >> ls; e < n; e += (int)blockDim.x >> ls) {
+                        for (int e = tid >> ls; e < n; e += de) {
                             double *dd = od + (size_t)e * nx;
                             double2 v;
-                            fin(bs[fx_at(e, q & 7)], f, dd, &v.x, &v.y, 1);
+                            fin(bs[fx_at(e, q & 7)], f, &v.x, &v.y, dd, 1);
                             *reinterpret_cast<double2 *>(dd) = v;
                         }
                     }
@@ -454,19 +689,27 @@ static FxConst fx_const(long double v)
     c.h = (int)((q - (int)q) >> 32);
     return c;
 }
-// exp(-2 pi i e/n) in long double, exact at the quadrants
-static TwX tw_unit(long e, long n)
-{
-    e %= n;
-    const long q = (4 * e) / n, r = 4 * e - q * n;     // quadrant, and the angle (pi/2) r/n in it
-    const long double h = 1.57079632679489661923132169163975144L;
-    long double c, s;
-    if (2 * r <= n) { c = cosl(h * (long double)r / n); s = sinl(h * (long double)r / n); }
-    else { c = sinl(h * (long double)(n - r) / n); s = cosl(h * (long double)(n - r) / n); }
-    const long double cc[4] = { c, -s, -c, s }, ss[4] = { s, c, -s, -c };
-    const FxConst x = fx_const(cc[q]), y = fx_const(-ss[q]);
-    return TwX{ x.h, x.l, y.h, y.l };
-}
+// exp(-2 pi i e/n), computed in long double, exact at the quadrants; the angles
+// of an octant are computed once
+struct UnitCircle {
+    long n;
+    std::vector<FxConst> c, s;      // cos, sin of (pi/2) r/n, r = 0 .. n/2; c.h = 0: not yet
+    explicit UnitCircle(int n_) : n(n_), c(n_ / 2 + 1, FxConst{ 0, 0 }), s(n_ / 2 + 1) {}
+    TwX operator()(long e)
+    {
+        e %= n;
+        const long q = (4 * e) / n, r = 4 * e - q * n, a = 2 * r <= n ? r : n - r;
+        if (!c[a].h) {
+            const long double t = 1.57079632679489661923132169163975144L * (long double)a / n;
+            c[a] = fx_const(cosl(t));
+            s[a] = fx_const(sinl(t));
+        }
+        const FxConst cr = a == r ? c[a] : s[a], sr = a == r ? s[a] : c[a];
+        const FxConst cn = { -cr.h, -cr.l }, sn = { -sr.h, -sr.l };
+        const FxConst re[4] = { cr, sn, cn, sr }, im[4] = { sn, cn, sr, cr };     // exp(-i t): (c, -s) turned by -q
+        return TwX{ re[q].h, re[q].l, im[q].h, im[q].l };
+    }
+};
 
 int line_fx_configure()
 {
@@ -481,24 +724,25 @@ int line_fx_configure()
     return VEC_OK;
 }
 
-// the radices of n with the fewest passes, larger ones first
+// the radices of n with the fewest passes; 8 where it divides, and last: the
+// strides of the other passes are then multiples of 8 or 64
 static bool radices(int n, std::vector<int> &r)
 {
-    static const int all[] = { 8, 6, 5, 4, 3, 2 };
+    static const int all[] = { 2, 3, 4, 5, 6, 8 };
     std::vector<int> best;
     std::vector<int> cur;
     auto go = [&](auto &self, int m, int from) -> void {
         if (!best.empty() && cur.size() >= best.size()) return;
         if (m == 1) { best = cur; return; }
-        for (int q = from; q < 6; q++)
+        for (int q = from; q >= 0; q--)
             if (m % all[q] == 0) {
                 cur.push_back(all[q]);
                 self(self, m / all[q], q);
                 cur.pop_back();
             }
     };
-    go(go, n, 0);
-    r = best;
+    go(go, n, 5);
+    r.assign(best.rbegin(), best.rend());
     return !r.empty();
 }
 
@@ -511,13 +755,18 @@ int fx_plan_make(int n, FxPlan *pl)
     pl->nb = (n + 7) & ~7;
     pl->np = (int)r.size();
     pl->rn = 1.0f / (float)n;
-    pl->pow2 = (n & (n - 1)) == 0;
+    // (what the squares' unit leaves out, half of it at every wavenumber: with
+    // (x + y)^2 <= 1.25 x^2 + 5 y^2, and the mean of k^2 and k^4)
+    const double kmax = n / 2;
+    pl->floor1 = (float)(n * kmax * kmax);
+    pl->floor2 = (float)(n * kmax * kmax * kmax * kmax);
     int L = n;
     double P = 1.0, top = 0.0;     // growth sqrt(P) 2^-halvings
     for (int p = 0; p < pl->np; p++) {
         const int R = r[p], M = L / R;
         pl->R[p] = R; pl->L[p] = L; pl->M[p] = M;
         pl->mg[p] = (unsigned)(((1ull << 31) + M - 1) / M);
+        pl->kind[p] = M % 64 == 0 ? K64 : R == 8 && M == 8 ? K8 : R == 8 && M == 1 ? K1 : KG;
         pl->tw[p] = pl->ntw;
         if (M > 1) pl->ntw += (R - 1) * M;
         // sums inside the radix: 2 x 4 and 3 x 2 with a halving between
@@ -551,71 +800,52 @@ int fx_plan_make(int n, FxPlan *pl)
 }
 
 // the tables of one direction: the twiddles of each pass, the order of the
-// spectrum, and the multipliers of line_tables_make in that order, scaled by a
-// power of two per table to at most one in magnitude
-int fx_tables_make(int n, const FxPlan &pl, const double *k1, const double *k2, int icut, FxTables *tb)
+// spectrum, and the operators' constants (k1, k2: the multipliers' tables)
+int fx_tables_make(int n, FxPlan *pl, const double *k1, const double *k2, int icut, FxTables *tb)
 {
+    pl->cut = n / 2 - icut;
+    tb->c0 = 1.0 / n;
+    tb->c1 = k1[1] / n;
+    tb->c2 = k2[1] / n;
+    UnitCircle unit(n);
     std::vector<TwX> tw;
-    for (int p = 0; p < pl.np; p++)
-        if (pl.M[p] > 1)
-            for (int r = 1; r < pl.R[p]; r++)
-                for (int j = 0; j < pl.M[p]; j++) tw.push_back(tw_unit((long)j * r, pl.L[p]));
-    std::vector<unsigned short> pos(n), kof(n);
+    for (int p = 0; p < pl->np; p++)
+        if (pl->M[p] > 1)
+            for (int r = 1; r < pl->R[p]; r++)
+                for (int j = 0; j < pl->M[p]; j++) tw.push_back(unit((long)j * r * (n / pl->L[p])));
+    std::vector<unsigned short> pos(2 * n);       // and kof
     for (int k = 0; k < n; k++) {
         int rest = k, at = 0;
-        for (int p = 0; p < pl.np; p++) {
-            at += (rest % pl.R[p]) * pl.M[p];
-            rest /= pl.R[p];
+        for (int p = 0; p < pl->np; p++) {
+            at += (rest % pl->R[p]) * pl->M[p];
+            rest /= pl->R[p];
         }
         pos[k] = (unsigned short)at;
-        kof[at] = (unsigned short)k;
+        pos[n + at] = (unsigned short)k;
     }
-    std::vector<long double> m[4];
-    for (auto &v : m) v.assign(n, 0.0L);
-    for (int e = 0; e < n; e++) {
-        if (e > 0 && 2 * e < n) m[0][e] = (long double)k1[e] / n;
-        else if (2 * e > n) m[0][e] = -(long double)k1[e] / n;
-        if (e) m[1][e] = (long double)k2[e] / n;
-        const int kk = e <= n / 2 ? e : n - e;
-        m[2][e] = kk >= n / 2 - icut ? 0.0L : 1.0L / n;
-        m[3][e] = 1.0L / n;
+    const size_t bt = tw.size() * sizeof(TwX), bp = pos.size() * sizeof(short);
+    std::vector<char> all(bt + bp);
+    if (bt) memcpy(all.data(), tw.data(), bt);
+    memcpy(all.data() + bt, pos.data(), bp);
+    if (cudaMalloc(&tb->tw, all.size()) != cudaSuccess) {
+        cudaGetLastError();
+        return VEC_ERR_ALLOC;
     }
-    int2 **dst[4] = { &tb->m1, &tb->m2, &tb->mda, &tb->minv };
-    int *px[4] = { &tb->p1, &tb->p2, &tb->pda, &tb->pinv };
-    auto up = [](void **d, const void *s, size_t bytes) {
-        if (cudaMalloc(d, bytes ? bytes : 16) != cudaSuccess) { cudaGetLastError(); return (int)VEC_ERR_ALLOC; }
-        return cudaMemcpy(*d, s, bytes, cudaMemcpyHostToDevice) == cudaSuccess ? (int)VEC_OK : (int)VEC_ERR_CUDA;
-    };
-    int st;
-    if ((st = up((void **)&tb->tw, tw.data(), tw.size() * sizeof(TwX))) ||
-        (st = up((void **)&tb->pos, pos.data(), n * sizeof(short))) || (st = up((void **)&tb->kof, kof.data(), n * sizeof(short))))
-        return st;
-    for (int t = 0; t < 4; t++) {
-        long double mx = 0.0L;
-        for (auto v : m[t]) mx = fmaxl(mx, fabsl(v));
-        int p = 0;
-        if (mx > 0.0L && frexpl(mx, &p) == 0.5L) p--;     // mx = f 2^p, f in (1/2, 1]
-        *px[t] = p;
-        std::vector<int2> q(n);
-        for (int i = 0; i < n; i++) {
-            const FxConst c = fx_const(ldexpl(m[t][kof[i]], -p));
-            q[i] = make_int2(c.h, c.l);
-        }
-        if ((st = up((void **)dst[t], q.data(), n * sizeof(int2)))) return st;
-    }
+    tb->pos = reinterpret_cast<unsigned short *>(reinterpret_cast<char *>(tb->tw) + bt);
+    tb->kof = tb->pos + n;
+    CUDA_TRY(cudaMemcpy(tb->tw, all.data(), all.size(), cudaMemcpyHostToDevice));
     return VEC_OK;
 }
 void fx_tables_free(FxTables *tb)
 {
-    cudaFree(tb->tw); cudaFree(tb->m1); cudaFree(tb->m2); cudaFree(tb->mda); cudaFree(tb->minv);
-    cudaFree(tb->pos); cudaFree(tb->kof);
+    cudaFree(tb->tw);
     *tb = FxTables{};
 }
 
 template <int DIR>
 static int run_fx(Engine *E, const LineJob<double> *jobs, int nj)
 {
-    const FxPlan &pl = DIR == 0 ? E->fpx : E->fpy;
+    FxPlan pl = DIR == 0 ? E->fpx : E->fpy;
     FxPack pk;
     memset(&pk, 0, sizeof(pk));
     double fields = 0.0;
@@ -630,6 +860,16 @@ static int run_fx(Engine *E, const LineJob<double> *jobs, int nj)
     // warps per CTA: 8, fewer where the buffers do not fit half an SM or where
     // there would be less than a CTA per SM
     int W = FX_TPB / 32;
+    // fewer sequences per warp where the device would not be full (8 warps per
+    // SM): the time is then that of one warp's tile, which more lanes per
+    // sequence shorten if its passes take fewer rounds (30 x 30 x 60: 36 -> 26 us;
+    // 64 points take as many with 8 lanes as with 32, and lose: 23 -> 28 us)
+    auto rounds = [&](int q) {
+        int r = 0;
+        for (int p = 0; p < pl.np; p++) r += (pl.n / pl.R[p] * q + 31) / 32;
+        return r;
+    };
+    while (pl.Q > 1 && (long long)nj * E->nz * pairs < (long long)E->num_sms * 8 * pl.Q && rounds(pl.Q / 2) < rounds(pl.Q)) pl.Q >>= 1;
     auto smem_of = [&](int w) {
         const size_t S = (size_t)w * pl.Q;
         return sizeof(TwX) * pl.ntw + S * pl.nb * sizeof(X2) * (two ? 2 : 1) + S * sizeof(FxOut) + 16;
