@@ -410,7 +410,7 @@ extern "C" int vec_create(const vec_params *p, vec_ctx **out)
     E.red_blocks = 152 * 4;
     ALLOC(E.red, sizeof(double) * ((size_t)nz * 8 + 8 + (size_t)E.red_blocks * 25 + 64));
     ALLOC(E.ds, sizeof(DevScalars));
-    ALLOC(E.cdt, sizeof(float) * (4 + 3 * (size_t)cdt_chunks(E.n)));
+    ALLOC(E.cdt, sizeof(float) * (4 + 3 * (size_t)cdt_chunks(E.np, E.nz)));
     if ((st = cdt_init(E.cdt))) { vec_destroy(c); return st; }
     if (cudaHostAlloc((void **)&E.dev_err, sizeof(int) * 4, cudaHostAllocMapped | cudaHostAllocPortable) != cudaSuccess) {
         cudaGetLastError();
@@ -969,14 +969,19 @@ static int enqueue_step(Engine &E, bool diag_now)
     if ((st = E.split ? split_ab3(&E, mdeal, fold) : phys_ab3(&E, mdeal))) return st;
     const bool dealias_now = E.p.dalias && (E.nit % 10 == 0);
     if (dealias_now && (st = E.split ? split_dealias(&E) : phys_dealias_state(&E))) return st;
-    if (mag && (st = E.split ? split_bandj(&E, fold) : phys_bandj64(&E))) return st;
+    // (the boundary conditions ride on bandj's last kernel where its form takes them)
+    const bool bounds = E.split && mag && split_bandj_bounds(E);
+    if (mag && (st = E.split ? split_bandj(&E, fold, bounds) : phys_bandj64(&E))) return st;
     if (mag) {
-        if ((st = phys_boundaries(&E))) return st;   // boundary and mag_boundary (disjoint fields)
+        if (!bounds && (st = phys_boundaries(&E))) return st;   // boundary and mag_boundary (disjoint fields)
     } else if ((st = boundary_step(E))) {
         return st;
     }
     if (diag_now && (st = diag_step(E, nullptr))) return st;
-    if (E.nit % 10 == 0 && (st = E.split ? split_calcdt(&E) : phys_calcdt(&E))) return st;
+    if (E.nit % 10 == 0) {
+        Engine *e = &E;
+        if ((st = E.split ? split_calcdt_m(&e, 1) : phys_calcdt(&E))) return st;
+    }
     return VEC_OK;
 }
 
@@ -1043,8 +1048,7 @@ static int enqueue_step_batch_body(Engine *const *Es, int nE)
     if ((st = split_ab3_m(Es, nE, mdeal, folded))) return st;
     const int nit = Es[0]->nit;
     if (Es[0]->p.dalias && nit % 10 == 0 && (st = split_dealias_m(Es, nE))) return st;
-    if (nm && (st = split_bandj_m(mag, nm, true))) return st;
-    if (nm && (st = phys_boundaries_m(mag, nm))) return st;
+    if (nm && (st = split_bandj_m(mag, nm, true, true))) return st;
     if (no && (st = phys_boundary_m(off, no))) return st;
     if (nit % 10 == 0 && (st = split_calcdt_m(Es, nE))) return st;
     return VEC_OK;

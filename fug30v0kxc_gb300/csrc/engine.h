@@ -213,7 +213,7 @@ template <typename R> int launch_lines(Engine *E, int dir, const LineJob<R> *job
 template <> int launch_lines<double>(Engine *E, int dir, const LineJob<double> *jobs, int njobs);   // lines_fx.cu
 int line_kernels_configure();
 // physics.cu: calcdt scratch (floats per context, initialisation of its keys)
-int cdt_chunks(size_t n);
+int cdt_chunks(size_t np, int nz);
 int cdt_init(float *cdt);
 int line_ct_configure();
 int line_fx_configure();
@@ -265,7 +265,8 @@ int closure_apply_corr(Engine *E);
 // split form (split.cu)
 int split_setup(Engine *E);
 int split_refresh_coefs(Engine *E);   // after kappa / eta change
-const double *split_bg_t0(const Engine *E);   // T0(z), FP64
+const double *split_bg_t0(const Engine *E);     // T0(z), FP64
+const double *split_bg_rho0(const Engine *E);   // rho0(z)
 // FP32 mirrors written by the boundary kernels in the split form (null: FP64 form)
 struct BoundaryMirrors {
     float *u32, *v32, *w32, *t32, *pol32, *tor32;
@@ -279,7 +280,8 @@ int split_hydro(Engine *E, bool with_mag = false);
 // first kernel of split_bandj (rotate_hist); split_ab3 then runs the update
 // alone (folded).
 int split_mag(Engine *E, bool ab3_coef = false, bool spectra_done = false);
-int split_bandj(Engine *E, bool rotate_hist = false);
+bool split_bandj_bounds(const Engine &E);
+int split_bandj(Engine *E, bool rotate_hist = false, bool bounds = false);
 int split_refresh(Engine *E);
 int split_refresh_field(Engine *E, int field);   // one field's mirror (VEC_F_*)
 int split_refresh_planes(Engine *E, int mask);
@@ -297,11 +299,12 @@ int phys_boundary_m(Engine *const *Es, int nE);
 int phys_boundaries_m(Engine *const *Es, int nE);
 int phys_rotate_hist_m(Engine *const *Es, int nE);
 int phys_ab3_coef_m(Engine *const *Es, int nE);
-int phys_calcdt_m(Engine *const *Es, int nE);
+int phys_calcdt_m(Engine *const *Es, int nE, bool mirrors);
+bool cdt_mirrors_ok(const Engine &E);
 int split_hydro_m(Engine *const *Es, int nE, const bool *with_mag);
 int split_emf_m(Engine *const *Es, int nE);
 int split_mag_m(Engine *const *Es, int nE, bool ab3_coef, bool spectra_done);
-int split_bandj_m(Engine *const *Es, int nE, bool rotate_hist);
+int split_bandj_m(Engine *const *Es, int nE, bool rotate_hist, bool bounds);
 int split_ab3_m(Engine *const *Es, int nE, const int *magdealias, const bool *folded);
 int split_dealias_m(Engine *const *Es, int nE);
 int split_sync_b64_m(Engine *const *Es, int nE);

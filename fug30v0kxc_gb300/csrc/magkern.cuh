@@ -419,11 +419,8 @@ struct Jsq4Args {
     int nz;
     float h;
 };
-template <int NB>
-static __global__ void k_jsq4(const __grid_constant__ Batch<Jsq4Args, NB> bt)
+__device__ __forceinline__ void jsq4_row(const Jsq4Args &A, int k)
 {
-    PDL_WAIT();
-    const Jsq4Args &A = BATCH_MEMBER(bt, NB);
     const float *jz = A.jz, *dybz = A.dybz, *dxbz = A.dxbz, *bx = A.bx, *by = A.by;
     float *jsq = A.jsq;
     const size_t np = A.np;
@@ -432,12 +429,17 @@ static __global__ void k_jsq4(const __grid_constant__ Batch<Jsq4Args, NB> bt)
     const size_t np4 = np / 4;
     const size_t q4 = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (q4 >= np4) return;
-    const int k = blockIdx.y;
     const size_t i4 = (size_t)k * np4 + q4;
     const V4 wk1 = zd1(reinterpret_cast<const V4 *>(by) + q4, np4, k, nz, 5, V4(h));
     const V4 wk2 = zd1(reinterpret_cast<const V4 *>(bx) + q4, np4, k, nz, 5, V4(h));
     const V4 ez = ld4(jz, i4), ex = ld4(dybz, i4), ey = ld4(dxbz, i4);
     st4(jsq, i4, ez * ez + ((ex - wk1) * (ex - wk1)) + ((wk2 - ey) * (wk2 - ey)));
+}
+template <int NB>
+static __global__ void k_jsq4(const __grid_constant__ Batch<Jsq4Args, NB> bt)
+{
+    PDL_WAIT();
+    jsq4_row(BATCH_MEMBER(bt, NB), blockIdx.y);
 }
 
 // spectral truncation of the 2/3 rule, src/magnetic.f90:666-717

@@ -22,6 +22,7 @@
 #include "common.cuh"
 #include "engine.h"
 #include "fpconv.cuh"
+#include "boundary.cuh"
 #include "zstencil.cuh"
 #include "magkern.cuh"
 
@@ -394,73 +395,6 @@ int phys_magdealias(Engine *E)
 // ============================================================================
 // boundary conditions: src/dbydz.F90:3686-4197 and :4205-4791
 // ============================================================================
-// In the split form (m != nullptr) the FP32 mirrors of the two boundary
-// planes are written here too: m = {u32, v32, w32, t32}, t0 = T0(z).
-__device__ __forceinline__ void boundary_column(double *u, double *v, double *w, double *t, size_t np, int nz,
-                                                double theta, double dz, int radbc, int constflux,
-                                                const BoundaryMirrors &mb, size_t q)
-{
-    const double elf = 1.0 / 11.0;
-#define P(f, kk) f[(size_t)(kk) * np + q]
-    P(w, 0) = 0.0;
-    P(u, 0) = elf * (18.0 * P(u, 1) - 9.0 * P(u, 2) + 2.0 * P(u, 3));
-    P(v, 0) = elf * (18.0 * P(v, 1) - 9.0 * P(v, 2) + 2.0 * P(v, 3));
-    P(w, nz - 1) = 0.0;
-    P(u, nz - 1) = elf * (18.0 * P(u, nz - 2) - 9.0 * P(u, nz - 3) + 2.0 * P(u, nz - 4));
-    P(v, nz - 1) = elf * (18.0 * P(v, nz - 2) - 9.0 * P(v, nz - 3) + 2.0 * P(v, nz - 4));
-    if (radbc) {   // :4036-4055, Newton iterations on the radiative condition
-        double t1old = P(t, 0);
-        for (int it = 0; it < 10; it++) {
-            double ft1 = 6.0 * theta * dz * t1old * t1old * t1old * t1old + 11.0 * t1old - 18.0 * P(t, 1)
-                         + 9.0 * P(t, 2) - 2.0 * P(t, 3);
-            double dft1 = 24.0 * theta * dz * t1old * t1old * t1old + 11.0;
-            t1old = t1old - (ft1 / dft1);
-        }
-        P(t, 0) = t1old;
-    } else {
-        P(t, 0) = 1.0;
-    }
-    if (constflux)
-        P(t, nz - 1) = elf * (18.0 * P(t, nz - 2) - 9.0 * P(t, nz - 3) + 2.0 * P(t, nz - 4) + 6.0 * theta * dz);
-    else
-        P(t, nz - 1) = 1.0 + theta;
-    if (mb.u32) {
-        const int ks[2] = { 0, nz - 1 };
-        for (int e = 0; e < 2; e++) {
-            const int kk = ks[e];
-            mb.u32[(size_t)kk * np + q] = d2f_rn(P(u, kk));
-            mb.v32[(size_t)kk * np + q] = d2f_rn(P(v, kk));
-            mb.w32[(size_t)kk * np + q] = d2f_rn(P(w, kk));
-            mb.t32[(size_t)kk * np + q] = d2f_rn(P(t, kk) - mb.t0[kk]);
-        }
-    }
-#undef P
-}
-
-// arguments of k_boundary / k_boundaries
-struct BndArgs {
-    double *u, *v, *w, *t, *pol, *tor, *bxb, *byb;
-    size_t np;
-    int nz;
-    double theta, dz;
-    int radbc, constflux, perfect;
-    BoundaryMirrors mb;
-};
-
-static BndArgs bnd_args(Engine *E)
-{
-    BndArgs a;
-    BoundaryMirrors mb = {};
-    if (E->split) {
-        mb.u32 = E->u32; mb.v32 = E->v32; mb.w32 = E->w32; mb.t32 = E->t32; mb.t0 = split_bg_t0(E);
-        mb.pol32 = E->pol32; mb.tor32 = E->tor32;
-    }
-    a.u = E->u; a.v = E->v; a.w = E->w; a.t = E->t; a.pol = E->pol; a.tor = E->tor; a.bxb = E->bxbar; a.byb = E->bybar;
-    a.np = E->np; a.nz = E->nz; a.theta = E->p.theta; a.dz = E->k.dz;
-    a.radbc = E->p.radbc; a.constflux = E->p.constflux; a.perfect = E->p.perfect; a.mb = mb;
-    return a;
-}
-
 template <int NB>
 __global__ void k_boundary(const __grid_constant__ Batch<BndArgs, NB> bt)
 {
@@ -476,42 +410,6 @@ int phys_boundary_m(Engine *const *Es, int nE)
                                    k_boundary<BATCH_MAX>, bnd_args);
 }
 int phys_boundary(Engine *E) { return phys_boundary_m(&E, 1); }
-
-__device__ __forceinline__ void mag_boundary_column(double *pol, double *tor, double *bxb, double *byb, size_t np,
-                                                    int nz, int perfect, const BoundaryMirrors &mb, size_t q)
-{
-    const double elf = 1.0 / 11.0;
-    if (q == 0) {
-        if (perfect) {
-            bxb[0] = elf * (18.0 * bxb[1] - 9.0 * bxb[2] + 2.0 * bxb[3]);
-            byb[0] = elf * (18.0 * byb[1] - 9.0 * byb[2] + 2.0 * byb[3]);
-            bxb[nz - 1] = elf * (18.0 * bxb[nz - 2] - 9.0 * bxb[nz - 3] + 2.0 * bxb[nz - 4]);
-            byb[nz - 1] = elf * (18.0 * byb[nz - 2] - 9.0 * byb[nz - 3] + 2.0 * byb[nz - 4]);
-        } else {
-            bxb[0] = 0.0; byb[0] = 0.0; bxb[nz - 1] = 0.0; byb[nz - 1] = 0.0;
-        }
-    }
-    if (q >= np) return;
-#define P(f, kk) f[(size_t)(kk) * np + q]
-    if (perfect) {   // :4407-4560
-        P(pol, 0) = 0.0;
-        P(tor, 0) = elf * (18.0 * P(tor, 1) - 9.0 * P(tor, 2) + 2.0 * P(tor, 3));
-        P(pol, nz - 1) = 0.0;
-        P(tor, nz - 1) = elf * (18.0 * P(tor, nz - 2) - 9.0 * P(tor, nz - 3) + 2.0 * P(tor, nz - 4));
-    } else {         // :4663-4780
-        P(tor, 0) = 0.0;
-        P(pol, 0) = elf * (18.0 * P(pol, 1) - 9.0 * P(pol, 2) + 2.0 * P(pol, 3));
-        P(tor, nz - 1) = 0.0;
-        P(pol, nz - 1) = elf * (18.0 * P(pol, nz - 2) - 9.0 * P(pol, nz - 3) + 2.0 * P(pol, nz - 4));
-    }
-    if (mb.pol32) {
-        mb.pol32[q] = d2f_rn(P(pol, 0));
-        mb.tor32[q] = d2f_rn(P(tor, 0));
-        mb.pol32[(size_t)(nz - 1) * np + q] = d2f_rn(P(pol, nz - 1));
-        mb.tor32[(size_t)(nz - 1) * np + q] = d2f_rn(P(tor, nz - 1));
-    }
-#undef P
-}
 
 __global__ void k_mag_boundary(double *pol, double *tor, double *bxb, double *byb, size_t np, int nz, int perfect,
                                BoundaryMirrors mb)
@@ -681,7 +579,7 @@ __device__ __forceinline__ double okey_dec(unsigned long long e)
 // The maxima of src/utils.F90:190-214 need the FP64 expression only at the
 // points that can hold them, and GB300's FP64 square roots are slow.  So:
 //
-// pass 1 (k_calcdt_est): per chunk of CDT_CHUNK points, FP32 estimates of
+// pass 1 (k_calcdt_est): per chunk of a plane's points, FP32 estimates of
 //   xx = |u_h| + g1 sqrt(T) + sqrt(f B^2 / rho) and xz (|w| in place of |u_h|)
 //   and the minimum density, their chunk extrema, and the global extrema;
 // pass 2 (k_calcdt_exact): the few chunks whose estimate lies within
@@ -692,8 +590,19 @@ __device__ __forceinline__ double okey_dec(unsigned long long e)
 // non-negative), far below CDT_MARGIN, so the point holding the exact
 // maximum (minimum) always passes both filters.  Estimates only choose
 // points; the results are the same FP64 extrema as a full FP64 pass.
-#define CDT_CHUNK 8192
+//
+// In the split form's time step the estimates are formed from the FP32
+// mirrors (half the bytes), and the exact values take B from them too, which
+// saves bringing the FP64 copy of B up to date: 386 -> 135 us per call at
+// 256^2 x 129.  A mirror's rounding is 2^-24 of its background at most:
+// CDT_BG bounds the backgrounds for which that stays below the margin at the
+// density floor of 0.05 (the margin for the density has CDT_ABS added).
 #define CDT_MARGIN 1.0e-3f
+#define CDT_BG 64.0
+#define CDT_ABS 2.0e-5f
+// points per chunk: small grids need small chunks to fill the device (one chunk
+// is one CTA; 8192 points took 77 us for the exact pass of 64^2 x 65)
+static int cdt_chunk(size_t np) { return np <= 16384 ? 1024 : np <= 131072 ? 2048 : 4096; }
 
 // order-preserving keys of floats (as okey for doubles)
 __device__ __forceinline__ unsigned okey32(float x)
@@ -726,21 +635,32 @@ int cdt_init(float *cdt)
 
 struct CdtArgs {
     const double *u, *v, *w, *r, *t, *bx, *by, *bz;
-    size_t n;
+    const float *u32, *v32, *w32, *r32, *t32, *bx32, *by32, *bz32;   // mirrors, or null
+    const double *r0, *t0;  // the mirrors' backgrounds
+    double bzbar;
+    size_t np;
     double g1, f;
     float *chunk;           // [3][nchunks]: xx max, xz max, rho min estimates
     unsigned *gkey;         // [3]: keys of the global estimates
-    int nchunks;
+    int nchunks, cs;        // chunks in all; points per chunk
     DevScalars *ds;
 };
 
 struct CdtEst { float xx, xz, r; };
 
-__device__ __forceinline__ CdtEst cdt_estimate(const CdtArgs &a, size_t i)
+// (rb, tb, bb: the mirrors' backgrounds and mean field)
+template <bool MIR>
+__device__ __forceinline__ CdtEst cdt_estimate(const CdtArgs &a, size_t i, float rb, float tb, float bb)
 {
-    // (conversions by truncation on the integer pipe: relative error < 2^-23)
-    const float u0 = d2f_est(a.u[i]), v0 = d2f_est(a.v[i]), w0 = d2f_est(a.w[i]), r0 = d2f_est(a.r[i]);
-    const float t0 = d2f_est(a.t[i]), bx0 = d2f_est(a.bx[i]), by0 = d2f_est(a.by[i]), bz0 = d2f_est(a.bz[i]);
+    float u0, v0, w0, r0, t0, bx0, by0, bz0;
+    if (MIR) {
+        u0 = a.u32[i]; v0 = a.v32[i]; w0 = a.w32[i]; r0 = rb + a.r32[i];
+        t0 = tb + a.t32[i]; bx0 = a.bx32[i]; by0 = a.by32[i]; bz0 = bb + a.bz32[i];
+    } else {
+        // (conversions by truncation on the integer pipe: relative error < 2^-23)
+        u0 = d2f_est(a.u[i]); v0 = d2f_est(a.v[i]); w0 = d2f_est(a.w[i]); r0 = d2f_est(a.r[i]);
+        t0 = d2f_est(a.t[i]); bx0 = d2f_est(a.bx[i]); by0 = d2f_est(a.by[i]); bz0 = d2f_est(a.bz[i]);
+    }
     const float bsq = bx0 * bx0 + by0 * by0 + bz0 * bz0;
     const float c = (float)a.g1 * sqrtf(t0) + sqrtf((bsq * (float)a.f) / r0);
     CdtEst e;
@@ -765,23 +685,26 @@ __device__ __forceinline__ void block_reduce3(float &mx, float &mz, float &mn, f
     }
 }
 
-template <int NB>
+// (grid: chunks of a plane, planes; a chunk lies in one plane)
+template <int NB, bool MIR>
 __global__ void __launch_bounds__(256) k_calcdt_est(const __grid_constant__ Batch<CdtArgs, NB> bt)
 {
     PDL_WAIT();
     const CdtArgs &a = BATCH_MEMBER(bt, NB);
-    if ((int)blockIdx.x >= a.nchunks) return;
     __shared__ float sh[96];
-    const size_t i0 = (size_t)blockIdx.x * CDT_CHUNK;
-    const size_t i1 = i0 + CDT_CHUNK < a.n ? i0 + CDT_CHUNK : a.n;
+    const int k = blockIdx.y, c = k * gridDim.x + blockIdx.x;
+    const size_t p0 = (size_t)k * a.np, i0 = p0 + (size_t)blockIdx.x * a.cs;
+    const size_t i1 = i0 + a.cs < p0 + a.np ? i0 + a.cs : p0 + a.np;
+    const float rb = MIR ? (float)a.r0[k] : 0.0f, tb = MIR ? (float)a.t0[k] : 0.0f, bb = (float)a.bzbar;
     float mx = -INFINITY, mz = -INFINITY, mn = INFINITY;
     // A NaN or infinity in u, v, w, T, B makes the speed estimates non-finite,
     // and one in rho its own estimate (a negative T or rho gives a NaN square
     // root, as in the FP64 expression); fmaxf / fminf would skip NaNs, so they
     // are counted separately.
     int bad = 0;
+#pragma unroll 4
     for (size_t i = i0 + threadIdx.x; i < i1; i += blockDim.x) {
-        const CdtEst e = cdt_estimate(a, i);
+        const CdtEst e = cdt_estimate<MIR>(a, i, rb, tb, bb);
         mx = fmaxf(mx, e.xx);
         mz = fmaxf(mz, e.xz);
         mn = fminf(mn, e.r);
@@ -791,40 +714,42 @@ __global__ void __launch_bounds__(256) k_calcdt_est(const __grid_constant__ Batc
     block_reduce3(mx, mz, mn, sh);
     if (threadIdx.x == 0) {
         if (bad) atomicOr(&a.gkey[3], 1u);
-        a.chunk[blockIdx.x] = mx;
-        a.chunk[a.nchunks + blockIdx.x] = mz;
-        a.chunk[2 * a.nchunks + blockIdx.x] = mn;
+        a.chunk[c] = mx;
+        a.chunk[a.nchunks + c] = mz;
+        a.chunk[2 * a.nchunks + c] = mn;
         atomicMax(&a.gkey[0], okey32(mx));
         atomicMax(&a.gkey[1], okey32(mz));
         atomicMin(&a.gkey[2], okey32(mn));
     }
 }
 
-template <int NB>
+template <int NB, bool MIR>
 __global__ void __launch_bounds__(256) k_calcdt_exact(const __grid_constant__ Batch<CdtArgs, NB> bt)
 {
     PDL_WAIT();
     const CdtArgs &a = BATCH_MEMBER(bt, NB);
-    if ((int)blockIdx.x >= a.nchunks) return;
     const float gx = okey32_dec(a.gkey[0]), gz = okey32_dec(a.gkey[1]), gr = okey32_dec(a.gkey[2]);
     // thresholds a relative margin below (above) the estimates; scaling
     // keeps infinite estimates infinite
     const float tx = gx * (gx >= 0.0f ? 1.0f - CDT_MARGIN : 1.0f + CDT_MARGIN);
     const float tz = gz * (gz >= 0.0f ? 1.0f - CDT_MARGIN : 1.0f + CDT_MARGIN);
-    const float tr = gr * (gr >= 0.0f ? 1.0f + CDT_MARGIN : 1.0f - CDT_MARGIN);
-    const int c = blockIdx.x;
+    const float tr = gr * (gr >= 0.0f ? 1.0f + CDT_MARGIN : 1.0f - CDT_MARGIN) + (MIR ? CDT_ABS : 0.0f);
+    const int k = blockIdx.y, c = k * gridDim.x + blockIdx.x;
     const bool fx = a.chunk[c] >= tx, fz = a.chunk[a.nchunks + c] >= tz, fr = a.chunk[2 * a.nchunks + c] <= tr;
     if (!(fx || fz || fr)) return;
-    const size_t i0 = (size_t)c * CDT_CHUNK;
-    const size_t i1 = i0 + CDT_CHUNK < a.n ? i0 + CDT_CHUNK : a.n;
+    const size_t p0 = (size_t)k * a.np, i0 = p0 + (size_t)blockIdx.x * a.cs;
+    const size_t i1 = i0 + a.cs < p0 + a.np ? i0 + a.cs : p0 + a.np;
+    const float rb = MIR ? (float)a.r0[k] : 0.0f, tb = MIR ? (float)a.t0[k] : 0.0f, bb = (float)a.bzbar;
     double mxx = -1.0e-50, mxz = -1.0e-50, mn = 1.0e300;
     for (size_t i = i0 + threadIdx.x; i < i1; i += blockDim.x) {
-        const CdtEst e = cdt_estimate(a, i);
+        const CdtEst e = cdt_estimate<MIR>(a, i, rb, tb, bb);
         const bool px = fx && e.xx >= tx, pz = fz && e.xz >= tz;
         if (px || pz) {
             // src/utils.F90:190-205, in FP64
             const double u0 = a.u[i], v0 = a.v[i], w0 = a.w[i], r0 = a.r[i], t0 = a.t[i];
-            const double bz0 = a.bz[i], bx0 = a.bx[i], by0 = a.by[i];
+            // (the mirrors of B are the newer ones, bz32 without bzbar)
+            const double bz0 = MIR ? a.bzbar + (double)a.bz32[i] : a.bz[i];
+            const double bx0 = MIR ? (double)a.bx32[i] : a.bx[i], by0 = MIR ? (double)a.by32[i] : a.by[i];
             const double bsq0 = bx0 * bx0 + by0 * by0 + bz0 * bz0;
             const double cc = a.g1 * sqrt(t0);
             const double cb = sqrt((bsq0 * a.f) / r0);
@@ -882,30 +807,42 @@ __global__ void k_calcdt_fin(const __grid_constant__ Batch<CdtFinArgs, NB> bt)
     cdt_reset_keys(gkey);
 }
 
-int cdt_chunks(size_t n) { return (int)((n + CDT_CHUNK - 1) / CDT_CHUNK); }
+int cdt_chunks(size_t np, int nz) { return (int)((np + cdt_chunk(np) - 1) / cdt_chunk(np)) * nz; }
 
 static CdtArgs cdt_args(Engine *E)
 {
     CdtArgs a;
     a.u = E->u; a.v = E->v; a.w = E->w; a.r = E->r; a.t = E->t; a.bx = E->bx; a.by = E->by; a.bz = E->bz;
-    a.n = E->n; a.g1 = E->k.g1; a.f = E->k.f;
-    a.nchunks = cdt_chunks(E->n);
+    a.u32 = E->u32; a.v32 = E->v32; a.w32 = E->w32; a.r32 = E->r32; a.t32 = E->t32;
+    a.bx32 = E->bx32; a.by32 = E->by32; a.bz32 = E->bz32; a.bzbar = E->bzbar;
+    a.r0 = E->split ? split_bg_rho0(E) : nullptr; a.t0 = E->split ? split_bg_t0(E) : nullptr;
+    a.np = E->np; a.g1 = E->k.g1; a.f = E->k.f;
+    a.nchunks = cdt_chunks(E->np, E->nz);
+    a.cs = cdt_chunk(E->np);
     a.gkey = reinterpret_cast<unsigned *>(E->cdt);
     a.chunk = E->cdt + 4;
     a.ds = E->ds;
     return a;
 }
 
-int phys_calcdt_m(Engine *const *Es, int nE)
+bool cdt_mirrors_ok(const Engine &E)
+{
+    return E.split && 1.0 + E.p.theta <= CDT_BG && pow(1.0 + E.p.theta, E.p.cm) <= CDT_BG && E.p.theta >= 0.0 && E.p.cm >= 0.0;
+}
+
+// mirrors: of the split form's time step (every member's mirrors are current)
+int phys_calcdt_m(Engine *const *Es, int nE, bool mirrors)
 {
     Engine *E = Es[0];
-    const unsigned nch = (unsigned)cdt_chunks(E->n);
+    const dim3 grid((unsigned)((E->np + cdt_chunk(E->np) - 1) / cdt_chunk(E->np)), (unsigned)E->nz);
     int st;
-    if ((st = launch_members<CdtArgs>(Es, nE, "calcdt_est_f64", FB(E, 8, 8), dim3(nch), dim3(256), 0,
-                                      k_calcdt_est<1>, k_calcdt_est<BATCH_MAX>, cdt_args)))
+    if ((st = launch_members<CdtArgs>(Es, nE, "calcdt_est", FB(E, 8, mirrors ? 4 : 8), grid, dim3(256), 0,
+                                      mirrors ? k_calcdt_est<1, true> : k_calcdt_est<1, false>,
+                                      mirrors ? k_calcdt_est<BATCH_MAX, true> : k_calcdt_est<BATCH_MAX, false>, cdt_args)))
         return st;
-    if ((st = launch_members<CdtArgs>(Es, nE, "calcdt_exact", 0.0, dim3(nch), dim3(256), 0, k_calcdt_exact<1>,
-                                      k_calcdt_exact<BATCH_MAX>, cdt_args)))
+    if ((st = launch_members<CdtArgs>(Es, nE, "calcdt_exact", 0.0, grid, dim3(256), 0,
+                                      mirrors ? k_calcdt_exact<1, true> : k_calcdt_exact<1, false>,
+                                      mirrors ? k_calcdt_exact<BATCH_MAX, true> : k_calcdt_exact<BATCH_MAX, false>, cdt_args)))
         return st;
     return launch_members<CdtFinArgs>(Es, nE, "calcdt_fin", 0.0, dim3(1), dim3(1), 0, k_calcdt_fin<1>,
                                       k_calcdt_fin<BATCH_MAX>, [](Engine *e) {
@@ -915,7 +852,7 @@ int phys_calcdt_m(Engine *const *Es, int nE)
                                                              c.var_eta, c.eta_max };
                                       });
 }
-int phys_calcdt(Engine *E) { return phys_calcdt_m(&E, 1); }
+int phys_calcdt(Engine *E) { return phys_calcdt_m(&E, 1, false); }
 
 // ============================================================================
 // diagnostics: GlobalAverages (src/utils.F90:22-139), nusselt

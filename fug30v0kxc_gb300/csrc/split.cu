@@ -27,6 +27,7 @@
 
 #include <vector>
 
+#include "boundary.cuh"
 #include "common.cuh"
 #include "engine.h"
 #include "fpconv.cuh"
@@ -82,6 +83,7 @@ __global__ void k_make_pcf(const double *bg, const double *kappa, const double *
 }
 
 const double *split_bg_t0(const Engine *E) { return E->hres + (size_t)BG_T0 * E->nz; }
+const double *split_bg_rho0(const Engine *E) { return E->hres + (size_t)BG_RHO0 * E->nz; }
 
 // (re)builds the FP32 plane coefficients from the FP64 profiles
 int split_refresh_coefs(Engine *E)
@@ -904,7 +906,20 @@ static void mag_fwd_jobs(Engine *E, LineJob<float> *fx, LineJob<float> *fy)
     fy[2] = ljob<float>(W[W_EZ], W[W_EZ], OP_FWD);
 }
 
-static SplitHydroArgs hydro_args(Engine *E)
+// planes per z chunk of passes 2 and 4: about kc_pass2 (tunable), less where the
+// chunks of all nE members would not give every SM two CTAs (64^2 x 65: 40 CTAs
+// of 16 planes took 39 us, 264 of 2 take 13 us, although a chunk of 2 planes
+// reads four times as many); balanced over nz
+static int z_chunk(const Engine *E, int nE)
+{
+    int kt = E->kc_pass2 > 0 ? E->kc_pass2 : 16;
+    const long long tiles = (long long)nE * (E->zpencil && E->np % 512 == 0 ? E->np / 512 : nblk(E->np));
+    while (kt > 2 && tiles * ((E->nz + kt - 1) / kt) < 2LL * E->num_sms) kt /= 2;
+    const int nch = (E->nz + kt - 1) / kt;
+    return (E->nz + nch - 1) / nch;
+}
+
+static SplitHydroArgs hydro_args(Engine *E, int nE)
 {
     float *W[W_COUNT];
     for (int i = 0; i < W_COUNT; i++) W[i] = E->W<float>(i);
@@ -927,10 +942,7 @@ static SplitHydroArgs hydro_args(Engine *E)
     a.ho12 = (float)c.ho12; a.sc1 = (float)c.sc1; a.bzbar = (float)E->bzbar;
     a.var_eta = c.var_eta; a.np = E->np; a.nz = E->nz;
     a.mag = split_mag_on(*E);
-    // chunks of about kc_pass2 planes (tunable), balanced over nz
-    const int kt = E->kc_pass2 > 0 ? E->kc_pass2 : 16;
-    const int nch = (E->nz + kt - 1) / kt;
-    a.kc = (E->nz + nch - 1) / nch;
+    a.kc = z_chunk(E, nE);
     a.err = E->dev_err;
     return a;
 }
@@ -944,7 +956,7 @@ static SplitHydroArgs hydro_args(Engine *E)
 #define DYV W_UYY
 #define DYW W_VYY
 
-static SplitHydro4Args hydro4_args(Engine *E)
+static SplitHydro4Args hydro4_args(Engine *E, int nE)
 {
     float *W[W_COUNT];
     for (int i = 0; i < W_COUNT; i++) W[i] = E->W<float>(i);
@@ -955,7 +967,7 @@ static SplitHydro4Args hydro4_args(Engine *E)
     b.ht = E->ht;
     b.ho12 = (float)E->k.ho12; b.np = E->np; b.nz = E->nz;
     b.mag = split_mag_on(*E);
-    b.kc = hydro_args(E).kc;
+    b.kc = z_chunk(E, nE);
     b.err = E->dev_err;
     return b;
 }
@@ -1018,8 +1030,8 @@ int split_hydro_m(Engine *const *Es, int nE, const bool *with_mag)
     // pass 2 (with E = u x B for the members whose mag branch shares the
     // transforms: 3 fields more)
     int im = 0;
-    auto p2args = [&im, with_mag](Engine *e) {
-        SplitHydroArgs a = hydro_args(e);
+    auto p2args = [&im, with_mag, nE](Engine *e) {
+        SplitHydroArgs a = hydro_args(e, nE);
         if (with_mag[im++]) {
             a.e1 = e->W<float>(W_M1);
             a.e2 = e->W<float>(W_M2);
@@ -1037,7 +1049,7 @@ int split_hydro_m(Engine *const *Es, int nE, const bool *with_mag)
                                           (int)smem));
             attr = true;
         }
-        const int kc = hydro_args(E).kc;
+        const int kc = z_chunk(E, nE);
         st = launch_members<SplitHydroArgs>(Es, nE, "hydro_pass2_f32", p2b,
                                             dim3((unsigned)(E->np / ZT_TILE), (unsigned)((E->nz + kc - 1) / kc)),
                                             dim3(ZT_TILE / 2), smem, k_split_pass2_zt<1>, k_split_pass2_zt<BATCH_MAX>,
@@ -1065,6 +1077,7 @@ int split_hydro_m(Engine *const *Es, int nE, const bool *with_mag)
     // (the z-pencil form pays where the per-plane form's z neighbours fall
     // out of L2: 4.8 against 3.9 TB/s at 1024^2 x 513; at 512^2 x 257 and
     // below its two CTAs per SM lose to four: 4.6 against 5.6 TB/s)
+    auto p4args = [nE](Engine *e) { return hydro4_args(e, nE); };
     const bool zt4 = E->zpencil4 == 1 || (E->zpencil4 < 0 && E->np >= (size_t)1024 * 1024);
     if (E->nx % 4 == 0 && E->vec4 && E->zpencil && zt4 && E->np % ZT_TILE == 0 && E->nz >= 6) {
         static bool attr4 = false;
@@ -1075,19 +1088,19 @@ int split_hydro_m(Engine *const *Es, int nE, const bool *with_mag)
                                           (int)smem));
             attr4 = true;
         }
-        const int kc = hydro4_args(E).kc;
+        const int kc = z_chunk(E, nE);
         if ((st = launch_members<SplitHydro4Args>(Es, nE, "hydro_pass4_f32", FB(E, split_mag_on(*E) ? 21 : 15, 4),
                                                   dim3((unsigned)(E->np / ZT_TILE), (unsigned)((E->nz + kc - 1) / kc)),
                                                   dim3(ZT_TILE / 2), smem, k_split_pass4_zt<1>,
-                                                  k_split_pass4_zt<BATCH_MAX>, hydro4_args)))
+                                                  k_split_pass4_zt<BATCH_MAX>, p4args)))
             return st;
     } else if (E->nx % 4 == 0 && E->vec4) {
         if ((st = launch_members<SplitHydro4Args>(Es, nE, "hydro_pass4_f32", FB(E, split_mag_on(*E) ? 21 : 15, 4),
                                                   dim3((unsigned)nblk(E->np / 4), (unsigned)E->nz), dim3(TPB), 0,
-                                                  k_split_pass4_v4<1>, k_split_pass4_v4<BATCH_MAX>, hydro4_args)))
+                                                  k_split_pass4_v4<1>, k_split_pass4_v4<BATCH_MAX>, p4args)))
             return st;
     } else {
-        const SplitHydro4Args b = hydro4_args(E);
+        const SplitHydro4Args b = p4args(E);
         KLAUNCHB(E, "hydro_pass4_f32", FB(E, split_mag_on(*E) ? 21 : 15, 4), k_split_pass4, plane_grid(*E), TPB, b);
     }
     return VEC_OK;
@@ -1227,8 +1240,33 @@ __global__ void __launch_bounds__(256) k_d1z4(const __grid_constant__ Batch<D1z4
     reinterpret_cast<V4 *>(out)[(size_t)k * np4 + q4] = zd1(reinterpret_cast<const V4 *>(in) + q4, np4, k, nz, fl, V4(h));
 }
 
-// bandj of the members (equally sized; one launch per kernel for all)
-int split_bandj_m(Engine *const *Es, int nE, bool rotate_hist)
+// jsq with the step's boundary conditions in BND_ROWS extra first CTA rows (a
+// CTA covers 1024 points of jsq and 256 columns of the boundaries).  jsq reads
+// B and what bandj derived; the boundaries change the walls of u, v, w, T, pol
+// and tor.  One launch less per step.
+#define BND_ROWS 4
+struct JsqBndArgs { Jsq4Args j; BndArgs b; };
+template <int NB>
+static __global__ void __launch_bounds__(256, 6) k_jsq4_bnd(const __grid_constant__ Batch<JsqBndArgs, NB> bt)
+{
+    PDL_WAIT();
+    const JsqBndArgs &A = BATCH_MEMBER(bt, NB);
+    if (blockIdx.y >= BND_ROWS) {
+        jsq4_row(A.j, (int)blockIdx.y - BND_ROWS);
+        return;
+    }
+    const BndArgs &a = A.b;
+    const size_t q = ((size_t)blockIdx.y * gridDim.x + blockIdx.x) * blockDim.x + threadIdx.x;
+    if (q < a.np) boundary_column(a.u, a.v, a.w, a.t, a.np, a.nz, a.theta, a.dz, a.radbc, a.constflux, a.mb, q);
+    mag_boundary_column(a.pol, a.tor, a.bxb, a.byb, a.np, a.nz, a.perfect, a.mb, q);
+}
+
+// whether split_bandj_m applies the boundary conditions too when asked
+bool split_bandj_bounds(const Engine &E) { return E.nx % 4 == 0 && E.vec4; }
+
+// bandj of the members (equally sized; one launch per kernel for all); bounds:
+// with boundary and mag_boundary of the step
+int split_bandj_m(Engine *const *Es, int nE, bool rotate_hist, bool bounds)
 {
     Engine *E = Es[0];
     int st;
@@ -1286,13 +1324,18 @@ int split_bandj_m(Engine *const *Es, int nE, bool rotate_hist)
     }
     if ((st = launch_lines<float>(E, 0, ix.data(), (int)ix.size()))) return st;
     if ((st = launch_lines<float>(E, 1, iy.data(), (int)iy.size()))) return st;
-    if (v4) {
+    auto jq = [](Engine *e) {
+        return Jsq4Args{ e->W<float>(W_M4), e->W<float>(W_M2), e->W<float>(W_M3), e->bx32, e->by32, e->jsq32, e->np,
+                         e->nz, (float)e->k.ho12 };
+    };
+    if (v4 && bounds) {
+        if ((st = launch_members<JsqBndArgs>(Es, nE, "jsq_f32", FB(E, 6, 4), dim3(g4.x, g4.y + BND_ROWS), dim3(TPB), 0,
+                                             k_jsq4_bnd<1>, k_jsq4_bnd<BATCH_MAX>,
+                                             [&jq](Engine *e) { return JsqBndArgs{ jq(e), bnd_args(e) }; })))
+            return st;
+    } else if (v4) {
         if ((st = launch_members<Jsq4Args>(Es, nE, "jsq_f32", FB(E, 6, 4), g4, dim3(TPB), 0, k_jsq4<1>,
-                                           k_jsq4<BATCH_MAX>, [](Engine *e) {
-                                               return Jsq4Args{ e->W<float>(W_M4), e->W<float>(W_M2),
-                                                                e->W<float>(W_M3), e->bx32, e->by32, e->jsq32, e->np,
-                                                                e->nz, (float)e->k.ho12 };
-                                           })))
+                                           k_jsq4<BATCH_MAX>, jq)))
             return st;
     } else {
         KLAUNCHB(E, "jsq_f32", FB(E, 6, 4), k_jsq<float>, plane_grid(*E), TPB, E->W<float>(W_M4), E->W<float>(W_M2),
@@ -1301,7 +1344,7 @@ int split_bandj_m(Engine *const *Es, int nE, bool rotate_hist)
     for (int i = 0; i < nE; i++) Es[i]->b32_auth = 1;
     return VEC_OK;
 }
-int split_bandj(Engine *E, bool rotate_hist) { return split_bandj_m(&E, 1, rotate_hist); }
+int split_bandj(Engine *E, bool rotate_hist, bool bounds) { return split_bandj_m(&E, 1, rotate_hist, bounds); }
 
 // ---- AB3 update in FP64 with FP32 histories ------------------------------------------
 struct SplitAb3Args {
@@ -1571,14 +1614,18 @@ int split_calcdt(Engine *E)
     return phys_calcdt(E);
 }
 
-// calcdt of the members (equally sized)
+// calcdt of the members (equally sized), in the time step: on the mirrors where
+// the backgrounds allow it, for all of them or none
 int split_calcdt_m(Engine *const *Es, int nE)
 {
+    bool mirrors = true;
+    for (int i = 0; i < nE; i++) mirrors = mirrors && cdt_mirrors_ok(*Es[i]);
     Engine *sync[BATCH_MAX];
     int ns = 0;
-    for (int i = 0; i < nE; i++)
-        if (Es[i]->b32_auth) sync[ns++] = Es[i];
+    if (!mirrors)
+        for (int i = 0; i < nE; i++)
+            if (Es[i]->b32_auth) sync[ns++] = Es[i];
     int st;
     if (ns && (st = split_sync_b64_m(sync, ns))) return st;
-    return phys_calcdt_m(Es, nE);
+    return phys_calcdt_m(Es, nE, mirrors);
 }
