@@ -279,7 +279,7 @@ extern "C" int vec_create(const vec_params *p, vec_ctx **out)
     }
     set_consts(E);
     int st;
-    if ((st = line_plan_make(E.nx, E.ny, 8, &E.plx)) || (st = line_plan_make(E.ny, E.nx, 8, &E.ply))) {
+    if ((st = fx_plan_make(E.nx, &E.fpx)) || (st = fx_plan_make(E.ny, &E.fpy))) {
         vec_set_error("line lengths nx=%d ny=%d are not supported (2^a 3^b 5^c <= 2048)", E.nx, E.ny);
         delete c;
         return st;
@@ -320,9 +320,10 @@ extern "C" int vec_create(const vec_params *p, vec_ctx **out)
         }
         aky2[E.ny / 2] = -(double)(E.ny / 2) * (double)(E.ny / 2) * cy * cy;
     }
-    if ((st = fx_plan_make(E.nx, &E.fpx)) || (st = fx_plan_make(E.ny, &E.fpy)) ||
-        (st = fx_tables_make(E.nx, &E.fpx, akx1.data(), akx2.data(), E.k.icutoffx, &E.fxx)) ||
+    if ((st = fx_tables_make(E.nx, &E.fpx, akx1.data(), akx2.data(), E.k.icutoffx, &E.fxx)) ||
         (st = fx_tables_make(E.ny, &E.fpy, aky1.data(), aky2.data(), E.k.icutoffy, &E.fxy)) ||
+        (st = fs_tables_make(E.nx, E.fpx, E.fxx, akx1.data(), akx2.data(), E.k.icutoffx, &E.fsx)) ||
+        (st = fs_tables_make(E.ny, E.fpy, E.fxy, aky1.data(), aky2.data(), E.k.icutoffy, &E.fsy)) ||
         (st = line_tables_make<float>(E.nx, akx1.data(), akx2.data(), E.k.icutoffx, &E.tx32)) ||
         (st = line_tables_make<float>(E.ny, aky1.data(), aky2.data(), E.k.icutoffy, &E.ty32))) {
         vec_destroy(c);
@@ -449,6 +450,8 @@ extern "C" int vec_destroy(vec_ctx *c)
     if (E.ht) cudaFree(E.ht);
     if (E.wblock) cudaFree(E.wblock);
     for (int i = 0; i < 6; i++) if (E.s64[i]) cudaFree(E.s64[i]);
+    fs_tables_free(&E.fsx);
+    fs_tables_free(&E.fsy);
     fx_tables_free(&E.fxx);
     fx_tables_free(&E.fxy);
     if (E.tx32.tw) line_tables_free(&E.tx32);

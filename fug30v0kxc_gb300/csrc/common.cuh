@@ -11,19 +11,6 @@ template <typename R> struct CT;
 template <> struct CT<double> { using T = double2; };
 template <> struct CT<float> { using T = float2; };
 
-// ---- line-transform (horizontal FFT) plan -------------------------------
-#define LP_MAXST 16
-struct LinePlan {
-    int n;                  // line length (nx or ny)
-    int nst;                // number of Stockham stages
-    int radix[LP_MAXST];    // radix of each stage (2,3,4,5,8)
-    int P;                  // complex sequences (= pairs of real lines) per CTA
-    int lines;              // real lines per plane (ny for x lines, nx for y lines)
-    int tiles;              // CTAs per plane = ceil(lines / (2P))
-    int threads;            // block size
-    size_t smem;            // dynamic shared memory bytes for the precision in use
-};
-
 // operations of one line job
 enum LineOp {
     OP_NONE = 0,
@@ -60,7 +47,7 @@ struct LineTables {
     R *mda;                 // dealias mask (1/n or 0)
 };
 
-// the FP64 line kernel's passes for a length n (lines_fx.cu): radix, block and
+// the general line kernels' passes for a length n (lines_fx.cu): radix, block and
 // stride of each, ceil(2^31 / stride), and where its twiddles start
 struct FxPlan {
     int n, nb;              // length; elements of a buffer (n rounded up to 8)
@@ -82,6 +69,13 @@ struct FxTables {
     TwX *tw;                // (one allocation with pos and kof)
     unsigned short *pos, *kof;
     double c0, c1, c2;
+};
+
+// the FP32 general line kernel's tables: twiddles by pass, multipliers by position
+struct FsTables {
+    float2 *tw;             // (one allocation with the multipliers)
+    const unsigned short *pos, *kof;    // the FxTables'
+    float *m1, *m2, *mda;
 };
 
 // horizontal wavenumber tables in one precision: akx1, aky1 and the

@@ -51,10 +51,9 @@ struct Engine {
     int dev = 0;                // the context's device
     int generic_lines = 0;      // force the generic line kernel (VEC_GENERIC_LINES=1)
 
-    LinePlan plx, ply;          // precision of the bulk path
-    LinePlan plx64, ply64;      // FP64 plans (per-operator entry points)
-    FxPlan fpx = {}, fpy = {};  // FP64 line passes and tables
-    FxTables fxx = {}, fxy = {};
+    FxPlan fpx = {}, fpy = {};  // passes of the general line kernels
+    FxTables fxx = {}, fxy = {};        // FP64
+    FsTables fsx = {}, fsy = {};        // FP32
     LineTables<float> tx32, ty32;
 
     // FP64 state (src/arrays.f90)
@@ -206,11 +205,11 @@ template <> inline const LineTables<float> &Engine::tables<float>(int dir) const
 // lines.cu
 // exp(-2 pi i e/n) on the host in double, exact at multiples of n/4
 void sincos2pi_host(long e, long n, double *c, double *s);
-int line_plan_make(int n, int lines, int elem_bytes, LinePlan *pl, int force_p = 0);
 template <typename R> int line_tables_make(int n, const double *k1, const double *k2, int icut, LineTables<R> *tb);
 template <typename R> void line_tables_free(LineTables<R> *tb);
 template <typename R> int launch_lines(Engine *E, int dir, const LineJob<R> *jobs, int njobs);
 template <> int launch_lines<double>(Engine *E, int dir, const LineJob<double> *jobs, int njobs);   // lines_fx.cu
+template <> int launch_lines<float>(Engine *E, int dir, const LineJob<float> *jobs, int njobs);
 int line_kernels_configure();
 // physics.cu: calcdt scratch (floats per context, initialisation of its keys)
 int cdt_chunks(size_t np, int nz);
@@ -220,6 +219,15 @@ int line_fx_configure();
 int fx_plan_make(int n, FxPlan *pl);
 int fx_tables_make(int n, FxPlan *pl, const double *k1, const double *k2, int icut, FxTables *tb);
 void fx_tables_free(FxTables *tb);
+// rounds of a group of 32 / q lanes through a plan's passes
+inline int fx_rounds(const FxPlan &pl, int q)
+{
+    int r = 0;
+    for (int p = 0; p < pl.np; p++) r += (pl.n / pl.R[p] * q + 31) / 32;
+    return r;
+}
+int fs_tables_make(int n, const FxPlan &pl, const FxTables &fx, const double *k1, const double *k2, int icut, FsTables *tb);
+void fs_tables_free(FsTables *tb);
 template <typename R> int launch_lines_ct(Engine *E, int dir, const LineJob<R> *jobs, int njobs);
 
 template <typename R>

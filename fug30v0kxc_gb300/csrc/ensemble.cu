@@ -299,8 +299,8 @@ extern "C" int vec_ensemble_tune(vec_ens *e, int steps, const char *cache)
             // chunk, or the z-marching kernel's where nx % 4 != 0)
             const int kcs[3] = { 8, 16, 32 };
             // sequences per tile: the register-FFT kernel's default, or its
-            // alternative (8 for n <= 256, 4 for n >= 768); the generic
-            // kernel's default, 4 or 8
+            // alternative (8 for n <= 256, 4 for n >= 768); the general kernel
+            // has no choice
             auto ct_len = [](int n) {
                 return n == 64 || n == 96 || n == 128 || n == 192 || n == 256 || n == 384 || n == 512 || n == 768 ||
                        n == 1024;
@@ -309,8 +309,6 @@ extern "C" int vec_ensemble_tune(vec_ens *e, int steps, const char *cache)
             if (ct_len(E.nx) && ct_len(E.ny)) {
                 if (E.nx <= 256 || E.ny <= 256) ss.push_back(8);
                 if (E.nx >= 768 || E.ny >= 768) ss.push_back(4);
-            } else {
-                ss = { 0, 4, 8 };
             }
             Entry best = { k, 16, 0 };
             float best_ms = 1e30f;

@@ -1,26 +1,30 @@
-// lines.cu -- horizontal spectral operators of src/fft.F90 as batched
-// shared-memory FFT kernels for sm_103a, in FP32 (FP64: lines_fx.cu).
+// lines.cu -- horizontal spectral operators of src/fft.F90 in FP32 for every
+// line length 2^a 3^b 5^c (FP64: lines_fx.cu; the lengths of the split step's
+// usual grids: lines_ct.cu).
 //
-// One CTA takes 2P real lines of one z-plane (rows of nx values for the x
-// direction, columns of ny values at stride nx for the y direction), packs
-// them pairwise as P complex sequences z = a + i b, and runs a mixed-radix
-// (8/4/2/3/5) Stockham FFT on them in shared memory.  Because every
-// spectral operator of the reference (+ik, -k^2, the 2/3 truncation) is a
-// Hermitian-symmetric multiplier, it acts on Z = A + iB directly and the
-// inverse transform returns both real lines at once; only the 2-D
-// forward/inverse transforms (halfcomplex storage) separate A and B.
+// The passes of lines_fx.cu in FP32: a group of G = 32 / Q lanes owns a sequence
+// z = a + i b of two real lines in shared memory and runs radix-8/6/5/4/3/2
+// passes on it in place, decimating in frequency forward and in time back, so
+// that the spectrum stays in digit-reversed order and the operators' Hermitian
+// multipliers (+ik, -k^2, the 2/3 truncation) are tables in that order.  Only the
+// halfcomplex transforms go through the permutation.  Warps synchronise their
+// passes alone; the CTA meets for the row-by-row loads and stores of y lines.
 //
-// A launch carries up to MAX_JOBS jobs (input field, one or two outputs, an
-// operator per output, optional accumulate epilogue); blockIdx.y selects the
-// job, so all fields needing the same direction share one launch.
+// Measured at 240^2 x 129, against a Stockham kernel that kept 2048 elements
+// per CTA, synchronised it between all stages and took 8 elements per thread
+// through a call per stage: d2bydx 226 -> 53 us, d2bydy 237 -> 58 us; at
+// 480^2 x 65 420 -> 102 us and 449 -> 126 us.  (The register kernel of lines_ct.cu
+// is faster at its own lengths: 256^2 x 129 36 against 52 us.)
 #include <math.h>
 #include <stdio.h>
 #include <string.h>
 
+#include <vector>
+
 #include "common.cuh"
 #include "engine.h"
 
-template <typename R> struct JobPack { LineJob<R> j[MAX_JOBS]; };
+struct JobPack { LineJob<float> j[MAX_JOBS]; };
 
 // ---- radix kernels (natural order outputs X_0..X_{R-1}) ----------------------
 template <typename C>
@@ -103,228 +107,309 @@ template <bool INV, typename C> struct Dft<5, INV, C> {
         v[0] = x0; v[1] = cadd(a1, b1); v[4] = csub(a1, b1); v[2] = cadd(a2, b2); v[3] = csub(a2, b2);
     }
 };
+// even and odd elements by 3, then by 2
+template <bool INV, typename C> struct Dft<6, INV, C> {
+    static __device__ __forceinline__ void run(C *v) {
+        using R = decltype(v[0].x);
+        C a[3] = { v[0], v[2], v[4] }, b[3] = { v[1], v[3], v[5] };
+        Dft<3, INV, C>::run(a);
+        Dft<3, INV, C>::run(b);
+        // b_k W_6^k, W_6 = (1 - i sqrt 3) / 2 forward
+        const R h = (R)0.5, q = (R)0.86602540378443864676372317075293618;
+        const C r1 = rot90<INV>(b[1]), r2 = rot90<INV>(b[2]);
+        C w1, w2;
+        w1.x = h * b[1].x + q * r1.x; w1.y = h * b[1].y + q * r1.y;
+        w2.x = q * r2.x - h * b[2].x; w2.y = q * r2.y - h * b[2].y;
+        v[0] = cadd(a[0], b[0]); v[3] = csub(a[0], b[0]);
+        v[1] = cadd(a[1], w1); v[4] = csub(a[1], w1);
+        v[2] = cadd(a[2], w2); v[5] = csub(a[2], w2);
+    }
+};
 
-// ---- one Stockham stage over nseq sequences of length n (stride ld) ----------
-// EPT: complex elements held per thread per stage (bounds the register use)
-#define EPT 8
-template <int RAD, bool INV, typename C>
-__device__ __noinline__ void fft_stage(C *buf, int nseq, int ld, int n, int Ns, const C *tw)
+#define FS_TPB 256
+// element i of a sequence's buffer: one word of padding per 16, against the bank
+// conflicts of even strides
+__device__ __forceinline__ int fs_at(int i) { return i + (i >> 4); }
+
+// words of a sequence's buffer: odd, so that the same element of a CTA's
+// sequences falls on different banks
+__host__ __device__ constexpr int fs_buf(int n) { return (n + n / 16 + 1) | 1; }
+
+struct FsPass { int n, L, M, G, l; unsigned mg; const float2 *tw; };
+
+template <int R>
+__device__ __forceinline__ int fs_places(const FsPass &a, int b, int *at)
 {
-    constexpr int MAXB = (EPT + RAD - 1) / RAD;
-    const int nb = n / RAD, total = nb * nseq;
-    const int ts = n / (Ns * RAD);
-    C v[MAXB][RAD];
+    const int q = (int)(((unsigned long long)(unsigned)b * a.mg) >> 31), j = b - q * a.M, i = q * a.L + j;
 #pragma unroll
-    for (int c = 0; c < MAXB; c++) {
-        int b = threadIdx.x + c * blockDim.x;
-        if (b < total) {
-            int s = b / nb, j = b - s * nb;
-            int k = j % Ns;
-            const C *sq = buf + s * ld;
+    for (int m = 0; m < R; m++) at[m] = fs_at(i + m * a.M);
+    return j;
+}
+// DFT_R over the elements j + m M of every block of L, then W_L^(j r) (not in the
+// last pass, M = 1)
+template <int R, bool LAST>
+__device__ __forceinline__ void fs_fwd(float2 *buf, const FsPass &a)
+{
+    for (int b = a.l; b < a.n / R; b += a.G) {
+        int at[R];
+        float2 v[R];
+        const int j = fs_places<R>(a, b, at);
 #pragma unroll
-            for (int r = 0; r < RAD; r++) v[c][r] = sq[j + r * nb];
-            if (Ns > 1) {
+        for (int m = 0; m < R; m++) v[m] = buf[at[m]];
+        Dft<R, false, float2>::run(v);
+        buf[at[0]] = v[0];
 #pragma unroll
-                for (int r = 1; r < RAD; r++) {
-                    C w = tw[r * k * ts];
-                    if (INV) w.y = -w.y;
-                    v[c][r] = cmul(v[c][r], w);
+        for (int r = 1; r < R; r++) buf[at[r]] = LAST ? v[r] : cmul(v[r], a.tw[(r - 1) * a.M + j]);
+    }
+    __syncwarp();
+}
+// the reverse.  FIRST (M = 1): from src, times the multipliers mul (d1: i times)
+// unless mul is null.  OUT (L = n, x lines): the results to the two rows.
+struct FsOut { float *a, *b; float sc, add; };
+template <int R, bool FIRST, bool OUT>
+__device__ __forceinline__ void fs_inv(float2 *buf, const float2 *src, const FsPass &a, const float *mul, bool d1, const FsOut &o)
+{
+    for (int b = a.l; b < a.n / R; b += a.G) {
+        int at[R];
+        float2 v[R];
+        const int j = fs_places<R>(a, b, at);
+#pragma unroll
+        for (int r = 0; r < R; r++) {
+            if (FIRST) {
+                v[r] = src[at[r]];
+                if (mul) {
+                    const float m = __ldg(mul + b * R + r);
+                    const float2 z = v[r];
+                    v[r].x = d1 ? -m * z.y : m * z.x;
+                    v[r].y = d1 ? m * z.x : m * z.y;
+                }
+            } else {
+                v[r] = buf[at[r]];
+                if (r) {
+                    float2 w = a.tw[(r - 1) * a.M + j];
+                    w.y = -w.y;
+                    v[r] = cmul(v[r], w);
                 }
             }
-            Dft<RAD, INV, C>::run(v[c]);
         }
-    }
-    __syncthreads();
+        Dft<R, true, float2>::run(v);
 #pragma unroll
-    for (int c = 0; c < MAXB; c++) {
-        int b = threadIdx.x + c * blockDim.x;
-        if (b < total) {
-            int s = b / nb, j = b - s * nb;
-            int k = j % Ns;
-            C *sq = buf + s * ld;
-            int d = (j / Ns) * Ns * RAD + k;
-#pragma unroll
-            for (int r = 0; r < RAD; r++) sq[d + r * Ns] = v[c][r];
+        for (int r = 0; r < R; r++) {
+            if (OUT) {
+                o.a[j + r * a.M] = v[r].x * o.sc + o.add;
+                o.b[j + r * a.M] = v[r].y * o.sc + o.add;
+            } else {
+                buf[at[r]] = v[r];
+            }
         }
     }
-    __syncthreads();
+    __syncwarp();
 }
-
-template <bool INV, typename C>
-__device__ void fft_run(C *buf, int nseq, int ld, const LinePlan &pl, const C *tw)
-{
-    int Ns = 1;
-    for (int st = 0; st < pl.nst; st++) {
-        switch (pl.radix[st]) {
-        case 8: fft_stage<8, INV>(buf, nseq, ld, pl.n, Ns, tw); break;
-        case 4: fft_stage<4, INV>(buf, nseq, ld, pl.n, Ns, tw); break;
-        case 2: fft_stage<2, INV>(buf, nseq, ld, pl.n, Ns, tw); break;
-        case 3: fft_stage<3, INV>(buf, nseq, ld, pl.n, Ns, tw); break;
-        default: fft_stage<5, INV>(buf, nseq, ld, pl.n, Ns, tw); break;
-        }
-        Ns *= pl.radix[st];
+#define FS_SWITCH(R, CALL)                                                                 \
+    switch (R) {                                                                           \
+    case 8: CALL(8); break;                                                                \
+    case 6: CALL(6); break;                                                                \
+    case 5: CALL(5); break;                                                                \
+    case 4: CALL(4); break;                                                                \
+    case 3: CALL(3); break;                                                                \
+    default: CALL(2); break;                                                               \
     }
-}
 
-// ---- the line kernel --------------------------------------------------------
-// DIR 0: lines along x (contiguous); DIR 1: lines along y (stride nx).
-template <typename R, int DIR>
-__global__ void __launch_bounds__(512, 1)
-line_kernel(JobPack<R> jobs, LinePlan pl, LineTables<R> tb, int nx, int ny, int nz)
+// DIR 0: x lines (sequence = two rows), DIR 1: y lines (two columns).  tpp tiles
+// per plane: of Q sequences (one warp's, x) or S = warps Q (a CTA's, y).
+template <int DIR>
+__global__ void __launch_bounds__(FS_TPB, 4)
+line_kernel(const __grid_constant__ JobPack jobs, const __grid_constant__ FxPlan pl, FsTables tb, int nx, int ny, int nz,
+            int tpp, int total, int two)
 {
     PDL_WAIT();
-    using C = typename CT<R>::T;
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    const int n = pl.n, P = pl.P, ld = n + 1;
-    C *A = reinterpret_cast<C *>(smem_raw);
-    C *B = A + (size_t)P * ld;
-    C *tw = B + (size_t)P * ld;
-
-    const LineJob<R> &jb = jobs.j[blockIdx.y];
-    const int plane = blockIdx.x / pl.tiles;
-    const int l0 = (blockIdx.x - plane * pl.tiles) * 2 * P;
+    const int n = pl.n, Q = pl.Q, G = 32 / Q, W = (int)blockDim.x / 32, S = W * Q, nb = fs_buf(n);
+    float2 *bufA = reinterpret_cast<float2 *>(smem_raw);
+    float2 *bufB = bufA + (size_t)S * nb;              // (two)
+    float2 *tw = bufB + (two ? (size_t)S * nb : 0);
+    const int tid = threadIdx.x, wid = tid >> 5, g = (tid & 31) / G, l = (tid & 31) % G, s = wid * Q + g;
+    float2 *A = bufA + (size_t)s * nb, *B = two ? bufB + (size_t)s * nb : A;
     const size_t np = (size_t)nx * ny;
-    const size_t pbase = (size_t)plane * np;
-    const int L = pl.lines;
-    const int tid = threadIdx.x, nt = blockDim.x;
+    const int pairs = (DIR == 0 ? ny : nx) / 2;
+    const int ls = 31 - __clz(S), yq = tid & (S - 1), ye = tid >> ls, de = (int)blockDim.x >> ls;   // y: row by row
+    for (int e = tid; e < pl.ntw; e += blockDim.x) tw[e] = tb.tw[e];
+    __syncthreads();
+    auto args = [&](int p) {
+        FsPass a;
+        a.n = n; a.L = pl.L[p]; a.M = pl.M[p]; a.G = G; a.l = l; a.mg = pl.mg[p]; a.tw = tw + pl.tw[p];
+        return a;
+    };
+    const int t0 = DIR == 0 ? blockIdx.x * W + wid : blockIdx.x, dt = DIR == 0 ? gridDim.x * W : gridDim.x;
+    for (int t = t0; t < total; t += dt) {
+        const int job = t / (nz * tpp), rem = t - job * (nz * tpp);
+        const int plane = rem / tpp, tile = rem - plane * tpp;
+        const LineJob<float> &jb = jobs.j[job];
+        const int op1 = jb.op1, op2 = jb.op2;
+        const bool inv = op1 == OP_INV;
+        const size_t pb = (size_t)plane * np;
+        const int pair = tile * (DIR == 0 ? Q : S) + (DIR == 0 ? g : s);
+        const bool valid = pair < pairs, yvalid = tile * S + yq < pairs;
+        const size_t xoff = pb + 2 * (size_t)pair * nx, yoff = pb + 2 * ((size_t)tile * S + yq);
 
-    for (int e = tid; e < n; e += nt) tw[e] = tb.tw[e];
-
-    // element (line l, position e) -> offset in the plane
-#define LOFF(l, e) (DIR == 0 ? (size_t)(l) * nx + (e) : (size_t)(e) * nx + (l))
-
-    const int op1 = jb.op1, op2 = jb.op2;
-    if (op1 == OP_INV) {
-        // assemble Z_k = A_k + i B_k from two halfcomplex lines
-        for (int idx = tid; idx < P * n; idx += nt) {
-            int s, k;
-            if (DIR == 0) { s = idx / n; k = idx - s * n; } else { k = idx / P; s = idx - k * P; }
-            int la = l0 + 2 * s, lb = la + 1;
-            R ar = 0, ai = 0, br = 0, bi = 0;
-            int kk = k <= n / 2 ? k : n - k;
-            bool edge = (kk == 0) || (2 * kk == n);
-            if (la < L) {
-                R x = jb.in[pbase + LOFF(la, kk)];
-                R y = edge ? (R)0 : jb.in[pbase + LOFF(la, n - kk)];
-                ar = x; ai = k <= n / 2 ? y : -y;
+        // ---- load
+        if (DIR == 0) {
+            const float *r0 = jb.in + (valid ? xoff : 0);
+            for (int e0 = l; e0 < n; e0 += 8 * G) {
+                float2 v[8];
+#pragma unroll
+                for (int c = 0; c < 8; c++) {
+                    const int e = e0 + c * G;
+                    const bool in = valid && e < n;
+                    v[c].x = in ? r0[e] : 0.0f;
+                    v[c].y = in ? r0[e + nx] : 0.0f;
+                }
+#pragma unroll
+                for (int c = 0; c < 8; c++)
+                    if (e0 + c * G < n) A[fs_at(e0 + c * G)] = v[c];
             }
-            if (lb < L) {
-                R x = jb.in[pbase + LOFF(lb, kk)];
-                R y = edge ? (R)0 : jb.in[pbase + LOFF(lb, n - kk)];
-                br = x; bi = k <= n / 2 ? y : -y;
+            __syncwarp();
+        } else {
+            const float *in = jb.in + yoff;
+            float2 *to = bufA + (size_t)yq * nb;
+            for (int e0 = ye; e0 < n; e0 += 8 * de) {
+                float2 v[8];
+#pragma unroll
+                for (int c = 0; c < 8; c++) {
+                    const int e = e0 + c * de;
+                    v[c] = make_float2(0.0f, 0.0f);
+                    if (yvalid && e < n) v[c] = *reinterpret_cast<const float2 *>(in + (size_t)e * nx);
+                }
+#pragma unroll
+                for (int c = 0; c < 8; c++)
+                    if (e0 + c * de < n) to[fs_at(e0 + c * de)] = v[c];
             }
-            C z; z.x = ar - bi; z.y = ai + br;
-            A[s * ld + k] = z;
-        }
-        // op2 OP_D1: also the derivative of the inverse, B <- m1 * Z
-        const bool two = op2 == OP_D1;
-        if (two) {
             __syncthreads();
-            for (int idx = tid; idx < P * n; idx += nt) {
-                const int s = idx / n, k = idx - s * n;
-                const C z = A[s * ld + k];
-                const R m = tb.m1[k];
-                C y; y.x = -m * z.y; y.y = m * z.x;
-                B[s * ld + k] = y;
+        }
+
+        // ---- forward
+        if (!inv) {
+            for (int p = 0; p < pl.np - 1; p++) {
+                const FsPass a = args(p);
+#define CALL(R) fs_fwd<R, false>(A, a)
+                FS_SWITCH(pl.R[p], CALL)
+#undef CALL
+            }
+            const FsPass a = args(pl.np - 1);
+#define CALL(R) fs_fwd<R, true>(A, a)
+            FS_SWITCH(pl.R[pl.np - 1], CALL)
+#undef CALL
+        }
+
+        if (op1 == OP_FWD) {
+            // separate Z into the halfcomplex spectra of the two real lines
+            auto sep = [&](const float2 *Z, int p) {
+                const float2 zp = Z[fs_at(__ldg(tb.pos + p))], zq = Z[fs_at(__ldg(tb.pos + (p == 0 ? 0 : n - p)))];
+                float2 v;
+                if (2 * p <= n) { v.x = 0.5f * (zp.x + zq.x); v.y = 0.5f * (zp.y + zq.y); }
+                else { v.x = 0.5f * (zq.y - zp.y); v.y = 0.5f * (zp.x - zq.x); }
+                v.x *= jb.alpha1;
+                v.y *= jb.alpha1;
+                return v;
+            };
+            if (DIR == 0) {
+                if (valid) {
+                    float *oa = jb.out1 + xoff, *ob = oa + nx;
+                    for (int p = l; p < n; p += G) {
+                        const float2 v = sep(A, p);
+                        oa[p] = jb.acc1 ? oa[p] + v.x : v.x;
+                        ob[p] = jb.acc1 ? ob[p] + v.y : v.y;
+                    }
+                }
+                __syncwarp();
+            } else {
+                __syncthreads();
+                if (yvalid)
+                    for (int p = ye; p < n; p += de) {
+                        float2 v = sep(bufA + (size_t)yq * nb, p);
+                        float2 *dd = reinterpret_cast<float2 *>(jb.out1 + yoff + (size_t)p * nx);
+                        if (jb.acc1) { const float2 w = *dd; v.x = w.x + v.x; v.y = w.y + v.y; }
+                        *dd = v;
+                    }
+                __syncthreads();
+            }
+            continue;
+        }
+
+        // ---- one or two inverse transforms
+        const int nout = op2 != OP_NONE && (!inv || op2 == OP_D1) ? 2 : 1;
+        for (int o = 0; o < nout; o++) {
+            const int op = o == 0 ? op1 : op2;
+            const float2 *src = A;
+            float2 *dst = o + 1 < nout ? B : A;
+            if (inv) {
+                // Z_k = A_k + i B_k from the halfcomplex lines a (re), b (im)
+                for (int i = l; i < n; i += G) {
+                    const int k = __ldg(tb.kof + i), kk = min(k, n - k);
+                    const bool edge = kk == 0 || 2 * kk == n;
+                    const float2 pa = A[fs_at(kk)];
+                    float2 pc = edge ? make_float2(0.0f, 0.0f) : A[fs_at(n - kk)];
+                    if (2 * k > n) { pc.x = -pc.x; pc.y = -pc.y; }
+                    B[fs_at(i)] = make_float2(pa.x - pc.y, pc.x + pa.y);
+                }
+                __syncwarp();
+                src = dst = B;
+            }
+            const float *mul = op == OP_D1 ? tb.m1 : op == OP_D2 ? tb.m2 : op == OP_DEALIAS ? tb.mda : nullptr;
+            const float alpha = o == 0 ? jb.alpha1 : jb.alpha2;
+            const int acc = o == 0 ? jb.acc1 : jb.acc2;
+            float *ot = o == 0 ? jb.out1 : jb.out2;
+            const float sc = op == OP_INV ? 1.0f / (float)n : 1.0f;
+            float addv = 0.0f;
+            if (op == OP_INV && jb.addk) addv = (float)jb.addk[plane];
+            if (op == OP_INV) addv = addv + (float)jb.addc;
+            // x lines: the last pass stores its results
+            const bool fused = DIR == 0 && pl.np > 1 && __all_sync(0xffffffffu, valid && !acc && alpha == 1.0f);
+            const FsOut to = { ot + xoff, ot + xoff + nx, sc, addv };
+            {
+                const FsPass a = args(pl.np - 1);
+#define CALL(R) fs_inv<R, true, false>(dst, src, a, mul, op == OP_D1, to)
+                FS_SWITCH(pl.R[pl.np - 1], CALL)
+#undef CALL
+            }
+            for (int p = pl.np - 2; p >= (fused ? 1 : 0); p--) {
+                const FsPass a = args(p);
+#define CALL(R) fs_inv<R, false, false>(dst, dst, a, nullptr, false, to)
+                FS_SWITCH(pl.R[p], CALL)
+#undef CALL
+            }
+            if (fused) {
+                const FsPass a = args(0);
+#define CALL(R) fs_inv<R, false, true>(dst, dst, a, nullptr, false, to)
+                FS_SWITCH(pl.R[0], CALL)
+#undef CALL
+                continue;
+            }
+            if (DIR == 0) {
+                if (valid)
+                    for (int e = l; e < n; e += G) {
+                        const float2 z = dst[fs_at(e)];
+                        float va = alpha * (z.x * sc), vb = alpha * (z.y * sc);
+                        if (acc) { va = to.a[e] + va; vb = to.b[e] + vb; }
+                        to.a[e] = va + addv;
+                        to.b[e] = vb + addv;
+                    }
+                __syncwarp();
+            } else {
+                __syncthreads();
+                const float2 *bs = (dst == A ? bufA : bufB) + (size_t)yq * nb;
+                if (yvalid)
+                    for (int e = ye; e < n; e += de) {
+                        const float2 z = bs[fs_at(e)];
+                        float2 *dd = reinterpret_cast<float2 *>(ot + yoff + (size_t)e * nx);
+                        float va = alpha * (z.x * sc), vb = alpha * (z.y * sc);
+                        if (acc) { const float2 w = *dd; va = w.x + va; vb = w.y + vb; }
+                        *dd = make_float2(va + addv, vb + addv);
+                    }
+                __syncthreads();
             }
         }
-        __syncthreads();
-        fft_run<true>(A, two ? 2 * P : P, ld, pl, tw);
-        const R sc = (R)1 / (R)n;
-        for (int idx = tid; idx < 2 * P * n; idx += nt) {
-            int l, e;
-            if (DIR == 0) { l = idx / n; e = idx - l * n; } else { e = idx / (2 * P); l = idx - e * (2 * P); }
-            int gl = l0 + l;
-            if (gl >= L) continue;
-            C z = A[(l >> 1) * ld + e];
-            R val = (l & 1) ? z.y : z.x;
-            val = val * sc;
-            R *o = jb.out1 + pbase + LOFF(gl, e);
-            R res = jb.alpha1 * val;
-            res = jb.acc1 ? *o + res : res;
-            if (jb.addk) res = res + (R)jb.addk[plane];
-            if (jb.addc != 0.0) res = res + (R)jb.addc;
-            *o = res;
-            if (two) {
-                const C y = B[(l >> 1) * ld + e];
-                R *o2 = jb.out2 + pbase + LOFF(gl, e);
-                const R r2 = jb.alpha2 * ((l & 1) ? y.y : y.x);
-                *o2 = jb.acc2 ? *o2 + r2 : r2;
-            }
-        }
-        return;
     }
-
-    // load 2P real lines as P complex sequences
-    for (int idx = tid; idx < 2 * P * n; idx += nt) {
-        int l, e;
-        if (DIR == 0) { l = idx / n; e = idx - l * n; } else { e = idx / (2 * P); l = idx - e * (2 * P); }
-        int gl = l0 + l;
-        R val = gl < L ? jb.in[pbase + LOFF(gl, e)] : (R)0;
-        R *dst = reinterpret_cast<R *>(&A[(l >> 1) * ld + e]);
-        dst[l & 1] = val;
-    }
-    __syncthreads();
-    fft_run<false>(A, P, ld, pl, tw);
-
-    if (op1 == OP_FWD) {
-        // separate Z into the halfcomplex spectra of the two real lines
-        for (int idx = tid; idx < 2 * P * n; idx += nt) {
-            int l, p;
-            if (DIR == 0) { l = idx / n; p = idx - l * n; } else { p = idx / (2 * P); l = idx - p * (2 * P); }
-            int gl = l0 + l;
-            if (gl >= L) continue;
-            const C *sq = A + (l >> 1) * ld;
-            int q = p == 0 ? 0 : n - p;
-            C zp = sq[p], zq = sq[q];
-            R val;
-            if (2 * p <= n) val = (l & 1) ? (R)0.5 * (zp.y + zq.y) : (R)0.5 * (zp.x + zq.x);
-            else            val = (l & 1) ? (R)0.5 * (zp.x - zq.x) : (R)0.5 * (zq.y - zp.y);
-            R *o = jb.out1 + pbase + LOFF(gl, p);
-            R res = jb.alpha1 * val;
-            *o = jb.acc1 ? *o + res : res;
-        }
-        return;
-    }
-
-    // spectral multipliers: A <- m1 * Z, B <- m2 * Z
-    const bool two = op2 != OP_NONE;
-    for (int idx = tid; idx < P * n; idx += nt) {
-        int s = idx / n, k = idx - s * n;
-        C z = A[s * ld + k];
-        if (two) {
-            C y;
-            if (op2 == OP_D1) { R m = tb.m1[k]; y.x = -m * z.y; y.y = m * z.x; }
-            else { R m = op2 == OP_D2 ? tb.m2[k] : tb.mda[k]; y.x = m * z.x; y.y = m * z.y; }
-            B[s * ld + k] = y;
-        }
-        C y;
-        if (op1 == OP_D1) { R m = tb.m1[k]; y.x = -m * z.y; y.y = m * z.x; }
-        else { R m = op1 == OP_D2 ? tb.m2[k] : tb.mda[k]; y.x = m * z.x; y.y = m * z.y; }
-        A[s * ld + k] = y;
-    }
-    __syncthreads();
-    // A and B are contiguous: one inverse pass over 2P sequences
-    fft_run<true>(A, two ? 2 * P : P, ld, pl, tw);
-
-    for (int idx = tid; idx < 2 * P * n; idx += nt) {
-        int l, e;
-        if (DIR == 0) { l = idx / n; e = idx - l * n; } else { e = idx / (2 * P); l = idx - e * (2 * P); }
-        int gl = l0 + l;
-        if (gl >= L) continue;
-        size_t off = pbase + LOFF(gl, e);
-        C z = A[(l >> 1) * ld + e];
-        R val = (l & 1) ? z.y : z.x;
-        R res = jb.alpha1 * val;
-        jb.out1[off] = jb.acc1 ? jb.out1[off] + res : res;
-        if (two) {
-            C y = B[(l >> 1) * ld + e];
-            R v2 = (l & 1) ? y.y : y.x;
-            R r2 = jb.alpha2 * v2;
-            jb.out2[off] = jb.acc2 ? jb.out2[off] + r2 : r2;
-        }
-    }
-#undef LOFF
 }
 
 // ---- host side ------------------------------------------------------------------
@@ -344,39 +429,6 @@ void sincos2pi_host(long e, long n, double *c, double *s)
     case 2: *c = -cf; *s = -sf; break;
     default: *c = sf; *s = -cf; break;
     }
-}
-
-int line_plan_make(int n, int lines, int elem_bytes, LinePlan *pl, int force_p)
-{
-    memset(pl, 0, sizeof(*pl));
-    pl->n = n;
-    int m = n;
-    while (m % 8 == 0 && pl->nst < LP_MAXST) { pl->radix[pl->nst++] = 8; m /= 8; }
-    while (m % 4 == 0 && pl->nst < LP_MAXST) { pl->radix[pl->nst++] = 4; m /= 4; }
-    while (m % 2 == 0 && pl->nst < LP_MAXST) { pl->radix[pl->nst++] = 2; m /= 2; }
-    while (m % 3 == 0 && pl->nst < LP_MAXST) { pl->radix[pl->nst++] = 3; m /= 3; }
-    while (m % 5 == 0 && pl->nst < LP_MAXST) { pl->radix[pl->nst++] = 5; m /= 5; }
-    if (m != 1) return VEC_ERR_SIZE;      // only 2^a 3^b 5^c line lengths
-    if (n > 2048) return VEC_ERR_SIZE;
-    // P complex sequences per CTA: about 2048 complex elements per buffer
-    int P = 2048 / n;
-    if (P < 1) P = 1;
-    if (P > 16) P = 16;
-    if (force_p > 0) P = force_p;
-    if (P > lines / 2) P = lines / 2;
-    if (P < 1) P = 1;
-    pl->P = P;
-    pl->lines = lines;
-    pl->tiles = (lines + 2 * P - 1) / (2 * P);
-    // threads: at most EPT complex elements per thread in every stage
-    // (inverse passes may run 2P sequences)
-    int th = (2 * P * n + EPT - 1) / EPT;
-    th = ((th + 31) / 32) * 32;
-    if (th < 64) th = 64;
-    if (th > 512) return VEC_ERR_SIZE;
-    pl->threads = th;
-    pl->smem = (size_t)(2 * P * (n + 1) + n) * 2 * elem_bytes;
-    return VEC_OK;
 }
 
 // multipliers for a direction: k1 = akx1-like table, k2 = akx2-like table
@@ -415,6 +467,54 @@ int line_tables_make(int n, const double *k1, const double *k2, int icut, LineTa
     return st;
 }
 
+// the general kernel's tables: the plan's twiddles, and the multipliers of
+// line_tables_make in the spectrum's order
+int fs_tables_make(int n, const FxPlan &pl, const FxTables &fx, const double *k1, const double *k2, int icut, FsTables *tb)
+{
+    std::vector<float2> tw;
+    for (int p = 0; p < pl.np; p++)
+        if (pl.M[p] > 1)
+            for (int r = 1; r < pl.R[p]; r++)
+                for (int j = 0; j < pl.M[p]; j++) {
+                    double c, s;
+                    sincos2pi_host((long)j * r, pl.L[p], &c, &s);
+                    tw.push_back(make_float2((float)c, (float)-s));
+                }
+    std::vector<float> m(3 * n);
+    const double dn = (double)n;
+    for (int k = 0; k < n; k++) {
+        int rest = k, at = 0;
+        for (int p = 0; p < pl.np; p++) {
+            at += (rest % pl.R[p]) * pl.M[p];
+            rest /= pl.R[p];
+        }
+        m[at] = (float)(k > 0 && 2 * k < n ? k1[k] / dn : 2 * k > n ? -k1[k] / dn : 0.0);
+        m[n + at] = (float)(k == 0 ? 0.0 : k2[k] / dn);
+        const int kk = k <= n / 2 ? k : n - k;
+        m[2 * n + at] = (float)(kk >= n / 2 - icut ? 0.0 : 1.0 / dn);
+    }
+    const size_t bt = tw.size() * sizeof(float2), bm = m.size() * sizeof(float);
+    std::vector<char> all(bt + bm);
+    if (bt) memcpy(all.data(), tw.data(), bt);
+    memcpy(all.data() + bt, m.data(), bm);
+    if (cudaMalloc(&tb->tw, all.size()) != cudaSuccess) {
+        cudaGetLastError();
+        return VEC_ERR_ALLOC;
+    }
+    tb->m1 = reinterpret_cast<float *>(reinterpret_cast<char *>(tb->tw) + bt);
+    tb->m2 = tb->m1 + n;
+    tb->mda = tb->m2 + n;
+    tb->pos = fx.pos;
+    tb->kof = fx.kof;
+    CUDA_TRY(cudaMemcpy(tb->tw, all.data(), all.size(), cudaMemcpyHostToDevice));
+    return VEC_OK;
+}
+void fs_tables_free(FsTables *tb)
+{
+    cudaFree(tb->tw);
+    *tb = FsTables{};
+}
+
 template <typename R>
 void line_tables_free(LineTables<R> *tb)
 {
@@ -422,43 +522,62 @@ void line_tables_free(LineTables<R> *tb)
     memset(tb, 0, sizeof(*tb));
 }
 
-template <typename R>
-int launch_lines(Engine *E, int dir, const LineJob<R> *jobs, int njobs)
+template <int DIR>
+static int run_fs(Engine *E, const LineJob<float> *jobs, int nj)
+{
+    FxPlan pl = DIR == 0 ? E->fpx : E->fpy;
+    JobPack pk;
+    memset(&pk, 0, sizeof(pk));
+    double fields = 0.0;
+    int two = 0;
+    for (int j = 0; j < nj; j++) {
+        pk.j[j] = jobs[j];
+        fields += 2.0 + (jobs[j].acc1 ? 1.0 : 0.0);
+        if (jobs[j].op2 != OP_NONE) fields += 1.0 + (jobs[j].acc2 ? 1.0 : 0.0);
+        if (jobs[j].op2 != OP_NONE || jobs[j].op1 == OP_INV) two = 1;
+    }
+    const int pairs = (DIR == 0 ? E->ny : E->nx) / 2;
+    // (sequences per warp and warps per CTA as in the FP64 kernel)
+    while (pl.Q > 1 && (long long)nj * E->nz * pairs < (long long)E->num_sms * 8 * pl.Q && fx_rounds(pl, pl.Q / 2) < fx_rounds(pl, pl.Q))
+        pl.Q >>= 1;
+    int W = FS_TPB / 32;
+    auto smem_of = [&](int w) {
+        return sizeof(float2) * (pl.ntw + (size_t)w * pl.Q * fs_buf(pl.n) * (two ? 2 : 1));
+    };
+    auto tiles_of = [&](int w) {
+        const int S = DIR == 0 ? pl.Q : w * pl.Q;
+        return (long long)nj * E->nz * ((pairs + S - 1) / S);
+    };
+    while (W > 1 && (smem_of(W) > 75 * 1024 || (DIR == 0 ? tiles_of(W) / W : tiles_of(W)) < E->num_sms)) W >>= 1;
+    const size_t smem = smem_of(W);
+    int per_sm = 1;
+    CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, line_kernel<DIR>, W * 32, smem));
+    if (per_sm < 1) per_sm = 1;
+    const int S = DIR == 0 ? pl.Q : W * pl.Q, tpp = (pairs + S - 1) / S;
+    const long long total = tiles_of(W);
+    long long grid = DIR == 0 ? (total + W - 1) / W : total;
+    if (grid > (long long)E->num_sms * per_sm) grid = (long long)E->num_sms * per_sm;
+    E->prof_begin(DIR == 0 ? "line_x_f32" : "line_y_f32", fields * (double)E->n * sizeof(float));
+    CUDA_TRY(launch_k(*E, line_kernel<DIR>, dim3((unsigned)grid), dim3(W * 32), smem, pk, pl, DIR == 0 ? E->fsx : E->fsy, E->nx,
+                      E->ny, E->nz, tpp, (int)total, two));
+    E->prof_end();
+    CUDA_TRY(cudaGetLastError());
+    return VEC_OK;
+}
+
+template <>
+int launch_lines<float>(Engine *E, int dir, const LineJob<float> *jobs, int njobs)
 {
     if (njobs <= 0) return VEC_OK;
     if (!E->generic_lines) {
-        int h = launch_lines_ct<R>(E, dir, jobs, njobs);
+        const int h = launch_lines_ct<float>(E, dir, jobs, njobs);
         if (h == 1) return VEC_OK;
         if (h < 0) return h;
     }
-    LinePlan pl = dir == 0 ? E->plx : E->ply;
-    if (E->ct_s > 0 && E->ct_s != pl.P) {
-        // autotuned sequences per CTA for the generic kernel
-        LinePlan alt;
-        if (line_plan_make(pl.n, pl.lines, sizeof(R), &alt, E->ct_s) == VEC_OK) pl = alt;
-    }
-    const LineTables<R> &tb = E->tables<R>(dir);
     for (int j0 = 0; j0 < njobs; j0 += MAX_JOBS) {
-        JobPack<R> pk;
-        memset(&pk, 0, sizeof(pk));
-        int nj = njobs - j0 < MAX_JOBS ? njobs - j0 : MAX_JOBS;
-        for (int j = 0; j < nj; j++) pk.j[j] = jobs[j0 + j];
-        dim3 grid((unsigned)(pl.tiles * E->nz), (unsigned)nj);
-        size_t smem = (size_t)(2 * pl.P * (pl.n + 1) + pl.n) * sizeof(typename CT<R>::T);
-        const char *name = dir == 0 ? "line_x_f32" : "line_y_f32";
-        double fields = 0.0;
-        for (int j = 0; j < nj; j++) {
-            const LineJob<R> &q = pk.j[j];
-            fields += 1.0 + 1.0 + (q.acc1 ? 1.0 : 0.0);
-            if (q.op2 != OP_NONE) fields += 1.0 + (q.acc2 ? 1.0 : 0.0);
-        }
-        E->prof_begin(name, fields * (double)E->n * sizeof(R));
-        if (dir == 0)
-            line_kernel<R, 0><<<grid, pl.threads, smem, E->stream>>>(pk, pl, tb, E->nx, E->ny, E->nz);
-        else
-            line_kernel<R, 1><<<grid, pl.threads, smem, E->stream>>>(pk, pl, tb, E->nx, E->ny, E->nz);
-        E->prof_end();
-        CUDA_TRY(cudaGetLastError());
+        const int nj = njobs - j0 < MAX_JOBS ? njobs - j0 : MAX_JOBS;
+        const int st = dir == 0 ? run_fs<0>(E, jobs + j0, nj) : run_fs<1>(E, jobs + j0, nj);
+        if (st) return st;
     }
     return VEC_OK;
 }
@@ -467,11 +586,10 @@ int line_kernels_configure()
 {
     int st = line_ct_configure();
     if (st || (st = line_fx_configure())) return st;
-    CUDA_TRY(cudaFuncSetAttribute(line_kernel<float, 0>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
-    CUDA_TRY(cudaFuncSetAttribute(line_kernel<float, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
+    CUDA_TRY(cudaFuncSetAttribute(line_kernel<0>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
+    CUDA_TRY(cudaFuncSetAttribute(line_kernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
     return VEC_OK;
 }
 
 template int line_tables_make<float>(int, const double *, const double *, int, LineTables<float> *);
 template void line_tables_free<float>(LineTables<float> *);
-template int launch_lines<float>(Engine *, int, const LineJob<float> *, int);

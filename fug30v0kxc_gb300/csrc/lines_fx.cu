@@ -864,12 +864,8 @@ static int run_fx(Engine *E, const LineJob<double> *jobs, int nj)
     // SM): the time is then that of one warp's tile, which more lanes per
     // sequence shorten if its passes take fewer rounds (30 x 30 x 60: 36 -> 26 us;
     // 64 points take as many with 8 lanes as with 32, and lose: 23 -> 28 us)
-    auto rounds = [&](int q) {
-        int r = 0;
-        for (int p = 0; p < pl.np; p++) r += (pl.n / pl.R[p] * q + 31) / 32;
-        return r;
-    };
-    while (pl.Q > 1 && (long long)nj * E->nz * pairs < (long long)E->num_sms * 8 * pl.Q && rounds(pl.Q / 2) < rounds(pl.Q)) pl.Q >>= 1;
+    while (pl.Q > 1 && (long long)nj * E->nz * pairs < (long long)E->num_sms * 8 * pl.Q && fx_rounds(pl, pl.Q / 2) < fx_rounds(pl, pl.Q))
+        pl.Q >>= 1;
     auto smem_of = [&](int w) {
         const size_t S = (size_t)w * pl.Q;
         return sizeof(TwX) * pl.ntw + S * pl.nb * sizeof(X2) * (two ? 2 : 1) + S * sizeof(FxOut) + 16;

@@ -298,7 +298,7 @@ int vec_ensemble_tune(vec_ens *ens, int steps, const char *cache);
 int vec_tunables(vec_ctx *ctx, int *kc, int *s);
 /* sets them: kc in {8, 16, 32}; s in {0 (the kernel's default), 4, 8}
  * (FP32 register-FFT lines: 8 selects 8 sequences per tile for n <= 256,
- * 4 selects 4 for n >= 768; the generic kernel takes 4 or 8) */
+ * 4 selects 4 for n >= 768; other lengths choose for themselves) */
 int vec_set_tunables(vec_ctx *ctx, int kc, int s);
 
 /* ---- learned closure: the network ---------------------------------------
