@@ -337,32 +337,33 @@ extern "C" int vec_create(const vec_params *p, vec_ctx **out)
     }
     {
         // the wavenumber tables per precision; kh2 = akx2[i] + aky2[j] per plane point
-        std::vector<double> kh2(E.np);
+        std::vector<double> kh2(E.np), kh2i(E.np);
         std::vector<float> kx1f(E.nx), ky1f(E.ny), kh2f(E.np), kh2if(E.np);
         for (int j = 0; j < E.ny; j++)
             for (int i = 0; i < E.nx; i++) {
                 const size_t q = (size_t)j * E.nx + i;
                 kh2[q] = akx2[i] + aky2[j];
                 kh2f[q] = (float)kh2[q];
-                kh2if[q] = q == 0 ? 0.0f : (float)(1.0 / kh2[q]);
+                kh2i[q] = q == 0 ? 0.0 : 1.0 / kh2[q];
+                kh2if[q] = (float)kh2i[q];
             }
         for (int i = 0; i < E.nx; i++) kx1f[i] = (float)akx1[i];
         for (int j = 0; j < E.ny; j++) ky1f[j] = (float)aky1[j];
         float *fx = nullptr, *fy = nullptr, *fk = nullptr, *fki = nullptr;
-        double *dk = nullptr;
+        double *dk = nullptr, *dki = nullptr;
         ALLOC(fx, sizeof(float) * E.nx); E.hf.kx1 = fx;
         ALLOC(fy, sizeof(float) * E.ny); E.hf.ky1 = fy;
         ALLOC(fk, sizeof(float) * E.np); E.hf.kh2 = fk;
         ALLOC(fki, sizeof(float) * E.np); E.hf.kh2inv = fki;
-        E.hd.kh2inv = nullptr;
         ALLOC(dk, sizeof(double) * E.np); E.hd.kh2 = dk;
+        ALLOC(dki, sizeof(double) * E.np); E.hd.kh2inv = dki;
         E.hd.kx1 = E.akx1;
         E.hd.ky1 = E.aky1;
         if (cudaMemcpy(fx, kx1f.data(), sizeof(float) * E.nx, cudaMemcpyHostToDevice) != cudaSuccess ||
             cudaMemcpy(fy, ky1f.data(), sizeof(float) * E.ny, cudaMemcpyHostToDevice) != cudaSuccess ||
             cudaMemcpy(fk, kh2f.data(), sizeof(float) * E.np, cudaMemcpyHostToDevice) != cudaSuccess ||
             cudaMemcpy(fki, kh2if.data(), sizeof(float) * E.np, cudaMemcpyHostToDevice) != cudaSuccess ||
-            upload(dk, kh2)) {
+            upload(dk, kh2) || upload(dki, kh2i)) {
             vec_destroy(c);
             return VEC_ERR_CUDA;
         }
@@ -389,6 +390,8 @@ extern "C" int vec_create(const vec_params *p, vec_ctx **out)
         vec_destroy(c);
         return VEC_ERR_CUDA;
     }
+    ALLOC(E.pc64, sizeof(double) * 3 * nz);
+    if ((st = phys_refresh_coefs(&E))) { vec_destroy(c); return st; }
     // state
     double **st64[] = { &E.r, &E.t, &E.u, &E.v, &E.w, &E.bx, &E.by, &E.bz, &E.jsq, &E.pol, &E.tor };
     for (auto pp : st64) ALLOC(*pp, sizeof(double) * n);
@@ -443,7 +446,7 @@ extern "C" int vec_destroy(vec_ctx *c)
                      E.r32, E.t32, E.u32, E.v32, E.w32, E.bx32, E.by32, E.bz32, E.jsq32, E.pol32, E.tor32,
                      E.rho0, E.t0, E.hres, E.corr, E.corr_bx };
     for (void *q : ptrs) if (q) cudaFree(q);
-    const void *tabs[] = { E.hf.kx1, E.hf.ky1, E.hf.kh2, E.hf.kh2inv, E.hd.kh2, E.pcf };
+    const void *tabs[] = { E.hf.kx1, E.hf.ky1, E.hf.kh2, E.hf.kh2inv, E.hd.kh2, E.hd.kh2inv, E.pcf, E.pc64 };
     for (const void *q : tabs) if (q) cudaFree((void *)q);
     for (int f = 0; f < 7; f++) for (int s = 0; s < 3; s++) if (E.hbuf[f][s]) cudaFree(E.hbuf[f][s]);
     for (int s = 0; s < 3; s++) { if (E.bxd_buf[s]) cudaFree(E.bxd_buf[s]); if (E.byd_buf[s]) cudaFree(E.byd_buf[s]); }
@@ -645,8 +648,8 @@ extern "C" int vec_set_mean(vec_ctx *c, int m, const double *src)
     double *d = mean_ptr(c->E, m);
     if (!d) return VEC_ERR_ARG;
     int st = stage_in(c->E, d, src, c->E.nz);
-    if (!st && c->E.split && (m == VEC_M_KAPPA || m == VEC_M_DKAPPA || m == VEC_M_ETA || m == VEC_M_DETA))
-        st = split_refresh_coefs(&c->E);   // their FP32 per-plane copies
+    if (!st && (m == VEC_M_KAPPA || m == VEC_M_DKAPPA || m == VEC_M_ETA || m == VEC_M_DETA))
+        st = c->E.split ? split_refresh_coefs(&c->E) : phys_refresh_coefs(&c->E);   // what is formed of them per plane
     return st ? st : vec_sync(c);
 }
 

@@ -70,6 +70,7 @@ struct Engine {
     HTab<float> hf = {};        // the same wavenumbers in FP32 (kh2: np values)
     HTab<double> hd = {};       // FP64 (kx1, ky1 alias akx1, aky1)
     float *pcf = nullptr;       // split: per-plane FP32 coefficients [PC_COUNT][nz]
+    double *pc64 = nullptr;     // FP64 form: plane coefficients of hydro pass 2 [3][nz]
     double *w1d = nullptr;      // 1-D scratch (8 nz)
     double bzbar = 0.0;
     // work arrays (bulk precision), carved from one contiguous block
@@ -246,6 +247,7 @@ int op_d1z(Engine *E, const double *in, double *out, int flag, int np, int nz);
 int op_d1upz(Engine *E, const double *in, double *out, int flag);
 int op_d2z(Engine *E, const double *in, double *out, int flag, int np, int nz);
 int phys_hydro64(Engine *E);
+int phys_refresh_coefs(Engine *E);   // after kappa / eta change
 int phys_mag64(Engine *E);
 int phys_zero_mag_rhs(Engine *E);
 int phys_bandj64(Engine *E);

@@ -161,10 +161,11 @@ __device__ __forceinline__ void fx_inv_first(X2 *buf, const X2 *src, const FxPas
     }
     __syncwarp();
 }
-// conj(W_L^(j r)) / 2, then the inverse DFT_R.  With oa (the last pass of an x
-// line): the results times sc, plus c, to the two rows.
+// conj(W_L^(j r)) / 2, then the inverse DFT_R.  OUT (the last pass of an x line):
+// the results times sc to the two rows; plus ca, cb or what the rows hold.
+enum { FX_SET, FX_CONST, FX_ACC };
 template <int R, int KIND, bool OUT>
-__device__ __forceinline__ void fx_inv(X2 *buf, const FxPassArgs &a, double *oa, double *ob, double sc, double ca, double cb, bool con)
+__device__ __forceinline__ void fx_inv(X2 *buf, const FxPassArgs &a, double *oa, double *ob, double sc, double ca, double cb, int mode)
 {
     const int M = fx_stride<KIND>(a);
     for (int b = a.l; b < a.n / R; b += a.G) {
@@ -178,7 +179,16 @@ __device__ __forceinline__ void fx_inv(X2 *buf, const FxPassArgs &a, double *oa,
         XDft<R, true>::run(v);
         if (OUT) {
             // (one block: elements j + r M)
-            if (con) {
+            if (mode == FX_ACC) {
+                double xa[R], xb[R];
+#pragma unroll
+                for (int r = 0; r < R; r++) { xa[r] = oa[j + r * M]; xb[r] = ob[j + r * M]; }
+#pragma unroll
+                for (int r = 0; r < R; r++) {
+                    oa[j + r * M] = fma(__ll2double_rn(v[r].x), sc, xa[r]);
+                    ob[j + r * M] = fma(__ll2double_rn(v[r].y), sc, xb[r]);
+                }
+            } else if (mode == FX_CONST) {
 #pragma unroll
                 for (int r = 0; r < R; r++) {
                     oa[j + r * M] = fma(__ll2double_rn(v[r].x), sc, ca);
@@ -595,8 +605,8 @@ line_fx(const __grid_constant__ FxPack jobs, const __grid_constant__ FxPlan pl, 
             const int acc = o == 0 ? jb.acc1 : jb.acc2;
             double *ot = o == 0 ? jb.out1 : jb.out2;
             // what is added back: the mean of a dealiased line, the constant of an
-            // inverse, and its addk, addc.  (What is only stored takes paths of its
-            // own: FP64 operations, predicated off or not, would keep the FP64 pipe
+            // inverse, and its addk, addc.  (What is stored or accumulated as it is takes
+            // paths of its own: FP64 operations, predicated off or not, would keep the FP64 pipe
             // busier than the conversions do.)
             const bool add = op == OP_DEALIAS || op == OP_INV;
             double addv = 0.0;
@@ -605,18 +615,19 @@ line_fx(const __grid_constant__ FxPack jobs, const __grid_constant__ FxPlan pl, 
             double ca = out.cx, cb = out.cy;
             if (store && op == OP_INV) { ca += addv; cb += addv; }
             double *oa = ot + pb + 2 * (size_t)pair * nx, *ob = oa + nx;
-            const bool plain = store && safe && !out.bad;
+            const bool plain = alpha == 1.0 && !(acc && add) && safe && !out.bad;
+            const int mode = acc ? FX_ACC : add ? FX_CONST : FX_SET;
             // x lines: the last pass stores its results
             const bool fused = DIR == 0 && pl.np > 1 && __all_sync(0xffffffffu, plain && valid);
             for (int p = pl.np - 2; p >= (fused ? 1 : 0); p--) {
                 const FxPassArgs a = args(p);
-#define CALL(R, K) fx_inv<R, K, false>(dst, a, nullptr, nullptr, 0.0, 0.0, 0.0, false)
+#define CALL(R, K) fx_inv<R, K, false>(dst, a, nullptr, nullptr, 0.0, 0.0, 0.0, FX_SET)
                 FX_SWITCH(pl, p, CALL)
 #undef CALL
             }
             if (fused) {
                 const FxPassArgs a = args(0);
-#define CALL(R, K) fx_inv<R, K, true>(dst, a, oa, ob, out.sc, ca, cb, add)
+#define CALL(R, K) fx_inv<R, K, true>(dst, a, oa, ob, out.sc, ca, cb, mode)
                 FX_SWITCH(pl, 0, CALL)
 #undef CALL
                 continue;
@@ -650,7 +661,14 @@ line_fx(const __grid_constant__ FxPack jobs, const __grid_constant__ FxPlan pl, 
                 double *od = ot + pb + 2 * ((size_t)tile * S + q);
                 if (tile * S + q < pairs) {
                     const FxOut f = so[q];
-                    if (fast && add) {
+                    if (fast && acc) {
+                        for (int e = tid >> ls; e < n; e += de) {
+                            const X2 v = bs[fx_at(e, q & 7)];
+                            double2 *o2 = reinterpret_cast<double2 *>(od + (size_t)e * nx);
+                            const double2 x = *o2;
+                            *o2 = make_double2(fma(__ll2double_rn(v.x), f.sc, x.x), fma(__ll2double_rn(v.y), f.sc, x.y));
+                        }
+                    } else if (fast && add) {
                         for (int e = tid >> ls; e < n; e += de) {
                             const X2 v = bs[fx_at(e, q & 7)];
                             *reinterpret_cast<double2 *>(od + (size_t)e * nx) =

@@ -24,6 +24,7 @@
 #include "fpconv.cuh"
 #include "boundary.cuh"
 #include "zstencil.cuh"
+#include "zfx.cuh"
 #include "magkern.cuh"
 
 #define TPB 256
@@ -47,53 +48,39 @@ static inline unsigned nblk(size_t n, int tpb = TPB)
 // ============================================================================
 // z-derivative operators (per-operator entry points)
 // ============================================================================
-template <typename R>
-__global__ void k_d1z(const R *in, R *out, int fl, size_t np, int nz, R h)
+// (grid (np/256, nz); bound by integer issue with the sums in integers: d1 at
+// 256^2 x 129 72 -> 55 us, d2 88 -> 65 us against FP64 sums)
+template <int W>
+__global__ void __launch_bounds__(256) k_zderiv(const double *in, const double *w, double *out, int fl, size_t np, int nz, double h)
 {
     PDL_WAIT();
-    size_t idx = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (idx >= np * nz) return;
-    int k = (int)(idx / np);
-    size_t q = idx - (size_t)k * np;
-    out[idx] = zd1(in + q, np, k, nz, fl, h);
+    const size_t q = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (q >= np) return;
+    const int k = blockIdx.y;
+    const size_t idx = (size_t)k * np + q;
+    const ZSum z = zsum<W | ZPIPE>(in + q, np, k, nz, fl, fl, W == ZUP ? w[idx] : 0.0);
+    out[idx] = h * (W == ZD1 ? z.d1 : W == ZD2 ? z.d2 : z.up);
 }
-template <typename R>
-__global__ void k_d1upz(const R *in, const R *w, R *out, int fl, size_t np, int nz, R h)
-{
-    PDL_WAIT();
-    size_t idx = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (idx >= np * nz) return;
-    int k = (int)(idx / np);
-    size_t q = idx - (size_t)k * np;
-    out[idx] = zd1up(in + q, np, k, nz, fl, h, w[idx]);
-}
-template <typename R>
-__global__ void k_d2z(const R *in, R *out, int fl, size_t np, int nz, R s)
-{
-    PDL_WAIT();
-    size_t idx = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (idx >= np * nz) return;
-    int k = (int)(idx / np);
-    size_t q = idx - (size_t)k * np;
-    out[idx] = zd2(in + q, np, k, nz, fl, s);
-}
+static dim3 zgrid(size_t np, int nz) { return dim3(nblk(np), (unsigned)nz); }
 
 int op_d1z(Engine *E, const double *in, double *out, int flag, int np, int nz)
 {
     if (!(flag == 0 || flag == 1 || flag == 2 || flag == 5)) return VEC_ERR_FLAG;
-    KLAUNCHB(E, "d1bydz_f64", 2.0 * np * nz * 8, k_d1z<double>, nblk((size_t)np * nz), TPB, in, out, flag, (size_t)np, nz, E->k.ho12);
+    KLAUNCHB(E, "d1bydz_f64", 2.0 * np * nz * 8, k_zderiv<ZD1>, zgrid(np, nz), TPB, in, (const double *)nullptr, out, flag,
+             (size_t)np, nz, E->k.ho12);
     return VEC_OK;
 }
 int op_d1upz(Engine *E, const double *in, double *out, int flag)
 {
     if (!(flag == 0 || flag == 1 || flag == 2 || flag == 5)) return VEC_ERR_FLAG;
-    KLAUNCH(E, "d1upbydz_f64", k_d1upz<double>, nblk(E->n), TPB, in, E->w, out, flag, E->np, E->nz, E->k.ho12);
+    KLAUNCHB(E, "d1upbydz_f64", FB(E, 3, 8), k_zderiv<ZUP>, zgrid(E->np, E->nz), TPB, in, E->w, out, flag, E->np, E->nz, E->k.ho12);
     return VEC_OK;
 }
 int op_d2z(Engine *E, const double *in, double *out, int flag, int np, int nz)
 {
     if (!(flag == 0 || flag == 3)) return VEC_ERR_FLAG;
-    KLAUNCH(E, "d2bydz_f64", k_d2z<double>, nblk((size_t)np * nz), TPB, in, out, flag, (size_t)np, nz, E->k.sc1);
+    KLAUNCHB(E, "d2bydz_f64", 2.0 * np * nz * 8, k_zderiv<ZD2>, zgrid(np, nz), TPB, in, (const double *)nullptr, out, flag,
+             (size_t)np, nz, E->k.sc1);
     return VEC_OK;
 }
 
@@ -104,136 +91,155 @@ struct HydroArgs {
     const double *r, *t, *u, *v, *w, *bx, *by, *bz, *jsq;
     const double *rx, *tx, *txx, *ux, *uxx, *vx, *vxx, *wx, *wxx;
     const double *ry, *ty, *tyy, *uy, *uyy, *vy, *vyy, *wy, *wyy;
-    const double *kappa, *dkappa, *eta;
+    const double *pc;       // per plane: gck kappa, gck dkappa ho12, fzckg eta / zck (k_make_pc64)
     const HistTable *ht;    // tdot = newest slot of t
     double *racc, *uacc, *vacc, *wacc;
     double *p1, *p2, *q, *g, *hh, *p3, *p4;
-    double gck, fzckg, gm1, sckg, fo2, scko3, f, thmplus1, cor, cpsi, spsi, sck, zck, ho12, sc1;
-    int var_eta;
+    double *ri;             // 1 / rho, over rx
+    double gm1, sckg, scko3, f, thmplus1, cor, cpsi, spsi, sck, ho12, sc1;
+    int mag;                // 0: no magnetic field (Q = 0): J^2 and the Lorentz fluxes
+                            // are zero, neither read nor written
     size_t np;
     int nz;
 };
 
+// the plane coefficients of pass 2
+__global__ void k_make_pc64(const double *kappa, const double *dkappa, const double *eta, double gck, double fzckg, double zck,
+                            double ho12, int var_eta, int nz, double *pc)
+{
+    for (int k = threadIdx.x; k < nz; k += blockDim.x) {
+        pc[k] = gck * kappa[k];
+        pc[nz + k] = gck * dkappa[k] * ho12;
+        pc[2 * nz + k] = fzckg * (var_eta ? eta[k] / zck : 1.0);
+    }
+}
+int phys_refresh_coefs(Engine *E)
+{
+    const Consts &c = E->k;
+    k_make_pc64<<<1, 256, 0, E->stream>>>(E->kappa, E->dkappa, E->eta, c.gck, c.fzckg, c.zck, c.ho12, c.var_eta, E->nz, E->pc64);
+    CUDA_TRY(cudaGetLastError());
+    return VEC_OK;
+}
+
 // pass 2: src/hydro_deriv.f90:45-53, 82-110, 139-168, 201-219, 245-261,
 // 287-309, 360-367, 390-398, 421-432 (every term without a second-level
 // derivative); the energy equation is complete here.
-// (three CTAs per SM, 80 registers: 2.68 ms at 256^2 x 129 against 2.74 at
-// the compiler's own 96 registers and two CTAs, 2.84 at 120 registers)
+//
+// Bound by the FP64 pipe: about 90 operations per point, with the z stencils
+// summed in integers (zfx.cuh) and left without their factors ho12 and sc1,
+// which enter the products they are part of, common factors taken out and the
+// plane coefficients formed beforehand.  As the reference's expressions stand
+// they were 170: 2.68 -> 1.56 ms at 256^2 x 129.  1 / rho is kept for pass 4
+// (16 bytes against nine operations).
 __global__ void __launch_bounds__(256, 3) k_hydro_pass2(HydroArgs a)
 {
     PDL_WAIT();
-    size_t idx = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (idx >= a.np * a.nz) return;
-    const int nz = a.nz;
-    const size_t np = a.np;
-    const int k = (int)(idx / np);
-    const size_t q = idx - (size_t)k * np;
-    const double h = a.ho12, s = a.sc1;
-
-    const double rr = a.r[idx], tt = a.t[idx], u0 = a.u[idx], v0 = a.v[idx], w0 = a.w[idx];
-    const double bx = a.bx[idx], by = a.by[idx], bz = a.bz[idx];
-    const double rx = a.rx[idx], ry = a.ry[idx];
-    const double tx = a.tx[idx], txx = a.txx[idx], ty = a.ty[idx], tyy = a.tyy[idx];
-    const double ux = a.ux[idx], uxx = a.uxx[idx], uy = a.uy[idx], uyy = a.uyy[idx];
-    const double vx = a.vx[idx], vxx = a.vxx[idx], vy = a.vy[idx], vyy = a.vyy[idx];
-    const double wx = a.wx[idx], wxx = a.wxx[idx], wy = a.wy[idx], wyy = a.wyy[idx];
+    const size_t np = a.np, q = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (q >= np) return;
+    const int nz = a.nz, k = blockIdx.y;
+    const size_t idx = (size_t)k * np + q;
+    const double h = a.ho12;
 
     // z derivatives (flags: src/hydro_deriv.f90:66-68, 124-125, 233, 275, 349-350)
-    const double tzu = zd1up(a.t + q, np, k, nz, 5, h, w0);
-    const double tz = zd1(a.t + q, np, k, nz, 5, h);
-    const double tzz = zd2(a.t + q, np, k, nz, 0, s);
-    const double wzu = zd1up(a.w + q, np, k, nz, 1, h, w0);
-    const double wz = zd1(a.w + q, np, k, nz, 1, h);
-    const double uzu = zd1up(a.u + q, np, k, nz, 2, h, w0);
-    const double vzu = zd1up(a.v + q, np, k, nz, 2, h, w0);
-    const double uzz = zd2(a.u + q, np, k, nz, 3, s);
-    const double vzz = zd2(a.v + q, np, k, nz, 3, s);
+    const double w0 = a.w[idx], hw = h * w0;
+    const ZSum zt = zsum<ZD1 | ZD2 | ZUP>(a.t + q, np, k, nz, 5, 0, w0), zw = zsum<ZD1 | ZUP>(a.w + q, np, k, nz, 1, 0, w0);
+    const ZSum zu = zsum<ZD2 | ZUP>(a.u + q, np, k, nz, 2, 3, w0), zv = zsum<ZD2 | ZUP>(a.v + q, np, k, nz, 2, 3, w0);
 
-    const double third = 1.0 / 3.0;
-    const double ohm = a.var_eta ? a.eta[k] / a.zck : 1.0;
-    const double divu = ux + vy + wz;
+    const double rr = a.r[idx], tt = a.t[idx], u0 = a.u[idx], v0 = a.v[idx];
+    const double rx = a.rx[idx], ry = a.ry[idx], tx = a.tx[idx], ty = a.ty[idx];
+    const double ux = a.ux[idx], uy = a.uy[idx], vx = a.vx[idx], vy = a.vy[idx], wx = a.wx[idx], wy = a.wy[idx];
+    const double ri = 1.0 / rr;
+    a.ri[idx] = ri;
+    const double wz = h * zw.d1, dh = ux + vy, divu = dh + wz;
 
     // continuity: :48, :149 (the w d(rho)/dz term is added in pass 4)
-    a.racc[idx] = -u0 * rx - v0 * ry - rr * divu;
+    a.racc[idx] = -(u0 * rx + v0 * ry + rr * divu);
 
     // energy (rho * dT/dt): :88-102, :150-151, :216, :258, :300, then / rho
-    double td = -rr * (u0 * tx + v0 * ty + w0 * tzu)
-                + a.gck * a.kappa[k] * (txx + tyy + tzz)
-                + a.gck * a.dkappa[k] * tzu
-                + a.fzckg * ohm * a.jsq[idx];
-    td = td - a.gm1 * tt * divu * rr + 2 * a.sckg * (ux * ux + vy * vy + wz * wz - third * divu * divu);
-    td = td + a.sckg * (uy + vx) * (uy + vx);
-    td = td + a.sckg * (wx + uzu) * (wx + uzu);
-    td = td + a.sckg * (wy + vzu) * (wy + vzu);
-    ((double *)a.ht->p[1][2])[idx] = td * (1.0 / rr);
+    const double at = u0 * tx + v0 * ty + hw * zt.up;
+    double td = a.pc[k] * ((a.txx[idx] + a.tyy[idx]) + a.sc1 * zt.d2) + a.pc[nz + k] * zt.up;
+    if (a.mag) td += a.pc[2 * nz + k] * a.jsq[idx];
+    td = td - rr * (at + (a.gm1 * tt) * divu);
+    const double sxy = uy + vx, sxz = wx + h * zu.up, syz = wy + h * zv.up;
+    const double dil = ux * ux + vy * vy + wz * wz - (1.0 / 3.0) * divu * divu;
+    td = td + a.sckg * (2.0 * dil + (sxy * sxy + sxz * sxz + syz * syz));
+    ((double *)a.ht->p[1][2])[idx] = td * ri;
 
     // momentum: :103-105, :159-161, :213-214, :253-254, :292-306, :363-364, :393-395, :424-426
-    double ud = -tt * rx - rr * tx;
-    ud = ud - rr * u0 * ux - rr * v0 * uy - rr * w0 * uzu;
-    ud = ud - rr * a.cor * (w0 * a.cpsi + v0 * a.spsi);
-    ud = ud + a.sck * uzz + a.sck * uxx + a.sck * uyy;
-    double vd = -tt * ry - rr * ty;
-    vd = vd - rr * v0 * vy - rr * u0 * vx - rr * w0 * vzu;
-    vd = vd - rr * a.cor * (-u0 * a.spsi);
-    vd = vd + a.sck * vzz + a.sck * vxx + a.sck * vyy;
-    double wd = -rr * tz;
-    wd = wd - rr * w0 * wzu + a.thmplus1 * rr - rr * u0 * wx - rr * v0 * wy;
-    wd = wd - rr * a.cor * (-u0 * a.cpsi);
-    wd = wd + a.sck * wxx + a.sck * wyy;
-    a.uacc[idx] = ud;
-    a.vacc[idx] = vd;
-    a.wacc[idx] = wd;
+    double au = tx + (u0 * ux + v0 * uy + hw * zu.up), av = ty + (u0 * vx + v0 * vy + hw * zv.up);
+    double aw = h * zt.d1 + (u0 * wx + v0 * wy + hw * zw.up) - a.thmplus1;
+    if (a.cor != 0.0) {
+        au += a.cor * (w0 * a.cpsi + v0 * a.spsi);
+        av -= a.cor * (u0 * a.spsi);
+        aw -= a.cor * (u0 * a.cpsi);
+    }
+    a.uacc[idx] = a.sck * ((a.uxx[idx] + a.uyy[idx]) + a.sc1 * zu.d2) - tt * rx - rr * au;
+    a.vacc[idx] = a.sck * ((a.vxx[idx] + a.vyy[idx]) + a.sc1 * zv.d2) - tt * ry - rr * av;
+    a.wacc[idx] = a.sck * (a.wxx[idx] + a.wyy[idx]) - rr * aw;
 
     // second-level inputs: :152-165, :215, :255-257, :297-299
-    const double temp1 = a.fo2 * bx * bx, temp2 = a.fo2 * by * by, temp3 = a.fo2 * bz * bz;
     const double dv = a.scko3 * divu;
-    a.p1[idx] = dv + temp1 - temp2 - temp3;
-    a.p2[idx] = dv + temp2 - temp1 - temp3;
-    a.p3[idx] = a.scko3 * ux + a.scko3 * vy + temp3 - temp1 - temp2;
-    a.p4[idx] = 4.0 * a.scko3 * wz;
-    a.q[idx] = a.f * by * bx;
-    a.g[idx] = a.f * bz * bx;
-    a.hh[idx] = a.f * bz * by;
+    if (!a.mag) {
+        a.p1[idx] = dv;
+        a.p2[idx] = dv;
+        a.p3[idx] = a.scko3 * dh;
+        a.p4[idx] = (4.0 * a.scko3) * wz;
+        return;
+    }
+    const double bx = a.bx[idx], by = a.by[idx], bz = a.bz[idx];
+    const double fx = a.f * bx, fy = a.f * by;
+    const double m1 = fx * bx, m2 = fy * by, m3 = a.f * bz * bz;
+    a.p1[idx] = dv + 0.5 * (m1 - (m2 + m3));
+    a.p2[idx] = dv + 0.5 * (m2 - (m1 + m3));
+    a.p3[idx] = a.scko3 * dh + 0.5 * (m3 - (m1 + m2));
+    a.p4[idx] = (4.0 * a.scko3) * wz;
+    a.q[idx] = fx * by;
+    a.g[idx] = fx * bz;
+    a.hh[idx] = fy * bz;
 }
 
 struct Hydro4Args {
-    const double *r, *t, *w, *p3, *p4, *g, *hh, *racc, *uacc, *vacc, *wacc;
+    const double *r, *t, *w, *p3, *p4, *g, *hh, *racc, *uacc, *vacc, *wacc, *ri;
     const HistTable *ht;    // rdot, udot, vdot, wdot = newest slots
     double ho12;
+    int mag;                // 0: g, hh are zero (not read)
     size_t np;
     int nz;
 };
 
 // pass 4: :183-184, :272, :321 (z derivatives of second-level inputs),
-// :443-497 (d(rho)/dz with the boundary override, division by rho)
-__global__ void k_hydro_pass4(Hydro4Args a)
+// :443-497 (d(rho)/dz with the boundary override, division by rho).  With the
+// z stencils summed in integers and 1 / rho from pass 2, 11 FP64 operations per
+// point are left of 53: 0.72 -> 0.41 ms at 256^2 x 129.
+__global__ void __launch_bounds__(256) k_hydro_pass4(Hydro4Args a)
 {
     PDL_WAIT();
-    size_t idx = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (idx >= a.np * a.nz) return;
-    const int nz = a.nz;
-    const size_t np = a.np;
-    const int k = (int)(idx / np);
-    const size_t q = idx - (size_t)k * np;
-    const double h = a.ho12;
-    const double w0 = a.w[idx], tt = a.t[idx], rr = a.r[idx];
-    double wd = a.wacc[idx] + zd1(a.p3 + q, np, k, nz, 2, h) + zd1(a.p4 + q, np, k, nz, 5, h);
-    double ud = a.uacc[idx] + zd1(a.g + q, np, k, nz, 5, h);
-    double vd = a.vacc[idx] + zd1(a.hh + q, np, k, nz, 5, h);
-    double rzu, rz;
-    if (k == 0 || k == nz - 1) {
-        rzu = wd / tt;
-        rz = wd / tt;
-    } else {
-        rzu = zd1up(a.r + q, np, k, nz, 0, h, w0);
-        rz = zd1(a.r + q, np, k, nz, 0, h);
+    const size_t np = a.np, q = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (q >= np) return;
+    const int nz = a.nz, k = blockIdx.y;
+    const size_t idx = (size_t)k * np + q;
+    const double h = a.ho12, w0 = a.w[idx], tt = a.t[idx], ri = a.ri[idx];
+    const double d3 = zsum<ZD1 | ZPIPE>(a.p3 + q, np, k, nz, 2, 0).d1, d4 = zsum<ZD1 | ZPIPE>(a.p4 + q, np, k, nz, 5, 0).d1;
+    double wd = a.wacc[idx] + h * (d3 + d4);
+    double ud = a.uacc[idx], vd = a.vacc[idx];
+    if (a.mag) {
+        ud += h * zsum<ZD1 | ZPIPE>(a.g + q, np, k, nz, 5, 0).d1;
+        vd += h * zsum<ZD1 | ZPIPE>(a.hh + q, np, k, nz, 5, 0).d1;
     }
-    ((double *)a.ht->p[0][2])[idx] = a.racc[idx] - w0 * rzu;
-    wd = wd - tt * rz;
-    const double ri = 1.0 / rr;
+    double wr, tr;      // w, T times the upwind and the central d(rho)/dz
+    if (k == 0 || k == nz - 1) {
+        const double rz = wd / tt;
+        wr = w0 * rz;
+        tr = tt * rz;
+    } else {
+        const ZSum z = zsum<ZD1 | ZUP | ZPIPE>(a.r + q, np, k, nz, 0, 0, w0);
+        wr = (h * w0) * z.up;
+        tr = (h * tt) * z.d1;
+    }
+    ((double *)a.ht->p[0][2])[idx] = a.racc[idx] - wr;
     ((double *)a.ht->p[2][2])[idx] = ud * ri;
     ((double *)a.ht->p[3][2])[idx] = vd * ri;
-    ((double *)a.ht->p[4][2])[idx] = wd * ri;
+    ((double *)a.ht->p[4][2])[idx] = (wd - tr) * ri;
 }
 
 int phys_hydro64(Engine *E)
@@ -267,17 +273,18 @@ int phys_hydro64(Engine *E)
     a.vx = W[W_VX]; a.vxx = W[W_VXX]; a.wx = W[W_WX]; a.wxx = W[W_WXX];
     a.ry = W[W_RY]; a.ty = W[W_TY]; a.tyy = W[W_TYY]; a.uy = W[W_UY]; a.uyy = W[W_UYY];
     a.vy = W[W_VY]; a.vyy = W[W_VYY]; a.wy = W[W_WY]; a.wyy = W[W_WYY];
-    a.kappa = E->kappa; a.dkappa = E->dkappa; a.eta = E->eta;
+    a.pc = E->pc64; a.ri = W[W_RX];
     a.racc = W[W_RACC]; a.ht = E->ht;
     a.uacc = W[W_UACC]; a.vacc = W[W_VACC]; a.wacc = W[W_WACC];
     a.p1 = W[W_P1]; a.p2 = W[W_P2]; a.q = W[W_Q]; a.g = W[W_G]; a.hh = W[W_H];
     a.p3 = W[W_P3]; a.p4 = W[W_P4];
     const Consts &c = E->k;
-    a.gck = c.gck; a.fzckg = c.fzckg; a.gm1 = c.gm1; a.sckg = c.sckg; a.fo2 = c.fo2;
+    a.gm1 = c.gm1; a.sckg = c.sckg;
     a.scko3 = c.scko3; a.f = c.f; a.thmplus1 = c.thmplus1; a.cor = c.cor; a.cpsi = c.cpsi;
-    a.spsi = c.spsi; a.sck = c.sck; a.zck = c.zck; a.ho12 = c.ho12; a.sc1 = c.sc1;
-    a.var_eta = c.var_eta; a.np = E->np; a.nz = E->nz;
-    KLAUNCHB(E, "hydro_pass2_f64", FB(E, 39, 8), k_hydro_pass2, nblk(E->n), TPB, a);
+    a.spsi = c.spsi; a.sck = c.sck; a.ho12 = c.ho12; a.sc1 = c.sc1;
+    const int mag = E->p.f != 0.0 || E->p.kinematic;
+    a.mag = mag; a.np = E->np; a.nz = E->nz;
+    KLAUNCHB(E, "hydro_pass2_f64", FB(E, mag ? 40 : 33, 8), k_hydro_pass2, zgrid(E->np, E->nz), TPB, a);
 
     // pass 3: d/dx, d/dy of the second-level inputs into the accumulators
     // (:181-182, :230-231, :273, :320)
@@ -286,20 +293,21 @@ int phys_hydro64(Engine *E)
         ljob<double>(W[W_Q], W[W_VACC], OP_D1, nullptr, OP_NONE, 1),
         ljob<double>(W[W_G], W[W_WACC], OP_D1, nullptr, OP_NONE, 1),
     };
-    if ((st = launch_lines<double>(E, 0, kx, 3))) return st;
+    // (p1; with a magnetic field also q and g)
+    if ((st = launch_lines<double>(E, 0, kx, mag ? 3 : 1))) return st;
     LineJob<double> ky[3] = {
         ljob<double>(W[W_P2], W[W_VACC], OP_D1, nullptr, OP_NONE, 1),
         ljob<double>(W[W_Q], W[W_UACC], OP_D1, nullptr, OP_NONE, 1),
         ljob<double>(W[W_H], W[W_WACC], OP_D1, nullptr, OP_NONE, 1),
     };
-    if ((st = launch_lines<double>(E, 1, ky, 3))) return st;
+    if ((st = launch_lines<double>(E, 1, ky, mag ? 3 : 1))) return st;
 
     Hydro4Args b;
     b.r = E->r; b.t = E->t; b.w = E->w; b.p3 = W[W_P3]; b.p4 = W[W_P4]; b.g = W[W_G]; b.hh = W[W_H];
     b.racc = W[W_RACC]; b.uacc = W[W_UACC]; b.vacc = W[W_VACC]; b.wacc = W[W_WACC];
-    b.ht = E->ht;
-    b.ho12 = c.ho12; b.np = E->np; b.nz = E->nz;
-    KLAUNCHB(E, "hydro_pass4_f64", FB(E, 15, 8), k_hydro_pass4, nblk(E->n), TPB, b);
+    b.ht = E->ht; b.ri = W[W_RX];
+    b.ho12 = c.ho12; b.mag = mag; b.np = E->np; b.nz = E->nz;
+    KLAUNCHB(E, "hydro_pass4_f64", FB(E, mag ? 16 : 14, 8), k_hydro_pass4, zgrid(E->np, E->nz), TPB, b);
     return VEC_OK;
 }
 
@@ -362,21 +370,22 @@ int phys_bandj64(Engine *E)
     if ((st = op_d1z(E, E->pol, W[W_M1], 5, (int)E->np, E->nz))) return st;   // :519
     BandjArgs<double> a;
     a.dzs = W[W_M1]; a.pol = E->pol; a.tor = E->tor; a.h = E->hd;
-    a.bxh = W[W_EX]; a.byh = W[W_EY]; a.bzh = W[W_EZ]; a.dybz = W[W_M2]; a.dxbz = W[W_M3]; a.jzh = W[W_M4];
+    a.bxh = W[W_EX]; a.byh = W[W_EY]; a.bzh = W[W_EZ]; a.dybz = nullptr; a.dxbz = nullptr; a.jzh = W[W_M4];
     a.nx = E->nx; a.ny = E->ny; a.nz = E->nz;
-    KLAUNCHB(E, "bandj_spec_f64", FB(E, 9, 8), k_bandj_spec<double>, plane_grid(*E), TPB, a);
-    // six inverse 2-D transforms (:575-577, :623-625): x pass in place, then y
-    LineJob<double> ix[6] = { ljob<double>(W[W_EX], W[W_EX], OP_INV), ljob<double>(W[W_EY], W[W_EY], OP_INV),
-                              ljob<double>(W[W_EZ], W[W_EZ], OP_INV), ljob<double>(W[W_M2], W[W_M2], OP_INV),
-                              ljob<double>(W[W_M3], W[W_M3], OP_INV), ljob<double>(W[W_M4], W[W_M4], OP_INV) };
-    if ((st = launch_lines<double>(E, 0, ix, 6))) return st;
-    LineJob<double> iy[6] = { ljob<double>(W[W_EX], E->bx, OP_INV), ljob<double>(W[W_EY], E->by, OP_INV),
-                              ljob<double>(W[W_EZ], E->bz, OP_INV), ljob<double>(W[W_M2], W[W_M2], OP_INV),
+    KLAUNCHB(E, "bandj_spec_f64", FB(E, 7, 8), k_bandj_spec<double>, plane_grid(*E), TPB, a);
+    // the inverse 2-D transforms (:575-577, :623-625): x pass in place, then y.  The
+    // x inverse of bz's spectrum also gives that of d(bz)/dx (into M3), the y
+    // inverse of the former bz and d(bz)/dy (into M2): two spectra less to form
+    LineJob<double> ix[4] = { ljob<double>(W[W_EX], W[W_EX], OP_INV), ljob<double>(W[W_EY], W[W_EY], OP_INV),
+                              ljob<double>(W[W_EZ], W[W_EZ], OP_INV, W[W_M3], OP_D1), ljob<double>(W[W_M4], W[W_M4], OP_INV) };
+    if ((st = launch_lines<double>(E, 0, ix, 4))) return st;
+    LineJob<double> iy[5] = { ljob<double>(W[W_EX], E->bx, OP_INV), ljob<double>(W[W_EY], E->by, OP_INV),
+                              ljob<double>(W[W_EZ], E->bz, OP_INV, W[W_M2], OP_D1),
                               ljob<double>(W[W_M3], W[W_M3], OP_INV), ljob<double>(W[W_M4], W[W_M4], OP_INV) };
     iy[0].addk = E->bxbar;       // :587-589
     iy[1].addk = E->bybar;
     iy[2].addc = E->bzbar;
-    if ((st = launch_lines<double>(E, 1, iy, 6))) return st;
+    if ((st = launch_lines<double>(E, 1, iy, 5))) return st;
     KLAUNCHB(E, "jsq_f64", FB(E, 6, 8), k_jsq<double>, plane_grid(*E), TPB, W[W_M4], W[W_M2], W[W_M3], E->bx,
              E->by, E->jsq, E->np, E->nz, E->k.ho12);
     return VEC_OK;
