@@ -215,7 +215,6 @@ int line_kernels_configure();
 // physics.cu: calcdt scratch (floats per context, initialisation of its keys)
 int cdt_chunks(size_t np, int nz);
 int cdt_init(float *cdt);
-int line_ct_configure();
 int line_fx_configure();
 int fx_plan_make(int n, FxPlan *pl);
 int fx_tables_make(int n, FxPlan *pl, const double *k1, const double *k2, int icut, FxTables *tb);
@@ -229,7 +228,7 @@ inline int fx_rounds(const FxPlan &pl, int q)
 }
 int fs_tables_make(int n, const FxPlan &pl, const FxTables &fx, const double *k1, const double *k2, int icut, FsTables *tb);
 void fs_tables_free(FsTables *tb);
-template <typename R> int launch_lines_ct(Engine *E, int dir, const LineJob<R> *jobs, int njobs);
+int launch_lines_ct(Engine *E, int dir, const LineJob<float> *jobs, int njobs);
 
 template <typename R>
 inline LineJob<R> ljob(const R *in, R *out1, int op1, R *out2 = nullptr, int op2 = OP_NONE,

@@ -570,7 +570,7 @@ int launch_lines<float>(Engine *E, int dir, const LineJob<float> *jobs, int njob
 {
     if (njobs <= 0) return VEC_OK;
     if (!E->generic_lines) {
-        const int h = launch_lines_ct<float>(E, dir, jobs, njobs);
+        const int h = launch_lines_ct(E, dir, jobs, njobs);
         if (h == 1) return VEC_OK;
         if (h < 0) return h;
     }
@@ -584,8 +584,8 @@ int launch_lines<float>(Engine *E, int dir, const LineJob<float> *jobs, int njob
 
 int line_kernels_configure()
 {
-    int st = line_ct_configure();
-    if (st || (st = line_fx_configure())) return st;
+    int st = line_fx_configure();
+    if (st) return st;
     CUDA_TRY(cudaFuncSetAttribute(line_kernel<0>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
     CUDA_TRY(cudaFuncSetAttribute(line_kernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
     return VEC_OK;
