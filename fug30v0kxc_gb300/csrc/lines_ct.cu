@@ -47,11 +47,7 @@
 #include "tma.cuh"
 
 // the jobs of one launch, and for y lines one TMA descriptor per input (3-D view
-// nx x ny x nz).  Parameters cost a launch time by their size: with room for MAX_JOBS
-// jobs and descriptors, 24 KB, a derivative pair at 64^2 x 65 took 11.2 us, without
-// the descriptors 9.7, with room for eight jobs 8.7.  So launches of a few jobs (one
-// solver's; a batch of members has more) have kernels of their own.
-#define NJ_SMALL 8
+// nx x ny x nz)
 template <int NJ> struct JobPackCT { LineJob<float> j[NJ]; };
 template <int DIR, int NJ> struct TmapPack { CUtensorMap m[NJ]; };
 template <int NJ> struct TmapPack<0, NJ> {};
@@ -264,13 +260,14 @@ struct CtShape {
     // (the other side reads down the rows); with three both sides read along them
     static constexpr int XS = C > 1 ? M : B + 1;
     static constexpr int GX = A * XS;
-    // twiddle rows: W^(j x) for j = 1, 2, 3, 4, 8, 12, the others are products of two;
-    // 1024 points have all rows of the second exchange (with products in both the
-    // error of a transform against FP64 was 0.6 % larger than with two levels, with
-    // them in one 2.5 % smaller; up to 768 it is smaller either way, and loads in place
-    // of products cost the 512-point launches 2 %)
-    static constexpr bool ALL2 = A > 8;
-    static constexpr int H1 = A / 4 - 1, R1 = 3 + H1, H2 = (B + 3) / 4 - 1, R2 = C == 1 ? 0 : ALL2 ? B - 1 : 3 + H2;
+    // twiddle rows: all, or W^(j x) for j = 1, 2, 3, 4, 8, 12 and the others as products
+    // of two.  Three levels take products where they can: loads in their place cost
+    // the 512-point launches 2 %.  They err more (a transform against FP64 with
+    // products in both exchanges 2.5-3 %): 1024 points have them in one exchange only,
+    // two levels in none, and every length errs less than two levels with products did.
+    static constexpr bool ALL1 = C == 1, ALL2 = A > 8;
+    static constexpr int H1 = A / 4 - 1, R1 = ALL1 ? A - 1 : 3 + H1;
+    static constexpr int H2 = (B + 3) / 4 - 1, R2 = C == 1 ? 0 : ALL2 ? B - 1 : 3 + H2;
     static constexpr size_t SMEM = 4 * (2 * (size_t)TILE + 4 * (size_t)NG * GX + 4 * (size_t)(R1 * M + R2 * C) + 6 * (size_t)N);
     static constexpr int MINB = NT <= 256 && 2 * (SMEM + 1152) <= 233472 ? 2 : 1;
     static_assert(T >= M && (C == 1 || C == 8) && SMEM + 128 <= 232448, "shape");
@@ -317,7 +314,7 @@ line_ct(const __grid_constant__ JobPackCT<NJ> jobs, const __grid_constant__ Tmap
         const bool first = e < P::R1 * M;
         const int q = first ? e : e - P::R1 * M, w = first ? M : C;
         const int r = q / w, x = q - r * w;
-        const int j = (!first && P::ALL2) || r < 3 ? r + 1 : 4 * (r - 2);
+        const int j = (first ? P::ALL1 : P::ALL2) || r < 3 ? r + 1 : 4 * (r - 2);
         const float2 v = tb.tw[(first ? j * x : A * j * x) % N];
         tw1[e] = Tw{ bc2(v.x), bc2(-v.y) };
     }
@@ -440,10 +437,10 @@ line_ct(const __grid_constant__ JobPackCT<NJ> jobs, const __grid_constant__ Tmap
                 for (int m = 0; m < A; m++) a[m] = tile_z(lane + M * m);
                 ZDft<A, false>::run(a);
                 Tw lo[3], hi[P::H1];
-                twrow(tw1, M, lane, P::H1, lo, hi);
+                if constexpr (!P::ALL1) twrow(tw1, M, lane, P::H1, lo, hi);
                 exg[ST * lane] = a[0];
 #pragma unroll
-                for (int k = 1; k < A; k++) exg[ST * (k * XS + lane)] = ztw<false>(a[k], twk(k, lo, hi));
+                for (int k = 1; k < A; k++) exg[ST * (k * XS + lane)] = ztw<false>(a[k], P::ALL1 ? tw1[(k - 1) * M + lane] : twk(k, lo, hi));
             }
             sync();
             if constexpr (L3) {
@@ -580,10 +577,10 @@ line_ct(const __grid_constant__ JobPackCT<NJ> jobs, const __grid_constant__ Tmap
             if (M % T == 0 || lane < M) {
                 Z a[A];
                 Tw lo[3], hi[P::H1];
-                twrow(tw1, M, lane, P::H1, lo, hi);
+                if constexpr (!P::ALL1) twrow(tw1, M, lane, P::H1, lo, hi);
                 a[0] = exg[ST * lane];
 #pragma unroll
-                for (int k = 1; k < A; k++) a[k] = ztw<true>(exg[ST * (k * XS + lane)], twk(k, lo, hi));
+                for (int k = 1; k < A; k++) a[k] = ztw<true>(exg[ST * (k * XS + lane)], P::ALL1 ? tw1[(k - 1) * M + lane] : twk(k, lo, hi));
                 ZDft<A, true>::run(a);
                 const float f = op == OP_INV ? alpha / (float)N : alpha;
                 float addv = 0.0f;
