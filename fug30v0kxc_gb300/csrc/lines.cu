@@ -24,7 +24,7 @@
 #include "common.cuh"
 #include "engine.h"
 
-struct JobPack { LineJob<float> j[MAX_JOBS]; };
+template <int NJ> struct JobPack { LineJob<float> j[NJ]; };
 
 // ---- radix kernels (natural order outputs X_0..X_{R-1}) ----------------------
 template <typename C>
@@ -217,9 +217,9 @@ __device__ __forceinline__ void fs_inv(float2 *buf, const float2 *src, const FsP
 
 // DIR 0: x lines (sequence = two rows), DIR 1: y lines (two columns).  tpp tiles
 // per plane: of Q sequences (one warp's, x) or S = warps Q (a CTA's, y).
-template <int DIR>
+template <int DIR, int NJ>
 __global__ void __launch_bounds__(FS_TPB, 4)
-line_kernel(const __grid_constant__ JobPack jobs, const __grid_constant__ FxPlan pl, FsTables tb, int nx, int ny, int nz,
+line_kernel(const __grid_constant__ JobPack<NJ> jobs, const __grid_constant__ FxPlan pl, FsTables tb, int nx, int ny, int nz,
             int tpp, int total, int two)
 {
     PDL_WAIT();
@@ -522,11 +522,11 @@ void line_tables_free(LineTables<R> *tb)
     memset(tb, 0, sizeof(*tb));
 }
 
-template <int DIR>
+template <int DIR, int NJ>
 static int run_fs(Engine *E, const LineJob<float> *jobs, int nj)
 {
     FxPlan pl = DIR == 0 ? E->fpx : E->fpy;
-    JobPack pk;
+    JobPack<NJ> pk;
     memset(&pk, 0, sizeof(pk));
     double fields = 0.0;
     int two = 0;
@@ -551,14 +551,14 @@ static int run_fs(Engine *E, const LineJob<float> *jobs, int nj)
     while (W > 1 && (smem_of(W) > 75 * 1024 || (DIR == 0 ? tiles_of(W) / W : tiles_of(W)) < E->num_sms)) W >>= 1;
     const size_t smem = smem_of(W);
     int per_sm = 1;
-    CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, line_kernel<DIR>, W * 32, smem));
+    CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, line_kernel<DIR, NJ>, W * 32, smem));
     if (per_sm < 1) per_sm = 1;
     const int S = DIR == 0 ? pl.Q : W * pl.Q, tpp = (pairs + S - 1) / S;
     const long long total = tiles_of(W);
     long long grid = DIR == 0 ? (total + W - 1) / W : total;
     if (grid > (long long)E->num_sms * per_sm) grid = (long long)E->num_sms * per_sm;
     E->prof_begin(DIR == 0 ? "line_x_f32" : "line_y_f32", fields * (double)E->n * sizeof(float));
-    CUDA_TRY(launch_k(*E, line_kernel<DIR>, dim3((unsigned)grid), dim3(W * 32), smem, pk, pl, DIR == 0 ? E->fsx : E->fsy, E->nx,
+    CUDA_TRY(launch_k(*E, line_kernel<DIR, NJ>, dim3((unsigned)grid), dim3(W * 32), smem, pk, pl, DIR == 0 ? E->fsx : E->fsy, E->nx,
                       E->ny, E->nz, tpp, (int)total, two));
     E->prof_end();
     CUDA_TRY(cudaGetLastError());
@@ -576,7 +576,9 @@ int launch_lines<float>(Engine *E, int dir, const LineJob<float> *jobs, int njob
     }
     for (int j0 = 0; j0 < njobs; j0 += MAX_JOBS) {
         const int nj = njobs - j0 < MAX_JOBS ? njobs - j0 : MAX_JOBS;
-        const int st = dir == 0 ? run_fs<0>(E, jobs + j0, nj) : run_fs<1>(E, jobs + j0, nj);
+        const LineJob<float> *j = jobs + j0;
+        const int st = nj <= NJ_SMALL ? (dir == 0 ? run_fs<0, NJ_SMALL>(E, j, nj) : run_fs<1, NJ_SMALL>(E, j, nj))
+                                      : (dir == 0 ? run_fs<0, MAX_JOBS>(E, j, nj) : run_fs<1, MAX_JOBS>(E, j, nj));
         if (st) return st;
     }
     return VEC_OK;
@@ -586,8 +588,10 @@ int line_kernels_configure()
 {
     int st = line_fx_configure();
     if (st) return st;
-    CUDA_TRY(cudaFuncSetAttribute(line_kernel<0>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
-    CUDA_TRY(cudaFuncSetAttribute(line_kernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
+    CUDA_TRY(cudaFuncSetAttribute(line_kernel<0, NJ_SMALL>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
+    CUDA_TRY(cudaFuncSetAttribute(line_kernel<1, NJ_SMALL>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
+    CUDA_TRY(cudaFuncSetAttribute(line_kernel<0, MAX_JOBS>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
+    CUDA_TRY(cudaFuncSetAttribute(line_kernel<1, MAX_JOBS>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
     return VEC_OK;
 }
 

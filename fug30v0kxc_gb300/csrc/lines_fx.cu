@@ -36,7 +36,7 @@
 #include "engine.h"
 #include "fx.cuh"
 
-struct FxPack { LineJob<double> j[MAX_JOBS]; };
+template <int NJ> struct FxPack { LineJob<double> j[NJ]; };
 
 #define FX_TPB 256
 
@@ -254,9 +254,9 @@ struct FxOut { double cx, cy, sc; int xe, bad; };
 
 // DIR 0: x lines (sequence = two rows), DIR 1: y lines (two columns).  tpp
 // tiles per plane: of Q sequences (one warp's, x) or S = warps Q (a CTA's, y).
-template <int DIR>
+template <int DIR, int NJ>
 __global__ void __launch_bounds__(FX_TPB, 3)
-line_fx(const __grid_constant__ FxPack jobs, const __grid_constant__ FxPlan pl, FxTables tb, int nx, int ny, int nz,
+line_fx(const __grid_constant__ FxPack<NJ> jobs, const __grid_constant__ FxPlan pl, FxTables tb, int nx, int ny, int nz,
         int tpp, int total, int two)
 {
     PDL_WAIT();
@@ -860,11 +860,11 @@ void fx_tables_free(FxTables *tb)
     *tb = FxTables{};
 }
 
-template <int DIR>
+template <int DIR, int NJ>
 static int run_fx(Engine *E, const LineJob<double> *jobs, int nj)
 {
     FxPlan pl = DIR == 0 ? E->fpx : E->fpy;
-    FxPack pk;
+    FxPack<NJ> pk;
     memset(&pk, 0, sizeof(pk));
     double fields = 0.0;
     int two = 0;                   // a second buffer per sequence
@@ -896,19 +896,19 @@ static int run_fx(Engine *E, const LineJob<double> *jobs, int nj)
     const size_t smem = smem_of(W);
     static bool attr = false;
     if (!attr) {
-        CUDA_TRY(cudaFuncSetAttribute(line_fx<DIR>, cudaFuncAttributeMaxDynamicSharedMemorySize, 226 * 1024));
+        CUDA_TRY(cudaFuncSetAttribute(line_fx<DIR, NJ>, cudaFuncAttributeMaxDynamicSharedMemorySize, 226 * 1024));
         attr = true;
     }
     if (smem > 226 * 1024) return VEC_ERR_SIZE;
     int per_sm = 1;
-    CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, line_fx<DIR>, W * 32, smem));
+    CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, line_fx<DIR, NJ>, W * 32, smem));
     if (per_sm < 1) per_sm = 1;
     const int S = DIR == 0 ? pl.Q : W * pl.Q, tpp = (pairs + S - 1) / S;
     const long long total = tiles_of(W);
     long long grid = DIR == 0 ? (total + W - 1) / W : total;
     if (grid > (long long)E->num_sms * per_sm) grid = (long long)E->num_sms * per_sm;
     E->prof_begin(DIR == 0 ? "line_x_f64" : "line_y_f64", fields * (double)E->n * 8.0);
-    CUDA_TRY(launch_k(*E, line_fx<DIR>, dim3((unsigned)grid), dim3(W * 32), smem, pk, pl, DIR == 0 ? E->fxx : E->fxy, E->nx,
+    CUDA_TRY(launch_k(*E, line_fx<DIR, NJ>, dim3((unsigned)grid), dim3(W * 32), smem, pk, pl, DIR == 0 ? E->fxx : E->fxy, E->nx,
                       E->ny, E->nz, tpp, (int)total, two));
     E->prof_end();
     CUDA_TRY(cudaGetLastError());
@@ -920,7 +920,9 @@ int launch_lines<double>(Engine *E, int dir, const LineJob<double> *jobs, int nj
 {
     for (int j0 = 0; j0 < njobs; j0 += MAX_JOBS) {
         const int nj = njobs - j0 < MAX_JOBS ? njobs - j0 : MAX_JOBS;
-        const int st = dir == 0 ? run_fx<0>(E, jobs + j0, nj) : run_fx<1>(E, jobs + j0, nj);
+        const LineJob<double> *j = jobs + j0;
+        const int st = nj <= NJ_SMALL ? (dir == 0 ? run_fx<0, NJ_SMALL>(E, j, nj) : run_fx<1, NJ_SMALL>(E, j, nj))
+                                      : (dir == 0 ? run_fx<0, MAX_JOBS>(E, j, nj) : run_fx<1, MAX_JOBS>(E, j, nj));
         if (st) return st;
     }
     return VEC_OK;
