@@ -30,13 +30,33 @@ struct MeanArgs {
     int nz;
     double xn, zck, ho12, sc1;
     int var_eta;
-    // k_mag_div4 only: with ds set, the mean-field CTA goes on with the AB3
-    // coefficient step and the mean update of ab3_coef_block on bxm, bym
-    // (the bxbar, bybar above), which read the history it has just written
+    // k_mag_final4 only: with ds set, the mean-field CTA does the AB3 coefficient
+    // step and the mean update of ab3_coef_block too, on bxm, bym (the bxbar, bybar
+    // above) and the history it has just written
     DevScalars *ds;
     double *bxm, *bym;
 };
 
+// the RHS at plane k from columns of E's means (times xn) and of the mean field
+template <typename R>
+__device__ __forceinline__ void mean_rhs(const MeanArgs<R> &a, const double *e1, const double *e2, const double *bx,
+                                         const double *by, int k, double &xd, double &yd)
+{
+    const int nz = a.nz;
+    double dey = zd1(e2, 1, k, nz, 5, a.ho12);   // :337
+    double dex = zd1(e1, 1, k, nz, 5, a.ho12);   // :338
+    double d2x = zd2(bx, 1, k, nz, 3, a.sc1);    // :343
+    double d2y = zd2(by, 1, k, nz, 3, a.sc1);    // :344
+    if (!a.var_eta) {
+        xd = a.zck * d2x - dey;                  // :350
+        yd = a.zck * d2y + dex;                  // :351
+    } else {
+        // extension: eta(z) d2b/dz2 + eta'(z) db/dz
+        double gx = zd1(bx, 1, k, nz, 5, a.ho12), gy = zd1(by, 1, k, nz, 5, a.ho12);
+        xd = a.eta[k] * d2x - dey + a.deta[k] * gx;
+        yd = a.eta[k] * d2y + dex + a.deta[k] * gy;
+    }
+}
 template <typename R>
 __device__ __forceinline__ void mean_rhs_block(const MeanArgs<R> &a)
 {
@@ -49,19 +69,10 @@ __device__ __forceinline__ void mean_rhs_block(const MeanArgs<R> &a)
     }
     __syncthreads();
     for (int k = threadIdx.x; k < nz; k += blockDim.x) {
-        double dey = zd1(e2, 1, k, nz, 5, a.ho12);   // :337
-        double dex = zd1(e1, 1, k, nz, 5, a.ho12);   // :338
-        double d2x = zd2(a.bxbar, 1, k, nz, 3, a.sc1); // :343
-        double d2y = zd2(a.bybar, 1, k, nz, 3, a.sc1); // :344
-        if (!a.var_eta) {
-            bxd[k] = a.zck * d2x - dey;              // :350
-            byd[k] = a.zck * d2y + dex;              // :351
-        } else {
-            // extension: eta(z) d2b/dz2 + eta'(z) db/dz
-            double gx = zd1(a.bxbar, 1, k, nz, 5, a.ho12), gy = zd1(a.bybar, 1, k, nz, 5, a.ho12);
-            bxd[k] = a.eta[k] * d2x - dey + a.deta[k] * gx;
-            byd[k] = a.eta[k] * d2y + dex + a.deta[k] * gy;
-        }
+        double xd, yd;
+        mean_rhs(a, e1, e2, a.bxbar, a.bybar, k, xd, yd);
+        bxd[k] = xd;
+        byd[k] = yd;
     }
 }
 
@@ -90,24 +101,29 @@ static __global__ void k_mag_div(const R *ex, const R *ey, R *w1, int nx, int ny
     w1[pb + q] = sdx(ex + pb, i, j, nx, h.kx1) + sdy(ey + pb, i, j, nx, ny, h.ky1);
 }
 
-// the AB3 coefficients (src/main.F90:381-403), dt1/dt2 (:488-489), ttime
-// (:345) and the 1-D mean update (:469-476), by one whole CTA
-__device__ __forceinline__ void ab3_coef_block(DevScalars *ds, double *bxbar, double *bybar, const HistTable *ht,
-                                               int nz, int do_means)
+// the 1-D mean update (src/main.F90:469-476) with the coefficients c, by one whole CTA
+__device__ __forceinline__ void ab3_means(const double *cc, double *bxbar, double *bybar, const HistTable *ht, int nz)
 {
     const double *bxd0 = ht->bx[0], *bxd1 = ht->bx[1], *bxd2 = ht->bx[2];
     const double *byd0 = ht->by[0], *byd1 = ht->by[1], *byd2 = ht->by[2];
+    for (int k = threadIdx.x; k < nz; k += blockDim.x) {
+        bxbar[k] = bxbar[k] + cc[0] * bxd2[k] + cc[1] * bxd1[k] + cc[2] * bxd0[k];
+        bybar[k] = bybar[k] + cc[0] * byd2[k] + cc[1] * byd1[k] + cc[2] * byd0[k];
+    }
+}
+
+// the AB3 coefficients (src/main.F90:381-403), dt1/dt2 (:488-489), ttime
+// (:345) and the 1-D mean update, by one whole CTA
+__device__ __forceinline__ void ab3_coef_block(DevScalars *ds, double *bxbar, double *bybar, const HistTable *ht,
+                                               int nz, int do_means)
+{
     __shared__ double cc[3];
     if (threadIdx.x == 0) {
         ab3_coefs(ds, cc);
         ab3_advance(ds, cc);
     }
     __syncthreads();
-    if (!do_means) return;
-    for (int k = threadIdx.x; k < nz; k += blockDim.x) {
-        bxbar[k] = bxbar[k] + cc[0] * bxd2[k] + cc[1] * bxd1[k] + cc[2] * bxd0[k];
-        bybar[k] = bybar[k] + cc[0] * byd2[k] + cc[1] * byd1[k] + cc[2] * byd0[k];
-    }
+    if (do_means) ab3_means(cc, bxbar, bybar, ht, nz);
 }
 
 template <typename R>
@@ -313,17 +329,12 @@ static __global__ void k_emf4(const __grid_constant__ Batch<Emf4Args, NB> bt)
     st4(e3, i, U * BY - Vv * BX);
 }
 
-// (grid (np/4/256, nz + 1): the first CTA of the extra first row computes
-// the mean-field RHS, which reads the same spectra -- one launch instead of
-// two; the row is dispatched first, so that the CTA's serial FP64 work is
-// not the grid's tail.  No plane of this kernel, and none of k_mag_final4
-// that follows it, reads ds, bxbar, bybar or the bx/by histories.)
+// grid (np/4/256, nz)
 struct MagDiv4Args {
     const float *ex, *ey;
     float *w1;
     int nx, ny;
     HTab<float> h;
-    MeanArgs<float> ma;
 };
 template <int NB>
 static __global__ void k_mag_div4(const __grid_constant__ Batch<MagDiv4Args, NB> bt)
@@ -334,37 +345,78 @@ static __global__ void k_mag_div4(const __grid_constant__ Batch<MagDiv4Args, NB>
     float *w1 = A.w1;
     const int nx = A.nx, ny = A.ny;
     const HTab<float> &h = A.h;
-    const MeanArgs<float> &ma = A.ma;
-    if (blockIdx.y == 0) {
-        if (blockIdx.x == 0) {
-            mean_rhs_block(ma);
-            if (ma.ds) {
-                __syncthreads();   // the new history is written, bxbar and bybar are read
-                ab3_coef_block(ma.ds, ma.bxm, ma.bym, ma.ht, ma.nz, 1);
-            }
-        }
-        return;
-    }
     const unsigned np4 = (unsigned)nx * ny / 4;
     const unsigned q4 = blockIdx.x * blockDim.x + threadIdx.x;
     if (q4 >= np4) return;
-    const size_t pb = (size_t)(blockIdx.y - 1) * np4 * 4;
+    const size_t pb = (size_t)blockIdx.y * np4 * 4;
     const unsigned q = 4 * q4;
     const int j = (int)(q / (unsigned)nx), i0 = (int)(q - (unsigned)j * nx);
     st4(w1 + pb, q4, sdx4(ex + pb, i0, j, nx, h.kx1) + sdy4(ey + pb, i0, j, nx, ny, h.ky1));
 }
 
+// The mean-field RHS and, with ds set, the AB3 coefficients, the scalars' advance and
+// the means' update: one CTA, whose time is a chain of loads and FP64 latencies.  Its
+// last thread does the coefficients' divisions meanwhile, and where a thread has at
+// most one plane all it reads is asked for at the start.
+static __device__ __noinline__ void mean_block(const MeanArgs<float> &a)
+{
+    __shared__ double cc[3];
+    __shared__ double col[4][256];
+    const int nz = a.nz, k = threadIdx.x;
+    const bool one = nz <= 256 && nz <= blockDim.x;
+    double b0x = 0.0, b0y = 0.0, b1x = 0.0, b1y = 0.0;
+    double *xd = a.ht->bx[2], *yd = a.ht->by[2];
+    if (one && k < nz) {
+        const double *x0 = a.ht->bx[0], *x1 = a.ht->bx[1], *y0 = a.ht->by[0], *y1 = a.ht->by[1];
+        const float ex = a.ex[(size_t)k * a.np], ey = a.ey[(size_t)k * a.np];
+        const double bx = a.bxbar[k], by = a.bybar[k];
+        if (a.ds) { b0x = x0[k]; b1x = x1[k]; b0y = y0[k]; b1y = y1[k]; }
+        col[0][k] = a.xn * (double)ex; col[1][k] = a.xn * (double)ey; col[2][k] = bx; col[3][k] = by;
+    }
+    if (a.ds && threadIdx.x == blockDim.x - 1) {
+        ab3_coefs(a.ds, cc);
+        ab3_advance(a.ds, cc);
+    }
+    if (!one) {
+        mean_rhs_block(a);
+        if (!a.ds) return;
+        __syncthreads();   // cc is written, bxbar and bybar are read
+        ab3_means(cc, a.bxm, a.bym, a.ht, nz);
+        return;
+    }
+    __syncthreads();
+    if (k >= nz) return;
+    double x, y;
+    mean_rhs(a, col[0], col[1], col[2], col[3], k, x, y);
+    xd[k] = x;
+    yd[k] = y;
+    if (!a.ds) return;
+    a.bxm[k] = col[2][k] + cc[0] * x + cc[1] * b1x + cc[2] * b0x;
+    a.bym[k] = col[3][k] + cc[0] * y + cc[1] * b1y + cc[2] * b0y;
+}
+
+// grid (np/4/256, nz + 1): the first CTA of the extra first row is mean_block's, which
+// reads the same spectra; no plane of this kernel reads ds, bxbar, bybar or the bx/by
+// histories.  The row is dispatched first and this is the longest of the spectral
+// kernels, so that the CTA's serial work hides (in k_mag_div4, and with
+// the coefficients after the means, it was that grid's tail: the two launches of
+// 64^2 x 65 16.2 + 8.5 us, now 6.1 + 12.3; of 256^2 x 129 25.0 + 74, now 19.0 + 75).
 // (four CTAs per SM: 3.4 TB/s against 2.1 at the compiler's own 90 registers
 // and 3.0 at three CTAs per SM with 80 registers and no spills)
+struct MagFinal4Args { MagArgs<float> m; MeanArgs<float> ma; };
 template <int NB>
-static __global__ void __launch_bounds__(256, 4) k_mag_final4(const __grid_constant__ Batch<MagArgs<float>, NB> bt)
+static __global__ void __launch_bounds__(256, 4) k_mag_final4(const __grid_constant__ Batch<MagFinal4Args, NB> bt)
 {
     PDL_WAIT();
-    const MagArgs<float> &a = BATCH_MEMBER(bt, NB);
+    if (blockIdx.y == 0) {
+        if (blockIdx.x == 0) mean_block(BATCH_MEMBER(bt, NB).ma);
+        return;
+    }
+    const MagArgs<float> &a = BATCH_MEMBER(bt, NB).m;
     const unsigned np = (unsigned)a.nx * a.ny, np4 = np / 4;
     const unsigned q4 = blockIdx.x * blockDim.x + threadIdx.x;
     if (q4 >= np4) return;
-    const int k = blockIdx.y;
+    const int k = (int)blockIdx.y - 1;
     const size_t pb = (size_t)k * np, i4 = (size_t)k * np4 + q4;
     const unsigned q = 4 * q4;
     const int j = (int)(q / (unsigned)a.nx), i0 = (int)(q - (unsigned)j * a.nx);

@@ -1167,15 +1167,16 @@ int split_mag_m(Engine *const *Es, int nE, bool ab3_coef, bool spectra_done)
         if ((st = launch_lines<float>(E, 1, fy.data(), 3 * nE))) return st;
     }
     if (v4) {
-        if ((st = launch_members<MagDiv4Args>(Es, nE, "mag_div_f32", FB(E, 3, 4), dim3(g4.x, g4.y + 1), dim3(TPB), 0,
-                                              k_mag_div4<1>, k_mag_div4<BATCH_MAX>, [ab3_coef](Engine *e) {
+        if ((st = launch_members<MagDiv4Args>(Es, nE, "mag_div_f32", FB(E, 3, 4), g4, dim3(TPB), 0, k_mag_div4<1>,
+                                              k_mag_div4<BATCH_MAX>, [](Engine *e) {
                                                   return MagDiv4Args{ e->W<float>(W_EX), e->W<float>(W_EY),
-                                                                      e->W<float>(W_M4), e->nx, e->ny, e->hf,
-                                                                      mean_args(e, ab3_coef) };
+                                                                      e->W<float>(W_M4), e->nx, e->ny, e->hf };
                                               })))
             return st;
-        return launch_members<MagArgs<float>>(Es, nE, "mag_final_f32", FB(E, 8, 4), g4, dim3(TPB), 0,
-                                              k_mag_final4<1>, k_mag_final4<BATCH_MAX>, mag_args);
+        return launch_members<MagFinal4Args>(Es, nE, "mag_final_f32", FB(E, 8, 4), dim3(g4.x, g4.y + 1), dim3(TPB), 0,
+                                             k_mag_final4<1>, k_mag_final4<BATCH_MAX>, [ab3_coef](Engine *e) {
+                                                 return MagFinal4Args{ mag_args(e), mean_args(e, ab3_coef) };
+                                             });
     }
     const MeanArgs<float> ma = mean_args(E, ab3_coef);
     KLAUNCHB(E, "mean_rhs", 0, k_mean_rhs<float>, 1, 256, ma);
