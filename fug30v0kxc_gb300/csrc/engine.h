@@ -228,7 +228,9 @@ inline int fx_rounds(const FxPlan &pl, int q)
 }
 int fs_tables_make(int n, const FxPlan &pl, const FxTables &fx, const double *k1, const double *k2, int icut, FsTables *tb);
 void fs_tables_free(FsTables *tb);
+int line_ct_configure();
 int launch_lines_ct(Engine *E, int dir, const LineJob<float> *jobs, int njobs);
+int launch_lines_cp(Engine *E, int dir, const LineJob<float> *jobs, int nj, int S, const char *name);   // lines_cp.cu
 
 template <typename R>
 inline LineJob<R> ljob(const R *in, R *out1, int op1, R *out2 = nullptr, int op2 = OP_NONE,

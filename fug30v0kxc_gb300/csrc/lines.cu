@@ -586,8 +586,8 @@ int launch_lines<float>(Engine *E, int dir, const LineJob<float> *jobs, int njob
 
 int line_kernels_configure()
 {
-    int st = line_fx_configure();
-    if (st) return st;
+    int st = line_ct_configure();
+    if (st || (st = line_fx_configure())) return st;
     CUDA_TRY(cudaFuncSetAttribute(line_kernel<0, NJ_SMALL>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
     CUDA_TRY(cudaFuncSetAttribute(line_kernel<1, NJ_SMALL>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
     CUDA_TRY(cudaFuncSetAttribute(line_kernel<0, MAX_JOBS>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));

@@ -1,40 +1,23 @@
 // lines_ct.cu -- horizontal spectral operators (src/fft.F90) in FP32 for line
-// lengths n = 2^a or 3*2^a (64..1024), the hot path of the split step.
+// lengths n = N1*N2 = 2^a or 3*2^a (64..256), the hot path of the split step
+// (384..1024 points: lines_cp.cu).
 //
-// Per tile a CTA owns 2S real lines of one z-plane.  The tile is brought into
-// shared memory by TMA bulk copies (cp.async.bulk + mbarrier): one copy per four
-// contiguous x rows, or a 2S-wide box of y columns.  CTAs are persistent over
-// tiles and the next tile is prefetched into the second buffer while the current
-// one is transformed.
+// Per tile a CTA owns 2S real lines of one z-plane (S complex sequences
+// z = a + ib).  The tile is brought into shared memory by TMA bulk copies
+// (cp.async.bulk + mbarrier): one copy for 2S contiguous x rows, or one
+// 2S-wide copy per row for y columns.  CTAs are persistent over tiles and the
+// next tile is prefetched into the second buffer while the current one is
+// transformed.
 //
-// Each length-n FFT is held in registers, in two levels n = A B (64 to 256 points)
-// or three n = A B C (384 to 1024): with m = BC m1 + C b + c and k = k1 + A k2 +
-// AB k3, thread m' = C b + c does an A-point DFT over m1 and applies W_n^(m' k1);
-// thread (k1, c) a B-point DFT over b and W_BC^(c k2); thread (k1, k2) a C-point DFT
-// over c.  The spectral operator (k, -k^2, 2/3 truncation, all Hermitian-symmetric
-// multipliers) is a product in registers, and the inverse runs the same levels
-// backwards, so that every thread writes to an exchange what it read from it and one
-// barrier per exchange is enough.
-//
-// A group of threads transforms two complex sequences together, of four adjacent
-// lines l + i (l+2) and (l+1) + i (l+3): a point is a pair of real parts and a pair
-// of imaginary parts (Z), every butterfly is an FP32x2 instruction on a pair (a sign
-// is an operand modifier and free), an exchange moves 16 bytes per point and a y
-// line's store as many.  Instructions bound the kernel, not memory: one sequence per
-// group in scalar FP32 took 150 per complex point and 65 % of the issue slots for a
-// derivative pair at 256^2 x 129, and pairs halve the arithmetic, the exchanges and
-// the stores at once.  Three levels of 8 keep all 64 threads of a 512-point line
-// busy with 32 registers per spectrum; two levels of 32 x 16 left half of them idle
-// on the first.  One sequence per group with sums on (re, im) pairs, twice the
-// threads: 512^2 y lines 17 % slower; groups of eight y columns with barriers of
-// their own: 32-byte rows, 8-30 % slower; 256 = 8 x 4 x 8: 3-8 % slower.  Nothing may
-// spill: what shared memory leaves of L1 does not hold it (28 bytes a thread: 512^2 y
-// lines 12-20 % slower).  A derivative pair, x and y, before -> now (us, two runs of
-// one side differ by 3 %):
-//     64^2 x 65    12.0 10.4 ->  9.2  8.2      384^2 x 65    53.1  48.9 ->  44.5  41.0
-//    128^2 x 65    14.6 12.3 -> 10.7 10.3      512^2 x 65    92.6  67.4 ->  61.0  61.9
-//    192^2 x 129   26.5 25.4 -> 23.0 22.0      768^2 x 33   104.1 100.0 ->  76.2  83.1
-//    256^2 x 129   34.4 34.4 -> 31.7 31.5     1024^2 x 33   153.3 140.2 -> 120.0 133.1
+// Each length-n FFT is a two-level four-step decomposition held in
+// registers: n = N1*N2, m = N2*m1 + m2, k = k1 + N1*k2.  Thread m2 does an
+// N1-point DFT over m1 (itself a four-step of radix-2/4/8 kernels), applies
+// the twiddle W_n^(m2 k1) and hands its results to thread k1 through one
+// padded, bank-conflict-free shared-memory exchange; thread k1 then does the
+// N2-point DFT over m2 and holds X[k1 + N1 k2] for all k2.  The spectral
+// operator (+ik, -k^2, 2/3 truncation, all Hermitian-symmetric multipliers)
+// is applied in registers and the inverse runs the same two levels in the
+// opposite order, so each transform costs one exchange.
 #include <math.h>
 #include <stdint.h>
 #include <string.h>
@@ -46,282 +29,211 @@
 #include "engine.h"
 #include "tma.cuh"
 
-// the jobs of one launch, and for y lines one TMA descriptor per input (3-D view
-// nx x ny x nz)
-template <int NJ> struct JobPackCT { LineJob<float> j[NJ]; };
+template <typename R, int NJ> struct JobPackCT { LineJob<R> j[NJ]; };
+// y lines: one TMA descriptor per job input (3-D view nx x ny x nz)
 template <int DIR, int NJ> struct TmapPack { CUtensorMap m[NJ]; };
 template <int NJ> struct TmapPack<0, NJ> {};
 
-// ---- arithmetic on points ------------------------------------------------------------
-// a point of two sequences: their real parts and their imaginary parts
-struct __align__(16) Z { float2 r, i; };
+// W_32^q = exp(-2 pi i q/32), q = 0..31, and W_96^q (the in-register radix
+// kernels; radix-3 factors take their twiddles from the second table)
+__constant__ float2 c_tw32f[32];
+__constant__ float2 c_tw96f[96];
 
-__device__ __forceinline__ float2 bc2(float v) { return make_float2(v, v); }
-__device__ __forceinline__ float2 add2(float2 a, float2 b) { return __fadd2_rn(a, b); }
-// (the sign is an operand modifier: no instruction)
-__device__ __forceinline__ float2 neg2(float2 a) { return make_float2(-a.x, -a.y); }
-__device__ __forceinline__ float2 sub2(float2 a, float2 b) { return __fadd2_rn(a, neg2(b)); }
-// q quarter turns (-i)^q, or i^q in the inverse
-template <bool INV> __host__ __device__ constexpr int turns(int q) { return INV ? (4 - (q & 3)) & 3 : q & 3; }
-// a + (-i)^q b
-template <bool INV, int Q> __device__ __forceinline__ Z zadd(const Z &a, const Z &b)
-{
-    constexpr int q = turns<INV>(Q);
-    if constexpr (q == 0) return Z{ add2(a.r, b.r), add2(a.i, b.i) };
-    else if constexpr (q == 1) return Z{ add2(a.r, b.i), sub2(a.i, b.r) };
-    else if constexpr (q == 2) return Z{ sub2(a.r, b.r), sub2(a.i, b.i) };
-    else return Z{ sub2(a.r, b.i), add2(a.i, b.r) };
-}
-// a + h (-i)^q b, h real
-template <bool INV, int Q> __device__ __forceinline__ Z zfma(const Z &a, const Z &b, float h)
-{
-    constexpr int q = turns<INV>(Q);
-    const float2 p = bc2(h), n = neg2(p);
-    if constexpr (q == 0) return Z{ __ffma2_rn(b.r, p, a.r), __ffma2_rn(b.i, p, a.i) };
-    else if constexpr (q == 1) return Z{ __ffma2_rn(b.i, p, a.r), __ffma2_rn(b.r, n, a.i) };
-    else if constexpr (q == 2) return Z{ __ffma2_rn(b.r, n, a.r), __ffma2_rn(b.i, n, a.i) };
-    else return Z{ __ffma2_rn(b.i, n, a.r), __ffma2_rn(b.r, p, a.i) };
-}
-// sqrt(2) W_8 b: the factor is left to the sum that takes it
-template <bool INV> __device__ __forceinline__ Z zw8(const Z &b)
-{
-    if constexpr (INV) return Z{ sub2(b.r, b.i), add2(b.r, b.i) };
-    else return Z{ add2(b.r, b.i), sub2(b.i, b.r) };
-}
-// (c - i s) b, (c + i s) b in the inverse
-template <bool INV> __device__ __forceinline__ Z ztw(const Z &b, float c, float s)
-{
-    const float2 t = INV ? neg2(bc2(s)) : bc2(s);
-    return Z{ __ffma2_rn(b.i, t, __fmul2_rn(b.r, bc2(c))), __ffma2_rn(b.r, neg2(t), __fmul2_rn(b.i, bc2(c))) };
-}
-// the same with a factor from a table, both elements of each pair alike
-struct __align__(16) Tw { float2 c, s; };
-template <bool INV> __device__ __forceinline__ Z ztw(const Z &b, const Tw &w)
-{
-    const float2 n = neg2(w.s);
-    if constexpr (INV) return Z{ __ffma2_rn(b.i, n, __fmul2_rn(b.r, w.c)), __ffma2_rn(b.r, w.s, __fmul2_rn(b.i, w.c)) };
-    else return Z{ __ffma2_rn(b.i, w.s, __fmul2_rn(b.r, w.c)), __ffma2_rn(b.r, n, __fmul2_rn(b.i, w.c)) };
-}
-__device__ __forceinline__ Tw twmul(const Tw &a, const Tw &b)
-{
-    return Tw{ __ffma2_rn(neg2(a.s), b.s, __fmul2_rn(a.c, b.c)), __ffma2_rn(a.s, b.c, __fmul2_rn(a.c, b.s)) };
-}
+template <typename C> __device__ __forceinline__ C tw32(int q);
+template <> __device__ __forceinline__ float2 tw32<float2>(int q) { return c_tw32f[q]; }
+template <typename C> __device__ __forceinline__ C tw96(int q);
+template <> __device__ __forceinline__ float2 tw96<float2>(int q) { return c_tw96f[q]; }
 
-// f v, f v + o, v + c, i v
-__device__ __forceinline__ Z zscale(const Z &v, float f) { return Z{ __fmul2_rn(v.r, bc2(f)), __fmul2_rn(v.i, bc2(f)) }; }
-__device__ __forceinline__ Z zscale(const Z &v, float2 f) { return Z{ __fmul2_rn(v.r, f), __fmul2_rn(v.i, f) }; }
-__device__ __forceinline__ Z zaxpy(float f, const Z &v, const Z &o)
-{
-    return Z{ __ffma2_rn(v.r, bc2(f), o.r), __ffma2_rn(v.i, bc2(f), o.i) };
-}
-__device__ __forceinline__ Z zaddc(const Z &v, float c) { return Z{ add2(v.r, bc2(c)), add2(v.i, bc2(c)) }; }
-__device__ __forceinline__ Z zi(const Z &v) { return Z{ neg2(v.i), v.r }; }
+// x mod N for x >= 0 (N a compile-time constant)
+template <int N> __device__ __forceinline__ int modn(int x) { return (N & (N - 1)) == 0 ? (x & (N - 1)) : x % N; }
 
-// ---- DFTs in registers, natural order ------------------------------------------------
-// DFT of four points of which v2 is (-i)^Q2 times what is given, v1 and v3 (-i)^Q1
-// and (-i)^Q3; h2, h13: real factors still to be applied to v2 and to v1, v3
-template <bool INV, int Q1, int Q2, int Q3, bool H2, bool H13>
-__device__ __forceinline__ void dft4(const Z &v0, const Z &v1, const Z &v2, const Z &v3, float h, Z &o0, Z &o1, Z &o2, Z &o3)
+template <typename C>
+__device__ __forceinline__ C cmul_(C a, C b) { C r; r.x = a.x * b.x - a.y * b.y; r.y = a.x * b.y + a.y * b.x; return r; }
+template <typename C>
+__device__ __forceinline__ C cadd_(C a, C b) { C r; r.x = a.x + b.x; r.y = a.y + b.y; return r; }
+template <typename C>
+__device__ __forceinline__ C csub_(C a, C b) { C r; r.x = a.x - b.x; r.y = a.y - b.y; return r; }
+template <bool INV, typename C>
+__device__ __forceinline__ C rot_(C a) { C r; if (INV) { r.x = -a.y; r.y = a.x; } else { r.x = a.y; r.y = -a.x; } return r; }
+
+// multiply by W_N^e (e compile-time after unrolling); conjugate for INV
+template <int N, bool INV, typename C>
+__device__ __forceinline__ C twc(C a, int e)
 {
-    Z a0, a1;
-    if constexpr (H2) { a0 = zfma<INV, Q2>(v0, v2, h); a1 = zfma<INV, Q2 + 2>(v0, v2, h); }
-    else { a0 = zadd<INV, Q2>(v0, v2); a1 = zadd<INV, Q2 + 2>(v0, v2); }
-    const Z b0 = zadd<INV, Q3 - Q1 + 4>(v1, v3), b1 = zadd<INV, Q3 - Q1 + 6>(v1, v3);
-    if constexpr (H13) {
-        o0 = zfma<INV, Q1>(a0, b0, h); o2 = zfma<INV, Q1 + 2>(a0, b0, h);
-        o1 = zfma<INV, Q1 + 1>(a1, b1, h); o3 = zfma<INV, Q1 + 3>(a1, b1, h);
+    if constexpr (32 % N == 0) {
+        const int q = (e * (32 / N)) & 31;
+        if (q == 0) return a;
+        if (q == 8) return rot_<INV>(a);                           // -i (fwd)
+        if (q == 16) { C r; r.x = -a.x; r.y = -a.y; return r; }
+        if (q == 24) return rot_<!INV>(a);                         // +i (fwd)
+        C w = tw32<C>(q);
+        if (INV) w.y = -w.y;
+        return cmul_(a, w);
     } else {
-        o0 = zadd<INV, Q1>(a0, b0); o2 = zadd<INV, Q1 + 2>(a0, b0);
-        o1 = zadd<INV, Q1 + 1>(a1, b1); o3 = zadd<INV, Q1 + 3>(a1, b1);
+        static_assert(96 % N == 0, "radix kernels cover divisors of 32 and 96");
+        const int q = (e * (96 / N)) % 96;
+        if (q == 0) return a;
+        if (q == 24) return rot_<INV>(a);
+        if (q == 48) { C r; r.x = -a.x; r.y = -a.y; return r; }
+        if (q == 72) return rot_<!INV>(a);
+        C w = tw96<C>(q);
+        if (INV) w.y = -w.y;
+        return cmul_(a, w);
     }
 }
-template <bool INV> __device__ __forceinline__ void dft4(Z &a, Z &b, Z &c, Z &d)
-{
-    Z o0, o1, o2, o3;
-    dft4<INV, 0, 0, 0, false, false>(a, b, c, d, 1.0f, o0, o1, o2, o3);
-    a = o0; b = o1; c = o2; d = o3;
-}
-template <bool INV> __device__ __forceinline__ void dft3(Z &a, Z &b, Z &c)
-{
-    const float h = 0.8660254037844386f;
-    const Z t = zadd<INV, 0>(b, c), d = zadd<INV, 2>(b, c);
-    const Z u = zfma<INV, 2>(a, t, 0.5f);
-    a = zadd<INV, 0>(a, t);
-    b = zfma<INV, 1>(u, d, h);
-    c = zfma<INV, 3>(u, d, h);
-}
-template <int N, bool INV> struct ZDft;
-template <bool INV> struct ZDft<4, INV> { static __device__ __forceinline__ void run(Z *v) { dft4<INV>(v[0], v[1], v[2], v[3]); } };
-template <bool INV> struct ZDft<8, INV> {
-    static __device__ __forceinline__ void run(Z *v)
-    {
-        const float h = 0.7071067811865476f;
-        dft4<INV>(v[0], v[2], v[4], v[6]);
-        dft4<INV>(v[1], v[3], v[5], v[7]);
-        const Z e0 = v[0], e1 = v[2], e2 = v[4], e3 = v[6], o0 = v[1], o2 = v[5];
-        const Z o1 = zw8<INV>(v[3]), o3 = zw8<INV>(v[7]);
-        v[0] = zadd<INV, 0>(e0, o0); v[4] = zadd<INV, 2>(e0, o0);
-        v[1] = zfma<INV, 0>(e1, o1, h); v[5] = zfma<INV, 2>(e1, o1, h);
-        v[2] = zadd<INV, 1>(e2, o2); v[6] = zadd<INV, 3>(e2, o2);
-        v[3] = zfma<INV, 1>(e3, o3, h); v[7] = zfma<INV, 3>(e3, o3, h);
-    }
-};
-template <bool INV> struct ZDft<16, INV> {
-    static __device__ __forceinline__ void run(Z *v)
-    {
-        const float h = 0.7071067811865476f, c = 0.9238795325112867f, s = 0.3826834323650898f;   // W_8, W_16
-#pragma unroll
-        for (int m = 0; m < 4; m++) dft4<INV>(v[m], v[4 + m], v[8 + m], v[12 + m]);
-        // v[4 k1 + m2] now
-        Z o[16];
-        dft4<INV, 0, 0, 0, false, false>(v[0], v[1], v[2], v[3], h, o[0], o[4], o[8], o[12]);
-        dft4<INV, 0, 0, 0, true, false>(v[4], ztw<INV>(v[5], c, s), zw8<INV>(v[6]), ztw<INV>(v[7], s, c), h, o[1], o[5], o[9], o[13]);
-        dft4<INV, 0, 1, 1, false, true>(v[8], zw8<INV>(v[9]), v[10], zw8<INV>(v[11]), h, o[2], o[6], o[10], o[14]);
-        dft4<INV, 0, 1, 2, true, false>(v[12], ztw<INV>(v[13], s, c), zw8<INV>(v[14]), ztw<INV>(v[15], c, s), h, o[3], o[7], o[11], o[15]);
-#pragma unroll
-        for (int k = 0; k < 16; k++) v[k] = o[k];
-    }
-};
-// 6 = 2 x 3 and 12 = 3 x 4 by the map of coprime factors (no twiddles)
-template <bool INV> struct ZDft<6, INV> {
-    static __device__ __forceinline__ void run(Z *v)
-    {
-        Z a[3], b[3];
-#pragma unroll
-        for (int n2 = 0; n2 < 3; n2++) {
-            const Z x = v[(2 * n2) % 6], y = v[(3 + 2 * n2) % 6];
-            a[n2] = zadd<INV, 0>(x, y);
-            b[n2] = zadd<INV, 2>(x, y);
-        }
-        dft3<INV>(a[0], a[1], a[2]);
-        dft3<INV>(b[0], b[1], b[2]);
-#pragma unroll
-        for (int k2 = 0; k2 < 3; k2++) { v[(4 * k2) % 6] = a[k2]; v[(3 + 4 * k2) % 6] = b[k2]; }
-    }
-};
-template <bool INV> struct ZDft<12, INV> {
-    static __device__ __forceinline__ void run(Z *v)
-    {
-        Z a[12];
-#pragma unroll
-        for (int n1 = 0; n1 < 3; n1++) {
-            Z *t = a + 4 * n1;
-#pragma unroll
-            for (int n2 = 0; n2 < 4; n2++) t[n2] = v[(4 * n1 + 3 * n2) % 12];
-            dft4<INV>(t[0], t[1], t[2], t[3]);
-        }
-#pragma unroll
-        for (int k2 = 0; k2 < 4; k2++) {
-            dft3<INV>(a[k2], a[4 + k2], a[8 + k2]);
-#pragma unroll
-            for (int k1 = 0; k1 < 3; k1++) v[(4 * k1 + 9 * k2) % 12] = a[4 * k1 + k2];
-        }
-    }
-};
 
-// ---- TMA helpers (tma.cuh) and the 3-D tiled load of the y tiles -------------------
-// 3-D tiled TMA load of one box (c0 innermost) into shared memory
-__device__ __forceinline__ void tma_load_3d(void *dst, const CUtensorMap *map, int c0, int c1, int c2, uint64_t *bar)
-{
-    asm volatile("cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4}], [%5];"
-                 ::"r"(smem_u32(dst)), "l"(map), "r"(c0), "r"(c1), "r"(c2), "r"(smem_u32(bar)) : "memory");
-}
-// this thread's writes to shared memory before later copies into it
-__device__ __forceinline__ void fence_async() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
-// rows per TMA box of a y tile: TMA boxes are at most 256 rows, and the box
-// must divide the line length
-__host__ __device__ constexpr int ybox_rows(int n) { return n <= 256 ? n : (n % 256 == 0 ? 256 : n / 2); }
-
-// ---- shape ---------------------------------------------------------------------------
-// DIR 0: x lines (a tile = 2S contiguous rows), DIR 1: y lines (a tile = 2S adjacent
-// columns over all ny rows).  C = 1: two levels.
-template <int DIR, int A, int B, int C, int S>
-struct CtShape {
-    static constexpr int cmax(int a, int b) { return a > b ? a : b; }
-    static constexpr int N = A * B * C;
-    static constexpr int NG = S / 2;                      // groups of four lines
-    static constexpr int RL = C > 1 ? C : B;              // radix of the last level
-    static constexpr int M = N / A, NL = N / RL;          // DFTs of the first and the last level
-    // threads per group: one DFT each on the first level (128 = 16 x 8: 8 threads,
-    // two DFTs of 8; 384: 64 rather than 48, whole warps)
-    static constexpr int T = C > 1 ? (DIR == 0 ? (M + 31) / 32 * 32 : M) : (N == 128 ? 8 : cmax(A, B));
-    static constexpr int NT = NG * T;
-    // groups side by side, lane by lane: all of a y tile (what a warp stores is then as
-    // wide as the tile)
-    static constexpr int ST = DIR == 0 ? 1 : NG, U = ST * T;
-    // barriers per unit where units are whole warps or divide one
-    static constexpr bool LOCAL = DIR == 0 && NT % 32 == 0 && (32 % U == 0 || U % 32 == 0);
-    static constexpr int D2 = C > 1 ? (A * C + T - 1) / T : 1, DL = (NL + T - 1) / T;
-    // reals of a group in the tile; x tiles: groups of T < 32 threads share a warp
-    // and a padding of T reals keeps their rows on different banks
-    static constexpr int GT = 4 * N + (DIR == 0 && T < 32 ? T : 0);
-    static constexpr int TILE = NG * GT;
-    // exchange rows of the first level, in points: an odd stride with two levels
-    // (the other side reads down the rows); with three both sides read along them
-    static constexpr int XS = C > 1 ? M : B + 1;
-    static constexpr int GX = A * XS;
-    // twiddle rows: all, or W^(j x) for j = 1, 2, 3, 4, 8, 12 and the others as products
-    // of two.  Three levels take products where they can: loads in their place cost
-    // the 512-point launches 2 %.  They err more (a transform against FP64 with
-    // products in both exchanges 2.5-3 %): 1024 points have them in one exchange only,
-    // two levels in none, and every length errs less than two levels with products did.
-    static constexpr bool ALL1 = C == 1, ALL2 = A > 8;
-    static constexpr int H1 = A / 4 - 1, R1 = ALL1 ? A - 1 : 3 + H1;
-    static constexpr int H2 = (B + 3) / 4 - 1, R2 = C == 1 ? 0 : ALL2 ? B - 1 : 3 + H2;
-    static constexpr size_t SMEM = 4 * (2 * (size_t)TILE + 4 * (size_t)NG * GX + 4 * (size_t)(R1 * M + R2 * C) + 6 * (size_t)N);
-    static constexpr int MINB = NT <= 256 && 2 * (SMEM + 1152) <= 233472 ? 2 : 1;
-    static_assert(T >= M && (C == 1 || C == 8) && SMEM + 128 <= 232448, "shape");
-    static_assert(GX >= N, "spectra fit the exchange");
+// in-register natural-order DFT of N points
+template <int N, bool INV> struct RDft;
+template <bool INV> struct RDft<1, INV> { template <typename C> static __device__ __forceinline__ void run(C *) {} };
+template <bool INV> struct RDft<2, INV> {
+    template <typename C> static __device__ __forceinline__ void run(C *v) { C a = v[0], b = v[1]; v[0] = cadd_(a, b); v[1] = csub_(a, b); }
 };
+// X1,2 = a - (b+c)/2 -+ i (sqrt(3)/2)(b-c) (forward; conjugate for INV)
+template <bool INV> struct RDft<3, INV> {
+    template <typename C> static __device__ __forceinline__ void run(C *v) {
+        using R = decltype(v[0].x);
+        const R h = (R)0.8660254037844386;
+        C t1 = cadd_(v[1], v[2]), d = csub_(v[1], v[2]);
+        C t2; t2.x = v[0].x - (R)0.5 * t1.x; t2.y = v[0].y - (R)0.5 * t1.y;
+        C r = rot_<INV>(d);
+        r.x *= h; r.y *= h;
+        v[0] = cadd_(v[0], t1);
+        v[1] = cadd_(t2, r);
+        v[2] = csub_(t2, r);
+    }
+};
+template <bool INV> struct RDft<4, INV> {
+    template <typename C> static __device__ __forceinline__ void run(C *v) {
+        C a0 = cadd_(v[0], v[2]), a1 = csub_(v[0], v[2]);
+        C b0 = cadd_(v[1], v[3]), b1 = rot_<INV>(csub_(v[1], v[3]));
+        v[0] = cadd_(a0, b0); v[1] = cadd_(a1, b1); v[2] = csub_(a0, b0); v[3] = csub_(a1, b1);
+    }
+};
+// four-step in registers: N = A*B, m = B*m1 + m2, k = k1 + A*k2
+template <int A, int B, bool INV, typename C>
+__device__ __forceinline__ void reg_ct(C *v)
+{
+    constexpr int N = A * B;
+    C t[N];
+#pragma unroll
+    for (int m2 = 0; m2 < B; m2++) {
+        C a[A];
+#pragma unroll
+        for (int m1 = 0; m1 < A; m1++) a[m1] = v[B * m1 + m2];
+        RDft<A, INV>::run(a);
+#pragma unroll
+        for (int k1 = 0; k1 < A; k1++) t[m2 * A + k1] = twc<N, INV>(a[k1], m2 * k1);
+    }
+#pragma unroll
+    for (int k1 = 0; k1 < A; k1++) {
+        C b[B];
+#pragma unroll
+        for (int m2 = 0; m2 < B; m2++) b[m2] = t[m2 * A + k1];
+        RDft<B, INV>::run(b);
+#pragma unroll
+        for (int k2 = 0; k2 < B; k2++) v[k1 + A * k2] = b[k2];
+    }
+}
+template <bool INV> struct RDft<8, INV> { template <typename C> static __device__ __forceinline__ void run(C *v) { reg_ct<2, 4, INV>(v); } };
+template <bool INV> struct RDft<16, INV> { template <typename C> static __device__ __forceinline__ void run(C *v) { reg_ct<4, 4, INV>(v); } };
+template <bool INV> struct RDft<12, INV> { template <typename C> static __device__ __forceinline__ void run(C *v) { reg_ct<4, 3, INV>(v); } };
 
 // ---- the kernel --------------------------------------------------------------------
-// wsync: x lines' groups sit in one warp or are whole warps, so the exchanges need
-// only warp or named barriers (0: CTA-wide ones).  The groups then run through their tiles
-// independently; an "empty" mbarrier per tile buffer (one arrival per warp once it
-// is done with the buffer) tells the thread that issues the TMA copies when a
-// buffer may be refilled.
-template <int DIR, int A, int B, int C, int S, int NJ>
-__global__ void __launch_bounds__(CtShape<DIR, A, B, C, S>::NT, CtShape<DIR, A, B, C, S>::MINB)
-line_ct(const __grid_constant__ JobPackCT<NJ> jobs, const __grid_constant__ TmapPack<DIR, NJ> tmaps, LineTables<float> tb,
-        int nx, int ny, int nz, int tpp, int total, int wsync, int *err)
+// DIR 0: x lines (a tile = 2S contiguous rows), DIR 1: y lines (a tile = 2S
+// adjacent columns over all ny rows).
+//
+// WS (x lines with NP dividing 32): the NP threads of a sequence sit in one
+// warp, so the exchanges need only warp barriers.  The warps then run
+// through their tiles independently; an "empty" mbarrier per tile buffer
+// (one arrival per warp once it has read the tile) tells the thread that
+// issues the TMA copies when a buffer may be refilled.
+// Per-sequence stride of the exchange rows, in complex elements.  The
+// forward exchange holds N1 rows of N2 + 1, the inverse one N2 rows of
+// N1 + 1, the spectra's separation N + N/32 padded elements: the stride
+// covers the largest.  A shared-memory wavefront serves U = 128 /
+// sizeof(complex) consecutive elements.  x lines: the threads of a
+// half-warp belong to one or two sequences, and a
+// stride of 1 mod 16 keeps them on distinct banks.  y lines: thread tid is
+// lane tid / S of sequence tid % S, so a wavefront's threads are G = U / S
+// lanes of U / G sequences; a stride of G mod U puts them on distinct banks
+// (exchange element sidx * stride + lane * 1 or lane * (odd row) + const).
+template <typename R, int DIR, int N1, int N2, int S>
+__host__ __device__ constexpr int ct_lds()
+{
+    constexpr int U = 128 / (2 * (int)sizeof(R));
+    constexpr int G = U / S > 1 ? U / S : 1;
+    constexpr int MF = N1 * (N2 + 1), MI = N2 * (N1 + 1), MS = N1 * N2 + (N1 * N2) / 32 + 1;
+    constexpr int M = MF > MI ? (MF > MS ? MF : MS) : (MI > MS ? MI : MS);
+    return DIR == 0 ? ((M + 15) / 16) * 16 + 1 : ((M + U - 1) / U) * U + G;
+}
+
+// dynamic shared memory of one CTA: two tile buffers, the exchange rows,
+// the twiddle table(s) and the three multiplier tables
+template <typename R, int DIR, int N1, int N2, int S>
+__host__ __device__ constexpr size_t ct_smem_bytes()
+{
+    constexpr int N = N1 * N2;
+    constexpr int LDS = ct_lds<R, DIR, N1, N2, S>();
+    return 2 * (size_t)(2 * S * N) * sizeof(R) + ((size_t)S * LDS + 2 * (size_t)N) * 2 * sizeof(R)
+           + 3 * (size_t)N * sizeof(R);
+}
+// two CTAs per SM where their shared memory fits (227 KB per SM), else one
+// CTA with the whole register file
+template <typename R, int DIR, int N1, int N2, int S>
+__host__ __device__ constexpr int ct_min_blocks()
+{
+    return (S * (N1 > N2 ? N1 : N2) <= 256 && 2 * ct_smem_bytes<R, DIR, N1, N2, S>() <= 232448) ? 2 : 1;
+}
+
+template <typename R, int DIR, int N1, int N2, int S, bool WSYNC, int NJ>
+__global__ void __launch_bounds__(S * (N1 > N2 ? N1 : N2), (ct_min_blocks<R, DIR, N1, N2, S>()))
+line_ct(const __grid_constant__ JobPackCT<R, NJ> jobs, const __grid_constant__ TmapPack<DIR, NJ> tmaps, LineTables<R> tb, int nx, int ny, int nz,
+        int tpp, int total, int *err)
 {
     PDL_WAIT();
-    using P = CtShape<DIR, A, B, C, S>;
-    constexpr int N = P::N, T = P::T, NT = P::NT, M = P::M, NL = P::NL, RL = P::RL, XS = P::XS, TILE = P::TILE;
-    constexpr bool L3 = C > 1;
-    const bool WS = P::LOCAL && wsync;
+    using C = typename CT<R>::T;
+    constexpr int N = N1 * N2;
+    constexpr int NP = N1 > N2 ? N1 : N2;
+    constexpr int NT = S * NP;
+    constexpr int TILE = 2 * S * N;                   // reals per tile
+    constexpr int LXF = N2 + 1;                       // padded exchange rows: forward,
+    constexpr int LXI = N1 + 1;                       // inverse
+    constexpr int LDS = ct_lds<R, DIR, N1, N2, S>();  // per-sequence exchange stride
+    constexpr bool WS = WSYNC && DIR == 0 && (32 % NP == 0) && NT % 32 == 0;
 
     extern __shared__ __align__(128) unsigned char smem[];
-    float *tile0 = reinterpret_cast<float *>(smem);
-    Z *ex = reinterpret_cast<Z *>(tile0 + 2 * TILE);
-    Tw *tw1 = reinterpret_cast<Tw *>(ex + P::NG * P::GX);   // [row][m']
-    Tw *tw2 = tw1 + P::R1 * M;                                 // [row][c]
-    float2 *mul = reinterpret_cast<float2 *>(tw2 + P::R2 * C);  // multipliers: d1, d2, dealias
-    __shared__ __align__(8) uint64_t bar[4];                   // full[2], empty[2]
+    R *tile0 = reinterpret_cast<R *>(smem);
+    R *tile1 = tile0 + TILE;
+    C *ex = reinterpret_cast<C *>(tile1 + TILE);
+    // twiddles W_N^(m2 k1) as two N1 x N2 tables, one row per value of
+    // the loop index, so that the 16 threads of a sequence read consecutive
+    // entries (indexed by (m2 k1) mod N, a thread stride of k1 made up to
+    // eight-way bank conflicts)
+    static_assert(N1 % 4 == 0 && N2 % 4 == 0, "twiddles factor the index as 4 a + b");
+    C *twf = ex + (size_t)S * LDS;                    // twf[k1 N2 + m2]
+    C *twi = twf + N;                                 // twi[m2 N1 + k1]
+    R *sm1 = reinterpret_cast<R *>(twi + N);   // spectral multipliers
+    R *sm2 = sm1 + N;
+    R *smda = sm2 + N;
+    __shared__ __align__(8) uint64_t bar[4];          // full[2], empty[2]
 
     const int tid = threadIdx.x;
-    constexpr int ST = P::ST, U = P::U;
-    const int unit = tid / U, side = tid % ST;
-    const int g = unit * ST + side, lane = (tid % U) / ST;
+    const int sidx = DIR == 0 ? tid / NP : tid % S;
+    const int lane = DIR == 0 ? tid % NP : tid / S;
     const size_t np = (size_t)nx * ny;
     auto sync = [&]() {
-        if (!P::LOCAL || !wsync) __syncthreads();
-        else if constexpr (U <= 32) __syncwarp();
-        else asm volatile("bar.sync %0, %1;" ::"r"(unit + 1), "n"(U) : "memory");
+        if constexpr (WS) __syncwarp();
+        else __syncthreads();
     };
 
-    for (int e = tid; e < P::R1 * M + P::R2 * C; e += NT) {
-        const bool first = e < P::R1 * M;
-        const int q = first ? e : e - P::R1 * M, w = first ? M : C;
-        const int r = q / w, x = q - r * w;
-        const int j = (first ? P::ALL1 : P::ALL2) || r < 3 ? r + 1 : 4 * (r - 2);
-        const float2 v = tb.tw[(first ? j * x : A * j * x) % N];
-        tw1[e] = Tw{ bc2(v.x), bc2(-v.y) };
-    }
     for (int e = tid; e < N; e += NT) {
-        mul[e] = bc2(tb.m1[e]);
-        mul[N + e] = bc2(tb.m2[e]);
-        mul[2 * N + e] = bc2(tb.mda[e]);
+        const int k1 = e / N2, m2 = e - k1 * N2;
+        twf[e] = tb.tw[modn<N>(m2 * k1)];
+        const int m2i = e / N1, k1i = e - m2i * N1;
+        twi[e] = tb.tw[modn<N>(m2i * k1i)];
+        sm1[e] = tb.m1[e];
+        sm2[e] = tb.m2[e];
+        smda[e] = tb.mda[e];
     }
     if (tid == 0) {
         mbar_init(&bar[0], 1);
@@ -329,194 +241,177 @@ line_ct(const __grid_constant__ JobPackCT<NJ> jobs, const __grid_constant__ Tmap
         mbar_init(&bar[2], NT / 32);
         mbar_init(&bar[3], NT / 32);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-        fence_async();
+        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     }
     __syncthreads();
 
-    // (thread 0)
-    auto issue = [&](int t, int buf) {
+    auto issue = [&](int t, R *dst, uint64_t *b) {
         const int job = t / (nz * tpp);
         const int rem = t - job * (nz * tpp);
         const int plane = rem / tpp;
         const int l0 = (rem - plane * tpp) * 2 * S;
-        float *dst = tile0 + buf * TILE;
-        mbar_expect_tx(&bar[buf], 2 * S * N * 4);
         if constexpr (DIR == 0) {
-            const float *src = jobs.j[job].in + (size_t)plane * np + (size_t)l0 * nx;
+            const R *src = jobs.j[job].in + (size_t)plane * np;
+            if (tid == 0) {
+                mbar_expect_tx(b, TILE * (unsigned)sizeof(R));
+                tma_load(dst, src + (size_t)l0 * nx, TILE * (unsigned)sizeof(R), b);
+            }
+        } else if constexpr (DIR == 1) {
+            if (tid == 0) {
+                // boxes of 2S columns x (up to 256) rows of this plane
+                constexpr int BR = ybox_rows(N);
+                mbar_expect_tx(b, TILE * (unsigned)sizeof(R));
 #pragma unroll
-            for (int c = 0; c < P::NG; c++) tma_load(dst + c * P::GT, src + (size_t)c * 4 * N, 16 * N, &bar[buf]);
-        } else {
-            // boxes of 2S columns x (up to 256) rows
-            constexpr int BR = ybox_rows(N);
-#pragma unroll
-            for (int c = 0; c < N / BR; c++)
-                tma_load_3d(dst + (size_t)c * BR * 2 * S, &tmaps.m[job], l0, c * BR, plane, &bar[buf]);
-        }
-    };
-    // A wait that runs out is reported and taken as done; this thread then issues
-    // no more copies and waits for no more of them but those in flight
-    bool bad = false;
-    auto wait = [&](int b, int parity) {
-        if (!mbar_wait(&bar[b], parity, bad ? 1 : MBAR_POLLS)) {
-            atomicExch(err, 1);
-            bad = true;
-        }
-    };
-
-    Z *exg = ex + unit * ST * P::GX + side;
-    // twiddle rows of column x; the factor of index k
-    auto twrow = [](const Tw *tab, int w, int x, int nhi, Tw *lo, Tw *hi) {
-#pragma unroll
-        for (int j = 0; j < 3; j++) lo[j] = tab[j * w + x];
-#pragma unroll
-        for (int j = 0; j < nhi; j++) hi[j] = tab[(3 + j) * w + x];
-    };
-    auto twk = [](int k, const Tw *lo, const Tw *hi) {
-        return (k >> 2) == 0 ? lo[(k & 3) - 1] : ((k & 3) == 0 ? hi[(k >> 2) - 1] : twmul(hi[(k >> 2) - 1], lo[(k & 3) - 1]));
-    };
-    // places of the second exchange, which uses the tile's buffer
-    auto x2 = [](int k1, int k2, int c) { return (k2 * A + k1) * 8 + (c ^ (k1 & 7)); };
-
-    int issued = 0;
-    if (tid == 0) {
-        if (blockIdx.x < total) { issue(blockIdx.x, 0); issued = 1; }
-    }
-    int it = 0;
-    for (int t = blockIdx.x; t < total; t += gridDim.x, it++) {
-        float *cur = tile0 + (it & 1) * TILE;
-        if (tid == 0 && t + (int)gridDim.x < total && !bad) {
-            // every warp is done with the other buffer (its use in iteration it - 1)
-            if (WS && it >= 1) wait(2 + ((it + 1) & 1), ((it - 1) >> 1) & 1);
-            if (!bad) {
-                fence_async();
-                issue(t + gridDim.x, (it + 1) & 1);
-                issued++;
+                for (int c = 0; c < N / BR; c++)
+                    tma_load_3d(dst + (size_t)c * BR * 2 * S, &tmaps.m[job], l0, c * BR, plane, b);
             }
         }
-        wait(it & 1, (it >> 1) & 1);
+    };
+
+    if (blockIdx.x < total) issue(blockIdx.x, tile0, &bar[0]);
+    int it = 0;
+    for (int t = blockIdx.x; t < total; t += gridDim.x, it++) {
+        R *cur = (it & 1) ? tile1 : tile0;
+        R *nxt = (it & 1) ? tile0 : tile1;
+        bool issued_next = false;
+        if (t + (int)gridDim.x < total) {
+            if (WS && it >= 1 && tid == 0) {
+                // every warp has read buffer nxt (its use in iteration it - 1)
+                if (!mbar_wait(&bar[2 + ((it + 1) & 1)], ((it - 1) >> 1) & 1)) {
+                    // report, then let this tile's copy (still in flight)
+                    // land before the CTA's shared memory is released
+                    atomicExch(err, 1);
+                    mbar_wait(&bar[it & 1], (it >> 1) & 1);
+                    return;
+                }
+            }
+            if (tid == 0) asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+            issue(t + gridDim.x, nxt, &bar[(it + 1) & 1]);
+            issued_next = true;
+        }
+        if (!mbar_wait(&bar[it & 1], (it >> 1) & 1)) {
+            if (tid == 0) {
+                // report, then wait (bounded) for the copies this CTA issued
+                atomicExch(err, 1);
+                mbar_wait(&bar[it & 1], (it >> 1) & 1);
+                if (issued_next) mbar_wait(&bar[(it + 1) & 1], ((it + 1) >> 1) & 1);
+            }
+            return;
+        }
         const int job = t / (nz * tpp);
         const int rem = t - job * (nz * tpp);
         const int plane = rem / tpp;
-        const int la = (rem - plane * tpp) * 2 * S + 4 * g;   // the group's first line
-        const size_t base = (size_t)plane * np + (DIR == 0 ? (size_t)la * N : (size_t)la);
-        const LineJob<float> &jb = jobs.j[job];
+        const int l0 = (rem - plane * tpp) * 2 * S;
+        const LineJob<R> &jb = jobs.j[job];
+        const size_t pbase = (size_t)plane * np;
         const int op1 = jb.op1, op2 = jb.op2;
-        Z *xg = reinterpret_cast<Z *>(cur) + unit * ST * (P::GT / 4) + side;
+        C *ex_s = ex + (size_t)sidx * LDS;
 
-        // element e of the group's lines in the tile; its place in a field
-        auto tile_z = [&](int e) -> Z {
-            if constexpr (DIR == 0) {
-                const float *r = cur + g * P::GT + e;
-                return Z{ make_float2(r[0], r[N]), make_float2(r[2 * N], r[3 * N]) };
-            } else {
-                return xg[ST * e];
-            }
-        };
-        auto load = [&](const float *f, int e) -> Z {
-            if constexpr (DIR == 0) {
-                const float *r = f + base + e;
-                return Z{ make_float2(r[0], r[N]), make_float2(r[2 * N], r[3 * N]) };
-            } else {
-                return *reinterpret_cast<const Z *>(f + base + (unsigned)(e * nx));
-            }
-        };
-        auto store = [&](float *f, int e, const Z &v) {
-            if constexpr (DIR == 0) {
-                float *r = f + base + e;
-                r[0] = v.r.x; r[N] = v.r.y; r[2 * N] = v.i.x; r[3 * N] = v.i.y;
-            } else {
-                *reinterpret_cast<Z *>(f + base + (unsigned)(e * nx)) = v;
-            }
+        // element e of sequence sidx in the tile
+        auto tile_z = [&](int e) -> C {
+            C z;
+            if (DIR == 0) { z.x = cur[(2 * sidx) * N + e]; z.y = cur[(2 * sidx + 1) * N + e]; }
+            else { z = reinterpret_cast<const C *>(cur)[(size_t)e * S + sidx]; }
+            return z;
         };
 
-        Z X[P::DL][RL];   // X[d][k3] = spectrum at lane + T d + NL k3
+        // The two sequences a warp holds (x lines, 16 threads each) have rows
+        // that start on the same bank; the odd one reads its columns in pairs
+        // swapped (index ^ 1), so that the two half-warps hit different banks,
+        // and swaps the registers back.  The values are the same.
+        constexpr bool XSW = WS && DIR == 0 && NP == 16 && N1 % 2 == 0 && N2 % 2 == 0;
+        const int sw = XSW ? (sidx & 1) : 0;
+        auto unswap = [&](C *v, int n) {
+            if constexpr (XSW) {
+#pragma unroll
+                for (int i = 0; i < n; i += 2) {
+                    const C t0 = v[i], t1 = v[i + 1];
+                    v[i] = sw ? t1 : t0;
+                    v[i + 1] = sw ? t0 : t1;
+                }
+            }
+        };
+
+        C X[N2];   // thread lane = k1 holds X[k1 + N1 k2], k2 = 0..N2-1
         if (op1 != OP_INV) {
-            if (M % T == 0 || lane < M) {
-                Z a[A];
+            // forward, first level: thread m2 = lane, N1-point DFT over m1
+            if (lane < N2) {
+                C a[N1];
 #pragma unroll
-                for (int m = 0; m < A; m++) a[m] = tile_z(lane + M * m);
-                ZDft<A, false>::run(a);
-                Tw lo[3], hi[P::H1];
-                if constexpr (!P::ALL1) twrow(tw1, M, lane, P::H1, lo, hi);
-                exg[ST * lane] = a[0];
+                for (int m1 = 0; m1 < N1; m1++) a[m1] = tile_z(N2 * (m1 ^ sw) + lane);
+                unswap(a, N1);
+                RDft<N1, false>::run(a);
+                // W^(lane k1) = W^(lane 4 (k1 / 4)) W^(lane (k1 % 4)): 3 + N1/4 - 1
+                // table reads instead of N1 - 1, one product more per twiddle
+                C lo[4], hi[N1 / 4];
 #pragma unroll
-                for (int k = 1; k < A; k++) exg[ST * (k * XS + lane)] = ztw<false>(a[k], P::ALL1 ? tw1[(k - 1) * M + lane] : twk(k, lo, hi));
+                for (int j = 1; j < 4; j++) lo[j] = twf[j * N2 + lane];
+#pragma unroll
+                for (int j = 1; j < N1 / 4; j++) hi[j] = twf[4 * j * N2 + lane];
+#pragma unroll
+                for (int k1 = 0; k1 < N1; k1++) {
+                    const int ja = k1 >> 2, jb = k1 & 3;
+                    const C w = ja == 0 ? lo[jb] : (jb == 0 ? hi[ja] : cmul_(hi[ja], lo[jb]));
+                    ex_s[k1 * LXF + lane] = k1 == 0 ? a[k1] : cmul_(a[k1], w);
+                }
             }
             sync();
-            if constexpr (L3) {
+            // second level: thread k1 = lane, N2-point DFT over m2
+            if (lane < N1) {
 #pragma unroll
-                for (int d = 0; d < P::D2; d++) {
-                    const int q = lane + T * d, k1 = q / C, c = q % C;
-                    if ((A * C) % T == 0 || q < A * C) {
-                        Z b[B];
-#pragma unroll
-                        for (int m = 0; m < B; m++) b[m] = exg[ST * (k1 * XS + C * m + c)];
-                        ZDft<B, false>::run(b);
-                        Tw lo[3], hi[P::H2 + 1];
-                        if constexpr (!P::ALL2) twrow(tw2, C, c, P::H2, lo, hi);
-                        xg[ST * x2(k1, 0, c)] = b[0];
-#pragma unroll
-                        for (int k = 1; k < B; k++) xg[ST * x2(k1, k, c)] = ztw<false>(b[k], P::ALL2 ? tw2[(k - 1) * C + c] : twk(k, lo, hi));
-                    }
-                }
-                sync();
+                for (int m2 = 0; m2 < N2; m2++) X[m2] = ex_s[lane * LXF + m2];
+                RDft<N2, false>::run(X);
             }
-#pragma unroll
-            for (int d = 0; d < P::DL; d++) {
-                const int q = lane + T * d;
-                if (NL % T == 0 || q < NL) {
-#pragma unroll
-                    for (int m = 0; m < RL; m++) X[d][m] = L3 ? xg[ST * x2(q % A, q / A, m)] : exg[ST * (q * XS + m)];
-                    ZDft<RL, false>::run(X[d]);
-                }
-            }
-        } else {
+            sync();
+        } else if (lane < N1) {
             // halfcomplex input lines a (re) and b (im): Z_k = A_k + i B_k
 #pragma unroll
-            for (int d = 0; d < P::DL; d++) {
-                const int q = lane + T * d;
-                if (NL % T == 0 || q < NL) {
-#pragma unroll
-                    for (int m = 0; m < RL; m++) {
-                        const int k = q + NL * m;
-                        const int kk = k <= N / 2 ? k : N - k;
-                        const bool edge = kk == 0 || 2 * kk == N;
-                        const Z pa = tile_z(kk), pb = tile_z(edge ? kk : N - kk);   // (ha, hb)
-                        X[d][m] = edge ? pa : zaxpy(k <= N / 2 ? 1.0f : -1.0f, zi(pb), pa);
-                    }
-                }
+            for (int k2 = 0; k2 < N2; k2++) {
+                const int k = lane + N1 * (k2 ^ sw);
+                const int kk = k <= N / 2 ? k : N - k;
+                const bool edge = kk == 0 || 2 * kk == N;
+                C pa = tile_z(kk);                     // (ha[kk], hb[kk])
+                C pb = edge ? C{0, 0} : tile_z(N - kk); // (ha[n-kk], hb[n-kk])
+                R ar = pa.x, br = pa.y, ai = k <= N / 2 ? pb.x : -pb.x, bi = k <= N / 2 ? pb.y : -pb.y;
+                X[k2].x = ar - bi;
+                X[k2].y = ai + br;
             }
-            // (the exchanges' last readers, and the tile's)
-            sync();
+            unswap(X, N2);
+        }
+        if constexpr (WS) {
+            // this warp is done with the tile buffer
+            __syncwarp();
+            if ((tid & 31) == 0) mbar_arrive(&bar[2 + (it & 1)]);
         }
 
-        // (two levels: the tile has been read)
-        if (WS && !L3 && op1 != OP_FWD && (tid & 31) == 0) mbar_arrive(&bar[2 + (it & 1)]);
         if (op1 == OP_FWD) {
-            // separate Z into the halfcomplex spectra of the two real lines, through
-            // whichever of the tile and the exchange no thread reads any more
-            Z *zg = L3 ? exg : xg;
+            // separate Z into the halfcomplex spectra of the two real lines
+            if (lane < N1) {
 #pragma unroll
-            for (int d = 0; d < P::DL; d++) {
-                const int q = lane + T * d;
-                if (NL % T == 0 || q < NL) {
-#pragma unroll
-                    for (int m = 0; m < RL; m++) zg[ST * (q + NL * m)] = X[d][m];
+                for (int k2 = 0; k2 < N2; k2++) ex_s[lane + N1 * k2 + ((lane + N1 * k2) >> 5)] = X[k2];
+            }
+            sync();
+            for (int p = lane; p < N; p += NP) {
+                const int q = p == 0 ? 0 : N - p;
+                C zp = ex_s[p + (p >> 5)], zq = ex_s[q + (q >> 5)];
+                R va, vb;
+                if (2 * p <= N) { va = (R)0.5 * (zp.x + zq.x); vb = (R)0.5 * (zp.y + zq.y); }
+                else { va = (R)0.5 * (zq.y - zp.y); vb = (R)0.5 * (zp.x - zq.x); }
+                const int la = l0 + 2 * sidx;
+                const R ra = jb.alpha1 * va, rb = jb.alpha1 * vb;
+                if (DIR == 0) {
+                    R *oa = jb.out1 + pbase + (size_t)la * nx + p, *ob = oa + nx;
+                    *oa = jb.acc1 ? *oa + ra : ra;
+                    *ob = jb.acc1 ? *ob + rb : rb;
+                } else {
+                    // the two lines are adjacent columns: one vector store
+                    C *o = reinterpret_cast<C *>(jb.out1 + pbase + (size_t)p * nx + la);
+                    C v = { ra, rb };
+                    if (jb.acc1) { const C q = *o; v.x += q.x; v.y += q.y; }
+                    *o = v;
                 }
             }
             sync();
-            const float f = 0.5f * jb.alpha1;
-#pragma unroll 4
-            for (int p = lane; p < N; p += T) {
-                const int q = p == 0 ? 0 : N - p;
-                const Z zp = zg[ST * p], zq = zg[ST * q];
-                Z v = 2 * p <= N ? zscale(zadd<false, 0>(zp, zq), f) : zscale(zi(zadd<false, 2>(zp, zq)), f);
-                if (jb.acc1) v = zadd<false, 0>(load(jb.out1, p), v);
-                store(jb.out1, p, v);
-            }
-            fence_async();
-            sync();
-            if (WS && (tid & 31) == 0) mbar_arrive(&bar[2 + (it & 1)]);
             continue;
         }
 
@@ -524,93 +419,70 @@ line_ct(const __grid_constant__ JobPackCT<NJ> jobs, const __grid_constant__ Tmap
         // halfcomplex input takes a second output only for OP_D1: the
         // derivative of its inverse)
         const int nout = (op2 != OP_NONE && (op1 != OP_INV || op2 == OP_D1)) ? 2 : 1;
-#pragma unroll 1
         for (int o = 0; o < nout; o++) {
             const int op = o == 0 ? op1 : op2;
-            float *out = o == 0 ? jb.out1 : jb.out2;
-            const float alpha = o == 0 ? jb.alpha1 : jb.alpha2;
+            R *out = o == 0 ? jb.out1 : jb.out2;
+            const R alpha = o == 0 ? jb.alpha1 : jb.alpha2;
             const int acc = o == 0 ? jb.acc1 : jb.acc2;
-            const float2 *mt = mul + (op == OP_D1 ? 0 : op == OP_D2 ? N : 2 * N);
-            if (!L3 && o == 1) sync();   // the first output's readers of the exchange
+            if (lane < N1) {
+                C Y[N2];
 #pragma unroll
-            for (int d = 0; d < P::DL; d++) {
-                const int q = lane + T * d;
-                if (NL % T == 0 || q < NL) {
-                    Z y[RL];
+                for (int k2 = 0; k2 < N2; k2++) {
+                    const int k = lane + N1 * k2;
+                    C z = X[k2], y;
+                    if (op == OP_D1) { R m = sm1[k]; y.x = -m * z.y; y.y = m * z.x; }
+                    else if (op == OP_INV) { y = z; }
+                    else { R m = op == OP_D2 ? sm2[k] : smda[k]; y.x = m * z.x; y.y = m * z.y; }
+                    Y[k2] = y;
+                }
+                // inverse, first level: thread k1 = lane, N2-point DFT over k2
+                RDft<N2, true>::run(Y);
+                // (the same factorisation of W^(m2 lane), m2 = 4 (m2 / 4) + m2 % 4)
+                C lo[4], hi[N2 / 4];
 #pragma unroll
-                    for (int m = 0; m < RL; m++) y[m] = X[d][m];
-                    if (op != OP_INV) {
+                for (int j = 1; j < 4; j++) lo[j] = twi[j * N1 + lane];
 #pragma unroll
-                        for (int m = 0; m < RL; m++) {
-                            y[m] = zscale(y[m], mt[q + NL * m]);
-                        }
-                    }
-                    ZDft<RL, true>::run(y);
+                for (int j = 1; j < N2 / 4; j++) hi[j] = twi[4 * j * N1 + lane];
 #pragma unroll
-                    for (int m = 0; m < RL; m++) {
-                        if constexpr (L3) xg[ST * x2(q % A, q / A, m)] = y[m];
-                        else exg[ST * (q * XS + m)] = y[m];
+                for (int m2 = 0; m2 < N2; m2++) {
+                    const int ja = m2 >> 2, jb = m2 & 3;
+                    C w = ja == 0 ? lo[jb] : (jb == 0 ? hi[ja] : cmul_(hi[ja], lo[jb]));
+                    w.y = -w.y;
+                    ex_s[m2 * LXI + lane] = m2 == 0 ? Y[m2] : cmul_(Y[m2], w);
+                }
+            }
+            sync();
+            // second level: thread m2 = lane, N1-point DFT over k1
+            if (lane < N2) {
+                C a[N1];
+#pragma unroll
+                for (int k1 = 0; k1 < N1; k1++) a[k1] = ex_s[lane * LXI + k1];
+                RDft<N1, true>::run(a);
+                const R sc = op == OP_INV ? (R)1 / (R)N : (R)1;
+                const int la = l0 + 2 * sidx;
+                R addv = (R)0;
+                if (op == OP_INV && jb.addk) addv = (R)jb.addk[plane];
+                if (op == OP_INV) addv = addv + (R)jb.addc;
+#pragma unroll
+                for (int m1 = 0; m1 < N1; m1++) {
+                    const int e = lane + N2 * m1;
+                    R va = alpha * (a[m1].x * sc), vb = alpha * (a[m1].y * sc);
+                    if (DIR == 0) {
+                        R *oa = out + pbase + (size_t)la * nx + e, *ob = oa + nx;
+                        if (acc) { va = *oa + va; vb = *ob + vb; }
+                        if (op == OP_INV) { va = va + addv; vb = vb + addv; }
+                        *oa = va;
+                        *ob = vb;
+                    } else {
+                        C *o = reinterpret_cast<C *>(out + pbase + (size_t)e * nx + la);
+                        if (acc) { const C q = *o; va = q.x + va; vb = q.y + vb; }
+                        if (op == OP_INV) { va = va + addv; vb = vb + addv; }
+                        *o = C{ va, vb };
                     }
                 }
             }
             sync();
-            if constexpr (L3) {
-#pragma unroll
-                for (int d = 0; d < P::D2; d++) {
-                    const int q = lane + T * d, k1 = q / C, c = q % C;
-                    if ((A * C) % T == 0 || q < A * C) {
-                        Z b[B];
-                        Tw lo[3], hi[P::H2 + 1];
-                        if constexpr (!P::ALL2) twrow(tw2, C, c, P::H2, lo, hi);
-                        b[0] = xg[ST * x2(k1, 0, c)];
-#pragma unroll
-                        for (int k = 1; k < B; k++) b[k] = ztw<true>(xg[ST * x2(k1, k, c)], P::ALL2 ? tw2[(k - 1) * C + c] : twk(k, lo, hi));
-                        ZDft<B, true>::run(b);
-#pragma unroll
-                        for (int m = 0; m < B; m++) exg[ST * (k1 * XS + C * m + c)] = b[m];
-                    }
-                }
-                fence_async();
-                sync();
-            }
-            if (WS && L3 && o == nout - 1 && (tid & 31) == 0) mbar_arrive(&bar[2 + (it & 1)]);
-            if (M % T == 0 || lane < M) {
-                Z a[A];
-                Tw lo[3], hi[P::H1];
-                if constexpr (!P::ALL1) twrow(tw1, M, lane, P::H1, lo, hi);
-                a[0] = exg[ST * lane];
-#pragma unroll
-                for (int k = 1; k < A; k++) a[k] = ztw<true>(exg[ST * (k * XS + lane)], P::ALL1 ? tw1[(k - 1) * M + lane] : twk(k, lo, hi));
-                ZDft<A, true>::run(a);
-                const float f = op == OP_INV ? alpha / (float)N : alpha;
-                float addv = 0.0f;
-                if (op == OP_INV && jb.addk) addv = (float)jb.addk[plane];
-                if (op == OP_INV) addv = addv + (float)jb.addc;
-                // (an accumulation's old values are asked for CH at a time; more cost
-                // y lines of 512 points spilled registers)
-                constexpr int CH = DIR == 0 ? 4 : 2;
-#pragma unroll
-                for (int m0 = 0; m0 < A; m0 += CH) {
-                    Z old[CH];
-                    if (acc) {
-#pragma unroll
-                        for (int m = 0; m < CH; m++) old[m] = load(out, lane + M * (m0 + m));
-                    }
-#pragma unroll
-                    for (int m = 0; m < CH; m++) {
-                        // (the derivative's factor i)
-                        Z v = op == OP_D1 ? zi(a[m0 + m]) : a[m0 + m];
-                        v = acc ? zaxpy(f, v, old[m]) : zscale(v, f);
-                        if (op == OP_INV) v = zaddc(v, addv);
-                        store(out, lane + M * (m0 + m), v);
-                    }
-                }
-            }
         }
-    }
-    if (tid == 0 && bad) {
-        // copies still in flight land before the CTA's shared memory is released
-        for (int i = issued > 2 ? issued - 2 : 0; i < issued; i++) mbar_wait(&bar[i & 1], (i >> 1) & 1);
     }
 }
 
@@ -637,6 +509,22 @@ extern "C" int vec_selftest_wait(vec_ctx *c, long long polls)
 }
 
 // ---- host side ------------------------------------------------------------------------
+int line_ct_configure()
+{
+    float2 tf[32], uf[96];
+    for (int q = 0; q < 96; q++) {
+        double c, v;
+        sincos2pi_host(q, 96, &c, &v);
+        uf[q].x = (float)c; uf[q].y = (float)(-v);
+        if (q >= 32) continue;
+        sincos2pi_host(q, 32, &c, &v);
+        tf[q].x = (float)c; tf[q].y = (float)(-v);
+    }
+    CUDA_TRY(cudaMemcpyToSymbol(c_tw32f, tf, sizeof(tf)));
+    CUDA_TRY(cudaMemcpyToSymbol(c_tw96f, uf, sizeof(uf)));
+    return VEC_OK;
+}
+
 static PFN_cuTensorMapEncodeTiled_v12000 g_encode = nullptr;
 static int get_encoder();
 
@@ -659,8 +547,10 @@ static int get_encoder()
 }
 
 // TMA descriptor of a (nx, ny, nz) field read in boxes of 2S columns x BR rows
-static int encode_ymap(CUtensorMap *m, const float *base, int nx, int ny, int nz, int S, int BR)
+int encode_ymap(CUtensorMap *m, const float *base, int nx, int ny, int nz, int S, int BR)
 {
+    const int st = get_encoder();
+    if (st) return st;
     cuuint64_t dims[3] = { (cuuint64_t)nx, (cuuint64_t)ny, (cuuint64_t)nz };
     cuuint64_t strides[2] = { (cuuint64_t)nx * sizeof(float), (cuuint64_t)nx * ny * sizeof(float) };
     cuuint32_t box[3] = { (cuuint32_t)(2 * S), (cuuint32_t)BR, 1 };
@@ -676,18 +566,28 @@ static int encode_ymap(CUtensorMap *m, const float *base, int nx, int ny, int nz
     return VEC_OK;
 }
 
-template <int DIR, int A, int B, int C, int S, int NJ>
-static int run_nj(Engine *E, const LineJob<float> *jobs, int nj, const char *name)
+template <typename R, int DIR, int N1, int N2, int S, bool WSYNC, int NJ>
+static int run_nj(Engine *E, const LineJob<R> *jobs, int nj, const char *name)
 {
-    using P = CtShape<DIR, A, B, C, S>;
+    using C = typename CT<R>::T;
+    constexpr int N = N1 * N2;
+    constexpr int NP = N1 > N2 ? N1 : N2;
+    constexpr int TILE = 2 * S * N;
+    constexpr int LDS = ct_lds<R, DIR, N1, N2, S>();
     static bool attr_set = false;
+    const size_t smem = ct_smem_bytes<R, DIR, N1, N2, S>();
+    static_assert(ct_smem_bytes<R, DIR, N1, N2, S>() == 2 * TILE * sizeof(R) + ((size_t)S * LDS + 2 * N) * sizeof(C) + 3 * (size_t)N * sizeof(R),
+                  "shared memory layout");
+    static_assert(ct_smem_bytes<R, DIR, N1, N2, S>() + 128 <= 232448, "tile does not fit one SM's shared memory");
+    static_assert(LDS >= N1 * (N2 + 1) && LDS >= N2 * (N1 + 1) && LDS >= N + N / 32 + 1, "exchange rows");
     if (!attr_set) {
-        CUDA_TRY(cudaFuncSetAttribute(line_ct<DIR, A, B, C, S, NJ>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)P::SMEM));
+        CUDA_TRY(cudaFuncSetAttribute(line_ct<R, DIR, N1, N2, S, WSYNC, NJ>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                      (int)smem));
         attr_set = true;
     }
     const int L = DIR == 0 ? E->ny : E->nx;
     const int tpp = L / (2 * S);
-    JobPackCT<NJ> pk;
+    JobPackCT<R, NJ> pk;
     memset(&pk, 0, sizeof(pk));
     double fields = 0.0;
     for (int j = 0; j < nj; j++) {
@@ -698,28 +598,30 @@ static int run_nj(Engine *E, const LineJob<float> *jobs, int nj, const char *nam
     TmapPack<DIR, NJ> tp;
     memset(&tp, 0, sizeof(tp));
     if constexpr (DIR == 1) {
-        int st = get_encoder();
-        if (st) return st;
+        constexpr int BR = ybox_rows(N);
+        int st;
         for (int j = 0; j < nj; j++)
-            if ((st = encode_ymap(&tp.m[j], jobs[j].in, E->nx, E->ny, E->nz, S, ybox_rows(P::N)))) return st;
+            if ((st = encode_ymap(&tp.m[j], jobs[j].in, E->nx, E->ny, E->nz, S, BR))) return st;
     }
     const int total = nj * E->nz * tpp;
     int per_sm = 1;
-    CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, line_ct<DIR, A, B, C, S, NJ>, P::NT, P::SMEM));
+    CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, line_ct<R, DIR, N1, N2, S, WSYNC, NJ>, S * NP, smem));
     if (per_sm < 1) per_sm = 1;
     int grid = E->num_sms * per_sm;
     if (grid > total) grid = total;
-    E->prof_begin(name, fields * (double)E->n * sizeof(float));
-    CUDA_TRY(launch_k(*E, line_ct<DIR, A, B, C, S, NJ>, dim3(grid), dim3(P::NT), P::SMEM, pk, tp, E->tables<float>(DIR), E->nx, E->ny,
-                      E->nz, tpp, total, (int)E->ct_warp, E->dev_err));
+    E->prof_begin(name, fields * (double)E->n * sizeof(R));
+    CUDA_TRY(launch_k(*E, line_ct<R, DIR, N1, N2, S, WSYNC, NJ>, dim3(grid), dim3(S * NP), smem, pk, tp,
+                      E->tables<R>(DIR), E->nx, E->ny, E->nz, tpp, total, E->dev_err));
     E->prof_end();
     CUDA_TRY(cudaGetLastError());
     return VEC_OK;
 }
-template <int DIR, int A, int B, int C, int S>
-static int run_ct(Engine *E, const LineJob<float> *jobs, int nj, const char *name)
+
+template <typename R, int DIR, int N1, int N2, int S, bool WSYNC>
+static int run_ct(Engine *E, const LineJob<R> *jobs, int nj, const char *name)
 {
-    return nj <= NJ_SMALL ? run_nj<DIR, A, B, C, S, NJ_SMALL>(E, jobs, nj, name) : run_nj<DIR, A, B, C, S, MAX_JOBS>(E, jobs, nj, name);
+    return nj <= NJ_SMALL ? run_nj<R, DIR, N1, N2, S, WSYNC, NJ_SMALL>(E, jobs, nj, name)
+                          : run_nj<R, DIR, N1, N2, S, WSYNC, MAX_JOBS>(E, jobs, nj, name);
 }
 
 static bool aligned16(const void *p) { return ((uintptr_t)p & 15) == 0; }
@@ -749,6 +651,7 @@ int launch_lines_ct(Engine *E, int dir, const LineJob<float> *jobs, int njobs)
         if (!aligned16(jobs[j].in) || !aligned16(jobs[j].out1) || (jobs[j].out2 && !aligned16(jobs[j].out2)))
             return 0;
     }
+    const bool ws = E->ct_warp;
     for (int j0 = 0; j0 < njobs; j0 += MAX_JOBS) {
         const int nj = njobs - j0 < MAX_JOBS ? njobs - j0 : MAX_JOBS;
         const LineJob<float> *jb = jobs + j0;
@@ -762,15 +665,16 @@ int launch_lines_ct(Engine *E, int dir, const LineJob<float> *jobs, int njobs)
             name = kinds[dir][kd];
         }
         int st = -1;
-#define CT_CASE(NN, A, B, C, SS)                                                                     \
-    if (n == NN && S == SS) st = dir == 0 ? run_ct<0, A, B, C, SS>(E, jb, nj, name) : run_ct<1, A, B, C, SS>(E, jb, nj, name);
-        CT_CASE(64, 8, 8, 1, 16) CT_CASE(96, 8, 12, 1, 16) CT_CASE(128, 16, 8, 1, 16)
-        CT_CASE(192, 16, 12, 1, 16) CT_CASE(256, 16, 16, 1, 16)
-        CT_CASE(64, 8, 8, 1, 8) CT_CASE(96, 8, 12, 1, 8) CT_CASE(128, 16, 8, 1, 8)
-        CT_CASE(192, 16, 12, 1, 8) CT_CASE(256, 16, 16, 1, 8)
-        CT_CASE(384, 8, 6, 8, 8) CT_CASE(512, 8, 8, 8, 8) CT_CASE(768, 8, 12, 8, 8) CT_CASE(1024, 16, 8, 8, 8)
-        CT_CASE(768, 8, 12, 8, 4) CT_CASE(1024, 16, 8, 8, 4)
+#define CT_CASE(NN, A, B, SS)                                                                       \
+    if (n == NN && S == SS)                                                                         \
+        st = dir == 1 ? run_ct<float, 1, A, B, SS, false>(E, jb, nj, name)                            \
+                      : (ws ? run_ct<float, 0, A, B, SS, true>(E, jb, nj, name)                       \
+                            : run_ct<float, 0, A, B, SS, false>(E, jb, nj, name));
+        CT_CASE(64, 8, 8, 16) CT_CASE(128, 16, 8, 16) CT_CASE(256, 16, 16, 16) CT_CASE(96, 8, 12, 16) CT_CASE(192, 16, 12, 16)
+        CT_CASE(64, 8, 8, 8) CT_CASE(128, 16, 8, 8) CT_CASE(256, 16, 16, 8) CT_CASE(96, 8, 12, 8) CT_CASE(192, 16, 12, 8)
 #undef CT_CASE
+        // three levels, pairs of sequences
+        if (n >= 384) st = launch_lines_cp(E, dir, jb, nj, S, name);
         if (st < 0) return 0;
         if (st) return st;
     }

@@ -3,6 +3,8 @@
 #pragma once
 #include <stdint.h>
 
+#include <cuda.h>
+
 __device__ __forceinline__ unsigned smem_u32(const void *p) { return (unsigned)__cvta_generic_to_shared(p); }
 
 __device__ __forceinline__ void mbar_init(uint64_t *bar, unsigned count)
@@ -38,3 +40,14 @@ __device__ __forceinline__ bool mbar_wait(uint64_t *bar, unsigned parity, long l
     }
     return false;
 }
+// 3-D tiled TMA load of one box (c0 innermost) into shared memory
+__device__ __forceinline__ void tma_load_3d(void *dst, const CUtensorMap *map, int c0, int c1, int c2, uint64_t *bar)
+{
+    asm volatile("cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4}], [%5];"
+                 ::"r"(smem_u32(dst)), "l"(map), "r"(c0), "r"(c1), "r"(c2), "r"(smem_u32(bar)) : "memory");
+}
+// this thread's writes to shared memory before later copies into it
+__device__ __forceinline__ void fence_async() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
+// rows per TMA box of a y tile: TMA boxes are at most 256 rows, and the box
+// must divide the line length
+__host__ __device__ constexpr int ybox_rows(int n) { return n <= 256 ? n : (n % 256 == 0 ? 256 : n / 2); }
