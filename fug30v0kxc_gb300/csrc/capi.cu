@@ -325,7 +325,10 @@ extern "C" int vec_create(const vec_params *p, vec_ctx **out)
         (st = fs_tables_make(E.nx, E.fpx, E.fxx, akx1.data(), akx2.data(), E.k.icutoffx, &E.fsx)) ||
         (st = fs_tables_make(E.ny, E.fpy, E.fxy, aky1.data(), aky2.data(), E.k.icutoffy, &E.fsy)) ||
         (st = line_tables_make<float>(E.nx, akx1.data(), akx2.data(), E.k.icutoffx, &E.tx32)) ||
-        (st = line_tables_make<float>(E.ny, aky1.data(), aky2.data(), E.k.icutoffy, &E.ty32))) {
+        (st = line_tables_make<float>(E.ny, aky1.data(), aky2.data(), E.k.icutoffy, &E.ty32)) ||
+        (E.split && ct64_length(E.nx) && ct64_length(E.ny) &&
+         ((st = line_tables_make<double>(E.nx, akx1.data(), akx2.data(), E.k.icutoffx, &E.tx64)) ||
+          (st = line_tables_make<double>(E.ny, aky1.data(), aky2.data(), E.k.icutoffy, &E.ty64))))) {
         vec_destroy(c);
         return st;
     }
@@ -457,6 +460,8 @@ extern "C" int vec_destroy(vec_ctx *c)
     fs_tables_free(&E.fsy);
     fx_tables_free(&E.fxx);
     fx_tables_free(&E.fxy);
+    if (E.tx64.tw) line_tables_free(&E.tx64);
+    if (E.ty64.tw) line_tables_free(&E.ty64);
     if (E.tx32.tw) line_tables_free(&E.tx32);
     if (E.ty32.tw) line_tables_free(&E.ty32);
     if (E.hs) cudaFreeHost(E.hs);

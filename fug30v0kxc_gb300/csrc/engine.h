@@ -55,6 +55,7 @@ struct Engine {
     FxTables fxx = {}, fxy = {};        // FP64
     FsTables fsx = {}, fsy = {};        // FP32
     LineTables<float> tx32, ty32;
+    LineTables<double> tx64, ty64;   // split, both lengths among lines_ct64.cu's: else null
 
     // FP64 state (src/arrays.f90)
     double *r = nullptr, *t = nullptr, *u = nullptr, *v = nullptr, *w = nullptr;
@@ -229,6 +230,10 @@ inline int fx_rounds(const FxPlan &pl, int q)
 int fs_tables_make(int n, const FxPlan &pl, const FxTables &fx, const double *k1, const double *k2, int icut, FsTables *tb);
 void fs_tables_free(FsTables *tb);
 int line_ct_configure();
+int line_ct64_configure();
+inline bool ct64_length(int n) { return n == 64 || n == 96 || n == 128 || n == 192 || n == 256; }
+int launch_lines_ct64(Engine *E, int dir, const LineJob<double> *jobs, int njobs);   // lines_ct64.cu
+void *tma_encode_fn();
 int launch_lines_ct(Engine *E, int dir, const LineJob<float> *jobs, int njobs);
 int launch_lines_cp(Engine *E, int dir, const LineJob<float> *jobs, int nj, int S, const char *name);   // lines_cp.cu
 

@@ -587,7 +587,7 @@ int launch_lines<float>(Engine *E, int dir, const LineJob<float> *jobs, int njob
 int line_kernels_configure()
 {
     int st = line_ct_configure();
-    if (st || (st = line_fx_configure())) return st;
+    if (st || (st = line_ct64_configure()) || (st = line_fx_configure())) return st;
     CUDA_TRY(cudaFuncSetAttribute(line_kernel<0, NJ_SMALL>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
     CUDA_TRY(cudaFuncSetAttribute(line_kernel<1, NJ_SMALL>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
     CUDA_TRY(cudaFuncSetAttribute(line_kernel<0, MAX_JOBS>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
@@ -595,5 +595,7 @@ int line_kernels_configure()
     return VEC_OK;
 }
 
+template int line_tables_make<double>(int, const double *, const double *, int, LineTables<double> *);
+template void line_tables_free<double>(LineTables<double> *);
 template int line_tables_make<float>(int, const double *, const double *, int, LineTables<float> *);
 template void line_tables_free<float>(LineTables<float> *);

@@ -241,7 +241,8 @@ static __global__ void k_bandj_spec(BandjArgs<R> a)
 
 // :630-645: jsq from Jz, dBz/dy, dBz/dx and the z derivatives of Bx, By
 // (grid (np/256, nz))
-template <typename R>
+// INT: the FP64 form's sums in integers (zfx.cuh)
+template <typename R, bool INT = sizeof(R) == 8>
 static __global__ void k_jsq(const R *jz, const R *dybz, const R *dxbz, const R *bx, const R *by, R *jsq,
                              size_t np, int nz, R h)
 {
@@ -251,7 +252,7 @@ static __global__ void k_jsq(const R *jz, const R *dybz, const R *dxbz, const R 
     const int k = blockIdx.y;
     const size_t idx = (size_t)k * np + q;
     R wk1, wk2;
-    if constexpr (sizeof(R) == 8) {
+    if constexpr (INT) {
         // (the sums in integers, zfx.cuh: 0.18 -> 0.13 ms at 256^2 x 129)
         wk1 = h * zsum<ZD1 | ZPIPE>(by + q, np, k, nz, 5, 0).d1;
         wk2 = h * zsum<ZD1 | ZPIPE>(bx + q, np, k, nz, 5, 0).d1;

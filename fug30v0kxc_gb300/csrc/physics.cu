@@ -1184,14 +1184,19 @@ int phys_mag_init(Engine *E)
     W[W_EX] = E->W64(0); W[W_EY] = E->W64(1); W[W_EZ] = E->W64(2);
     W[W_M1] = E->W64(3); W[W_M2] = E->W64(4); W[W_M3] = E->W64(5);
     int st;
+    // (a split context's: see lines_ct64.cu)
+    auto lines = [E](int dir, const LineJob<double> *j, int nj) {
+        const int h = E->split ? launch_lines_ct64(E, dir, j, nj) : 0;
+        return h == 1 ? VEC_OK : h < 0 ? h : launch_lines<double>(E, dir, j, nj);
+    };
     if (E->p.dynamo)
         KLAUNCH(E, "dynamo_seed", k_dynamo_seed, nblk(E->n), TPB, E->bx, E->by, E->bz, E->nx, E->ny, E->n, E->p.perfect);
     LineJob<double> fx[3] = { ljob<double>(E->bx, W[W_EX], OP_FWD), ljob<double>(E->by, W[W_EY], OP_FWD),
                               ljob<double>(E->bz, W[W_EZ], OP_FWD) };
-    if ((st = launch_lines<double>(E, 0, fx, 3))) return st;
+    if ((st = lines(0, fx, 3))) return st;
     LineJob<double> fy[3] = { ljob<double>(W[W_EX], W[W_EX], OP_FWD), ljob<double>(W[W_EY], W[W_EY], OP_FWD),
                               ljob<double>(W[W_EZ], W[W_EZ], OP_FWD) };
-    if ((st = launch_lines<double>(E, 1, fy, 3))) return st;
+    if ((st = lines(1, fy, 3))) return st;
     for (int f = 0; f < 3; f++)     // :70-103
         KLAUNCH(E, "truncate_f64", k_truncate<double>, plane_grid(*E), TPB, W[W_EX + f], (double *)nullptr, E->nx, E->ny,
                 E->nz, E->k.icutoffx, E->k.icutoffy);
@@ -1208,10 +1213,14 @@ int phys_mag_init(Engine *E)
     KLAUNCH(E, "mag_init_spec", k_mag_init_spec, nblk(E->n), TPB, a);
     LineJob<double> ix[3] = { ljob<double>(W[W_M1], W[W_M1], OP_INV), ljob<double>(W[W_M2], W[W_M2], OP_INV),
                               ljob<double>(W[W_M3], W[W_M3], OP_INV) };
-    if ((st = launch_lines<double>(E, 0, ix, 3))) return st;
-    if ((st = launch_lines<double>(E, 1, ix, 3))) return st;
+    if ((st = lines(0, ix, 3))) return st;
+    if ((st = lines(1, ix, 3))) return st;
     // jsq (:246-261): ex = inv(dBz/dy), ey = inv(dBz/dx), ez = inv(Jz)
-    KLAUNCH(E, "jsq_f64", k_jsq<double>, plane_grid(*E), TPB, W[W_M3], W[W_M1], W[W_M2], E->bx, E->by,
-            E->jsq, E->np, E->nz, E->k.ho12);
+    if (E->split)
+        KLAUNCH(E, "jsq_f64", (k_jsq<double, false>), plane_grid(*E), TPB, W[W_M3], W[W_M1], W[W_M2], E->bx, E->by,
+                E->jsq, E->np, E->nz, E->k.ho12);
+    else
+        KLAUNCH(E, "jsq_f64", k_jsq<double>, plane_grid(*E), TPB, W[W_M3], W[W_M1], W[W_M2], E->bx, E->by,
+                E->jsq, E->np, E->nz, E->k.ho12);
     return phys_mag_boundary(E);
 }
