@@ -31,8 +31,9 @@
 // runs of one side differ by 3 %; the error against FP64 falls by 2-8 %):
 //    384^2 x 65    53.1  48.9 ->  44.5  41.0      768^2 x 33   104.1 100.0 ->  76.2  83.1
 //    512^2 x 65    92.6  67.4 ->  60.4  61.7     1024^2 x 33   153.3 140.2 -> 122.7 135.8
-// (Up to 256 points the gain was 3-8 %, less than a change of rounding in every step,
-// restart and training set of those grids is worth: they keep two levels, bit for bit.)
+// (Up to 256 points pairs on two levels took 3-8 % less, 34.4 -> 31.5 at 256^2 x 129,
+// which is not worth other rounding in every step, restart and training set of those
+// grids: lines_ct.cu keeps their results bit for bit.)
 #include <math.h>
 #include <stdint.h>
 #include <string.h>

@@ -13,17 +13,17 @@
 // loaded and stored by all its threads row by row.
 //
 // Why passes through shared memory rather than 16-point DFTs in registers:
-// the work is bound by integer instructions, and with 8 elements a thread
-// three times as many warps fit and the code stays in the instruction cache.
-// The register form (the FP32 kernel's) issued in 20 % of the cycles, this one
-// in 57 % (three CTAs per SM at 80 registers).
+// the work is bound by integer instructions, and with 8 elements a thread three
+// times as many warps fit (three CTAs per SM at 80 registers).  The register form
+// (lines_ct.cu's, on integers) issued in 20 % of the cycles.
 //
 // Measured at 256^2 x 129, mean of d2bydx and d1bydx: 618 us in FP64 (the FP64
 // pipe 83 % busy) -> 150 us, y the same.  (168 us with every element's place
 // computed, a table of multipliers, and x results stored by a loop of their
 // own.)  It issues in 45 % of the cycles, the rest being instruction fetches and
 // the latency of shared memory and conversions; synchronising the passes of a
-// CTA's warps, so that they fetch the same code, changed nothing.  Error against
+// CTA's warps, so that they fetch the same code, changed nothing, nor did rolled
+// loops of twiddle products (13 % less code).  Error against
 // long double: 2 to 3 times smaller than in FP64 for white noise, 10^4 times for
 // a constant plus little.
 #include <math.h>
