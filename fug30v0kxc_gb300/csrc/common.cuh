@@ -37,10 +37,10 @@ struct LineJob {
 // jobs, and the Lorentz fluxes' and E's transforms, per member); the job
 // and tensor-map packs then take 24 KB of the 32 KB kernel parameter space
 #define MAX_JOBS 128
-// Parameters cost a launch time by their size: with room for MAX_JOBS jobs and, y
-// lines, their TMA descriptors, 24 KB, a derivative pair at 64^2 x 65 took 11.2 us,
-// without the descriptors 9.7, with room for eight jobs 8.7.  So launches of a few
-// jobs (one solver's; a batch of members has more) have kernels of their own.
+// Parameters cost a launch time by their size: with room for MAX_JOBS jobs and TMA
+// descriptors, 24 KB, a derivative pair at 64^2 x 65 took 12.0 (x) and 10.4 us (y),
+// with room for eight jobs 8.9 and 8.5.  So launches of a few jobs (one solver's; a
+// batch of members has more) have kernels of their own.
 #define NJ_SMALL 8
 
 // spectral tables of one direction (device pointers)
