@@ -163,8 +163,7 @@ __host__ __device__ constexpr size_t ct_smem_bytes()
 {
     constexpr int N = N1 * N2;
     constexpr int LDS = ct_lds<R, DIR, N1, N2, S>();
-    return 2 * (size_t)(2 * S * N) * sizeof(R) + ((size_t)S * LDS + (sizeof(R) == 4 ? 2 : 1) * (size_t)N) * 2 * sizeof(R)
-           + 3 * (size_t)N * sizeof(R);
+    return 2 * (size_t)(2 * S * N) * sizeof(R) + ((size_t)S * LDS + (size_t)N) * 2 * sizeof(R);
 }
 // two CTAs per SM where their shared memory fits (227 KB per SM), else one
 // CTA with the whole register file
@@ -194,18 +193,7 @@ line_ct64(JobPackCT<R> jobs, const __grid_constant__ TmapPack tmaps, LineTables<
     R *tile0 = reinterpret_cast<R *>(smem);
     R *tile1 = tile0 + TILE;
     C *ex = reinterpret_cast<C *>(tile1 + TILE);
-    // FP32: twiddles W_N^(m2 k1) as two N1 x N2 tables, one row per value of
-    // the loop index, so that the 16 threads of a sequence read consecutive
-    // entries (indexed by (m2 k1) mod N, a thread stride of k1 made up to
-    // eight-way bank conflicts).  FP64: one table of N (the second would
-    // cost the second CTA per SM).
-    constexpr bool TW2 = sizeof(R) == 4;
-    static_assert(!TW2 || (N1 % 4 == 0 && N2 % 4 == 0), "FP32 twiddles factor the index as 4 a + b");
-    C *twf = ex + (size_t)S * LDS;                    // twf[k1 N2 + m2] (FP64: tw[e])
-    C *twi = twf + N;                                 // twi[m2 N1 + k1]
-    R *sm1 = reinterpret_cast<R *>(twi + (TW2 ? N : 0));   // spectral multipliers
-    R *sm2 = sm1 + N;
-    R *smda = sm2 + N;
+    C *twf = ex + (size_t)S * LDS;                    // W_N^e
     __shared__ __align__(8) uint64_t bar[4];          // full[2], empty[2]
 
     const int tid = threadIdx.x;
@@ -218,17 +206,7 @@ line_ct64(JobPackCT<R> jobs, const __grid_constant__ TmapPack tmaps, LineTables<
     };
 
     for (int e = tid; e < N; e += NT) {
-        if constexpr (TW2) {
-            const int k1 = e / N2, m2 = e - k1 * N2;
-            twf[e] = tb.tw[modn<N>(m2 * k1)];
-            const int m2i = e / N1, k1i = e - m2i * N1;
-            twi[e] = tb.tw[modn<N>(m2i * k1i)];
-        } else {
-            twf[e] = tb.tw[e];
-        }
-        sm1[e] = tb.m1[e];
-        sm2[e] = tb.m2[e];
-        smda[e] = tb.mda[e];
+        twf[e] = tb.tw[e];
     }
     if (tid == 0) {
         mbar_init(&bar[0], 1);
@@ -298,7 +276,7 @@ line_ct64(JobPackCT<R> jobs, const __grid_constant__ TmapPack tmaps, LineTables<
         const int l0 = (rem - plane * tpp) * 2 * S;
         const LineJob<R> &jb = jobs.j[job];
         const size_t pbase = (size_t)plane * np;
-        const int op1 = jb.op1, op2 = jb.op2;
+        const int op1 = jb.op1;
         C *ex_s = ex + (size_t)sidx * LDS;
 
         // element e of sequence sidx in the tile
@@ -309,50 +287,17 @@ line_ct64(JobPackCT<R> jobs, const __grid_constant__ TmapPack tmaps, LineTables<
             return z;
         };
 
-        // The two sequences a warp holds (x lines, 16 threads each) have rows
-        // that start on the same bank; the odd one reads its columns in pairs
-        // swapped (index ^ 1), so that the two half-warps hit different banks,
-        // and swaps the registers back.  The values are the same.
-        constexpr bool XSW = WS && DIR == 0 && NP == 16 && sizeof(R) == 4 && N1 % 2 == 0 && N2 % 2 == 0;
-        const int sw = XSW ? (sidx & 1) : 0;
-        auto unswap = [&](C *v, int n) {
-            if constexpr (XSW) {
-#pragma unroll
-                for (int i = 0; i < n; i += 2) {
-                    const C t0 = v[i], t1 = v[i + 1];
-                    v[i] = sw ? t1 : t0;
-                    v[i + 1] = sw ? t0 : t1;
-                }
-            }
-        };
-
         C X[N2];   // thread lane = k1 holds X[k1 + N1 k2], k2 = 0..N2-1
         if (op1 != OP_INV) {
             // forward, first level: thread m2 = lane, N1-point DFT over m1
             if (lane < N2) {
                 C a[N1];
 #pragma unroll
-                for (int m1 = 0; m1 < N1; m1++) a[m1] = tile_z(N2 * (m1 ^ sw) + lane);
-                unswap(a, N1);
+                for (int m1 = 0; m1 < N1; m1++) a[m1] = tile_z(N2 * m1 + lane);
                 RDft<N1, false>::run(a);
-                // FP32: W^(lane k1) = W^(lane 4 (k1 / 4)) W^(lane (k1 % 4)): 3 + N1/4 - 1
-                // table reads instead of N1 - 1, one product more per twiddle
-                C lo[4], hi[N1 / 4];
-                if constexpr (TW2) {
-#pragma unroll
-                    for (int j = 1; j < 4; j++) lo[j] = twf[j * N2 + lane];
-#pragma unroll
-                    for (int j = 1; j < N1 / 4; j++) hi[j] = twf[4 * j * N2 + lane];
-                }
 #pragma unroll
                 for (int k1 = 0; k1 < N1; k1++) {
-                    C w;
-                    if constexpr (TW2) {
-                        const int ja = k1 >> 2, jb = k1 & 3;
-                        w = ja == 0 ? lo[jb] : (jb == 0 ? hi[ja] : cmul_(hi[ja], lo[jb]));
-                    } else {
-                        w = twf[modn<N>(lane * k1)];
-                    }
+                    const C w = twf[modn<N>(lane * k1)];
                     ex_s[k1 * LXF + lane] = k1 == 0 ? a[k1] : cmul_(a[k1], w);
                 }
             }
@@ -368,7 +313,7 @@ line_ct64(JobPackCT<R> jobs, const __grid_constant__ TmapPack tmaps, LineTables<
             // halfcomplex input lines a (re) and b (im): Z_k = A_k + i B_k
 #pragma unroll
             for (int k2 = 0; k2 < N2; k2++) {
-                const int k = lane + N1 * (k2 ^ sw);
+                const int k = lane + N1 * k2;
                 const int kk = k <= N / 2 ? k : N - k;
                 const bool edge = kk == 0 || 2 * kk == N;
                 C pa = tile_z(kk);                     // (ha[kk], hb[kk])
@@ -377,7 +322,6 @@ line_ct64(JobPackCT<R> jobs, const __grid_constant__ TmapPack tmaps, LineTables<
                 X[k2].x = ar - bi;
                 X[k2].y = ai + br;
             }
-            unswap(X, N2);
         }
         if constexpr (WS) {
             // this warp is done with the tile buffer
@@ -399,98 +343,56 @@ line_ct64(JobPackCT<R> jobs, const __grid_constant__ TmapPack tmaps, LineTables<
                 if (2 * p <= N) { va = (R)0.5 * (zp.x + zq.x); vb = (R)0.5 * (zp.y + zq.y); }
                 else { va = (R)0.5 * (zq.y - zp.y); vb = (R)0.5 * (zp.x - zq.x); }
                 const int la = l0 + 2 * sidx;
-                const R ra = jb.alpha1 * va, rb = jb.alpha1 * vb;
                 if (DIR == 0) {
                     R *oa = jb.out1 + pbase + (size_t)la * nx + p, *ob = oa + nx;
-                    *oa = jb.acc1 ? *oa + ra : ra;
-                    *ob = jb.acc1 ? *ob + rb : rb;
+                    *oa = va;
+                    *ob = vb;
                 } else {
                     // the two lines are adjacent columns: one vector store
-                    C *o = reinterpret_cast<C *>(jb.out1 + pbase + (size_t)p * nx + la);
-                    C v = { ra, rb };
-                    if (jb.acc1) { const C q = *o; v.x += q.x; v.y += q.y; }
-                    *o = v;
+                    *reinterpret_cast<C *>(jb.out1 + pbase + (size_t)p * nx + la) = C{ va, vb };
                 }
             }
             sync();
             continue;
         }
 
-        // one or two outputs: Y = m(X), inverse transform, store (a
-        // halfcomplex input takes a second output only for OP_D1: the
-        // derivative of its inverse)
-        const int nout = (op2 != OP_NONE && (op1 != OP_INV || op2 == OP_D1)) ? 2 : 1;
-        for (int o = 0; o < nout; o++) {
-            const int op = o == 0 ? op1 : op2;
-            R *out = o == 0 ? jb.out1 : jb.out2;
-            const R alpha = o == 0 ? jb.alpha1 : jb.alpha2;
-            const int acc = o == 0 ? jb.acc1 : jb.acc2;
-            if (lane < N1) {
-                C Y[N2];
+        // inverse transform, store
+        if (lane < N1) {
+            C Y[N2];
 #pragma unroll
-                for (int k2 = 0; k2 < N2; k2++) {
-                    const int k = lane + N1 * k2;
-                    C z = X[k2], y;
-                    if (op == OP_D1) { R m = sm1[k]; y.x = -m * z.y; y.y = m * z.x; }
-                    else if (op == OP_INV) { y = z; }
-                    else { R m = op == OP_D2 ? sm2[k] : smda[k]; y.x = m * z.x; y.y = m * z.y; }
-                    Y[k2] = y;
-                }
-                // inverse, first level: thread k1 = lane, N2-point DFT over k2
-                RDft<N2, true>::run(Y);
-                // (FP32: the same factorisation of W^(m2 lane), m2 = 4 (m2 / 4) + m2 % 4)
-                C lo[4], hi[N2 / 4];
-                if constexpr (TW2) {
+            for (int k2 = 0; k2 < N2; k2++) Y[k2] = X[k2];
+            // inverse, first level: thread k1 = lane, N2-point DFT over k2
+            RDft<N2, true>::run(Y);
 #pragma unroll
-                    for (int j = 1; j < 4; j++) lo[j] = twi[j * N1 + lane];
-#pragma unroll
-                    for (int j = 1; j < N2 / 4; j++) hi[j] = twi[4 * j * N1 + lane];
-                }
-#pragma unroll
-                for (int m2 = 0; m2 < N2; m2++) {
-                    C w;
-                    if constexpr (TW2) {
-                        const int ja = m2 >> 2, jb = m2 & 3;
-                        w = ja == 0 ? lo[jb] : (jb == 0 ? hi[ja] : cmul_(hi[ja], lo[jb]));
-                    } else {
-                        w = twf[modn<N>(m2 * lane)];
-                    }
-                    w.y = -w.y;
-                    ex_s[m2 * LXI + lane] = m2 == 0 ? Y[m2] : cmul_(Y[m2], w);
-                }
+            for (int m2 = 0; m2 < N2; m2++) {
+                C w = twf[modn<N>(m2 * lane)];
+                w.y = -w.y;
+                ex_s[m2 * LXI + lane] = m2 == 0 ? Y[m2] : cmul_(Y[m2], w);
             }
-            sync();
-            // second level: thread m2 = lane, N1-point DFT over k1
-            if (lane < N2) {
-                C a[N1];
-#pragma unroll
-                for (int k1 = 0; k1 < N1; k1++) a[k1] = ex_s[lane * LXI + k1];
-                RDft<N1, true>::run(a);
-                const R sc = op == OP_INV ? (R)1 / (R)N : (R)1;
-                const int la = l0 + 2 * sidx;
-                R addv = (R)0;
-                if (op == OP_INV && jb.addk) addv = (R)jb.addk[plane];
-                if (op == OP_INV) addv = addv + (R)jb.addc;
-#pragma unroll
-                for (int m1 = 0; m1 < N1; m1++) {
-                    const int e = lane + N2 * m1;
-                    R va = alpha * (a[m1].x * sc), vb = alpha * (a[m1].y * sc);
-                    if (DIR == 0) {
-                        R *oa = out + pbase + (size_t)la * nx + e, *ob = oa + nx;
-                        if (acc) { va = *oa + va; vb = *ob + vb; }
-                        if (op == OP_INV) { va = va + addv; vb = vb + addv; }
-                        *oa = va;
-                        *ob = vb;
-                    } else {
-                        C *o = reinterpret_cast<C *>(out + pbase + (size_t)e * nx + la);
-                        if (acc) { const C q = *o; va = q.x + va; vb = q.y + vb; }
-                        if (op == OP_INV) { va = va + addv; vb = vb + addv; }
-                        *o = C{ va, vb };
-                    }
-                }
-            }
-            sync();
         }
+        sync();
+        // second level: thread m2 = lane, N1-point DFT over k1
+        if (lane < N2) {
+            C a[N1];
+#pragma unroll
+            for (int k1 = 0; k1 < N1; k1++) a[k1] = ex_s[lane * LXI + k1];
+            RDft<N1, true>::run(a);
+            const R sc = (R)1 / (R)N;
+            const int la = l0 + 2 * sidx;
+#pragma unroll
+            for (int m1 = 0; m1 < N1; m1++) {
+                const int e = lane + N2 * m1;
+                const R va = a[m1].x * sc, vb = a[m1].y * sc;
+                if (DIR == 0) {
+                    R *oa = jb.out1 + pbase + (size_t)la * nx + e, *ob = oa + nx;
+                    *oa = va;
+                    *ob = vb;
+                } else {
+                    *reinterpret_cast<C *>(jb.out1 + pbase + (size_t)e * nx + la) = C{ va, vb };
+                }
+            }
+        }
+        sync();
     }
 }
 
@@ -542,15 +444,11 @@ static int encode_ymap64(CUtensorMap *m, const R *base, int nx, int ny, int nz, 
 template <typename R, int DIR, int N1, int N2, int S, bool WSYNC>
 static int run_ct(Engine *E, const LineJob<R> *jobs, int nj, const char *name)
 {
-    using C = typename CT<R>::T;
     constexpr int N = N1 * N2;
     constexpr int NP = N1 > N2 ? N1 : N2;
-    constexpr int TILE = 2 * S * N;
     constexpr int LDS = ct_lds<R, DIR, N1, N2, S>();
     static bool attr_set = false;
     const size_t smem = ct_smem_bytes<R, DIR, N1, N2, S>();
-    static_assert(ct_smem_bytes<R, DIR, N1, N2, S>() == 2 * TILE * sizeof(R) + ((size_t)S * LDS + (sizeof(R) == 4 ? 2 : 1) * N) * sizeof(C) + 3 * (size_t)N * sizeof(R),
-                  "shared memory layout");
     static_assert(ct_smem_bytes<R, DIR, N1, N2, S>() + 128 <= 232448, "tile does not fit one SM's shared memory");
     static_assert(LDS >= N1 * (N2 + 1) && LDS >= N2 * (N1 + 1) && LDS >= N + N / 32 + 1, "exchange rows");
     if (!attr_set) {
@@ -565,8 +463,7 @@ static int run_ct(Engine *E, const LineJob<R> *jobs, int nj, const char *name)
     double fields = 0.0;
     for (int j = 0; j < nj; j++) {
         pk.j[j] = jobs[j];
-        fields += 2.0 + (jobs[j].acc1 ? 1.0 : 0.0);
-        if (jobs[j].op2 != OP_NONE) fields += 1.0 + (jobs[j].acc2 ? 1.0 : 0.0);
+        fields += 2.0;
     }
     TmapPack tp;
     memset(&tp, 0, sizeof(tp));
@@ -592,7 +489,7 @@ static int run_ct(Engine *E, const LineJob<R> *jobs, int nj, const char *name)
 
 static bool aligned16(const void *p) { return ((uintptr_t)p & 15) == 0; }
 
-// up to CT64_JOBS jobs: 1 if done, 0 if the lengths or addresses are not its own, < 0
+// up to CT64_JOBS plain forward or inverse jobs: 1 if done, 0 if the lengths or addresses are not its own, < 0
 // on error
 int launch_lines_ct64(Engine *E, int dir, const LineJob<double> *jobs, int njobs)
 {
