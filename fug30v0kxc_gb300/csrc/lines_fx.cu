@@ -359,13 +359,19 @@ line_fx(const __grid_constant__ FxPack<NJ> jobs, const __grid_constant__ FxPlan 
                 out.cy = __shfl_sync(0xffffffffu, dcy, src) / (double)n;
                 return;
             }
+            // (an element is 2^21 at most, a lane's sum 2^27: the line's fits 32 bits up
+            // to 1024 elements, and without its last two bits above that)
+            const int cut = n > 1024 ? 2 : 0;
+            sx >>= cut;
+            sy >>= cut;
             for (int o = G >> 1; o > 0; o >>= 1) {
                 sx += __shfl_xor_sync(0xffffffffu, sx, o);
                 sy += __shfl_xor_sync(0xffffffffu, sy, o);
             }
             // (to 21 bits, a multiple of 2^41 units)
-            mx = (long long)(int)((float)sx * pl.rn) << 41;
-            my = (long long)(int)((float)sy * pl.rn) << 41;
+            const float rn = cut ? 4.0f * pl.rn : pl.rn;
+            mx = (long long)(int)((float)sx * rn) << 41;
+            my = (long long)(int)((float)sy * rn) << 41;
         };
         auto square = [&](const X2 &v) {     // in units of 2^41
             const float x = fx_float(fx_hi(v.x) >> 9), y = fx_float(fx_hi(v.y) >> 9);
