@@ -311,6 +311,9 @@ line_fx(const __grid_constant__ FxPack<NJ> jobs, const __grid_constant__ FxPlan 
             }
             __syncthreads();
         }
+        // (a spectrum's constant is kept apart: it must not set the exponent of a
+        // derivative that does not contain it)
+        double dcx = 0.0, dcy = 0.0;
         auto raw = [&](int e) -> X2 {
             X2 v;
             if (DIR == 0) {
@@ -318,6 +321,11 @@ line_fx(const __grid_constant__ FxPack<NJ> jobs, const __grid_constant__ FxPlan 
                 v.y = valid ? __double_as_longlong(r0[e + nx]) : 0;
             } else {
                 v = A[fx_at(e, s7)];
+            }
+            if (inv && e == 0) {
+                dcx = __longlong_as_double(v.x);
+                dcy = __longlong_as_double(v.y);
+                v.x = v.y = 0;
             }
             return v;
         };
@@ -339,13 +347,8 @@ line_fx(const __grid_constant__ FxPack<NJ> jobs, const __grid_constant__ FxPlan 
         out.cx = out.cy = 0.0;
         int E = 1, F = 0, sx = 0, sy = 0;
         long long mx = 0, my = 0;
-        double dcx = 0.0, dcy = 0.0;
         auto conv = [&](int e, X2 v) {
-            if (inv && e == 0) {
-                dcx = __longlong_as_double(v.x);
-                dcy = __longlong_as_double(v.y);
-                v.x = v.y = 0;
-            }
+            if (inv && e == 0) v.x = v.y = 0;
             v.x = fx_from((unsigned)fx_hi(v.x), (unsigned)v.x, E);
             v.y = fx_from((unsigned)fx_hi(v.y), (unsigned)v.y, E);
             sx += fx_hi(v.x) >> 9;
@@ -389,11 +392,7 @@ line_fx(const __grid_constant__ FxPack<NJ> jobs, const __grid_constant__ FxPlan 
         // the elements become integers one by one, in shared memory)
         auto conv_low = [&](int e) {
             X2 v = A[fx_at(e, s7)];
-            if (inv && e == 0) {
-                dcx = __longlong_as_double(v.x);
-                dcy = __longlong_as_double(v.y);
-                v.x = v.y = 0;
-            }
+            if (inv && e == 0) v.x = v.y = 0;
             v.x = fx_from_low((unsigned)fx_hi(v.x), (unsigned)v.x, E);
             v.y = fx_from_low((unsigned)fx_hi(v.y), (unsigned)v.y, E);
             sx += fx_hi(v.x) >> 9;
@@ -487,6 +486,7 @@ line_fx(const __grid_constant__ FxPack<NJ> jobs, const __grid_constant__ FxPlan 
             }
         }
         out.bad = E == 0x7ff;
+        if (inv) out.bad = out.bad || !(isfinite(out.cx) && isfinite(out.cy));
         if (op1 == OP_FWD || op1 == OP_DEALIAS || op2 == OP_DEALIAS) {
             const int ex = E - 1084;
             out.cx = fx_to(mx, ex, fx_safe(ex));
