@@ -100,7 +100,14 @@ static __device__ __noinline__ long long fx_from_low(unsigned h, unsigned l, int
     const long long p = (long long)((m << 9) >> min(E - (int)max(e, 1u), 63));
     return (int)h < 0 ? -p : p;
 }
+// 2^e in the normal range
+__device__ __forceinline__ double fx_pow2(int e) { return __hiloint2double((1023 + e) << 20, 0); }
 static __device__ __noinline__ double fx_to_slow(long long a, int ex) { return scalbn((double)a, ex); }
+// a con 2^ex for -1100 < ex < 1100 and 2^-400 < con < 2^400, rounded once where it leaves the normal range
+static __device__ __noinline__ double fx_to_far(long long a, int ex, double con)
+{
+    return (double)a * (con * fx_pow2(ex >> 1)) * fx_pow2(ex - (ex >> 1));
+}
 // a 2^ex rounded to double; safe: ex lies in [-1022, 960], where no result
 // with |a| < 2^62 leaves the normal range
 __device__ __forceinline__ bool fx_safe(int ex) { return ex >= -1022 && ex <= 960; }

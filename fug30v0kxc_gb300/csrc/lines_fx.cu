@@ -311,9 +311,6 @@ line_fx(const __grid_constant__ FxPack<NJ> jobs, const __grid_constant__ FxPlan 
             }
             __syncthreads();
         }
-        // (a spectrum's constant is kept apart: it must not set the exponent of a
-        // derivative that does not contain it)
-        double dcx = 0.0, dcy = 0.0;
         auto raw = [&](int e) -> X2 {
             X2 v;
             if (DIR == 0) {
@@ -322,19 +319,29 @@ line_fx(const __grid_constant__ FxPack<NJ> jobs, const __grid_constant__ FxPlan 
             } else {
                 v = A[fx_at(e, s7)];
             }
-            if (inv && e == 0) {
+            return v;
+        };
+        // (a spectrum's constant, lane 0's first element, is kept apart: it must not set
+        // the exponent of a derivative that does not contain it)
+        double dcx = 0.0, dcy = 0.0;
+        auto constant = [&](X2 &v) {
+            if (inv && l == 0) {
                 dcx = __longlong_as_double(v.x);
                 dcy = __longlong_as_double(v.y);
                 v.x = v.y = 0;
             }
-            return v;
         };
-        auto top = [](unsigned m, const X2 &v) {
+        // the largest high word; 0 only for a line of zeros (at rest, truncated, or a
+        // partial tile's), which takes the exponent of 1 and no slow path
+        unsigned low = 0u;
+        auto top = [&](unsigned m, const X2 &v) {
+            low |= (unsigned)v.x | (unsigned)v.y;
             return max(max(m, (unsigned)fx_hi(v.x) & 0x7fffffffu), (unsigned)fx_hi(v.y) & 0x7fffffffu);
         };
         auto group_max = [&](unsigned m) {
+            m = max(m, min(low, 1u));
             for (int o = G >> 1; o > 0; o >>= 1) m = max(m, __shfl_xor_sync(0xffffffffu, m, o));
-            return (int)max(m >> 20, 1u);
+            return m == 0 ? 1023 : (int)max(m >> 20, 1u);
         };
         auto group_sum = [&](float f) {
             for (int o = G >> 1; o > 0; o >>= 1) f += __shfl_xor_sync(0xffffffffu, f, o);
@@ -358,8 +365,11 @@ line_fx(const __grid_constant__ FxPack<NJ> jobs, const __grid_constant__ FxPlan 
         auto means = [&]() {
             if (inv) {
                 const int src = (tid & 31) - l;
-                out.cx = __shfl_sync(0xffffffffu, dcx, src) / (double)n;
-                out.cy = __shfl_sync(0xffffffffu, dcy, src) / (double)n;
+                out.cx = __shfl_sync(0xffffffffu, dcx, src);
+                out.cy = __shfl_sync(0xffffffffu, dcy, src);
+                // (the division takes zeros on a slow path)
+                if (out.cx != 0.0) out.cx /= (double)n;
+                if (out.cy != 0.0) out.cy /= (double)n;
                 return;
             }
             // (an element is 2^21 at most, a lane's sum 2^27: the line's fits 32 bits up
@@ -410,6 +420,7 @@ line_fx(const __grid_constant__ FxPack<NJ> jobs, const __grid_constant__ FxPlan 
                 if (e < n) v[c] = raw(e);
                 else v[c].x = v[c].y = 0;
             }
+            constant(v[0]);
 #pragma unroll
             for (int c = 0; c < CH; c++) m = top(m, v[c]);
             E = group_max(m);
@@ -458,6 +469,7 @@ line_fx(const __grid_constant__ FxPack<NJ> jobs, const __grid_constant__ FxPlan 
                     if (e < n) v[c] = raw(e);
                     else v[c].x = v[c].y = 0;
                 }
+                if (e0 == l) constant(v[0]);
 #pragma unroll
                 for (int c = 0; c < 8; c++) {
                     m = top(m, v[c]);
@@ -606,7 +618,7 @@ line_fx(const __grid_constant__ FxPack<NJ> jobs, const __grid_constant__ FxPlan 
             const double con = op == OP_D1 ? tb.c1 : op == OP_D2 ? tb.c2 : tb.c0;
             // (con 2^xe, and with it every result, in the normal range)
             const bool safe = out.xe >= -700 && out.xe <= 700;
-            out.sc = safe ? con * __hiloint2double((1023 + out.xe) << 20, 0) : 0.0;
+            out.sc = safe ? con * fx_pow2(out.xe) : 0.0;
             const double alpha = o == 0 ? jb.alpha1 : jb.alpha2;
             const int acc = o == 0 ? jb.acc1 : jb.acc2;
             double *ot = o == 0 ? jb.out1 : jb.out2;
@@ -640,8 +652,8 @@ line_fx(const __grid_constant__ FxPack<NJ> jobs, const __grid_constant__ FxPlan 
             }
             auto fin = [&](const X2 v, const FxOut &q, double *va, double *vb, const double *old, size_t step) {
                 const bool ok = q.xe >= -700 && q.xe <= 700;
-                *va = ok ? __ll2double_rn(v.x) * q.sc : fx_to_slow(v.x, q.xe) * con;
-                *vb = ok ? __ll2double_rn(v.y) * q.sc : fx_to_slow(v.y, q.xe) * con;
+                *va = ok ? __ll2double_rn(v.x) * q.sc : fx_to_far(v.x, q.xe, con);
+                *vb = ok ? __ll2double_rn(v.y) * q.sc : fx_to_far(v.y, q.xe, con);
                 if (add) { *va += q.cx; *vb += q.cy; }
                 if (q.bad) *va = *vb = FX_NAN;
                 *va *= alpha;
