@@ -48,20 +48,34 @@ static inline unsigned nblk(size_t n, int tpb = TPB)
 // ============================================================================
 // z-derivative operators (per-operator entry points)
 // ============================================================================
-// (grid (np/256, nz); bound by integer issue with the sums in integers: d1 at
+// A thread's point of the plane kernels: grid (np/256, nz), or one row of CTAs over all
+// points where there are more planes than a grid has rows.
+__device__ __forceinline__ bool zpoint(size_t np, int nz, size_t &q, int &k)
+{
+    q = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
+    k = blockIdx.y;
+    if (gridDim.y == 1) {
+        if (q >= np * nz) return false;
+        k = (int)(q / np);
+        q -= (size_t)k * np;
+    }
+    return q < np;
+}
+static dim3 zgrid(size_t np, int nz) { return nz <= 65535 ? dim3(nblk(np), (unsigned)nz) : dim3(nblk(np * nz)); }
+
+// (bound by integer issue with the sums in integers: d1 at
 // 256^2 x 129 72 -> 55 us, d2 88 -> 65 us against FP64 sums)
 template <int W>
 __global__ void __launch_bounds__(256) k_zderiv(const double *in, const double *w, double *out, int fl, size_t np, int nz, double h)
 {
     PDL_WAIT();
-    const size_t q = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (q >= np) return;
-    const int k = blockIdx.y;
+    size_t q;
+    int k;
+    if (!zpoint(np, nz, q, k)) return;
     const size_t idx = (size_t)k * np + q;
     const ZSum z = zsum<W | ZPIPE>(in + q, np, k, nz, fl, fl, W == ZUP ? w[idx] : 0.0);
     out[idx] = h * (W == ZD1 ? z.d1 : W == ZD2 ? z.d2 : z.up);
 }
-static dim3 zgrid(size_t np, int nz) { return dim3(nblk(np), (unsigned)nz); }
 
 int op_d1z(Engine *E, const double *in, double *out, int flag, int np, int nz)
 {
@@ -134,9 +148,11 @@ int phys_refresh_coefs(Engine *E)
 __global__ void __launch_bounds__(256, 3) k_hydro_pass2(HydroArgs a)
 {
     PDL_WAIT();
-    const size_t np = a.np, q = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (q >= np) return;
-    const int nz = a.nz, k = blockIdx.y;
+    const size_t np = a.np;
+    const int nz = a.nz;
+    size_t q;
+    int k;
+    if (!zpoint(np, nz, q, k)) return;
     const size_t idx = (size_t)k * np + q;
     const double h = a.ho12;
 
@@ -214,9 +230,11 @@ struct Hydro4Args {
 __global__ void __launch_bounds__(256) k_hydro_pass4(Hydro4Args a)
 {
     PDL_WAIT();
-    const size_t np = a.np, q = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (q >= np) return;
-    const int nz = a.nz, k = blockIdx.y;
+    const size_t np = a.np;
+    const int nz = a.nz;
+    size_t q;
+    int k;
+    if (!zpoint(np, nz, q, k)) return;
     const size_t idx = (size_t)k * np + q;
     const double h = a.ho12, w0 = a.w[idx], tt = a.t[idx], ri = a.ri[idx];
     const double d3 = zsum<ZD1 | ZPIPE>(a.p3 + q, np, k, nz, 2, 0).d1, d4 = zsum<ZD1 | ZPIPE>(a.p4 + q, np, k, nz, 5, 0).d1;
@@ -651,7 +669,7 @@ struct CdtArgs {
     double g1, f;
     float *chunk;           // [3][nchunks]: xx max, xz max, rho min estimates
     unsigned *gkey;         // [3]: keys of the global estimates
-    int nchunks, cs;        // chunks in all; points per chunk
+    int nchunks, cpp, cs;   // chunks in all, per plane; points per chunk
     DevScalars *ds;
 };
 
@@ -694,15 +712,15 @@ __device__ __forceinline__ void block_reduce3(float &mx, float &mz, float &mn, f
     }
 }
 
-// (grid: chunks of a plane, planes; a chunk lies in one plane)
+// (grid: the chunks, plane by plane)
 template <int NB, bool MIR>
 __global__ void __launch_bounds__(256) k_calcdt_est(const __grid_constant__ Batch<CdtArgs, NB> bt)
 {
     PDL_WAIT();
     const CdtArgs &a = BATCH_MEMBER(bt, NB);
     __shared__ float sh[96];
-    const int k = blockIdx.y, c = k * gridDim.x + blockIdx.x;
-    const size_t p0 = (size_t)k * a.np, i0 = p0 + (size_t)blockIdx.x * a.cs;
+    const int c = blockIdx.x, k = c / a.cpp;
+    const size_t p0 = (size_t)k * a.np, i0 = p0 + (size_t)(c - k * a.cpp) * a.cs;
     const size_t i1 = i0 + a.cs < p0 + a.np ? i0 + a.cs : p0 + a.np;
     const float rb = MIR ? (float)a.r0[k] : 0.0f, tb = MIR ? (float)a.t0[k] : 0.0f, bb = (float)a.bzbar;
     float mx = -INFINITY, mz = -INFINITY, mn = INFINITY;
@@ -743,10 +761,10 @@ __global__ void __launch_bounds__(256) k_calcdt_exact(const __grid_constant__ Ba
     const float tx = gx * (gx >= 0.0f ? 1.0f - CDT_MARGIN : 1.0f + CDT_MARGIN);
     const float tz = gz * (gz >= 0.0f ? 1.0f - CDT_MARGIN : 1.0f + CDT_MARGIN);
     const float tr = gr * (gr >= 0.0f ? 1.0f + CDT_MARGIN : 1.0f - CDT_MARGIN) + (MIR ? CDT_ABS : 0.0f);
-    const int k = blockIdx.y, c = k * gridDim.x + blockIdx.x;
+    const int c = blockIdx.x, k = c / a.cpp;
     const bool fx = a.chunk[c] >= tx, fz = a.chunk[a.nchunks + c] >= tz, fr = a.chunk[2 * a.nchunks + c] <= tr;
     if (!(fx || fz || fr)) return;
-    const size_t p0 = (size_t)k * a.np, i0 = p0 + (size_t)blockIdx.x * a.cs;
+    const size_t p0 = (size_t)k * a.np, i0 = p0 + (size_t)(c - k * a.cpp) * a.cs;
     const size_t i1 = i0 + a.cs < p0 + a.np ? i0 + a.cs : p0 + a.np;
     const float rb = MIR ? (float)a.r0[k] : 0.0f, tb = MIR ? (float)a.t0[k] : 0.0f, bb = (float)a.bzbar;
     double mxx = -1.0e-50, mxz = -1.0e-50, mn = 1.0e300;
@@ -827,6 +845,7 @@ static CdtArgs cdt_args(Engine *E)
     a.r0 = E->split ? split_bg_rho0(E) : nullptr; a.t0 = E->split ? split_bg_t0(E) : nullptr;
     a.np = E->np; a.g1 = E->k.g1; a.f = E->k.f;
     a.nchunks = cdt_chunks(E->np, E->nz);
+    a.cpp = a.nchunks / E->nz;
     a.cs = cdt_chunk(E->np);
     a.gkey = reinterpret_cast<unsigned *>(E->cdt);
     a.chunk = E->cdt + 4;
@@ -843,7 +862,7 @@ bool cdt_mirrors_ok(const Engine &E)
 int phys_calcdt_m(Engine *const *Es, int nE, bool mirrors)
 {
     Engine *E = Es[0];
-    const dim3 grid((unsigned)((E->np + cdt_chunk(E->np) - 1) / cdt_chunk(E->np)), (unsigned)E->nz);
+    const dim3 grid((unsigned)cdt_chunks(E->np, E->nz));
     int st;
     if ((st = launch_members<CdtArgs>(Es, nE, "calcdt_est", FB(E, 8, mirrors ? 4 : 8), grid, dim3(256), 0,
                                       mirrors ? k_calcdt_est<1, true> : k_calcdt_est<1, false>,
