@@ -199,7 +199,7 @@ static void set_consts(Engine &E)
     c.dtdiff0z = 0.2 * c.dz * c.dz / p.gamma / p.ck * (1.0 + p.theta / 7.0);
     // src/dbydz.F90:360-361
     c.ho12 = (double)(E.nz - 1) / 12.0;
-    c.sc1 = (double)((E.nz - 1) * (E.nz - 1)) / 12.0;
+    c.sc1 = (double)(E.nz - 1) * (double)(E.nz - 1) / 12.0;
     c.f = p.f; c.gamma = p.gamma; c.theta = p.theta; c.sf = p.sf;
     c.var_eta = p.eta_contrast != 1.0;
     c.icutoffx = (E.nx / 2) / 3;

@@ -45,3 +45,14 @@ def test_step(nz):
     assert np.isfinite(dt) and dt > 0.0
     assert g.step(1) == 0
     g.close()
+
+
+@pytest.mark.parametrize("nz", [46341, 46342, 70000])
+def test_second_derivative(nz):
+    """(nz - 1)^2 does not fit 32 bits above 46341 planes."""
+    g = P3D(convection_params(4, 4, nz))
+    f = np.random.default_rng(nz).standard_normal((nz, 4, 4))
+    s, x = (nz - 1) ** 2 / 12.0, f.astype(np.longdouble)
+    d2 = s * (-x[:-4] + 16 * x[1:-3] - 30 * x[2:-2] + 16 * x[3:-1] - x[4:])
+    assert np.abs(g.d2bydz(f, 3)[2:-2] - d2).max() <= s * 700 * 2.0 ** -52 * np.abs(f).max()
+    g.close()
