@@ -4,6 +4,9 @@ hydro right-hand sides, calcdt and a step.
 The operators against their own stencils in long double on interior planes (bound: that
 of the z stencil tests), the right-hand sides of a state that repeats every 40 planes by
 planes 40 apart: away from the walls they have equal bits."""
+import ctypes as C
+import time
+
 import numpy as np
 import pytest
 
@@ -56,3 +59,23 @@ def test_second_derivative(nz):
     d2 = s * (-x[:-4] + 16 * x[1:-3] - 30 * x[2:-2] + 16 * x[3:-1] - x[4:])
     assert np.abs(g.d2bydz(f, 3)[2:-2] - d2).max() <= s * 700 * 2.0 ** -52 * np.abs(f).max()
     g.close()
+
+
+def test_columns_fill_their_blocks():
+    """A column of 60000 values takes a call's fixed time, as one of 1000 does (with a CTA per
+    value it took three times as long)."""
+    torch = pytest.importorskip("torch")
+    ts = []
+    for nz in (1000, 60000):
+        g = P3D(convection_params(4, 4, nz))
+        f = torch.randn(nz, dtype=torch.float64, device="cuda")
+        o = torch.empty_like(f)
+        t = []
+        for _ in range(100):
+            torch.cuda.synchronize()
+            t0 = time.perf_counter()
+            assert g.L.vec_d1bydz1d(g.h, C.c_void_p(f.data_ptr()), C.c_void_p(o.data_ptr()), 5) == 0
+            t.append(time.perf_counter() - t0)
+        ts.append(sorted(t)[25])
+        g.close()
+    assert ts[1] <= 1.8 * ts[0], ts
