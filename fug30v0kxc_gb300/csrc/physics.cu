@@ -67,37 +67,40 @@ static dim3 zgrid(size_t np, int nz) { return nz <= 65535 && np >= TPB / 2 ? dim
 
 // (bound by integer issue with the sums in integers: d1 at
 // 256^2 x 129 72 -> 55 us, d2 88 -> 65 us against FP64 sums)
-template <int W>
+template <int W, bool ROW>
 __global__ void __launch_bounds__(256) k_zderiv(const double *in, const double *w, double *out, int fl, size_t np, int nz, double h)
 {
     PDL_WAIT();
-    size_t q;
-    int k;
-    if (!zpoint(np, nz, q, k)) return;
+    size_t q = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
+    int k = blockIdx.y;
+    if (ROW ? !zpoint(np, nz, q, k) : q >= np) return;
     const size_t idx = (size_t)k * np + q;
     const ZSum z = zsum<W | ZPIPE>(in + q, np, k, nz, fl, fl, W == ZUP ? w[idx] : 0.0);
     out[idx] = h * (W == ZD1 ? z.d1 : W == ZD2 ? z.d2 : z.up);
 }
 
+template <int W>
+static int zderiv(Engine *E, const char *name, double bytes, const double *in, double *out, int flag, size_t np, int nz, double h)
+{
+    const dim3 g = zgrid(np, nz);
+    if (g.y == 1) KLAUNCHB(E, name, bytes, (k_zderiv<W, true>), g, TPB, in, E->w, out, flag, np, nz, h);
+    else KLAUNCHB(E, name, bytes, (k_zderiv<W, false>), g, TPB, in, E->w, out, flag, np, nz, h);
+    return VEC_OK;
+}
 int op_d1z(Engine *E, const double *in, double *out, int flag, int np, int nz)
 {
     if (!(flag == 0 || flag == 1 || flag == 2 || flag == 5)) return VEC_ERR_FLAG;
-    KLAUNCHB(E, "d1bydz_f64", 2.0 * np * nz * 8, k_zderiv<ZD1>, zgrid(np, nz), TPB, in, (const double *)nullptr, out, flag,
-             (size_t)np, nz, E->k.ho12);
-    return VEC_OK;
+    return zderiv<ZD1>(E, "d1bydz_f64", 2.0 * np * nz * 8, in, out, flag, np, nz, E->k.ho12);
 }
 int op_d1upz(Engine *E, const double *in, double *out, int flag)
 {
     if (!(flag == 0 || flag == 1 || flag == 2 || flag == 5)) return VEC_ERR_FLAG;
-    KLAUNCHB(E, "d1upbydz_f64", FB(E, 3, 8), k_zderiv<ZUP>, zgrid(E->np, E->nz), TPB, in, E->w, out, flag, E->np, E->nz, E->k.ho12);
-    return VEC_OK;
+    return zderiv<ZUP>(E, "d1upbydz_f64", FB(E, 3, 8), in, out, flag, E->np, E->nz, E->k.ho12);
 }
 int op_d2z(Engine *E, const double *in, double *out, int flag, int np, int nz)
 {
     if (!(flag == 0 || flag == 3)) return VEC_ERR_FLAG;
-    KLAUNCHB(E, "d2bydz_f64", 2.0 * np * nz * 8, k_zderiv<ZD2>, zgrid(np, nz), TPB, in, (const double *)nullptr, out, flag,
-             (size_t)np, nz, E->k.sc1);
-    return VEC_OK;
+    return zderiv<ZD2>(E, "d2bydz_f64", 2.0 * np * nz * 8, in, out, flag, np, nz, E->k.sc1);
 }
 
 // ============================================================================
@@ -229,7 +232,7 @@ struct Hydro4Args {
 // :443-497 (d(rho)/dz with the boundary override, division by rho).  With the
 // z stencils summed in integers and 1 / rho from pass 2, 11 FP64 operations per
 // point are left of 53: 0.72 -> 0.41 ms at 256^2 x 129.
-__global__ void __launch_bounds__(256) k_hydro_pass4(Hydro4Args a)
+__global__ void __launch_bounds__(256, 5) k_hydro_pass4(Hydro4Args a)
 {
     PDL_WAIT();
     const size_t np = a.np;

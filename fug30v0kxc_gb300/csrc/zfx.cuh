@@ -4,11 +4,12 @@
 // or five FP64 operations of 37 issue slots each on GB300 (2 per clock and SM).
 // Here the neighbours are aligned to their largest exponent (14 integer
 // instructions each, shared by all the stencils of a field at a point), summed
-// exactly, and the sum rounded once (20 instructions).  Three bits below the
+// in integers, and the sum rounded once (20 instructions).  Three bits below the
 // largest value's last one are kept, so that neighbours of up to an eighth of it
-// enter whole; the weights' absolute sum is at most 64, and the sum below 2^62.
-// The result's error is that of one rounding, where the FP64 sum has one per
-// operation.
+// enter whole; what smaller ones lose, less than a unit of 2^-3 each, enters with
+// the weights (their absolute sum is at most 64, and the sum below 2^62): at most 8
+// units in the last place of the largest neighbour, and the one rounding, where the
+// FP64 sum has a rounding per operation.
 #pragma once
 #include <stdint.h>
 
@@ -79,22 +80,51 @@ struct ZSum { double d1, d2, up; };
 
 // the stencils W of one column at plane k without their factors (F(k): plane k
 // of the column; the wall rows' flags f1, f2 for d1 and up, d2)
+//
+// The stencils share one alignment, to the largest of all planes that any of them
+// reads.  One whose own planes are more than four times smaller would lose bits to a
+// plane it does not read, more than its FP64 sum rounds off (at four times as large
+// the truncation is at most 4 / 8 of the weights' sum in the last bits of its own
+// largest plane, 9, 32 and 19, and the FP64 sums' intermediate results round off 17,
+// 57 and 35): there all are summed in FP64.
 template <int W, typename A>
 __device__ __forceinline__ ZSum zsum(const A &F, int k, int nz, int f1, int f2, double w0)
 {
     ZSum z = { 0.0, 0.0, 0.0 };
     if (k >= 3 && k <= nz - 4) {
+        const bool pos = w0 >= 0.0;
+        int E;
+        if constexpr ((W & (ZD1 | ZD2 | ZUP)) == ZUP) {
+            // (the five planes it reads, against the flow in mirror image)
+            double f[5];
+            long long v[5];
+#pragma unroll
+            for (int d = 0; d < 5; d++) f[d] = F(pos ? k - 3 + d : k + 3 - d);
+            if (zi_align<5>(f, v, E)) {
+                const long long t = v[1] - v[2] - (v[2] << 1);
+                const long long s = (t << 2) + (t << 1) - v[0] + (v[3] << 3) + (v[3] << 1) + v[4] + (v[4] << 1);
+                z.up = W & ZPIPE ? zi_to_pipe(pos ? s : -s, E) : zi_to(pos ? s : -s, E);
+                return z;
+            }
+            z.up = zd1upa(F, k, nz, f1, 1.0, w0);
+            return z;
+        }
         double f[7];
         long long v[7];
-        int E;
         // (the planes the wanted stencils do not read count as zero)
 #pragma unroll
         for (int d = 0; d < 7; d++) f[d] = (d == 0 || d == 6) && !(W & ZUP) ? 0.0 : d == 3 && !(W & (ZD2 | ZUP)) ? 0.0 : F(k - 3 + d);
-        if (zi_align<7>(f, v, E)) {
+        // the smallest of the stencils' own largest planes
+        auto top = [&](int d) { return (unsigned)__double2hiint(f[d]) & 0x7fffffffu; };
+        unsigned m = 0xffffffffu;
+        if (W & ZUP) m = max(max(max(top(2), top(4)), top(3)), pos ? max(top(0), top(1)) : max(top(5), top(6)));
+        if ((W & ZD1) && (W & (ZD2 | ZUP))) m = min(m, max(max(top(1), top(5)), max(top(2), top(4))));
+        else if ((W & ZD2) && (W & ZUP)) m = min(m, max(max(max(top(1), top(5)), max(top(2), top(4))), top(3)));
+        if (zi_align<7>(f, v, E) && (m >= (unsigned)(E - 2) << 20 || E <= 66)) {     // (E = 64: all zeros)
             auto to = [&](long long s) { return W & ZPIPE ? zi_to_pipe(s, E) : zi_to(s, E); };
             if (W & ZD1) z.d1 = to(zi_sum1(v));
             if (W & ZD2) z.d2 = to(zi_sum2(v));
-            if (W & ZUP) z.up = to(zi_sumup(v, w0 >= 0.0));
+            if (W & ZUP) z.up = to(zi_sumup(v, pos));
             return z;
         }
     }
