@@ -23,14 +23,21 @@
 // group in scalar FP32 and two levels (lines_ct.cu) took 65 % of the issue slots, with
 // half of a 512-point line's threads idle on the first of 32 x 16 levels.  Pairs halve
 // the arithmetic, the exchanges and the stores at once, and three levels of 8 keep
-// all 64 threads busy with 32 registers per spectrum.  One sequence per group with
+// all 64 threads busy with 32 registers per spectrum.  (A factor of 3 is in the last level,
+// C = 6 or 12, and an 8 ends on fours: what a last stage rounds off repeats at n / its
+// radix, and a second derivative weighs it by the fourth power.  With the 3 in the middle
+// the second derivative of a smooth 384- or 768-point line erred 6 % more than with two
+// levels, of a constant plus little 9 to 38 %.)  One sequence per group with
 // sums on (re, im) pairs, twice the threads: 512^2 y lines 17 % slower; groups of
 // eight y columns with barriers of their own: 32-byte rows, 8-30 % slower.  Nothing
 // may spill: what shared memory leaves of L1 does not hold it (28 bytes a thread:
 // 512^2 y lines 12-20 % slower).  A derivative pair, x and y, before -> now (us, two
-// runs of one side differ by 3 %; the error against FP64 falls by 2-8 %):
-//    384^2 x 65    53.1  48.9 ->  44.5  41.0      768^2 x 33   104.1 100.0 ->  76.2  83.1
-//    512^2 x 65    92.6  67.4 ->  60.4  61.7     1024^2 x 33   153.3 140.2 -> 122.7 135.8
+// runs of one side differ by 3 %):
+//    384^2 x 65    53.1  48.9 ->  43.5  41.6      768^2 x 33   104.1 100.0 ->  73.0  82.5
+//    512^2 x 65    92.6  67.4 ->  60.1  62.0     1024^2 x 33   153.3 140.2 -> 122.4 133.7
+// The error against FP64 (rms of d1, d2 and dealias) falls by 6 to 13 % for white noise, by
+// 1 to 13 % for lines of few waves with and without noise, and stays for a constant plus
+// little.
 // (Up to 256 points pairs on two levels took 3-8 % less, 34.4 -> 31.5 at 256^2 x 129,
 // which is not worth other rounding in every step, restart and training set of those
 // grids: lines_ct.cu keeps their results bit for bit.)
@@ -152,18 +159,23 @@ template <bool INV> __device__ __forceinline__ void dft3(Z &a, Z &b, Z &c)
     c = zfma<INV, 3>(u, d, h);
 }
 template <int N, bool INV> struct ZDft;
+// 8 = 2 x 4 and 16 = 4 x 4, the fours last: what a last stage of twos rounds off lies at
+// the highest wavenumbers, where a second derivative weighs it most
 template <bool INV> struct ZDft<8, INV> {
     static __device__ __forceinline__ void run(Z *v)
     {
         const float h = 0.7071067811865476f;
-        dft4<INV>(v[0], v[2], v[4], v[6]);
-        dft4<INV>(v[1], v[3], v[5], v[7]);
-        const Z e0 = v[0], e1 = v[2], e2 = v[4], e3 = v[6], o0 = v[1], o2 = v[5];
-        const Z o1 = zw8<INV>(v[3]), o3 = zw8<INV>(v[7]);
-        v[0] = zadd<INV, 0>(e0, o0); v[4] = zadd<INV, 2>(e0, o0);
-        v[1] = zfma<INV, 0>(e1, o1, h); v[5] = zfma<INV, 2>(e1, o1, h);
-        v[2] = zadd<INV, 1>(e2, o2); v[6] = zadd<INV, 3>(e2, o2);
-        v[3] = zfma<INV, 1>(e3, o3, h); v[7] = zfma<INV, 3>(e3, o3, h);
+        Z b[4];
+#pragma unroll
+        for (int m = 0; m < 4; m++) {
+            b[m] = zadd<INV, 2>(v[m], v[m + 4]);
+            v[m] = zadd<INV, 0>(v[m], v[m + 4]);
+        }
+        Z o[8];
+        dft4<INV, 0, 0, 0, false, false>(v[0], v[1], v[2], v[3], h, o[0], o[2], o[4], o[6]);
+        dft4<INV, 0, 1, 1, false, true>(b[0], zw8<INV>(b[1]), b[2], zw8<INV>(b[3]), h, o[1], o[3], o[5], o[7]);
+#pragma unroll
+        for (int k = 0; k < 8; k++) v[k] = o[k];
     }
 };
 template <bool INV> struct ZDft<16, INV> {
@@ -221,10 +233,9 @@ template <bool INV> struct ZDft<12, INV> {
 
 // ---- shape ---------------------------------------------------------------------------
 // DIR 0: x lines (a tile = 2S contiguous rows), DIR 1: y lines (a tile = 2S adjacent
-// columns over all ny rows).  C = 1: two levels.
+// columns over all ny rows).
 template <int DIR, int A, int B, int C, int S>
 struct CpShape {
-    static constexpr int cmax(int a, int b) { return a > b ? a : b; }
     static constexpr int N = A * B * C;
     static constexpr int NG = S / 2;                      // groups of four lines
     static constexpr int RL = C;                          // radix of the last level
@@ -239,17 +250,15 @@ struct CpShape {
     static constexpr int D2 = (A * C + T - 1) / T, DL = (NL + T - 1) / T;
     static constexpr int GT = 4 * N;                      // reals of a group in the tile
     static constexpr int TILE = NG * GT;
-    static constexpr int XS = M, GX = A * XS;             // rows of the first exchange, in points
-    // twiddle rows: W^(j x) for j = 1, 2, 3, 4, 8, 12 and the others as products of two
-    // (loads in their place cost the 512-point launches 2 %).  Products err more: a
-    // transform against FP64 with them in both exchanges 2.5-3 %, and 1024 points have
-    // all rows of the second one, so that every length errs less than with two levels.
-    static constexpr bool ALL2 = A > 8;
-    static constexpr int H1 = A / 4 - 1, R1 = 3 + H1;
-    static constexpr int H2 = (B + 3) / 4 - 1, R2 = ALL2 ? B - 1 : 3 + H2;
-    static constexpr size_t SMEM = 4 * (2 * (size_t)TILE + 4 * (size_t)NG * GX + 4 * (size_t)(R1 * M + R2 * C) + 6 * (size_t)N);
+    // rows of the first exchange, in points; the lanes of its second level run over k1
+    // (unless C = 8, where they run over c first), an odd row apart
+    static constexpr int XS = C == 8 ? M : M + 1, GX = A * XS;
+    // twiddle rows W^(j x), all of them (products of two of them in place of some err 2-3 %
+    // more per exchange)
+    static constexpr int R1 = A - 1, R2 = B - 1;
+    static constexpr size_t SMEM = 4 * (2 * (size_t)TILE + 4 * (size_t)NG * GX + 2 * (size_t)(R1 * M) + 4 * (size_t)(R2 * C) + 6 * (size_t)N);
     static constexpr int MINB = NT <= 256 && 2 * (SMEM + 1152) <= 233472 ? 2 : 1;
-    static_assert(T >= M && C == 8 && SMEM + 128 <= 232448, "shape");
+    static_assert(T >= M && (C == 8 || M % 2 == 0) && SMEM + 128 <= 232448, "shape");
     static_assert(GX >= N, "spectra fit the exchange");
 };
 
@@ -272,9 +281,9 @@ line_cp(const __grid_constant__ JobPackCP<NJ> jobs, const __grid_constant__ Tmap
     extern __shared__ __align__(128) unsigned char smem[];
     float *tile0 = reinterpret_cast<float *>(smem);
     Z *ex = reinterpret_cast<Z *>(tile0 + 2 * TILE);
-    Tw *tw1 = reinterpret_cast<Tw *>(ex + P::NG * P::GX);   // [row][m']
-    Tw *tw2 = tw1 + P::R1 * M;                                 // [row][c]
-    float2 *mul = reinterpret_cast<float2 *>(tw2 + P::R2 * C);  // multipliers: d1, d2, dealias
+    Tw *tw2 = reinterpret_cast<Tw *>(ex + P::NG * P::GX);   // [row][c]
+    float2 *tw1 = reinterpret_cast<float2 *>(tw2 + P::R2 * C);  // [row][m']: cosine and sine
+    float2 *mul = tw1 + P::R1 * M;  // multipliers: d1, d2, dealias
     __shared__ __align__(8) uint64_t bar[4];                   // full[2], empty[2]
 
     const int tid = threadIdx.x;
@@ -291,9 +300,10 @@ line_cp(const __grid_constant__ JobPackCP<NJ> jobs, const __grid_constant__ Tmap
         const bool first = e < P::R1 * M;
         const int q = first ? e : e - P::R1 * M, w = first ? M : C;
         const int r = q / w, x = q - r * w;
-        const int j = (!first && P::ALL2) || r < 3 ? r + 1 : 4 * (r - 2);
+        const int j = r + 1;
         const float2 v = tb.tw[(first ? j * x : A * j * x) % N];
-        tw1[e] = Tw{ bc2(v.x), bc2(-v.y) };
+        if (first) tw1[q] = make_float2(v.x, -v.y);
+        else tw2[q] = Tw{ bc2(v.x), bc2(-v.y) };
     }
     for (int e = tid; e < N; e += NT) {
         mul[e] = bc2(tb.m1[e]);
@@ -341,18 +351,13 @@ line_cp(const __grid_constant__ JobPackCP<NJ> jobs, const __grid_constant__ Tmap
     };
 
     Z *exg = ex + unit * ST * P::GX + side;
-    // twiddle rows of column x; the factor of index k
-    auto twrow = [](const Tw *tab, int w, int x, int nhi, Tw *lo, Tw *hi) {
-#pragma unroll
-        for (int j = 0; j < 3; j++) lo[j] = tab[j * w + x];
-#pragma unroll
-        for (int j = 0; j < nhi; j++) hi[j] = tab[(3 + j) * w + x];
+    // the second level's k1 and c; the places of the second exchange, which uses the tile's
+    // buffer
+    auto lev2 = [](int q, int &k1, int &c) {
+        k1 = C == 8 ? q / C : q % A;
+        c = C == 8 ? q % C : q / A;
     };
-    auto twk = [](int k, const Tw *lo, const Tw *hi) {
-        return (k >> 2) == 0 ? lo[(k & 3) - 1] : ((k & 3) == 0 ? hi[(k >> 2) - 1] : twmul(hi[(k >> 2) - 1], lo[(k & 3) - 1]));
-    };
-    // places of the second exchange, which uses the tile's buffer
-    auto x2 = [](int k1, int k2, int c) { return (k2 * A + k1) * 8 + (c ^ (k1 & 7)); };
+    auto x2 = [](int k1, int k2, int c) { return C == 8 ? (k2 * A + k1) * 8 + (c ^ (k1 & 7)) : c * NL + k2 * A + k1; };
 
     int issued = 0;
     if (tid == 0) {
@@ -413,26 +418,24 @@ line_cp(const __grid_constant__ JobPackCP<NJ> jobs, const __grid_constant__ Tmap
 #pragma unroll
                 for (int m = 0; m < A; m++) a[m] = tile_z(lane + M * m);
                 ZDft<A, false>::run(a);
-                Tw lo[3], hi[P::H1];
-                twrow(tw1, M, lane, P::H1, lo, hi);
                 exg[ST * lane] = a[0];
 #pragma unroll
-                for (int k = 1; k < A; k++) exg[ST * (k * XS + lane)] = ztw<false>(a[k], twk(k, lo, hi));
+                for (int k = 1; k < A; k++) exg[ST * (k * XS + lane)] = ztw<false>(a[k], tw1[(k - 1) * M + lane].x, tw1[(k - 1) * M + lane].y);
             }
             sync();
 #pragma unroll
             for (int d = 0; d < P::D2; d++) {
-                const int q = lane + T * d, k1 = q / C, c = q % C;
+                const int q = lane + T * d;
+                int k1, c;
+                lev2(q, k1, c);
                 if ((A * C) % T == 0 || q < A * C) {
                     Z b[B];
 #pragma unroll
                     for (int m = 0; m < B; m++) b[m] = exg[ST * (k1 * XS + C * m + c)];
                     ZDft<B, false>::run(b);
-                    Tw lo[3], hi[P::H2 + 1];
-                    if constexpr (!P::ALL2) twrow(tw2, C, c, P::H2, lo, hi);
                     xg[ST * x2(k1, 0, c)] = b[0];
 #pragma unroll
-                    for (int k = 1; k < B; k++) xg[ST * x2(k1, k, c)] = ztw<false>(b[k], P::ALL2 ? tw2[(k - 1) * C + c] : twk(k, lo, hi));
+                    for (int k = 1; k < B; k++) xg[ST * x2(k1, k, c)] = ztw<false>(b[k], tw2[(k - 1) * C + c]);
                 }
             }
             sync();
@@ -526,14 +529,14 @@ line_cp(const __grid_constant__ JobPackCP<NJ> jobs, const __grid_constant__ Tmap
             sync();
 #pragma unroll
             for (int d = 0; d < P::D2; d++) {
-                const int q = lane + T * d, k1 = q / C, c = q % C;
+                const int q = lane + T * d;
+                int k1, c;
+                lev2(q, k1, c);
                 if ((A * C) % T == 0 || q < A * C) {
                     Z b[B];
-                    Tw lo[3], hi[P::H2 + 1];
-                    if constexpr (!P::ALL2) twrow(tw2, C, c, P::H2, lo, hi);
                     b[0] = xg[ST * x2(k1, 0, c)];
 #pragma unroll
-                    for (int k = 1; k < B; k++) b[k] = ztw<true>(xg[ST * x2(k1, k, c)], P::ALL2 ? tw2[(k - 1) * C + c] : twk(k, lo, hi));
+                    for (int k = 1; k < B; k++) b[k] = ztw<true>(xg[ST * x2(k1, k, c)], tw2[(k - 1) * C + c]);
                     ZDft<B, true>::run(b);
 #pragma unroll
                     for (int m = 0; m < B; m++) exg[ST * (k1 * XS + C * m + c)] = b[m];
@@ -544,11 +547,9 @@ line_cp(const __grid_constant__ JobPackCP<NJ> jobs, const __grid_constant__ Tmap
             if (WS && o == nout - 1 && (tid & 31) == 0) mbar_arrive(&bar[2 + (it & 1)]);
             if (M % T == 0 || lane < M) {
                 Z a[A];
-                Tw lo[3], hi[P::H1];
-                twrow(tw1, M, lane, P::H1, lo, hi);
                 a[0] = exg[ST * lane];
 #pragma unroll
-                for (int k = 1; k < A; k++) a[k] = ztw<true>(exg[ST * (k * XS + lane)], twk(k, lo, hi));
+                for (int k = 1; k < A; k++) a[k] = ztw<true>(exg[ST * (k * XS + lane)], tw1[(k - 1) * M + lane].x, tw1[(k - 1) * M + lane].y);
                 ZDft<A, true>::run(a);
                 const float f = op == OP_INV ? alpha / (float)N : alpha;
                 float addv = 0.0f;
@@ -633,8 +634,8 @@ int launch_lines_cp(Engine *E, int dir, const LineJob<float> *jobs, int nj, int 
     const int n = dir == 0 ? E->nx : E->ny;
 #define CP_CASE(NN, A, B, C, SS)                                                                     \
     if (n == NN && S == SS) return dir == 0 ? run_cp<0, A, B, C, SS>(E, jobs, nj, name) : run_cp<1, A, B, C, SS>(E, jobs, nj, name);
-    CP_CASE(384, 8, 6, 8, 8) CP_CASE(512, 8, 8, 8, 8) CP_CASE(768, 8, 12, 8, 8) CP_CASE(1024, 16, 8, 8, 8)
-    CP_CASE(768, 8, 12, 8, 4) CP_CASE(1024, 16, 8, 8, 4)
+    CP_CASE(384, 8, 8, 6, 8) CP_CASE(512, 8, 8, 8, 8) CP_CASE(768, 8, 8, 12, 8) CP_CASE(1024, 16, 8, 8, 8)
+    CP_CASE(768, 8, 8, 12, 4) CP_CASE(1024, 16, 8, 8, 4)
 #undef CP_CASE
     return -1;
 }
