@@ -279,7 +279,8 @@ extern "C" int vec_create(const vec_params *p, vec_ctx **out)
     }
     set_consts(E);
     int st;
-    if ((st = fx_plan_make(E.nx, &E.fpx)) || (st = fx_plan_make(E.ny, &E.fpy))) {
+    if ((st = fx_plan_make(E.nx, &E.fpx)) || (st = fx_plan_make(E.ny, &E.fpy)) || (st = fs_plan_make(E.nx, &E.fspx)) ||
+        (st = fs_plan_make(E.ny, &E.fspy))) {
         vec_set_error("line lengths nx=%d ny=%d are not supported (2^a 3^b 5^c <= 2048)", E.nx, E.ny);
         delete c;
         return st;
@@ -322,8 +323,8 @@ extern "C" int vec_create(const vec_params *p, vec_ctx **out)
     }
     if ((st = fx_tables_make(E.nx, &E.fpx, akx1.data(), akx2.data(), E.k.icutoffx, &E.fxx)) ||
         (st = fx_tables_make(E.ny, &E.fpy, aky1.data(), aky2.data(), E.k.icutoffy, &E.fxy)) ||
-        (st = fs_tables_make(E.nx, E.fpx, E.fxx, akx1.data(), akx2.data(), E.k.icutoffx, &E.fsx)) ||
-        (st = fs_tables_make(E.ny, E.fpy, E.fxy, aky1.data(), aky2.data(), E.k.icutoffy, &E.fsy)) ||
+        (st = fs_tables_make(E.fspx, akx1.data(), akx2.data(), E.k.icutoffx, &E.fsx)) ||
+        (st = fs_tables_make(E.fspy, aky1.data(), aky2.data(), E.k.icutoffy, &E.fsy)) ||
         (st = line_tables_make<float>(E.nx, akx1.data(), akx2.data(), E.k.icutoffx, &E.tx32)) ||
         (st = line_tables_make<float>(E.ny, aky1.data(), aky2.data(), E.k.icutoffy, &E.ty32)) ||
         (E.split && ct64_length(E.nx) && ct64_length(E.ny) &&

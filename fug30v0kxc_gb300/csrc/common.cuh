@@ -52,7 +52,7 @@ struct LineTables {
     R *mda;                 // dealias mask (1/n or 0)
 };
 
-// the general line kernels' passes for a length n (lines_fx.cu): radix, block and
+// the FP64 line kernel's passes for a length n (lines_fx.cu): radix, block and
 // stride of each, ceil(2^31 / stride), and where its twiddles start
 struct FxPlan {
     int n, nb;              // length; elements of a buffer (n rounded up to 8)
@@ -76,11 +76,22 @@ struct FxTables {
     double c0, c1, c2;
 };
 
-// the FP32 general line kernel's tables: twiddles by pass, multipliers by position
+// the FP32 general line kernel's passes (lines.cu): radices, the strides of the forward and
+// the inverse pass of each, ceil(2^31 / stride), and where their twiddles start
+struct FsPlan {
+    int n, np, R[8];
+    int fM[8], iM[8], ftw[8], itw[8];
+    unsigned fmg[8], img[8];
+    int ntw;                // twiddles in all
+    int Q;                  // sequences per warp
+    int nb, sha, shb;       // words of a buffer; padding of the first and the second one
+};
+// its tables: twiddles by pass; multipliers, wavenumber and place in the spectrum by the
+// element of the first inverse pass
 struct FsTables {
-    float2 *tw;             // (one allocation with the multipliers)
-    const unsigned short *pos, *kof;    // the FxTables'
+    float2 *tw;             // (one allocation with the others)
     float *m1, *m2, *mda;
+    unsigned short *pos, *gat;
 };
 
 // horizontal wavenumber tables in one precision: akx1, aky1 and the

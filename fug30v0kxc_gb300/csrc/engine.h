@@ -51,9 +51,10 @@ struct Engine {
     int dev = 0;                // the context's device
     int generic_lines = 0;      // force the generic line kernel (VEC_GENERIC_LINES=1)
 
-    FxPlan fpx = {}, fpy = {};  // passes of the general line kernels
-    FxTables fxx = {}, fxy = {};        // FP64
-    FsTables fsx = {}, fsy = {};        // FP32
+    FxPlan fpx = {}, fpy = {};          // FP64 lines
+    FxTables fxx = {}, fxy = {};
+    FsPlan fspx = {}, fspy = {};        // FP32 lines, general kernel
+    FsTables fsx = {}, fsy = {};
     LineTables<float> tx32, ty32;
     LineTables<double> tx64, ty64;   // split, both lengths among lines_ct64.cu's: else null
 
@@ -221,13 +222,14 @@ int fx_plan_make(int n, FxPlan *pl);
 int fx_tables_make(int n, FxPlan *pl, const double *k1, const double *k2, int icut, FxTables *tb);
 void fx_tables_free(FxTables *tb);
 // rounds of a group of 32 / q lanes through a plan's passes
-inline int fx_rounds(const FxPlan &pl, int q)
+template <typename P> inline int fx_rounds(const P &pl, int q)
 {
     int r = 0;
     for (int p = 0; p < pl.np; p++) r += (pl.n / pl.R[p] * q + 31) / 32;
     return r;
 }
-int fs_tables_make(int n, const FxPlan &pl, const FxTables &fx, const double *k1, const double *k2, int icut, FsTables *tb);
+int fs_plan_make(int n, FsPlan *pl);
+int fs_tables_make(const FsPlan &pl, const double *k1, const double *k2, int icut, FsTables *tb);
 void fs_tables_free(FsTables *tb);
 int line_ct_configure();
 int line_ct64_configure();

@@ -2,19 +2,27 @@
 // line length 2^a 3^b 5^c (FP64: lines_fx.cu; the lengths of the split step's
 // usual grids: lines_ct.cu).
 //
-// The passes of lines_fx.cu in FP32: a group of G = 32 / Q lanes owns a sequence
-// z = a + i b of two real lines in shared memory and runs radix-8/6/5/4/3/2
-// passes on it in place, decimating in frequency forward and in time back, so
-// that the spectrum stays in digit-reversed order and the operators' Hermitian
-// multipliers (+ik, -k^2, the 2/3 truncation) are tables in that order.  Only the
-// halfcomplex transforms go through the permutation.  Warps synchronise their
-// passes alone; the CTA meets for the row-by-row loads and stores of y lines.
+// A group of G = 32 / Q lanes owns a sequence z = a + i b of two real lines in shared
+// memory and runs radix-8/4/2/3/5 passes on it in place, decimating in time both ways:
+// forward from natural to digit-reversed order, and back through a second buffer, whose
+// first pass gathers the spectrum in the order it needs and applies the operators'
+// Hermitian multipliers (+ik, -k^2, the 2/3 truncation; tables in that order).  Warps
+// synchronise their passes alone; the CTA meets for the row-by-row loads and stores of y
+// lines.
 //
-// Measured at 240^2 x 129, against a Stockham kernel that kept 2048 elements
-// per CTA, synchronised it between all stages and took 8 elements per thread
-// through a call per stage: d2bydx 226 -> 53 us, d2bydy 237 -> 58 us; at
-// 480^2 x 65 420 -> 102 us and 449 -> 126 us.  (The register kernel of lines_ct.cu
-// is faster at its own lengths: 256^2 x 129 36 against 52 us.)
+// The eights come first and the fives last, both ways, and twiddles before the DFTs: what
+// the last stages round off lies at multiples of n / radix, and a second derivative weighs it
+// by the fourth power, while the first passes of the inverse meet a smooth line's spectrum
+// mostly in zeros.  The errors are those of plain Stockham stages of 8, 4, 2, 3 and 5 points,
+// or up to 6 % less where a two or four takes a three along.  Passes in place both ways (no
+// gathering, no second buffer for a single output) with the eights last take 5 to 30 % less
+// time, but err up to 20 % more on smooth lines and up to 60 % on a constant plus little.
+//
+// Measured (d2bydx, d2bydy) against the Stockham kernel, which kept 2048 elements per CTA,
+// synchronised it between all stages and took 8 elements per thread through a call per
+// stage: 240^2 x 129 220 227 -> 58 63 us, 480^2 x 65 419 446 -> 105 130, 1000^2 x 33
+// 898 968 -> 314 384.  (The register kernel of lines_ct.cu is faster at its own lengths:
+// 256^2 x 129 34 us.)
 #include <math.h>
 #include <stdio.h>
 #include <string.h>
@@ -107,89 +115,118 @@ template <bool INV, typename C> struct Dft<5, INV, C> {
         v[0] = x0; v[1] = cadd(a1, b1); v[4] = csub(a1, b1); v[2] = cadd(a2, b2); v[3] = csub(a2, b2);
     }
 };
-// even and odd elements by 3, then by 2
-template <bool INV, typename C> struct Dft<6, INV, C> {
-    static __device__ __forceinline__ void run(C *v) {
-        using R = decltype(v[0].x);
-        C a[3] = { v[0], v[2], v[4] }, b[3] = { v[1], v[3], v[5] };
-        Dft<3, INV, C>::run(a);
-        Dft<3, INV, C>::run(b);
-        // b_k W_6^k, W_6 = (1 - i sqrt 3) / 2 forward
-        const R h = (R)0.5, q = (R)0.86602540378443864676372317075293618;
-        const C r1 = rot90<INV>(b[1]), r2 = rot90<INV>(b[2]);
-        C w1, w2;
-        w1.x = h * b[1].x + q * r1.x; w1.y = h * b[1].y + q * r1.y;
-        w2.x = q * r2.x - h * b[2].x; w2.y = q * r2.y - h * b[2].y;
-        v[0] = cadd(a[0], b[0]); v[3] = csub(a[0], b[0]);
-        v[1] = cadd(a[1], w1); v[4] = csub(a[1], w1);
-        v[2] = cadd(a[2], w2); v[5] = csub(a[2], w2);
+// 6 = 2 x 3 and 12 = 4 x 3 by the map of coprime factors (no twiddles)
+template <int A, bool INV, typename C>
+__device__ __forceinline__ void dft_a3(C *v)
+{
+    constexpr int N = 3 * A, E = A == 2 ? 3 : 9;      // 1 mod A, 0 mod 3
+    C a[3][A];
+#pragma unroll
+    for (int m = 0; m < 3; m++) {
+#pragma unroll
+        for (int j = 0; j < A; j++) a[m][j] = v[(3 * j + A * m) % N];
+        Dft<A, INV, C>::run(a[m]);
     }
-};
+#pragma unroll
+    for (int k = 0; k < A; k++) {
+        C b[3] = { a[0][k], a[1][k], a[2][k] };
+        Dft<3, INV, C>::run(b);
+#pragma unroll
+        for (int m = 0; m < 3; m++) v[(E * k + 4 * m) % N] = b[m];
+    }
+}
+template <bool INV, typename C> struct Dft<6, INV, C> { static __device__ __forceinline__ void run(C *v) { dft_a3<2, INV>(v); } };
+template <bool INV, typename C> struct Dft<12, INV, C> { static __device__ __forceinline__ void run(C *v) { dft_a3<4, INV>(v); } };
 
 #define FS_TPB 256
-// element i of a sequence's buffer: one word of padding per 16, against the bank
-// conflicts of even strides
-__device__ __forceinline__ int fs_at(int i) { return i + (i >> 4); }
+// element i of a sequence's buffer: a word of padding per 2^sh, against the bank conflicts
+// of even strides (FsPlan: the best for the length, of either buffer)
+__device__ __forceinline__ int fs_at(int i, int sh) { return i + (i >> sh); }
 
-// words of a sequence's buffer: odd, so that the same element of a CTA's
-// sequences falls on different banks
-__host__ __device__ constexpr int fs_buf(int n) { return (n + n / 16 + 1) | 1; }
-
-struct FsPass { int n, L, M, G, l; unsigned mg; const float2 *tw; };
+// one pass: radix R over the elements j + m M of every block of R M; tw: its twiddles
+struct FsPass { int n, M, G, l, sh; unsigned mg; const float2 *tw; };
 
 template <int R>
-__device__ __forceinline__ int fs_places(const FsPass &a, int b, int *at)
+__device__ __forceinline__ void fs_places(const FsPass &a, int b, int &q, int &j, int *at)
 {
-    const int q = (int)(((unsigned long long)(unsigned)b * a.mg) >> 31), j = b - q * a.M, i = q * a.L + j;
+    q = (int)(((unsigned long long)(unsigned)b * a.mg) >> 31);
+    j = b - q * a.M;
+    const int i = q * R * a.M + j;
 #pragma unroll
-    for (int m = 0; m < R; m++) at[m] = fs_at(i + m * a.M);
-    return j;
+    for (int m = 0; m < R; m++) at[m] = fs_at(i + m * a.M, a.sh);
 }
-// DFT_R over the elements j + m M of every block of L, then W_L^(j r) (not in the
-// last pass, M = 1)
-template <int R, bool LAST>
+// W^(r K) for block q of wavenumber K so far (not in the FIRST pass), then DFT_R
+template <int R, bool FIRST>
 __device__ __forceinline__ void fs_fwd(float2 *buf, const FsPass &a)
 {
+    const int nb = a.n / (R * a.M);
     for (int b = a.l; b < a.n / R; b += a.G) {
-        int at[R];
+        int q, j, at[R];
         float2 v[R];
-        const int j = fs_places<R>(a, b, at);
+        fs_places<R>(a, b, q, j, at);
 #pragma unroll
-        for (int m = 0; m < R; m++) v[m] = buf[at[m]];
+        for (int r = 0; r < R; r++) {
+            v[r] = buf[at[r]];
+            if (!FIRST && r) v[r] = cmul(v[r], a.tw[(r - 1) * nb + q]);
+        }
         Dft<R, false, float2>::run(v);
-        buf[at[0]] = v[0];
 #pragma unroll
-        for (int r = 1; r < R; r++) buf[at[r]] = LAST ? v[r] : cmul(v[r], a.tw[(r - 1) * a.M + j]);
+        for (int r = 0; r < R; r++) buf[at[r]] = v[r];
     }
     __syncwarp();
 }
-// the reverse.  FIRST (M = 1): from src, times the multipliers mul (d1: i times)
-// unless mul is null.  OUT (L = n, x lines): the results to the two rows.
-struct FsOut { float *a, *b; float sc, add; };
-template <int R, bool FIRST, bool OUT>
-__device__ __forceinline__ void fs_inv(float2 *buf, const float2 *src, const FsPass &a, const float *mul, bool d1, const FsOut &o)
+// the first inverse pass (M = 1), from the spectrum src in the forward passes' order,
+// times the multipliers mul (d1: i times), or from a halfcomplex line pair (HC):
+// Z_k = A_k + i B_k
+template <int R, bool HC>
+__device__ __forceinline__ void fs_inv_first(float2 *buf, const float2 *src, const FsPass &a, int sha, const unsigned short *tab,
+                                             const float *mul, bool d1)
 {
     for (int b = a.l; b < a.n / R; b += a.G) {
-        int at[R];
         float2 v[R];
-        const int j = fs_places<R>(a, b, at);
 #pragma unroll
         for (int r = 0; r < R; r++) {
-            if (FIRST) {
-                v[r] = src[at[r]];
-                if (mul) {
-                    const float m = __ldg(mul + b * R + r);
-                    const float2 z = v[r];
-                    v[r].x = d1 ? -m * z.y : m * z.x;
-                    v[r].y = d1 ? m * z.x : m * z.y;
-                }
+            const int i = b * R + r, t = __ldg(tab + i);
+            if (HC) {
+                const int kk = min(t, a.n - t);
+                const bool edge = kk == 0 || 2 * kk == a.n;
+                const float2 pa = src[fs_at(kk, sha)];
+                float2 pc = src[fs_at(edge ? 0 : a.n - kk, sha)];
+                if (edge) pc = make_float2(0.0f, 0.0f);
+                if (2 * t > a.n) { pc.x = -pc.x; pc.y = -pc.y; }
+                v[r] = make_float2(pa.x - pc.y, pc.x + pa.y);
             } else {
-                v[r] = buf[at[r]];
-                if (r) {
-                    float2 w = a.tw[(r - 1) * a.M + j];
-                    w.y = -w.y;
-                    v[r] = cmul(v[r], w);
-                }
+                v[r] = src[fs_at(t, sha)];
+            }
+            if (mul) {
+                const float m = __ldg(mul + i);
+                const float2 z = v[r];
+                v[r].x = d1 ? -m * z.y : m * z.x;
+                v[r].y = d1 ? m * z.x : m * z.y;
+            }
+        }
+        Dft<R, true, float2>::run(v);
+#pragma unroll
+        for (int r = 0; r < R; r++) buf[fs_at(b * R + r, a.sh)] = v[r];
+    }
+    __syncwarp();
+}
+// the others; OUT (the last one of x lines): the results to the two rows
+struct FsOut { float *a, *b; float sc, add; };
+template <int R, bool OUT>
+__device__ __forceinline__ void fs_inv(float2 *buf, const FsPass &a, const FsOut &o)
+{
+    for (int b = a.l; b < a.n / R; b += a.G) {
+        int q, j, at[R];
+        float2 v[R];
+        fs_places<R>(a, b, q, j, at);
+#pragma unroll
+        for (int r = 0; r < R; r++) {
+            v[r] = buf[at[r]];
+            if (r) {
+                float2 w = a.tw[(r - 1) * a.M + j];
+                w.y = -w.y;
+                v[r] = cmul(v[r], w);
             }
         }
         Dft<R, true, float2>::run(v);
@@ -207,6 +244,7 @@ __device__ __forceinline__ void fs_inv(float2 *buf, const float2 *src, const FsP
 }
 #define FS_SWITCH(R, CALL)                                                                 \
     switch (R) {                                                                           \
+    case 12: CALL(12); break;                                                              \
     case 8: CALL(8); break;                                                                \
     case 6: CALL(6); break;                                                                \
     case 5: CALL(5); break;                                                                \
@@ -219,12 +257,12 @@ __device__ __forceinline__ void fs_inv(float2 *buf, const float2 *src, const FsP
 // per plane: of Q sequences (one warp's, x) or S = warps Q (a CTA's, y).
 template <int DIR, int NJ>
 __global__ void __launch_bounds__(FS_TPB, 4)
-line_kernel(const __grid_constant__ JobPack<NJ> jobs, const __grid_constant__ FxPlan pl, FsTables tb, int nx, int ny, int nz,
+line_kernel(const __grid_constant__ JobPack<NJ> jobs, const __grid_constant__ FsPlan pl, FsTables tb, int nx, int ny, int nz,
             int tpp, int total, int two)
 {
     PDL_WAIT();
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    const int n = pl.n, Q = pl.Q, G = 32 / Q, W = (int)blockDim.x / 32, S = W * Q, nb = fs_buf(n);
+    const int n = pl.n, Q = pl.Q, G = 32 / Q, W = (int)blockDim.x / 32, S = W * Q, nb = pl.nb, sha = pl.sha, shb = pl.shb;
     float2 *bufA = reinterpret_cast<float2 *>(smem_raw);
     float2 *bufB = bufA + (size_t)S * nb;              // (two)
     float2 *tw = bufB + (two ? (size_t)S * nb : 0);
@@ -235,9 +273,12 @@ line_kernel(const __grid_constant__ JobPack<NJ> jobs, const __grid_constant__ Fx
     const int ls = 31 - __clz(S), yq = tid & (S - 1), ye = tid >> ls, de = (int)blockDim.x >> ls;   // y: row by row
     for (int e = tid; e < pl.ntw; e += blockDim.x) tw[e] = tb.tw[e];
     __syncthreads();
-    auto args = [&](int p) {
+    auto args = [&](int p, bool inverse) {
         FsPass a;
-        a.n = n; a.L = pl.L[p]; a.M = pl.M[p]; a.G = G; a.l = l; a.mg = pl.mg[p]; a.tw = tw + pl.tw[p];
+        a.n = n; a.G = G; a.l = l; a.sh = inverse ? shb : sha;
+        a.M = inverse ? pl.iM[p] : pl.fM[p];
+        a.mg = inverse ? pl.img[p] : pl.fmg[p];
+        a.tw = tw + (inverse ? pl.itw[p] : pl.ftw[p]);
         return a;
     };
     const int t0 = DIR == 0 ? blockIdx.x * W + wid : blockIdx.x, dt = DIR == 0 ? gridDim.x * W : gridDim.x;
@@ -266,7 +307,7 @@ line_kernel(const __grid_constant__ JobPack<NJ> jobs, const __grid_constant__ Fx
                 }
 #pragma unroll
                 for (int c = 0; c < 8; c++)
-                    if (e0 + c * G < n) A[fs_at(e0 + c * G)] = v[c];
+                    if (e0 + c * G < n) A[fs_at(e0 + c * G, sha)] = v[c];
             }
             __syncwarp();
         } else {
@@ -282,29 +323,29 @@ line_kernel(const __grid_constant__ JobPack<NJ> jobs, const __grid_constant__ Fx
                 }
 #pragma unroll
                 for (int c = 0; c < 8; c++)
-                    if (e0 + c * de < n) to[fs_at(e0 + c * de)] = v[c];
+                    if (e0 + c * de < n) to[fs_at(e0 + c * de, sha)] = v[c];
             }
             __syncthreads();
         }
 
         // ---- forward
         if (!inv) {
-            for (int p = 0; p < pl.np - 1; p++) {
-                const FsPass a = args(p);
+            const FsPass a0 = args(0, false);
+#define CALL(R) fs_fwd<R, true>(A, a0)
+            FS_SWITCH(pl.R[0], CALL)
+#undef CALL
+            for (int p = 1; p < pl.np; p++) {
+                const FsPass a = args(p, false);
 #define CALL(R) fs_fwd<R, false>(A, a)
                 FS_SWITCH(pl.R[p], CALL)
 #undef CALL
             }
-            const FsPass a = args(pl.np - 1);
-#define CALL(R) fs_fwd<R, true>(A, a)
-            FS_SWITCH(pl.R[pl.np - 1], CALL)
-#undef CALL
         }
 
         if (op1 == OP_FWD) {
             // separate Z into the halfcomplex spectra of the two real lines
             auto sep = [&](const float2 *Z, int p) {
-                const float2 zp = Z[fs_at(__ldg(tb.pos + p))], zq = Z[fs_at(__ldg(tb.pos + (p == 0 ? 0 : n - p)))];
+                const float2 zp = Z[fs_at(__ldg(tb.pos + p), sha)], zq = Z[fs_at(__ldg(tb.pos + (p == 0 ? 0 : n - p)), sha)];
                 float2 v;
                 if (2 * p <= n) { v.x = 0.5f * (zp.x + zq.x); v.y = 0.5f * (zp.y + zq.y); }
                 else { v.x = 0.5f * (zq.y - zp.y); v.y = 0.5f * (zp.x - zq.x); }
@@ -340,21 +381,6 @@ line_kernel(const __grid_constant__ JobPack<NJ> jobs, const __grid_constant__ Fx
         const int nout = op2 != OP_NONE && (!inv || op2 == OP_D1) ? 2 : 1;
         for (int o = 0; o < nout; o++) {
             const int op = o == 0 ? op1 : op2;
-            const float2 *src = A;
-            float2 *dst = o + 1 < nout ? B : A;
-            if (inv) {
-                // Z_k = A_k + i B_k from the halfcomplex lines a (re), b (im)
-                for (int i = l; i < n; i += G) {
-                    const int k = __ldg(tb.kof + i), kk = min(k, n - k);
-                    const bool edge = kk == 0 || 2 * kk == n;
-                    const float2 pa = A[fs_at(kk)];
-                    float2 pc = edge ? make_float2(0.0f, 0.0f) : A[fs_at(n - kk)];
-                    if (2 * k > n) { pc.x = -pc.x; pc.y = -pc.y; }
-                    B[fs_at(i)] = make_float2(pa.x - pc.y, pc.x + pa.y);
-                }
-                __syncwarp();
-                src = dst = B;
-            }
             const float *mul = op == OP_D1 ? tb.m1 : op == OP_D2 ? tb.m2 : op == OP_DEALIAS ? tb.mda : nullptr;
             const float alpha = o == 0 ? jb.alpha1 : jb.alpha2;
             const int acc = o == 0 ? jb.acc1 : jb.acc2;
@@ -367,28 +393,34 @@ line_kernel(const __grid_constant__ JobPack<NJ> jobs, const __grid_constant__ Fx
             const bool fused = DIR == 0 && pl.np > 1 && __all_sync(0xffffffffu, valid && !acc && alpha == 1.0f);
             const FsOut to = { ot + xoff, ot + xoff + nx, sc, addv };
             {
-                const FsPass a = args(pl.np - 1);
-#define CALL(R) fs_inv<R, true, false>(dst, src, a, mul, op == OP_D1, to)
-                FS_SWITCH(pl.R[pl.np - 1], CALL)
+                const FsPass a = args(0, true);
+                if (inv) {
+#define CALL(R) fs_inv_first<R, true>(B, A, a, sha, tb.pos, mul, op == OP_D1)
+                    FS_SWITCH(pl.R[0], CALL)
 #undef CALL
+                } else {
+#define CALL(R) fs_inv_first<R, false>(B, A, a, sha, tb.gat, mul, op == OP_D1)
+                    FS_SWITCH(pl.R[0], CALL)
+#undef CALL
+                }
             }
-            for (int p = pl.np - 2; p >= (fused ? 1 : 0); p--) {
-                const FsPass a = args(p);
-#define CALL(R) fs_inv<R, false, false>(dst, dst, a, nullptr, false, to)
+            for (int p = 1; p < pl.np - (fused ? 1 : 0); p++) {
+                const FsPass a = args(p, true);
+#define CALL(R) fs_inv<R, false>(B, a, to)
                 FS_SWITCH(pl.R[p], CALL)
 #undef CALL
             }
             if (fused) {
-                const FsPass a = args(0);
-#define CALL(R) fs_inv<R, false, true>(dst, dst, a, nullptr, false, to)
-                FS_SWITCH(pl.R[0], CALL)
+                const FsPass a = args(pl.np - 1, true);
+#define CALL(R) fs_inv<R, true>(B, a, to)
+                FS_SWITCH(pl.R[pl.np - 1], CALL)
 #undef CALL
                 continue;
             }
             if (DIR == 0) {
                 if (valid)
                     for (int e = l; e < n; e += G) {
-                        const float2 z = dst[fs_at(e)];
+                        const float2 z = B[fs_at(e, shb)];
                         float va = alpha * (z.x * sc), vb = alpha * (z.y * sc);
                         if (acc) { va = to.a[e] + va; vb = to.b[e] + vb; }
                         to.a[e] = va + addv;
@@ -397,10 +429,10 @@ line_kernel(const __grid_constant__ JobPack<NJ> jobs, const __grid_constant__ Fx
                 __syncwarp();
             } else {
                 __syncthreads();
-                const float2 *bs = (dst == A ? bufA : bufB) + (size_t)yq * nb;
+                const float2 *bs = bufB + (size_t)yq * nb;
                 if (yvalid)
                     for (int e = ye; e < n; e += de) {
-                        const float2 z = bs[fs_at(e)];
+                        const float2 z = bs[fs_at(e, shb)];
                         float2 *dd = reinterpret_cast<float2 *>(ot + yoff + (size_t)e * nx);
                         float va = alpha * (z.x * sc), vb = alpha * (z.y * sc);
                         if (acc) { const float2 w = *dd; va = w.x + va; vb = w.y + vb; }
@@ -467,36 +499,129 @@ int line_tables_make(int n, const double *k1, const double *k2, int icut, LineTa
     return st;
 }
 
-// the general kernel's tables: the plan's twiddles, and the multipliers of
-// line_tables_make in the spectrum's order
-int fs_tables_make(int n, const FxPlan &pl, const FxTables &fx, const double *k1, const double *k2, int icut, FsTables *tb)
+// k with its digits in the radices reversed: the place of wavenumber k after the forward
+// passes, and the wavenumber at place k before the inverse ones
+static int fs_reverse(const FsPlan &pl, int k)
 {
-    std::vector<float2> tw;
-    for (int p = 0; p < pl.np; p++)
-        if (pl.M[p] > 1)
-            for (int r = 1; r < pl.R[p]; r++)
-                for (int j = 0; j < pl.M[p]; j++) {
-                    double c, s;
-                    sincos2pi_host((long)j * r, pl.L[p], &c, &s);
-                    tw.push_back(make_float2((float)c, (float)-s));
-                }
-    std::vector<float> m(3 * n);
-    const double dn = (double)n;
-    for (int k = 0; k < n; k++) {
-        int rest = k, at = 0;
-        for (int p = 0; p < pl.np; p++) {
-            at += (rest % pl.R[p]) * pl.M[p];
-            rest /= pl.R[p];
-        }
-        m[at] = (float)(k > 0 && 2 * k < n ? k1[k] / dn : 2 * k > n ? -k1[k] / dn : 0.0);
-        m[n + at] = (float)(k == 0 ? 0.0 : k2[k] / dn);
-        const int kk = k <= n / 2 ? k : n - k;
-        m[2 * n + at] = (float)(kk >= n / 2 - icut ? 0.0 : 1.0 / dn);
+    int M = pl.n, at = 0;
+    for (int p = 0; p < pl.np; p++) {
+        M /= pl.R[p];
+        at += (k % pl.R[p]) * M;
+        k /= pl.R[p];
     }
-    const size_t bt = tw.size() * sizeof(float2), bm = m.size() * sizeof(float);
-    std::vector<char> all(bt + bm);
+    return at;
+}
+// the general kernel's passes: the eights first, the fives last; a two or four takes one of
+// the threes along (above 64 points: below them a pass more does not show, and 60 = 12 x 5
+// errs 1 % more than 4 x 3 x 5)
+int fs_plan_make(int n, FsPlan *pl)
+{
+    *pl = FsPlan{};
+    int m = n;
+    auto add = [&](int r) {
+        if (pl->np < 8) pl->R[pl->np++] = r;
+        m /= r;
+    };
+    while (m % 8 == 0) add(8);
+    if (m % 2 == 0) add((m % 4 == 0 ? 4 : 2) * (m % 3 == 0 && n > 64 ? 3 : 1));
+    for (int r : { 3, 5 })
+        while (m % r == 0) add(r);
+    if (m != 1 || n > 2048 || pl->np == 0) return VEC_ERR_SIZE;
+    pl->n = n;
+    int nb = 1;      // blocks before a forward pass, elements of an inverse one's block
+    for (int p = 0; p < pl->np; p++) {
+        const int R = pl->R[p];
+        pl->fM[p] = n / (nb * R);
+        pl->iM[p] = nb;
+        pl->fmg[p] = (unsigned)(((1ull << 31) + pl->fM[p] - 1) / pl->fM[p]);
+        pl->img[p] = (unsigned)(((1ull << 31) + nb - 1) / nb);
+        pl->ftw[p] = pl->ntw;
+        if (p) pl->ntw += (R - 1) * nb;
+        pl->itw[p] = pl->ntw;
+        if (p) pl->ntw += (R - 1) * nb;
+        nb *= R;
+    }
+    pl->Q = n <= 32 ? 8 : n <= 64 ? 4 : n <= 128 ? 2 : 1;
+    // the paddings with the fewest wavefronts: half a warp's words of 8 bytes, in 16 banks,
+    // of every butterfly's accesses (first: a forward pass's, or the gathering one's and the
+    // separation's; second: an inverse pass's, and the gathering one's writes)
+    int best[2] = { 0, 0 };
+    for (int sh : { 31, 6, 5, 4, 3, 2 }) {
+        const int G = 32 / pl->Q, ld = (n + ((n - 1) >> sh)) | 1;
+        int cost[2] = { 0, 0 };
+        auto count = [&](int which, int R, auto place) {
+            for (int b0 = 0; b0 < n / R; b0 += G)
+                for (int r = 0; r < R; r++)
+                    for (int h = 0; h < 32; h += 16) {
+                        int used[16] = {}, top = 0;
+                        for (int t = h; t < h + 16; t++) {
+                            const int b = b0 + t % G;
+                            if (b >= n / R) continue;
+                            const int i = place(b, r), w = t / G * ld + i + (i >> sh);
+                            if (++used[w & 15] > top) top = used[w & 15];
+                        }
+                        cost[which] += top;
+                    }
+        };
+        for (int p = 0; p < pl->np; p++) {
+            const int R = pl->R[p];
+            for (int which = 0; which < 2; which++) {
+                const int M = which ? pl->iM[p] : pl->fM[p];
+                count(which, R, [&](int b, int r) { return b / M * R * M + b % M + r * M; });
+            }
+        }
+        count(0, pl->R[0], [&](int b, int r) { return fs_reverse(*pl, fs_reverse(*pl, b * pl->R[0] + r)); });
+        count(0, 1, [&](int b, int) { return fs_reverse(*pl, b); });
+        if (best[0] == 0 || cost[0] < best[0]) { best[0] = cost[0]; pl->sha = sh; }
+        if (best[1] == 0 || cost[1] < best[1]) { best[1] = cost[1]; pl->shb = sh; }
+    }
+    // (odd: the same element of a CTA's sequences on different banks)
+    pl->nb = (n + ((n - 1) >> (pl->sha < pl->shb ? pl->sha : pl->shb))) | 1;
+    return VEC_OK;
+}
+// its tables: the passes' twiddles, and the multipliers of line_tables_make in the order of
+// the first inverse pass
+int fs_tables_make(const FsPlan &pl, const double *k1, const double *k2, int icut, FsTables *tb)
+{
+    const int n = pl.n;
+    std::vector<float2> tw;
+    auto add = [&](long e) {
+        double c, s;
+        sincos2pi_host(e, n, &c, &s);
+        tw.push_back(make_float2((float)c, (float)-s));
+    };
+    for (int p = 1; p < pl.np; p++) {
+        const int R = pl.R[p], nb = pl.iM[p], ts = n / (nb * R);
+        for (int r = 1; r < R; r++)
+            for (int q = 0; q < nb; q++) {
+                int K = 0, M = nb, rest = q;     // the block's wavenumber so far
+                for (int s = 0, w = 1; s < p; w *= pl.R[s++]) {
+                    M /= pl.R[s];
+                    K += rest / M * w;
+                    rest %= M;
+                }
+                add((long)r * K * ts);
+            }
+        for (int r = 1; r < R; r++)
+            for (int j = 0; j < nb; j++) add((long)r * j * ts);
+    }
+    std::vector<float> m(3 * n);
+    std::vector<unsigned short> pos(2 * n);       // and gat
+    const double dn = (double)n;
+    for (int i = 0; i < n; i++) {
+        const int k = fs_reverse(pl, i);
+        pos[i] = (unsigned short)k;
+        pos[n + i] = (unsigned short)fs_reverse(pl, k);
+        m[i] = (float)(k > 0 && 2 * k < n ? k1[k] / dn : 2 * k > n ? -k1[k] / dn : 0.0);
+        m[n + i] = (float)(k == 0 ? 0.0 : k2[k] / dn);
+        const int kk = k <= n / 2 ? k : n - k;
+        m[2 * n + i] = (float)(kk >= n / 2 - icut ? 0.0 : 1.0 / dn);
+    }
+    const size_t bt = tw.size() * sizeof(float2), bm = m.size() * sizeof(float), bp = pos.size() * sizeof(short);
+    std::vector<char> all(bt + bm + bp);
     if (bt) memcpy(all.data(), tw.data(), bt);
     memcpy(all.data() + bt, m.data(), bm);
+    memcpy(all.data() + bt + bm, pos.data(), bp);
     if (cudaMalloc(&tb->tw, all.size()) != cudaSuccess) {
         cudaGetLastError();
         return VEC_ERR_ALLOC;
@@ -504,8 +629,8 @@ int fs_tables_make(int n, const FxPlan &pl, const FxTables &fx, const double *k1
     tb->m1 = reinterpret_cast<float *>(reinterpret_cast<char *>(tb->tw) + bt);
     tb->m2 = tb->m1 + n;
     tb->mda = tb->m2 + n;
-    tb->pos = fx.pos;
-    tb->kof = fx.kof;
+    tb->pos = reinterpret_cast<unsigned short *>(tb->mda + n);
+    tb->gat = tb->pos + n;
     CUDA_TRY(cudaMemcpy(tb->tw, all.data(), all.size(), cudaMemcpyHostToDevice));
     return VEC_OK;
 }
@@ -525,7 +650,7 @@ void line_tables_free(LineTables<R> *tb)
 template <int DIR, int NJ>
 static int run_fs(Engine *E, const LineJob<float> *jobs, int nj)
 {
-    FxPlan pl = DIR == 0 ? E->fpx : E->fpy;
+    FsPlan pl = DIR == 0 ? E->fspx : E->fspy;
     JobPack<NJ> pk;
     memset(&pk, 0, sizeof(pk));
     double fields = 0.0;
@@ -534,21 +659,30 @@ static int run_fs(Engine *E, const LineJob<float> *jobs, int nj)
         pk.j[j] = jobs[j];
         fields += 2.0 + (jobs[j].acc1 ? 1.0 : 0.0);
         if (jobs[j].op2 != OP_NONE) fields += 1.0 + (jobs[j].acc2 ? 1.0 : 0.0);
-        if (jobs[j].op2 != OP_NONE || jobs[j].op1 == OP_INV) two = 1;
+        if (jobs[j].op1 != OP_FWD) two = 1;
     }
     const int pairs = (DIR == 0 ? E->ny : E->nx) / 2;
     // (sequences per warp and warps per CTA as in the FP64 kernel)
     while (pl.Q > 1 && (long long)nj * E->nz * pairs < (long long)E->num_sms * 8 * pl.Q && fx_rounds(pl, pl.Q / 2) < fx_rounds(pl, pl.Q))
         pl.Q >>= 1;
-    int W = FS_TPB / 32;
     auto smem_of = [&](int w) {
-        return sizeof(float2) * (pl.ntw + (size_t)w * pl.Q * fs_buf(pl.n) * (two ? 2 : 1));
+        return sizeof(float2) * (pl.ntw + (size_t)w * pl.Q * pl.nb * (two ? 2 : 1));
     };
     auto tiles_of = [&](int w) {
         const int S = DIR == 0 ? pl.Q : w * pl.Q;
         return (long long)nj * E->nz * ((pairs + S - 1) / S);
     };
-    while (W > 1 && (smem_of(W) > 75 * 1024 || (DIR == 0 ? tiles_of(W) / W : tiles_of(W)) < E->num_sms)) W >>= 1;
+    // warps per CTA: the most warps per SM (32 by their registers), the largest CTA of equals,
+    // for wider rows of y tiles and fewer copies of the twiddles; fewer where there would be
+    // less than a CTA per SM
+    auto warps_of = [&](int w) {
+        const size_t fit = 227 * 1024 / (smem_of(w) + 1024);
+        return w * (int)(fit < (size_t)(32 / w) ? fit : (size_t)(32 / w));
+    };
+    int W = FS_TPB / 32;
+    for (int w = W / 2; w >= 1; w >>= 1)
+        if (warps_of(w) > warps_of(W)) W = w;
+    while (W > 1 && (DIR == 0 ? tiles_of(W) / W : tiles_of(W)) < E->num_sms) W >>= 1;
     const size_t smem = smem_of(W);
     int per_sm = 1;
     CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, line_kernel<DIR, NJ>, W * 32, smem));
@@ -588,10 +722,10 @@ int line_kernels_configure()
 {
     int st = line_ct_configure();
     if (st || (st = line_ct64_configure()) || (st = line_fx_configure())) return st;
-    CUDA_TRY(cudaFuncSetAttribute(line_kernel<0, NJ_SMALL>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
-    CUDA_TRY(cudaFuncSetAttribute(line_kernel<1, NJ_SMALL>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
-    CUDA_TRY(cudaFuncSetAttribute(line_kernel<0, MAX_JOBS>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
-    CUDA_TRY(cudaFuncSetAttribute(line_kernel<1, MAX_JOBS>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
+    CUDA_TRY(cudaFuncSetAttribute(line_kernel<0, NJ_SMALL>, cudaFuncAttributeMaxDynamicSharedMemorySize, 226 * 1024));
+    CUDA_TRY(cudaFuncSetAttribute(line_kernel<1, NJ_SMALL>, cudaFuncAttributeMaxDynamicSharedMemorySize, 226 * 1024));
+    CUDA_TRY(cudaFuncSetAttribute(line_kernel<0, MAX_JOBS>, cudaFuncAttributeMaxDynamicSharedMemorySize, 226 * 1024));
+    CUDA_TRY(cudaFuncSetAttribute(line_kernel<1, MAX_JOBS>, cudaFuncAttributeMaxDynamicSharedMemorySize, 226 * 1024));
     return VEC_OK;
 }
 
