@@ -31,6 +31,7 @@
 #include <vector>
 
 #include "common.cuh"
+#include "smem_limit.h"
 #include "closure_net.h"
 
 namespace {
@@ -795,12 +796,8 @@ int run_conv_mt(vec_net *N, const NetGeom &gt, const bf16 *x, const bf16 *wt, co
                 bf16 *o_act, float *o_f32, int cout_real, const bf16 *gate)
 {
     const size_t sm = conv_smem<CIN, COUT>(gt);
-    static bool set = false;
-    if (!set) {
-        CUDA_TRY(cudaFuncSetAttribute(k_conv<CIN, COUT, EPI, MT, KS>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                      200 * 1024));
-        set = true;
-    }
+    static SmemLimit limit;
+    CUDA_TRY(limit.raise((const void *)k_conv<CIN, COUT, EPI, MT, KS>, 200 * 1024));
     long long grid = N->num_sms;
     if (grid > gt.tiles) grid = gt.tiles;
     k_conv<CIN, COUT, EPI, MT, KS><<<(int)grid, 256 * KS, sm, N->stream>>>(x, wt, bias, gt, o_pre, o_act, o_f32,
@@ -817,11 +814,8 @@ int run_conv_tc(vec_net *N, const bf16 *x, const bf16 *wt, const float *bias, bf
                 int cout_real, const bf16 *gate)
 {
     constexpr size_t sm = tc_smem_bytes<CIN, COUT>();
-    static bool set = false;
-    if (!set) {
-        CUDA_TRY(cudaFuncSetAttribute(k_conv_tc<CIN, COUT, EPI>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
-        set = true;
-    }
+    static SmemLimit limit;
+    CUDA_TRY(limit.raise((const void *)k_conv_tc<CIN, COUT, EPI>, (int)sm));
     // x as (8 channels, channel block, x, y, z and sample): boxes of 8 x 1 x 128 x 1 x 1
     PFN_cuTensorMapEncodeTiled_v12000 enc = (PFN_cuTensorMapEncodeTiled_v12000)tma_encode_fn();
     if (!enc) return VEC_ERR_CUDA;
@@ -873,11 +867,8 @@ template <int CI, int CO, int TPW>
 int run_wgrad_t(vec_net *N, const bf16 *x, const bf16 *dy, float *gout)
 {
     const size_t sm = wgrad_smem<CI, CO>(N->g);
-    static bool set = false;
-    if (!set) {
-        CUDA_TRY(cudaFuncSetAttribute(k_wgrad<CI, CO, TPW>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
-        set = true;
-    }
+    static SmemLimit limit;
+    CUDA_TRY(limit.raise((const void *)k_wgrad<CI, CO, TPW>, 200 * 1024));
     long long grid = N->num_sms;
     if (grid > N->g.tiles) grid = N->g.tiles;
     k_wgrad<CI, CO, TPW><<<(int)grid, 32 * (NTAP / TPW), sm, N->stream>>>(x, dy, N->g, N->part);

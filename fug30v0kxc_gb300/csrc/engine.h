@@ -11,6 +11,7 @@
 #include <vector>
 
 #include "common.cuh"
+#include "smem_limit.h"
 
 // work-array slots (FP64 form: double; split form: float)
 enum WorkSlot {

@@ -684,6 +684,8 @@ static int run_fs(Engine *E, const LineJob<float> *jobs, int nj)
         if (warps_of(w) > warps_of(W)) W = w;
     while (W > 1 && (DIR == 0 ? tiles_of(W) / W : tiles_of(W)) < E->num_sms) W >>= 1;
     const size_t smem = smem_of(W);
+    static SmemLimit limit;
+    CUDA_TRY(limit.raise((const void *)line_kernel<DIR, NJ>, 226 * 1024));
     int per_sm = 1;
     CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, line_kernel<DIR, NJ>, W * 32, smem));
     if (per_sm < 1) per_sm = 1;
@@ -722,10 +724,6 @@ int line_kernels_configure()
 {
     int st = line_ct_configure();
     if (st || (st = line_ct64_configure()) || (st = line_fx_configure())) return st;
-    CUDA_TRY(cudaFuncSetAttribute(line_kernel<0, NJ_SMALL>, cudaFuncAttributeMaxDynamicSharedMemorySize, 226 * 1024));
-    CUDA_TRY(cudaFuncSetAttribute(line_kernel<1, NJ_SMALL>, cudaFuncAttributeMaxDynamicSharedMemorySize, 226 * 1024));
-    CUDA_TRY(cudaFuncSetAttribute(line_kernel<0, MAX_JOBS>, cudaFuncAttributeMaxDynamicSharedMemorySize, 226 * 1024));
-    CUDA_TRY(cudaFuncSetAttribute(line_kernel<1, MAX_JOBS>, cudaFuncAttributeMaxDynamicSharedMemorySize, 226 * 1024));
     return VEC_OK;
 }
 

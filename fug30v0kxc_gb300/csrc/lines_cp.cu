@@ -587,11 +587,8 @@ template <int DIR, int A, int B, int C, int S, int NJ>
 static int run_nj(Engine *E, const LineJob<float> *jobs, int nj, const char *name)
 {
     using P = CpShape<DIR, A, B, C, S>;
-    static bool attr_set = false;
-    if (!attr_set) {
-        CUDA_TRY(cudaFuncSetAttribute(line_cp<DIR, A, B, C, S, NJ>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)P::SMEM));
-        attr_set = true;
-    }
+    static SmemLimit limit;
+    CUDA_TRY(limit.raise((const void *)line_cp<DIR, A, B, C, S, NJ>, (int)P::SMEM));
     const int L = DIR == 0 ? E->ny : E->nx;
     const int tpp = L / (2 * S);
     JobPackCP<NJ> pk;

@@ -574,17 +574,13 @@ static int run_nj(Engine *E, const LineJob<R> *jobs, int nj, const char *name)
     constexpr int NP = N1 > N2 ? N1 : N2;
     constexpr int TILE = 2 * S * N;
     constexpr int LDS = ct_lds<R, DIR, N1, N2, S>();
-    static bool attr_set = false;
+    static SmemLimit limit;
     const size_t smem = ct_smem_bytes<R, DIR, N1, N2, S>();
     static_assert(ct_smem_bytes<R, DIR, N1, N2, S>() == 2 * TILE * sizeof(R) + ((size_t)S * LDS + 2 * N) * sizeof(C) + 3 * (size_t)N * sizeof(R),
                   "shared memory layout");
     static_assert(ct_smem_bytes<R, DIR, N1, N2, S>() + 128 <= 232448, "tile does not fit one SM's shared memory");
     static_assert(LDS >= N1 * (N2 + 1) && LDS >= N2 * (N1 + 1) && LDS >= N + N / 32 + 1, "exchange rows");
-    if (!attr_set) {
-        CUDA_TRY(cudaFuncSetAttribute(line_ct<R, DIR, N1, N2, S, WSYNC, NJ>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                      (int)smem));
-        attr_set = true;
-    }
+    CUDA_TRY(limit.raise((const void *)line_ct<R, DIR, N1, N2, S, WSYNC, NJ>, (int)smem));
     const int L = DIR == 0 ? E->ny : E->nx;
     const int tpp = L / (2 * S);
     JobPackCT<R, NJ> pk;

@@ -447,15 +447,11 @@ static int run_ct(Engine *E, const LineJob<R> *jobs, int nj, const char *name)
     constexpr int N = N1 * N2;
     constexpr int NP = N1 > N2 ? N1 : N2;
     constexpr int LDS = ct_lds<R, DIR, N1, N2, S>();
-    static bool attr_set = false;
+    static SmemLimit limit;
     const size_t smem = ct_smem_bytes<R, DIR, N1, N2, S>();
     static_assert(ct_smem_bytes<R, DIR, N1, N2, S>() + 128 <= 232448, "tile does not fit one SM's shared memory");
     static_assert(LDS >= N1 * (N2 + 1) && LDS >= N2 * (N1 + 1) && LDS >= N + N / 32 + 1, "exchange rows");
-    if (!attr_set) {
-        CUDA_TRY(cudaFuncSetAttribute(line_ct64<R, DIR, N1, N2, S, WSYNC>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                      (int)smem));
-        attr_set = true;
-    }
+    CUDA_TRY(limit.raise((const void *)line_ct64<R, DIR, N1, N2, S, WSYNC>, (int)smem));
     const int L = DIR == 0 ? E->ny : E->nx;
     const int tpp = L / (2 * S);
     JobPackCT<R> pk;

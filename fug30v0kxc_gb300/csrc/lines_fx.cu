@@ -912,11 +912,8 @@ static int run_fx(Engine *E, const LineJob<double> *jobs, int nj)
     };
     while (W > 1 && (smem_of(W) > 75 * 1024 || (DIR == 0 ? tiles_of(W) / W : tiles_of(W)) < E->num_sms)) W >>= 1;
     const size_t smem = smem_of(W);
-    static bool attr = false;
-    if (!attr) {
-        CUDA_TRY(cudaFuncSetAttribute(line_fx<DIR, NJ>, cudaFuncAttributeMaxDynamicSharedMemorySize, 226 * 1024));
-        attr = true;
-    }
+    static SmemLimit limit;
+    CUDA_TRY(limit.raise((const void *)line_fx<DIR, NJ>, 226 * 1024));
     if (smem > 226 * 1024) return VEC_ERR_SIZE;
     int per_sm = 1;
     CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, line_fx<DIR, NJ>, W * 32, smem));

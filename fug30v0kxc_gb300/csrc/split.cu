@@ -1041,14 +1041,10 @@ int split_hydro_m(Engine *const *Es, int nE, const bool *with_mag)
     };
     const double p2b = FB(E, split_mag_on(*E) ? (with_mag[0] ? 42 : 39) : 32, 4);
     if (E->zpencil && E->np % ZT_TILE == 0 && E->nz >= 6) {
-        static bool attr = false;
+        static SmemLimit limit1, limit;
         const size_t smem = (size_t)ZT_SLOTS * 4 * ZT_TILE * sizeof(float);
-        if (!attr) {
-            CUDA_TRY(cudaFuncSetAttribute(k_split_pass2_zt<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-            CUDA_TRY(cudaFuncSetAttribute(k_split_pass2_zt<BATCH_MAX>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                          (int)smem));
-            attr = true;
-        }
+        CUDA_TRY(limit1.raise((const void *)k_split_pass2_zt<1>, (int)smem));
+        CUDA_TRY(limit.raise((const void *)k_split_pass2_zt<BATCH_MAX>, (int)smem));
         const int kc = z_chunk(E, nE);
         st = launch_members<SplitHydroArgs>(Es, nE, "hydro_pass2_f32", p2b,
                                             dim3((unsigned)(E->np / ZT_TILE), (unsigned)((E->nz + kc - 1) / kc)),
@@ -1080,14 +1076,10 @@ int split_hydro_m(Engine *const *Es, int nE, const bool *with_mag)
     auto p4args = [nE](Engine *e) { return hydro4_args(e, nE); };
     const bool zt4 = E->zpencil4 == 1 || (E->zpencil4 < 0 && E->np >= (size_t)1024 * 1024);
     if (E->nx % 4 == 0 && E->vec4 && E->zpencil && zt4 && E->np % ZT_TILE == 0 && E->nz >= 6) {
-        static bool attr4 = false;
+        static SmemLimit limit1, limit;
         const size_t smem = (size_t)ZT_SLOTS * Z4_FIELDS * ZT_TILE * sizeof(float);
-        if (!attr4) {
-            CUDA_TRY(cudaFuncSetAttribute(k_split_pass4_zt<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-            CUDA_TRY(cudaFuncSetAttribute(k_split_pass4_zt<BATCH_MAX>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                          (int)smem));
-            attr4 = true;
-        }
+        CUDA_TRY(limit1.raise((const void *)k_split_pass4_zt<1>, (int)smem));
+        CUDA_TRY(limit.raise((const void *)k_split_pass4_zt<BATCH_MAX>, (int)smem));
         const int kc = z_chunk(E, nE);
         if ((st = launch_members<SplitHydro4Args>(Es, nE, "hydro_pass4_f32", FB(E, split_mag_on(*E) ? 21 : 15, 4),
                                                   dim3((unsigned)(E->np / ZT_TILE), (unsigned)((E->nz + kc - 1) / kc)),
