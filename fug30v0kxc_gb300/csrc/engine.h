@@ -112,7 +112,8 @@ struct Engine {
     double *corr_bx = nullptr, *corr_by = nullptr;
     int corr_on = 0;
     // tunables (the ensemble autotuner sets them per grid)
-    int kc_pass2 = 16;          // planes per z chunk of hydro pass 2 (z-pencil or z-marching kernel)
+    int kc_pass2 = 16;          // planes per z chunk of hydro pass 2 (z-pencil or z-marching kernel), at most
+    int kc_members = 1;         // chunks as in launches of that many members (the tuner's contexts)
     int ct_s = 0;               // sequences per line tile (0: default for the size)
     bool ct_warp = true;        // x-line tiles synchronised per warp (FP32; VEC_CT_WARP=0: per CTA)
     bool prof_kinds = false;    // VEC_PROF_KINDS=1: line launches profiled per job kind
@@ -299,6 +300,7 @@ int split_hydro(Engine *E, bool with_mag = false);
 // first kernel of split_bandj (rotate_hist); split_ab3 then runs the update
 // alone (folded).
 int split_mag(Engine *E, bool ab3_coef = false, bool spectra_done = false);
+int split_z_chunk(const Engine *E, int kc, int nE);   // planes per chunk in launches of nE members
 bool split_bandj_bounds(const Engine &E);
 int split_bandj(Engine *E, bool rotate_hist = false, bool bounds = false);
 int split_refresh(Engine *E);

@@ -17,6 +17,7 @@
 // pass 2 and the sequences per tile of the line kernels by
 // timing a scratch context of that grid; results can be cached in a text
 // file (one line per grid: nx ny nz precision kc s).
+#include <algorithm>
 #include <stdio.h>
 #include <string.h>
 
@@ -247,13 +248,14 @@ static bool same(const TuneKey &a, const TuneKey &b)
     return a.nx == b.nx && a.ny == b.ny && a.nz == b.nz && a.prec == b.prec;
 }
 
-static int time_config(const vec_params &p, int kc, int s, int steps, float *ms)
+static int time_config(const vec_params &p, int kc, int members, int s, int steps, float *ms)
 {
     vec_ctx *c = nullptr;
     int st = vec_create(&p, &c);
     if (st) return st;
     Engine &E = engine_of(c);
     E.kc_pass2 = kc;
+    E.kc_members = members;
     E.ct_s = s;
     cudaEvent_t a = nullptr, b = nullptr;
     if ((st = vec_static(c)) || (st = vec_calcdt(c, nullptr))) goto out;
@@ -296,8 +298,18 @@ extern "C" int vec_ensemble_tune(vec_ens *e, int steps, const char *cache)
         for (auto &t : tab) if (same(t.k, k)) { hit = &t; break; }
         if (!hit) {
             // planes per z chunk of hydro pass 2 (the z-pencil kernel's
-            // chunk, or the z-marching kernel's where nx % 4 != 0)
-            const int kcs[3] = { 8, 16, 32 };
+            // chunk, or the z-marching kernel's where nx % 4 != 0): the default first, and
+            // only bounds that give the batch of this member another chunk
+            int members = 0;
+            for (auto m : e->m) members += m == c || engine_batchable(E, engine_of(m));
+            if (members > BATCH_MAX) members = BATCH_MAX;
+            std::vector<int> kcs, chunks;
+            for (int kc : { 16, 8, 32 }) {
+                const int ch = E.split ? split_z_chunk(&E, kc, members) : 0;
+                if (std::find(chunks.begin(), chunks.end(), ch) != chunks.end()) continue;
+                chunks.push_back(ch);
+                kcs.push_back(kc);
+            }
             // sequences per tile: the register-FFT kernel's default, or its
             // alternative (8 for n <= 256, 4 for n >= 768); the general kernel
             // has no choice
@@ -315,7 +327,7 @@ extern "C" int vec_ensemble_tune(vec_ens *e, int steps, const char *cache)
             for (int kc : kcs)
                 for (int s : ss) {
                     float ms = 0.0f;
-                    int st = time_config(E.p, kc, s, steps, &ms);
+                    int st = time_config(E.p, kc, members, s, steps, &ms);
                     if (st) return st;
                     if (ms < best_ms) { best_ms = ms; best.kc = kc; best.s = s; }
                 }

@@ -910,14 +910,15 @@ static void mag_fwd_jobs(Engine *E, LineJob<float> *fx, LineJob<float> *fy)
 // chunks of all nE members would not give every SM two CTAs (64^2 x 65: 40 CTAs
 // of 16 planes took 39 us, 264 of 2 take 13 us, although a chunk of 2 planes
 // reads four times as many); balanced over nz
-static int z_chunk(const Engine *E, int nE)
+int split_z_chunk(const Engine *E, int kc, int nE)
 {
-    int kt = E->kc_pass2 > 0 ? E->kc_pass2 : 16;
+    int kt = kc > 0 ? kc : 16;
     const long long tiles = (long long)nE * (E->zpencil && E->np % 512 == 0 ? E->np / 512 : nblk(E->np));
     while (kt > 2 && tiles * ((E->nz + kt - 1) / kt) < 2LL * E->num_sms) kt /= 2;
     const int nch = (E->nz + kt - 1) / kt;
     return (E->nz + nch - 1) / nch;
 }
+static int z_chunk(const Engine *E, int nE) { return split_z_chunk(E, E->kc_pass2, nE > E->kc_members ? nE : E->kc_members); }
 
 static SplitHydroArgs hydro_args(Engine *E, int nE)
 {

@@ -296,7 +296,8 @@ int vec_ensemble_sync(vec_ens *ens);
 int vec_ensemble_tune(vec_ens *ens, int steps, const char *cache);
 /* the tile shapes in use by a context */
 int vec_tunables(vec_ctx *ctx, int *kc, int *s);
-/* sets them: kc in {8, 16, 32}; s in {0 (the kernel's default), 4, 8}
+/* sets them: kc in {8, 16, 32}, the most planes per chunk (grids that would not
+ * fill the device take smaller ones); s in {0 (the kernel's default), 4, 8}
  * (FP32 register-FFT lines: 8 selects 8 sequences per tile for n <= 256,
  * 4 selects 4 for n >= 768; other lengths choose for themselves) */
 int vec_set_tunables(vec_ctx *ctx, int kc, int s);
