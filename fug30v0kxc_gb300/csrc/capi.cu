@@ -228,6 +228,18 @@ static int upload(double *d, const std::vector<double> &h)
     return VEC_OK;
 }
 
+// akx2[i] + aky2[j] per plane point and its inverse (0 at the mean), in FP64 and rounded to FP32
+__global__ void k_make_kh2(const double *akx2, const double *aky2, int nx, size_t np, double *k, float *kf, double *ki, float *kif)
+{
+    const size_t q = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (q >= np) return;
+    const double v = akx2[q % nx] + aky2[q / nx], w = q == 0 ? 0.0 : 1.0 / v;
+    k[q] = v;
+    kf[q] = (float)v;
+    ki[q] = w;
+    kif[q] = (float)w;
+}
+
 extern "C" int vec_create(const vec_params *p, vec_ctx **out)
 {
     if (!p || !out) return VEC_ERR_ARG;
@@ -340,17 +352,8 @@ extern "C" int vec_create(const vec_params *p, vec_ctx **out)
         return VEC_ERR_CUDA;
     }
     {
-        // the wavenumber tables per precision; kh2 = akx2[i] + aky2[j] per plane point
-        std::vector<double> kh2(E.np), kh2i(E.np);
-        std::vector<float> kx1f(E.nx), ky1f(E.ny), kh2f(E.np), kh2if(E.np);
-        for (int j = 0; j < E.ny; j++)
-            for (int i = 0; i < E.nx; i++) {
-                const size_t q = (size_t)j * E.nx + i;
-                kh2[q] = akx2[i] + aky2[j];
-                kh2f[q] = (float)kh2[q];
-                kh2i[q] = q == 0 ? 0.0 : 1.0 / kh2[q];
-                kh2if[q] = (float)kh2i[q];
-            }
+        // the wavenumber tables per precision; those of the plane are formed on the device
+        std::vector<float> kx1f(E.nx), ky1f(E.ny);
         for (int i = 0; i < E.nx; i++) kx1f[i] = (float)akx1[i];
         for (int j = 0; j < E.ny; j++) ky1f[j] = (float)aky1[j];
         float *fx = nullptr, *fy = nullptr, *fk = nullptr, *fki = nullptr;
@@ -364,10 +367,13 @@ extern "C" int vec_create(const vec_params *p, vec_ctx **out)
         E.hd.kx1 = E.akx1;
         E.hd.ky1 = E.aky1;
         if (cudaMemcpy(fx, kx1f.data(), sizeof(float) * E.nx, cudaMemcpyHostToDevice) != cudaSuccess ||
-            cudaMemcpy(fy, ky1f.data(), sizeof(float) * E.ny, cudaMemcpyHostToDevice) != cudaSuccess ||
-            cudaMemcpy(fk, kh2f.data(), sizeof(float) * E.np, cudaMemcpyHostToDevice) != cudaSuccess ||
-            cudaMemcpy(fki, kh2if.data(), sizeof(float) * E.np, cudaMemcpyHostToDevice) != cudaSuccess ||
-            upload(dk, kh2) || upload(dki, kh2i)) {
+            cudaMemcpy(fy, ky1f.data(), sizeof(float) * E.ny, cudaMemcpyHostToDevice) != cudaSuccess) {
+            vec_destroy(c);
+            return VEC_ERR_CUDA;
+        }
+        // (on the copies' stream, done before the context's own streams read them)
+        k_make_kh2<<<(unsigned)((E.np + 255) / 256), 256>>>(E.akx2, E.aky2, E.nx, E.np, dk, fk, dki, fki);
+        if (cudaGetLastError() != cudaSuccess || cudaStreamSynchronize(0) != cudaSuccess) {
             vec_destroy(c);
             return VEC_ERR_CUDA;
         }
@@ -420,14 +426,14 @@ extern "C" int vec_create(const vec_params *p, vec_ctx **out)
     ALLOC(E.ds, sizeof(DevScalars));
     ALLOC(E.cdt, sizeof(float) * (4 + 3 * (size_t)cdt_chunks(E.np, E.nz)));
     if ((st = cdt_init(E.cdt))) { vec_destroy(c); return st; }
-    if (cudaHostAlloc((void **)&E.dev_err, sizeof(int) * 4, cudaHostAllocMapped | cudaHostAllocPortable) != cudaSuccess) {
+    // the host's copy of the scalars, and behind it the error flag
+    if (cudaHostAlloc((void **)&E.hs, sizeof(DevScalars) + sizeof(int) * 4, cudaHostAllocMapped | cudaHostAllocPortable) != cudaSuccess) {
         cudaGetLastError();
         vec_destroy(c);
         return VEC_ERR_ALLOC;
     }
-    memset(E.dev_err, 0, sizeof(int) * 4);
-    if (cudaMallocHost(&E.hs, sizeof(DevScalars)) != cudaSuccess) { vec_destroy(c); return VEC_ERR_ALLOC; }
-    memset(E.hs, 0, sizeof(DevScalars));
+    memset((void *)E.hs, 0, sizeof(DevScalars) + sizeof(int) * 4);
+    E.dev_err = reinterpret_cast<int *>(E.hs + 1);
     E.hs->first = 1;
     E.hs->velmxx = OKEY_NEG_HUGE;
     E.hs->velmxz = OKEY_NEG_HUGE;
@@ -466,7 +472,6 @@ extern "C" int vec_destroy(vec_ctx *c)
     if (E.tx32.tw) line_tables_free(&E.tx32);
     if (E.ty32.tw) line_tables_free(&E.ty32);
     if (E.hs) cudaFreeHost(E.hs);
-    if (E.dev_err) cudaFreeHost(E.dev_err);
     for (auto &pd : E.pending) { cudaEventDestroy(pd.a); cudaEventDestroy(pd.b); }
     for (auto ev : E.ev_pool) cudaEventDestroy(ev);
     if (E.stream2) { cudaStreamSynchronize(E.stream2); cudaStreamDestroy(E.stream2); }

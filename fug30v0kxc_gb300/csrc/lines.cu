@@ -543,14 +543,16 @@ int fs_plan_make(int n, FsPlan *pl)
     }
     pl->Q = n <= 32 ? 8 : n <= 64 ? 4 : n <= 128 ? 2 : 1;
     // the paddings with the fewest wavefronts: half a warp's words of 8 bytes, in 16 banks,
-    // of every butterfly's accesses (first: a forward pass's, or the gathering one's and the
+    // of the accesses of 128 butterflies or all (first: a forward pass's, or the gathering one's and the
     // separation's; second: an inverse pass's, and the gathering one's writes)
     int best[2] = { 0, 0 };
+    std::vector<int> rev(n);
+    for (int k = 0; k < n; k++) rev[k] = fs_reverse(*pl, k);
     for (int sh : { 31, 6, 5, 4, 3, 2 }) {
         const int G = 32 / pl->Q, ld = (n + ((n - 1) >> sh)) | 1;
         int cost[2] = { 0, 0 };
         auto count = [&](int which, int R, auto place) {
-            for (int b0 = 0; b0 < n / R; b0 += G)
+            for (int b0 = 0; b0 < n / R && b0 < 128; b0 += G)
                 for (int r = 0; r < R; r++)
                     for (int h = 0; h < 32; h += 16) {
                         int used[16] = {}, top = 0;
@@ -570,8 +572,8 @@ int fs_plan_make(int n, FsPlan *pl)
                 count(which, R, [&](int b, int r) { return b / M * R * M + b % M + r * M; });
             }
         }
-        count(0, pl->R[0], [&](int b, int r) { return fs_reverse(*pl, fs_reverse(*pl, b * pl->R[0] + r)); });
-        count(0, 1, [&](int b, int) { return fs_reverse(*pl, b); });
+        count(0, pl->R[0], [&](int b, int r) { return rev[rev[b * pl->R[0] + r]]; });
+        count(0, 1, [&](int b, int) { return rev[b]; });
         if (best[0] == 0 || cost[0] < best[0]) { best[0] = cost[0]; pl->sha = sh; }
         if (best[1] == 0 || cost[1] < best[1]) { best[1] = cost[1]; pl->shb = sh; }
     }
@@ -584,12 +586,13 @@ int fs_plan_make(int n, FsPlan *pl)
 int fs_tables_make(const FsPlan &pl, const double *k1, const double *k2, int icut, FsTables *tb)
 {
     const int n = pl.n;
-    std::vector<float2> tw;
-    auto add = [&](long e) {
+    std::vector<float2> tw, unit(n);
+    for (int e = 0; e < n; e++) {
         double c, s;
         sincos2pi_host(e, n, &c, &s);
-        tw.push_back(make_float2((float)c, (float)-s));
-    };
+        unit[e] = make_float2((float)c, (float)-s);
+    }
+    auto add = [&](long e) { tw.push_back(unit[e % n]); };
     for (int p = 1; p < pl.np; p++) {
         const int R = pl.R[p], nb = pl.iM[p], ts = n / (nb * R);
         for (int r = 1; r < R; r++)
