@@ -321,14 +321,14 @@ line_fx(const __grid_constant__ FxPack<NJ> jobs, const __grid_constant__ FxPlan 
             }
             return v;
         };
-        // (a spectrum's constant, lane 0's first element, is kept apart: it must not set
-        // the exponent of a derivative that does not contain it)
+        // (a spectrum's constant, lane 0's first element, is kept apart; where a derivative
+        // is asked for, which does not contain it, it must not set the exponent either)
         double dcx = 0.0, dcy = 0.0;
         auto constant = [&](X2 &v) {
             if (inv && l == 0) {
                 dcx = __longlong_as_double(v.x);
                 dcy = __longlong_as_double(v.y);
-                v.x = v.y = 0;
+                if (op2 == OP_D1) v.x = v.y = 0;
             }
         };
         // the largest high word; 0 only for a line of zeros (at rest, truncated, or a
