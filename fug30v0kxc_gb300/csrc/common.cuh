@@ -60,7 +60,8 @@ struct FxPlan {
     int R[6], L[6], M[6], tw[6], kind[6];
     unsigned mg[6];
     int ntw;                // twiddles in all
-    int halvings;           // of one transform
+    int hf, hi;             // halvings of a forward, an inverse transform
+    unsigned fup, iup;      // passes (bits) that leave their halving out: lines_fx_long.cu
     int gb;                 // its values stay below 2^gb times the norm
     int Q;                  // sequences per warp
     int cut;                // wavenumbers below it survive the dealiasing

@@ -220,6 +220,8 @@ int line_kernels_configure();
 int cdt_chunks(size_t np, int nz);
 int cdt_init(float *cdt);
 int line_fx_configure();
+int line_fx_long_configure();
+int launch_lines_fx_long(Engine *E, int dir, const LineJob<double> *jobs, int njobs);   // lines_fx_long.cu
 int fx_plan_make(int n, FxPlan *pl);
 int fx_tables_make(int n, FxPlan *pl, const double *k1, const double *k2, int icut, FxTables *tb);
 void fx_tables_free(FxTables *tb);

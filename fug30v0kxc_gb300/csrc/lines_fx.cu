@@ -23,9 +23,10 @@
 // own.)  It issues in 45 % of the cycles, the rest being instruction fetches and
 // the latency of shared memory and conversions; synchronising the passes of a
 // CTA's warps, so that they fetch the same code, changed nothing, nor did rolled
-// loops of twiddle products (13 % less code).  Error against
-// long double: 2 to 3 times smaller than in FP64 for white noise, 10^4 times for
-// a constant plus little.
+// loops of twiddle products (13 % less code).  Error (rms) of
+// derivatives against long double, in parts of that of the register FFT in FP64: 0.3 to
+// 0.5 for white noise, 0.1 to 0.5 for lines of few waves, 10^-3 to 4 10^-3 for a constant plus
+// 1 % of waves.
 #include <math.h>
 #include <string.h>
 
@@ -39,6 +40,8 @@
 template <int NJ> struct FxPack { LineJob<double> j[NJ]; };
 
 #define FX_TPB 256
+// lines above that many points: lines_fx_long.cu, which compiles this file once more
+#define FX_SHORT 512
 
 // element i of a sequence's buffer: the eight 16-byte words of a 128-byte row
 // are permuted by the row (and, y lines, by the sequence), so that strides of
@@ -51,7 +54,18 @@ __device__ __forceinline__ int fx_at(int i, int s7) { return i ^ ((i >> 3) & 7) 
 // (the permutation of fx_at costs three instructions per element in general):
 // K64: M a multiple of 64, K8: R = M = 8, K1: R = 8, M = 1.
 enum { KG, K64, K8, K1 };
-struct FxPassArgs { int n, L, M, G, l, s7; unsigned mg; const TwX *tw; };
+struct FxPassArgs { int n, L, M, G, l, s7, up; unsigned mg; const TwX *tw; };
+// the value that a pass takes its twiddle product of (which halves it), and the one it
+// halves itself; long lines leave some halvings out
+__device__ __forceinline__ X2 fx_up(X2 v, const FxPassArgs &a)
+{
+#if FX_LONG
+    v.x <<= a.up;
+    v.y <<= a.up;
+#endif
+    return v;
+}
+__device__ __forceinline__ X2 fx_half(X2 v, const FxPassArgs &a) { return FX_LONG && a.up ? v : fx_half(v); }
 
 template <int R, int KIND>
 __device__ __forceinline__ void fx_places(const FxPassArgs &a, int b, int &j, int *at)
@@ -89,10 +103,10 @@ __device__ __forceinline__ void fx_fwd(X2 *buf, const FxPassArgs &a)
 #pragma unroll
         for (int m = 0; m < R; m++) v[m] = buf[at[m]];
         XDft<R, false>::run(v);
-        buf[at[0]] = fx_half(v[0]);
+        buf[at[0]] = fx_half(v[0], a);
         const TwX *w = a.tw + j;
 #pragma unroll
-        for (int r = 1; r < R; r++) buf[at[r]] = fx_mulc(v[r], w[(r - 1) * M]);
+        for (int r = 1; r < R; r++) buf[at[r]] = fx_mulc(fx_up(v[r], a), w[(r - 1) * M]);
     }
     __syncwarp();
 }
@@ -173,9 +187,9 @@ __device__ __forceinline__ void fx_inv(X2 *buf, const FxPassArgs &a, double *oa,
         X2 v[R];
         fx_places<R, KIND>(a, b, j, at);
         const TwX *w = a.tw + j;
-        v[0] = fx_half(buf[at[0]]);
+        v[0] = fx_half(buf[at[0]], a);
 #pragma unroll
-        for (int r = 1; r < R; r++) v[r] = fx_mulcj(buf[at[r]], w[(r - 1) * M]);
+        for (int r = 1; r < R; r++) v[r] = fx_mulcj(fx_up(buf[at[r]], a), w[(r - 1) * M]);
         XDft<R, true>::run(v);
         if (OUT) {
             // (one block: elements j + r M)
@@ -254,7 +268,7 @@ struct FxOut { double cx, cy, sc; int xe, bad; };
 
 // DIR 0: x lines (sequence = two rows), DIR 1: y lines (two columns).  tpp
 // tiles per plane: of Q sequences (one warp's, x) or S = warps Q (a CTA's, y).
-template <int DIR, int NJ>
+template <int DIR, int NJ, int LONG>
 __global__ void __launch_bounds__(FX_TPB, 3)
 line_fx(const __grid_constant__ FxPack<NJ> jobs, const __grid_constant__ FxPlan pl, FxTables tb, int nx, int ny, int nz,
         int tpp, int total, int two)
@@ -275,8 +289,9 @@ line_fx(const __grid_constant__ FxPack<NJ> jobs, const __grid_constant__ FxPlan 
 
     for (int e = tid; e < pl.ntw; e += blockDim.x) tw[e] = tb.tw[e];
     __syncthreads();
-    auto args = [&](int p) {
+    auto args = [&](int p, unsigned up) {
         FxPassArgs a;
+        a.up = (up >> p) & 1;
         a.n = n; a.L = pl.L[p]; a.M = pl.M[p]; a.G = G; a.l = l; a.s7 = s7; a.mg = pl.mg[p]; a.tw = tw + pl.tw[p];
         return a;
     };
@@ -510,13 +525,13 @@ line_fx(const __grid_constant__ FxPack<NJ> jobs, const __grid_constant__ FxPlan 
         float s1 = 0.0f, s2 = 0.0f;
         if (!inv) {
             for (int p = 0; p < pl.np - 1; p++) {
-                const FxPassArgs a = args(p);
+                const FxPassArgs a = args(p, pl.fup);
 #define CALL(R, K) fx_fwd<R, K>(A, a)
                 FX_SWITCH(pl, p, CALL)
 #undef CALL
             }
             const bool key = op1 == OP_D1 || op1 == OP_D2 || op2 == OP_D1 || op2 == OP_D2;
-            const FxPassArgs a = args(pl.np - 1);
+            const FxPassArgs a = args(pl.np - 1, 0);
 #define CALL(R, K) fx_last<R, K>(A, a, tb.kof, key, s1, s2)
             FX_SWITCH_LAST(pl, CALL)
 #undef CALL
@@ -528,7 +543,7 @@ line_fx(const __grid_constant__ FxPack<NJ> jobs, const __grid_constant__ FxPlan 
 
         if (op1 == OP_FWD) {
             // separate Z into the halfcomplex spectra of the two real lines
-            out.xe = F + pl.halvings - 1;
+            out.xe = F + pl.hf - 1;
             const bool scale = jb.alpha1 != 1.0;
             auto sep = [&](const X2 *Z, int z7, int p, const FxOut &o, double *va, double *vb) {
                 const X2 zp = Z[fx_at(__ldg(tb.pos + p), z7)], zq = Z[fx_at(__ldg(tb.pos + (p == 0 ? 0 : n - p)), z7)];
@@ -605,7 +620,7 @@ line_fx(const __grid_constant__ FxPack<NJ> jobs, const __grid_constant__ FxPlan 
             else if (op == OP_D2) sh = max(((fx_log2(s2 + pl.floor2) + 1) >> 1) + pl.gb - 22, -20);
             else if (op == OP_DEALIAS) sh = pl.gb;
             {
-                const FxPassArgs a = args(pl.np - 1);
+                const FxPassArgs a = args(pl.np - 1, 0);
                 if (op == OP_INV && pl.kind[pl.np - 1] == K1) {
                     fx_inv_first<8, K1>(dst, src, a, tb.kof, OP_INV, 0, 0);
                 } else {
@@ -614,7 +629,7 @@ line_fx(const __grid_constant__ FxPack<NJ> jobs, const __grid_constant__ FxPlan 
 #undef CALL
                 }
             }
-            out.xe = F + sh + (inv ? 1 : 2) * pl.halvings;
+            out.xe = F + sh + pl.hi + (inv ? 0 : pl.hf);
             const double con = op == OP_D1 ? tb.c1 : op == OP_D2 ? tb.c2 : tb.c0;
             // (con 2^xe, and with it every result, in the normal range)
             const bool safe = out.xe >= -700 && out.xe <= 700;
@@ -638,13 +653,13 @@ line_fx(const __grid_constant__ FxPack<NJ> jobs, const __grid_constant__ FxPlan 
             // x lines: the last pass stores its results
             const bool fused = DIR == 0 && pl.np > 1 && __all_sync(0xffffffffu, plain && valid);
             for (int p = pl.np - 2; p >= (fused ? 1 : 0); p--) {
-                const FxPassArgs a = args(p);
+                const FxPassArgs a = args(p, pl.iup);
 #define CALL(R, K) fx_inv<R, K, false>(dst, a, nullptr, nullptr, 0.0, 0.0, 0.0, FX_SET)
                 FX_SWITCH(pl, p, CALL)
 #undef CALL
             }
             if (fused) {
-                const FxPassArgs a = args(0);
+                const FxPassArgs a = args(0, pl.iup);
 #define CALL(R, K) fx_inv<R, K, true>(dst, a, oa, ob, out.sc, ca, cb, mode)
                 FX_SWITCH(pl, 0, CALL)
 #undef CALL
@@ -725,6 +740,7 @@ static FxConst fx_const(long double v)
     c.h = (int)((q - (int)q) >> 32);
     return c;
 }
+#if !FX_LONG
 // exp(-2 pi i e/n), computed in long double, exact at the quadrants; the angles
 // of an octant are computed once
 struct UnitCircle {
@@ -746,8 +762,13 @@ struct UnitCircle {
         return TwX{ re[q].h, re[q].l, im[q].h, im[q].l };
     }
 };
+#endif
 
+#if FX_LONG
+int line_fx_long_configure()
+#else
 int line_fx_configure()
+#endif
 {
     const long double h = 3.14159265358979323846264338327950288L;
     const FxConst r8 = fx_const(cosl(h / 4)), r3 = fx_const(sinl(h / 3));
@@ -757,9 +778,14 @@ int line_fx_configure()
     CUDA_TRY(cudaMemcpyToSymbol(c_fx_c5, &c5, sizeof(c5)));
     CUDA_TRY(cudaMemcpyToSymbol(c_fx_s5a, &sa, sizeof(sa)));
     CUDA_TRY(cudaMemcpyToSymbol(c_fx_s5b, &sb, sizeof(sb)));
+#if FX_LONG
     return VEC_OK;
+#else
+    return line_fx_long_configure();
+#endif
 }
 
+#if !FX_LONG
 // the radices of n with the fewest passes; 8 where it divides, and last: the
 // strides of the other passes are then multiples of 8 or 64
 static bool radices(int n, std::vector<int> &r)
@@ -796,8 +822,12 @@ int fx_plan_make(int n, FxPlan *pl)
     const double kmax = n / 2;
     pl->floor1 = (float)(n * kmax * kmax);
     pl->floor2 = (float)(n * kmax * kmax * kmax * kmax);
+    // the sums of a pass: 2 x 4 and 3 x 2 with a halving between
+    auto sums = [&](int p, int q) {
+        const int R = r[p];
+        return q == 0 ? (R == 8 ? 2 : R == 6 ? 3 : R) : R == 8 ? 4 : R == 6 ? 2 : 1;
+    };
     int L = n;
-    double P = 1.0, top = 0.0;     // growth sqrt(P) 2^-halvings
     for (int p = 0; p < pl->np; p++) {
         const int R = r[p], M = L / R;
         pl->R[p] = R; pl->L[p] = L; pl->M[p] = M;
@@ -805,31 +835,44 @@ int fx_plan_make(int n, FxPlan *pl)
         pl->kind[p] = M % 64 == 0 ? K64 : R == 8 && M == 8 ? K8 : R == 8 && M == 1 ? K1 : KG;
         pl->tw[p] = pl->ntw;
         if (M > 1) pl->ntw += (R - 1) * M;
-        // sums inside the radix: 2 x 4 and 3 x 2 with a halving between
-        const int in[2] = { R == 8 ? 2 : R == 6 ? 3 : R, R == 8 ? 4 : R == 6 ? 2 : 1 };
-        for (int q = 0; q < 2; q++) {
-            P *= in[q];
-            top = fmax(top, sqrt(P) * exp2(-(double)pl->halvings));
-            if (q == 0 && in[1] > 1) pl->halvings++;
-        }
-        if (p + 1 < pl->np) pl->halvings++;
         L = M;
     }
-    // (the inverse takes the radices backwards: the same bound on its growth
-    // from the other end)
-    P = 1.0;
-    int h = 0;
-    for (int p = pl->np - 1; p >= 0; p--) {
-        const int R = r[p], in[2] = { R == 8 ? 2 : R == 6 ? 3 : R, R == 8 ? 4 : R == 6 ? 2 : 1 };
-        for (int q = 0; q < 2; q++) {
-            P *= in[q];
-            top = fmax(top, sqrt(P) * exp2(-(double)h));
-            if (q == 0 && in[1] > 1) h++;
-        }
-        h++;
-    }
+    // growth sqrt(P) 2^-halvings along the forward passes, and along the inverse ones, which
+    // take the radices backwards; a halving between two passes.  Long lines leave out those
+    // that the bound does not need: each costs a bit
+    double top = 0.0;
+    for (int d = 0; d < 2; d++)
+        for (int o = 0; o < pl->np; o++)
+            for (int q = 0; q < 2; q++) {
+                double P = 1.0;
+                int h = 0;
+                for (int t = 0; t <= o; t++) {
+                    const int p = d ? pl->np - 1 - t : t;
+                    P *= sums(p, 0);
+                    if (t == o && q == 0) break;
+                    h += sums(p, 1) > 1;
+                    P *= sums(p, 1);
+                    if (t < o) h++;
+                }
+                top = fmax(top, sqrt(P) * exp2(-(double)h));
+            }
     pl->gb = top <= 2.0 ? 1 : 2;
     if (top > 4.0) return VEC_ERR_SIZE;
+    for (int d = 0; d < 2; d++) {
+        double P = 1.0;
+        int h = 0;
+        for (int t = 0; t < pl->np; t++) {
+            const int p = d ? pl->np - 1 - t : t, next = d ? p - 1 : p + 1;
+            P *= r[p];
+            h += sums(p, 1) > 1;
+            if (t + 1 == pl->np) break;
+            if (n > FX_SHORT && sqrt(P * sums(next, 0)) * exp2(-(double)h) <= exp2((double)pl->gb))
+                (d ? pl->iup : pl->fup) |= 1u << (d ? next : p);
+            else
+                h++;
+        }
+        (d ? pl->hi : pl->hf) = h;
+    }
     // sequences per warp: about 256 elements, at least four lanes each
     pl->Q = n <= 32 ? 8 : n <= 64 ? 4 : n <= 128 ? 2 : 1;
     return VEC_OK;
@@ -877,6 +920,7 @@ void fx_tables_free(FxTables *tb)
     cudaFree(tb->tw);
     *tb = FxTables{};
 }
+#endif
 
 template <int DIR, int NJ>
 static int run_fx(Engine *E, const LineJob<double> *jobs, int nj)
@@ -913,26 +957,32 @@ static int run_fx(Engine *E, const LineJob<double> *jobs, int nj)
     while (W > 1 && (smem_of(W) > 75 * 1024 || (DIR == 0 ? tiles_of(W) / W : tiles_of(W)) < E->num_sms)) W >>= 1;
     const size_t smem = smem_of(W);
     static SmemLimit limit;
-    CUDA_TRY(limit.raise((const void *)line_fx<DIR, NJ>, 226 * 1024));
+    CUDA_TRY(limit.raise((const void *)line_fx<DIR, NJ, FX_LONG>, 226 * 1024));
     if (smem > 226 * 1024) return VEC_ERR_SIZE;
     int per_sm = 1;
-    CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, line_fx<DIR, NJ>, W * 32, smem));
+    CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, line_fx<DIR, NJ, FX_LONG>, W * 32, smem));
     if (per_sm < 1) per_sm = 1;
     const int S = DIR == 0 ? pl.Q : W * pl.Q, tpp = (pairs + S - 1) / S;
     const long long total = tiles_of(W);
     long long grid = DIR == 0 ? (total + W - 1) / W : total;
     if (grid > (long long)E->num_sms * per_sm) grid = (long long)E->num_sms * per_sm;
     E->prof_begin(DIR == 0 ? "line_x_f64" : "line_y_f64", fields * (double)E->n * 8.0);
-    CUDA_TRY(launch_k(*E, line_fx<DIR, NJ>, dim3((unsigned)grid), dim3(W * 32), smem, pk, pl, DIR == 0 ? E->fxx : E->fxy, E->nx,
+    CUDA_TRY(launch_k(*E, line_fx<DIR, NJ, FX_LONG>, dim3((unsigned)grid), dim3(W * 32), smem, pk, pl, DIR == 0 ? E->fxx : E->fxy, E->nx,
                       E->ny, E->nz, tpp, (int)total, two));
     E->prof_end();
     CUDA_TRY(cudaGetLastError());
     return VEC_OK;
 }
 
+#if FX_LONG
+int launch_lines_fx_long(Engine *E, int dir, const LineJob<double> *jobs, int njobs)
+{
+#else
 template <>
 int launch_lines<double>(Engine *E, int dir, const LineJob<double> *jobs, int njobs)
 {
+    if ((dir == 0 ? E->nx : E->ny) > FX_SHORT) return launch_lines_fx_long(E, dir, jobs, njobs);
+#endif
     for (int j0 = 0; j0 < njobs; j0 += MAX_JOBS) {
         const int nj = njobs - j0 < MAX_JOBS ? njobs - j0 : MAX_JOBS;
         const LineJob<double> *j = jobs + j0;
