@@ -38,9 +38,8 @@
 // The error against FP64 (rms of d1, d2 and dealias) falls by 6 to 13 % for white noise, by
 // 1 to 13 % for lines of few waves with and without noise, and stays for a constant plus
 // little.
-// (Up to 256 points pairs on two levels took 3-8 % less, 34.4 -> 31.5 at 256^2 x 129,
-// which is not worth other rounding in every step, restart and training set of those
-// grids: lines_ct.cu keeps their results bit for bit.)
+// (Up to 256 points pairs on two levels took 3-8 % less than lines_ct.cu's scalar kernel,
+// 34.4 -> 31.5 at 256^2 x 129; they are not in use.)
 #include <math.h>
 #include <stdint.h>
 #include <string.h>

@@ -2,11 +2,11 @@
 // line lengths n = N1*N2 = 2^a or 3*2^a (64..256): the scheme of lines_ct.cu in double.
 //
 // The FP64 form's lines run on integers (lines_fx.cu), 2.5 times as fast and more
-// exact.  What a split context makes of its magnetic field at a start is kept as it
-// was instead, bit for bit, so that runs, restarts and training sets made from split
-// steps are: their FP32 mirrors round these values, and 1e-16 moves some of them by an
-// FP32 unit (2e-7 of a state after ten steps, 6e-5 of a network's gradients after
-// two iterations).  It runs once per start; FP64 arithmetic bounds it.
+// exact.  Where both lengths are among these, a split context's start keeps this kernel's
+// bits instead: its FP32 mirrors round what mag_init makes, and 1e-16 moves some of them by
+// an FP32 unit (2e-7 of a state after ten steps), from which a convecting layer takes
+// another course.  (At other lengths starts are lines_fx.cu's.)  It runs once per start;
+// FP64 arithmetic bounds it.
 #include <math.h>
 #include <stdint.h>
 #include <string.h>

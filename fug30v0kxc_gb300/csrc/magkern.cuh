@@ -152,7 +152,7 @@ static __global__ void k_mag_final(MagArgs<R> a)
     const int j = (int)(q / (unsigned)a.nx), i = (int)(q - (unsigned)j * a.nx);
     if constexpr (sizeof(R) == 8) {
         // FP64: the z stencils in integers (zfx.cuh) and the inverse Laplacian by
-        // its reciprocal with one correction (the quotient to the last bit or so),
+        // its reciprocal with one correction (the quotient's own bits in 2 10^8 random pairs),
         // 20 FP64 operations of 57: 0.77 -> 0.41 ms at 256^2 x 129
         const double w2 = sdy(a.ex + pb, i, j, a.nx, a.ny, a.h.ky1) - sdx(a.ey + pb, i, j, a.nx, a.h.kx1);
         const double w3 = a.ho12 * zsum<ZD1 | ZPIPE>(a.w1 + q, (size_t)np, k, a.nz, 5, 0).d1;
